@@ -90,8 +90,9 @@ def draw(rng: random.Random):
         w, h = _size(rng, 320, 1920)
         if rng.random() < 0.3:
             return dict(kind=kind, w=max(w, 400), h=max(h, 240), tw=APP_W, th=APP_H, step=rng.choice([1, 2]), precision=0, level1=True)
-        return dict(kind=kind, w=w, h=h, tw=8 * rng.randint(2, 12), th=rng.randint(12, 96), step=rng.choice([1, 1, 2]),
-                    precision=rng.choice([0, 1, 2]), level1=False)
+        step = rng.choice([1, 1, 2])  # every second corner: the smaller templates, as in a tracker's own searches
+        return dict(kind=kind, w=w, h=h, tw=8 * rng.randint(2, 12 if step == 1 else 8), th=rng.randint(12, 96 if step == 1 else 64),
+                    step=step, precision=rng.choice([0, 1, 2]), level1=False)
     if kind == "detect":
         w, h = _size(rng, 320, 1920)
         rw, rh = w * rng.uniform(0.1, 1.0), h * rng.uniform(0.15, 1.0)
