@@ -331,7 +331,9 @@ __global__ void __launch_bounds__(256, SUMS ? 6 : 1) ncc_map_f32q(const T *__res
     const int ccx0 = BC * bx, ccy0 = BC * by; /* the CTA's first cell column and row */
     const int X0 = p.x0 + ccx0 * NCC_CELL, Y0 = p.y0 + ccy0 * NCC_CELL;
     const int iw = nmq_cols(ST, p.tw), ip = nmq_pitch(ST, p.tw), ih = nmq_rows(ST, p.th);
-    float *s_app = sm, *s_img = sm + nmq_head(ST, p.tw, p.th); /* a multiple of 8 floats: s_img stays 16-byte aligned */
+    /* a multiple of 8 floats either way: s_img stays 16-byte aligned. Without SUMS nothing takes the template's place, and
+     * the launch sizes the head by the template alone (shorter than the column sums for a wide, low template). */
+    float *s_app = sm, *s_img = sm + (SUMS ? nmq_head(ST, p.tw, p.th) : p.tw * p.th);
     for (int i = threadIdx.x; i < p.tw * p.th; i += blockDim.x)
         s_app[i] = app[i];
     bool small = true; /* every value this thread staged converts to the same integer in 32 bits */
