@@ -15,7 +15,7 @@ struct vtg_search {
     char *mem;
     size_t bytes;
     float *app;       /* the template, max_tw x max_th floats */
-    float *sum_t;     /* [0]: BF16 band sum, [1]: FP16 band sum (device) */
+    NccBandStats *stats; /* [0]: the BF16 band's, [1]: the FP16 band's (device) */
     NccScratch sc;
     uint16_t *band[2]; /* BF16 and FP16 bands */
     vtg_found *found;  /* device result slot for host callers */
@@ -23,7 +23,7 @@ struct vtg_search {
     float *vals;
     int tw, th;
     float norm;
-    float host_sum[2];
+    NccBandStats host_stats[2];
     bool has_template;
 };
 
@@ -143,7 +143,7 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
         return VTG_ECUDA;
     }
     s->app = (float *)(s->mem + L.app);
-    s->sum_t = (float *)(s->mem + L.sum);
+    s->stats = (NccBandStats *)(s->mem + L.sum);
     s->sc.S1 = (long long *)(s->mem + L.S1);
     s->sc.S2 = (long long *)(s->mem + L.S2);
     s->sc.tp = L.tp;
@@ -165,6 +165,11 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
     s->sc.topblk = (unsigned long long *)(s->mem + L.topblk);
     s->sc.topblk_lists = L.lists;
     s->sc.arrive = (unsigned *)(s->mem + L.arrive);
+    s->sc.cand = (unsigned *)s->sc.S1;
+    s->sc.cand_elems = 2 * (size_t)L.tp * (max_h + 1);
+    s->sc.tol = (uint16_t *)s->sc.S2;
+    s->sc.tol_elems = 4 * (size_t)L.tp * (max_h + 1);
+    s->sc.ncand = s->sc.arrive + 2;
     s->sc.map_ev0 = s->sc.map_ev1 = nullptr;
     s->found = (vtg_found *)(s->mem + L.found);
     s->xy = nullptr;
@@ -206,9 +211,9 @@ extern "C" int vtg_search_template(vtg_search *s, const float *app, int tw, int 
     const cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
     CU(cudaMemcpyAsync(s->app, app, sizeof(float) * (size_t)tw * th,
                        where == VTG_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
-    CU(vtg_launch_ncc_band(s->app, tw, th, VTG_NCC_BF16, s->band[0], s->sum_t + 0, st));
-    CU(vtg_launch_ncc_band(s->app, tw, th, VTG_NCC_FP16, s->band[1], s->sum_t + 1, st));
-    CU(cudaMemcpyAsync(s->host_sum, s->sum_t, 2 * sizeof(float), cudaMemcpyDeviceToHost, st));
+    CU(vtg_launch_ncc_band(s->app, tw, th, VTG_NCC_BF16, s->band[0], s->stats + 0, st));
+    CU(vtg_launch_ncc_band(s->app, tw, th, VTG_NCC_FP16, s->band[1], s->stats + 1, st));
+    CU(cudaMemcpyAsync(s->host_stats, s->stats, sizeof s->host_stats, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st)); /* the band sums are kernel parameters of every later search */
     s->tw = tw;
     s->th = th;
@@ -230,7 +235,9 @@ static int make_prm(const vtg_search *s, int w, int h, int x0, int x1, int y0, i
     p->n = s->tw * s->th;
     p->norm = s->norm;
     ncc_thresholds(*p);
-    p->sum_t = precision == VTG_NCC_BF16 ? s->host_sum[0] : precision == VTG_NCC_FP16 ? s->host_sum[1] : 0.0f;
+    /* the F32 map's filter multiplies the FP16 band too */
+    p->sum_t = s->host_stats[precision == VTG_NCC_BF16 ? 0 : 1].sum_h;
+    vtg_ncc_filter_bound(*p, s->host_stats[1]);
     /* the reference's clamp of the window (search_slot, track.c:1665-1670) */
     const int lo_x = 1, hi_x = w - s->tw - 2, lo_y = 1, hi_y = h - s->th - 2;
     p->x0 = x0 < lo_x ? lo_x : x0;
@@ -269,7 +276,7 @@ extern "C" int vtg_search_run(vtg_search *s, const void *plane, int w, int h, in
         return VTG_OK;
     }
     NccScratch sc = s->sc;
-    sc.band = precision == VTG_NCC_BF16 ? s->band[0] : precision == VTG_NCC_FP16 ? s->band[1] : nullptr;
+    sc.band = s->band[precision == VTG_NCC_BF16 ? 0 : 1]; /* the F32 map's filter multiplies the FP16 band */
     CU(vtg_launch_ncc(plane, pitch, plane_type, s->app, p, sc, precision, dst, st));
     const size_t cells = (size_t)p.ccols * p.crows;
     const cudaMemcpyKind k = where == VTG_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
@@ -342,7 +349,7 @@ extern "C" int vtg_search_profile(vtg_search *s, const void *plane, int w, int h
     for (int k = 0; k < 4; k++)
         CU(cudaEventCreate(&ev[k]));
     NccScratch sc = s->sc;
-    sc.band = precision == VTG_NCC_BF16 ? s->band[0] : precision == VTG_NCC_FP16 ? s->band[1] : nullptr;
+    sc.band = s->band[precision == VTG_NCC_BF16 ? 0 : 1]; /* the F32 map's filter multiplies the FP16 band */
     sc.map_ev0 = ev[1];
     sc.map_ev1 = ev[2];
     std::vector<float> tm, tt;

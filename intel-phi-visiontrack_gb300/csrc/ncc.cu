@@ -11,7 +11,9 @@
  * norm <= 0, else st / sqrt(norm var). The window sums come from exact int64 integral images (sum J and sum J^2), so the
  * near-blank rule compares an exact integer n var with n norm / 16 and never lets a flat window through.
  *
- * Pipeline (all on one stream, no host round trip):
+ * Pipeline (all on one stream, no host round trip). The F32 map of an 8-bit plane at steps 1 and 2, large templates and
+ * windows (vtg_ncc_filters): ncc_prep and the FP16 tensor-core map (ncc_tc.cu) find the corners that could be their cell's
+ * best, ncc_rescore scores those in F32; every bit is the F32 map's. Otherwise:
  *   integral_rows / integral_cols  int64 tables of J and J^2 ((h + 1) x (w + 1)), exact: for the F32 map at steps 4 to
  *                                 16, and at steps 1 and 2 where ncc_sums_in_map leaves the window sums to them (the
  *                                 tensor-core map's preparation (ncc_prep) sums the window bytes directly)
@@ -510,6 +512,181 @@ static bool ncc_sums_in_map(const NccPrm &p)
     return p.tw * p.th <= 64 * 64 || 2 * win < (long long)p.w * (long long)p.h;
 }
 
+/* ---- the F32 map by filter: the corners that the FP16 tensor-core map could not rule out, scored exactly ---- */
+
+/* Two lanes a corner of the list, one for each of ncc_map_f32q's two chains (rows, then the even or the odd columns), so the
+ * score is that map's bit for bit, and into its cell's word. The chains are serial: a run of corners takes a warp n / 2
+ * dependent steps whatever the chip, and a map leaves fewer runs than the chip has warp schedulers, so what counts is a
+ * step's latency. The picture comes in by 16-byte asynchronous copies, NCR_DEPTH rows ahead, the pair's lanes taking a corner
+ * row's chunks in turn; a step is 32 columns, its words and template values read from shared memory while the step before
+ * runs. Byte b becomes the float 2^23 + b by one byte permute, then less 2^23 + first: b - first, exact. The window's sums
+ * are byte dot products, each lane of a pair on half the words. Measured at 1080p: 11 us at 32 x 32, 21 at 64 x 64, 53 at
+ * 96 x 96, three times less than a lane a corner reading the picture itself; the wait between a step's dependent
+ * instructions bounds it (an instruction every three cycles of a scheduler). Columns past the template's in a last step (not FULL) hold
+ * zeros in the staged template and are masked from the sums: they add exact zeros.
+ * The copies stay in the plane: a chunk starts at most 15 bytes before a corner's row and ends less than 64 past it, a row
+ * lies above (y >= 1) and below (y + th <= h - 2) it, and rows have at least 64 bytes (vtg_ncc_filters). */
+#define NCR_WARPS 8
+#define NCR_RUN 16
+#define NCR_DEPTH 4
+#define NCR_CTAS 152 /* one an SM: a whole 1080p map leaves some 500 runs */
+
+/* Steps of 32 columns; a corner's bytes of a row in 16-byte chunks at any offset, an odd number of them, so that the lanes
+ * spread over the banks. */
+static constexpr int ncr_stride(int steps) { return 16 * (2 * steps + 1); }
+
+/* the template and the warps' rings */
+static size_t ncr_smem(const NccPrm &p)
+{
+    const int steps = (p.tw + 31) / 32;
+    return sizeof(float) * 32 * (size_t)steps * p.th + (size_t)NCR_WARPS * NCR_DEPTH * NCR_RUN * ncr_stride(steps);
+}
+
+struct NcrStep {
+    unsigned w[9]; /* the words from the corner's first one of these 32 columns */
+    float4 t[4];   /* the template at the lane's columns */
+};
+
+template <int STEPS, bool FULL>
+__global__ void __launch_bounds__(32 * NCR_WARPS) ncc_rescore(const uint8_t *__restrict__ plane, int pitch,
+                                                              const float *__restrict__ app, NccPrm p,
+                                                              const unsigned *__restrict__ cand,
+                                                              const unsigned *__restrict__ ncand,
+                                                              unsigned long long *__restrict__ cellw)
+{
+    extern __shared__ __align__(16) float sm[]; /* the template, 32 columns at a time: 16 even ones, then 16 odd ones */
+    constexpr int COLS = 32 * STEPS, STRIDE = ncr_stride(STEPS), SLOT = NCR_RUN * STRIDE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, odd = lane & 1;
+    for (int i = threadIdx.x; i < COLS * p.th; i += 32 * NCR_WARPS) {
+        const int r = i / COLS, c = i % COLS;
+        sm[r * COLS + (c & ~31) + 16 * (c & 1) + ((c & 31) >> 1)] = c < p.tw ? __ldg(app + r * p.tw + c) : 0.0f;
+    }
+    __syncthreads();
+    /* the pair's rows in the warp's ring */
+    const uint8_t *const ring = reinterpret_cast<const uint8_t *>(sm + COLS * p.th) + warp * NCR_DEPTH * SLOT + (lane >> 1) * STRIDE;
+    const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring) + 16u * odd;
+    const int count = (int)__ldcg(ncand);
+    const int sh = __ffs(p.step) - 1, per = NCC_CELL >> sh;
+    const unsigned lo = 0x7440u + odd, hi = 0x7442u + odd; /* the lane's two bytes of a word */
+    const int groups = (p.tw - 32 * (STEPS - 1)) / 8;      /* of the last step; the others have 4 */
+    /* runs of 16 corners, one a CTA before any CTA takes a second */
+    for (int base = (warp * gridDim.x + blockIdx.x) * NCR_RUN; base < count; base += NCR_WARPS * gridDim.x * NCR_RUN) {
+        const int mine = base + (lane >> 1);
+        const bool on = mine < count;
+        const unsigned xy = __ldcg(cand + (on ? mine : base));
+        const int a = (int)(xy & 0xFFFFu), b = (int)(xy >> 16);
+        const uint8_t *const row0 = plane + (size_t)(p.y0 + b) * pitch + (p.x0 + a);
+        const uint8_t *next = row0; /* the row copied next, and its slot; the rows left to copy */
+        unsigned put = 0u;
+        int left = p.th;
+        auto fetch = [&]() {
+            if (left > 0) {
+                const uint8_t *src = reinterpret_cast<const uint8_t *>((uintptr_t)next & ~(uintptr_t)15) + 16 * odd;
+#pragma unroll
+                for (int k = 0; k <= STEPS; k++) /* the lane's chunks: 0, 2, .., or 1, 3, .. */
+                    if (k < STEPS || !odd)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(ring_s + put + 32 * k), "l"(src + 32 * k)
+                                     : "memory");
+                next += pitch;
+                put = put == (NCR_DEPTH - 1) * SLOT ? 0u : put + SLOT;
+                left--;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        __syncwarp(); /* every lane is done with the last run's rows */
+#pragma unroll
+        for (int r = 0; r < NCR_DEPTH - 1; r++)
+            fetch();
+        const float first = (float)__ldg(row0) + 8388608.0f; /* exact */
+        float acc = 0.0f;
+        unsigned s1 = 0u, s2 = 0u;
+        /* the row being read: its slot and address (for its offset in its first chunk), its template columns */
+        const float *t = sm + 16 * odd;
+        unsigned get = 0u, at = (unsigned)(uintptr_t)row0;
+        const unsigned *w = nullptr;
+        auto turn = [&]() {
+            asm volatile("cp.async.wait_group %0;" ::"n"(NCR_DEPTH - 2) : "memory");
+            __syncwarp(); /* every lane's copies of the row are there, and every lane is done with the row before */
+            fetch();
+            w = reinterpret_cast<const unsigned *>(ring + get + (at & 12u));
+            get = get == (NCR_DEPTH - 1) * SLOT ? 0u : get + SLOT;
+        };
+        auto read = [&](NcrStep &q, int c) {
+#pragma unroll
+            for (int k = 0; k < 9; k++)
+                q.w[k] = w[8 * c + k];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                q.t[k] = *reinterpret_cast<const float4 *>(t + 32 * c + 4 * k);
+        };
+        auto run = [&](const NcrStep &q, int c, int shift) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                unsigned v0 = __funnelshift_r(q.w[2 * k], q.w[2 * k + 1], shift);
+                unsigned v1 = __funnelshift_r(q.w[2 * k + 1], q.w[2 * k + 2], shift);
+                if (!FULL && c == STEPS - 1) {
+                    v0 = k < groups ? v0 : 0u;
+                    v1 = k < groups ? v1 : 0u;
+                }
+                const unsigned u = odd ? v1 : v0;
+                s1 = __dp4a(u, 0x01010101u, s1);
+                s2 = __dp4a(u, u, s2);
+                acc = __fmaf_rn(__uint_as_float(__byte_perm(v0, 0x4B000000u, lo)) - first, q.t[k].x, acc);
+                acc = __fmaf_rn(__uint_as_float(__byte_perm(v0, 0x4B000000u, hi)) - first, q.t[k].y, acc);
+                acc = __fmaf_rn(__uint_as_float(__byte_perm(v1, 0x4B000000u, lo)) - first, q.t[k].z, acc);
+                acc = __fmaf_rn(__uint_as_float(__byte_perm(v1, 0x4B000000u, hi)) - first, q.t[k].w, acc);
+            }
+        };
+        /* two steps in registers, one running while the next is read: step c of row i in q[(i STEPS + c) % 2] */
+        NcrStep q[2];
+        turn();
+        read(q[0], 0);
+        auto rows = [&](auto parity, int i) {
+            constexpr int PAR = decltype(parity)::value;
+            const int shift = 8 * (int)(at & 3u);
+#pragma unroll
+            for (int c = 0; c < STEPS; c++) {
+                if (c + 1 < STEPS) {
+                    read(q[(PAR + c + 1) & 1], c + 1);
+                } else if (i + 1 < p.th) {
+                    at += (unsigned)pitch;
+                    t += COLS;
+                    turn();
+                    read(q[(PAR + c + 1) & 1], 0);
+                }
+                run(q[(PAR + c) & 1], c, shift);
+            }
+        };
+        for (int i = 0; i < p.th; i += 2) {
+            rows(std::integral_constant<int, 0>(), i);
+            if (i + 1 < p.th)
+                rows(std::integral_constant<int, STEPS & 1>(), i + 1);
+        }
+        const float acc1 = __shfl_xor_sync(VTG_FULL, acc, 1);
+        s1 += __shfl_xor_sync(VTG_FULL, s1, 1);
+        s2 += __shfl_xor_sync(VTG_FULL, s2, 1);
+        if (on && !odd) {
+            const float v = ncc_score(acc + acc1, (long long)s1, (long long)s2, p) + 0.0f;
+            const int key = ((b % NCC_CELL) >> sh) * per + ((a % NCC_CELL) >> sh);
+            atomicMax(cellw + (size_t)(b / NCC_CELL) * p.ccols + a / NCC_CELL, ncc_cell_word(v, key));
+        }
+    }
+}
+
+template <int STEPS>
+static cudaError_t launch_rescore(const uint8_t *plane, int pitch, const float *app, const NccPrm &p, const NccScratch &s,
+                                  cudaStream_t st)
+{
+    auto kernel = p.tw % 32 ? ncc_rescore<STEPS, false> : ncc_rescore<STEPS, true>;
+    const size_t smem = ncr_smem(p);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+        return e;
+    /* an ordinary launch: as the map's programmatic dependent its CTAs would all start on the SMs that the map leaves free */
+    kernel<<<NCR_CTAS, 32 * NCR_WARPS, smem, st>>>(plane, pitch, app, p, s.cand, s.ncand, s.cellw);
+    return cudaGetLastError();
+}
+
 /* ---- the eight best cells ---- */
 
 /* The eight best cells. Each CTA takes NCC_TOPB_PER x NCC_TOPB_THREADS cells (a thread keeps its best eight in
@@ -836,7 +1013,23 @@ static cudaError_t launch_all(const T *plane, int pitch, const float *app, const
 {
     const int cells = p.ccols * p.crows;
     cudaError_t e = cudaSuccess;
-    if (map_kind == VTG_NCC_F32) {
+    bool filtered = false;
+    if (map_kind == VTG_NCC_F32 && sizeof(T) == 1 && vtg_ncc_filters(p, s)) {
+        /* the same map by the FP16 tensor-core map's filter */
+        filtered = true;
+        const uint8_t *u8 = (const uint8_t *)plane;
+        if ((e = vtg_launch_ncc_filter(u8, pitch, p, s, st)) != cudaSuccess)
+            return e;
+        const int steps = (p.tw + 31) / 32;
+        e = steps == 1   ? launch_rescore<1>(u8, pitch, app, p, s, st)
+            : steps == 2 ? launch_rescore<2>(u8, pitch, app, p, s, st)
+            : steps == 3 ? launch_rescore<3>(u8, pitch, app, p, s, st)
+                         : launch_rescore<4>(u8, pitch, app, p, s, st);
+        if (e != cudaSuccess)
+            return e;
+        if (s.map_ev1 && (e = cudaEventRecord(s.map_ev1, st)) != cudaSuccess)
+            return e;
+    } else if (map_kind == VTG_NCC_F32) {
         /* steps 1 and 2: four corners a thread, the window sums from the staged window; the other steps one corner a
          * thread, a CTA a cell, the window sums from the integral images (the tensor-core map's prep sums the bytes) */
         const bool quad = p.step == 1 || p.step == 2;
@@ -870,7 +1063,7 @@ static cudaError_t launch_all(const T *plane, int pitch, const float *app, const
     /* the tensor-core map's launcher ends with the top-8 pass over its cell words (ncc_tc.cu); the passes after the
      * map start as programmatic dependents, except when events around the map time it alone */
     const bool pdl = !s.map_ev1;
-    if (map_kind == VTG_NCC_F32 && (e = vtg_launch_ncc_top(p, s, false, st, pdl)) != cudaSuccess)
+    if (map_kind == VTG_NCC_F32 && (e = vtg_launch_ncc_top(p, s, filtered, st, pdl)) != cudaSuccess)
         return e;
     const int around = p.step > 1 ? 2 * p.step - 1 : 1, ring = 2 * around + 3;
     return vtg_launch_k(ncc_half_all<T>, dim3(NCC_TOP * ring * ring), dim3(NCC_TOP * 32), 0, st, pdl, plane, pitch, app, p,

@@ -100,42 +100,81 @@ __global__ void ncc_band_kernel(const float *__restrict__ app, int tw, int th, i
     }
 }
 
-/* The sum of the template as the tensor cores see it (its rounded values), in double. */
-__global__ void ncc_band_sum(const float *__restrict__ app, int count, int kind, float *__restrict__ out)
+/* What the band's rounding keeps and loses of the template, in double: h the 16-bit value, d = t - h (exact: a 16-bit
+ * and an F32 value's difference). */
+__global__ void ncc_band_sum(const float *__restrict__ app, int count, int kind, NccBandStats *__restrict__ out)
 {
-    __shared__ double s[256];
-    double a = 0.0;
-    for (int i = threadIdx.x; i < count; i += blockDim.x)
-        a += (double)from16(to16(app[i], kind), kind);
-    s[threadIdx.x] = a;
+    __shared__ double s[4][256];
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        const float t = app[i];
+        const double h = (double)from16(to16(t, kind), kind), d = (double)t - h;
+        a[0] += h;
+        a[1] += d;
+        a[2] += d * d;
+        a[3] += (double)t * (double)t;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        s[k][threadIdx.x] = a[k];
     __syncthreads();
     for (int h = 128; h >= 1; h >>= 1) {
         if (threadIdx.x < h)
-            s[threadIdx.x] += s[threadIdx.x + h];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                s[k][threadIdx.x] += s[k][threadIdx.x + h];
         __syncthreads();
     }
     if (threadIdx.x == 0)
-        *out = (float)s[0];
+        *out = NccBandStats{(float)s[0][0], (float)s[1][0], (float)s[2][0], (float)s[3][0]};
 }
 
-cudaError_t vtg_launch_ncc_band(const float *app, int tw, int th, int kind, uint16_t *band, float *sum_t, cudaStream_t st)
+cudaError_t vtg_launch_ncc_band(const float *app, int tw, int th, int kind, uint16_t *band, NccBandStats *stats,
+                                cudaStream_t st)
 {
     const int q = tc_q(tw, th), krow = tc_krow(tw), rows = q + th - 1;
     const size_t total = (size_t)8 * q * krow * rows;
     const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
     ncc_band_kernel<<<blocks, 256, 0, st>>>(app, tw, th, kind, krow, rows, q, band);
-    ncc_band_sum<<<1, 256, 0, st>>>(app, tw * th, kind, sum_t);
+    ncc_band_sum<<<1, 256, 0, st>>>(app, tw * th, kind, stats);
     return cudaGetLastError();
+}
+
+/* How far a corner's FP16 tensor-core score may lie from its F32 score (ncc_map_f32q's chains), on a byte picture. With v =
+ * sum (J - mean)^2 over the window, a score is a sum over sqrt(norm v); f is the window's first pixel, sigma = sqrt(v / n),
+ * d = t - h the template's FP16 rounding. By Cauchy-Schwarz, for any constant c,
+ *     sum |t (J - c)| <= |t| sqrt(v + n (mean - c)^2) <= |t| sqrt(v) (1 + |mean - c| / sigma),
+ * so errors relative to such a sum become, in the score, that many units of |t| / sqrt(norm) times the bracket:
+ *   - the rounding: sum d (J - f) = sum (d - mean d)(J - mean) + sum d (mean - f), at most |d - mean d| / sqrt(norm) and
+ *     |sum d| / sqrt(n norm) |mean - f| / sigma;
+ *   - the tensor core's accumulation of t (J - 128) (the picture is converted less 128): each MMA of 16 products taken as
+ *     rounded to 2^-21 of the sum of magnitudes, over the steps of one issuer (its accumulator holds more than an F32's 24
+ *     bits, so this is some ten times what it loses);
+ *   - the F32 chains of t (J - f): n / 2 additions each, rounded to 2^-24;
+ *   - the scores' own last operations: a few units in the last place of 1.
+ * flt_a = -1 where FP16 does not hold the template (d infinite, or more than a hundredth of t). */
+void vtg_ncc_filter_bound(NccPrm &p, const NccBandStats &b)
+{
+    const double n = p.n, sd = fabs((double)b.sum_d), norm = (double)p.norm;
+    const double steps = ((p.th + TC_QMAX) / TC_ISSUERS + 2) * (double)(tc_krow(p.tw) / 16) + 16.0;
+    const double spread = (double)b.sum_dd * 1.001 - sd * sd * 0.999 / n;
+    const double t = sqrt((double)b.sum_tt / norm); /* 1 for a caller's true norm */
+    const double core = t * steps * 0x1p-21, chain = t * (n * 0.5 + 16.0) * 0x1p-24;
+    const double a = sqrt((spread > 0.0 ? spread : 0.0) / norm) + core + chain + 4e-6;
+    const bool good = norm > 0.0 && a <= 0.01; /* false for NaN */
+    p.flt_a = good ? (float)(a * 1.02) : -1.0f;
+    p.flt_m = good ? (float)(core * 1.02) : 0.0f;
+    p.flt_f = good ? (float)((chain + sd / sqrt(n * norm)) * 1.02) : 0.0f;
 }
 
 /* ---- per-search preparation ---- */
 
-/* conv[r][i] = 16-bit J[r][x0 + i] (zero past the picture), for rows 0 .. rows - 1 and columns 0 .. cpitch - 1: the
+/* conv[r][i] = 16-bit J[r][x0 + i] - centre (minus the centre past the picture), for rows 0 .. rows - 1 and columns 0 .. cpitch - 1: the
  * CTA (bx, by) of 256 threads converts row by, eight elements a thread and one 16-byte store (cpitch is a multiple of 8
  * and rows start 16-byte aligned: 2 cpitch = 2048 tiles_x + 288 bytes). */
 template <int KIND>
 __device__ __forceinline__ void conv_cta(const uint8_t *__restrict__ plane, int pitch, int w, int h, int x0, int rows,
-                                         int cpitch, uint16_t *__restrict__ conv, int bx, int by)
+                                         int cpitch, float centre, uint16_t *__restrict__ conv, int bx, int by)
 {
     const int r = by, i0 = 8 * (bx * 256 + (int)threadIdx.x);
     if (r >= rows || i0 >= cpitch)
@@ -147,7 +186,7 @@ __device__ __forceinline__ void conv_cta(const uint8_t *__restrict__ plane, int 
 #pragma unroll
         for (int f = 0; f < 2; f++) {
             const int x = x0 + i0 + 2 * e + f;
-            const float v = (r < h && x < w) ? (float)__ldg(plane + (size_t)r * pitch + x) : 0.0f;
+            const float v = (r < h && x < w) ? (float)__ldg(plane + (size_t)r * pitch + x) - centre : -centre;
             pr |= (uint32_t)to16(v, KIND) << (16 * f);
         }
         o[e] = pr;
@@ -170,8 +209,9 @@ __device__ __forceinline__ void conv_cta(const uint8_t *__restrict__ plane, int 
 #endif
 /* corners a CTA across: the most, a multiple of 32, whose columns (+ T_w - 1) fit the CTA's 256 threads */
 static inline int bp_tx(int tw) { return ((257 - tw) / 32) * 32; }
+template <bool TOL>
 __device__ void box_cta(const uint8_t *__restrict__ plane, int pitch, const NccPrm &p, int fw, int fpitch, int btx,
-                        float *__restrict__ fac, int bx, int by)
+                        float *__restrict__ fac, uint16_t *__restrict__ tol, int bx, int by)
 {
     __shared__ unsigned P1[BP_TY][257], P2[BP_TY][257]; /* P[r][c]: columns 0 .. c - 1 of row r */
     __shared__ unsigned t1[8][BP_TY], t2[8][BP_TY];     /* each warp's column totals, then the earlier warps' */
@@ -254,7 +294,14 @@ __device__ void box_cta(const uint8_t *__restrict__ plane, int pitch, const NccP
             const long long s1 = (long long)(P1[r][x + p.tw] - P1[r][x]), s2 = (long long)(P2[r][x + p.tw] - P2[r][x]);
             const long long nvar = (long long)p.n * s2 - s1 * s1;
             /* 1 / sqrt(norm var) = sqrt(n / norm) / sqrt(n var) */
-            frow[x] = (nvar <= p.nthr || p.norm <= 0.0f) ? 0.0f : p.rnorm * rsqrtf((float)nvar);
+            const float rs = rsqrtf((float)nvar);
+            frow[x] = (nvar <= p.nthr || p.norm <= 0.0f) ? 0.0f : p.rnorm * rs;
+            if constexpr (TOL) { /* |mean - c| / sigma = |sum J - n c| / sqrt(n var); rounded up */
+                const int f = __ldg(plane + (size_t)(p.y0 + ty0 + r) * pitch + (p.x0 + tx0 + x));
+                const float zm = fabsf((float)(s1 - 128 * p.n)) * rs, zf = fabsf((float)(s1 - (long long)f * p.n)) * rs;
+                tol[(size_t)(ty0 + r) * fpitch + tx0 + x] =
+                    __half_as_ushort(__float2half_ru(p.flt_a + p.flt_m * zm + p.flt_f * zf));
+            }
         }
     }
 }
@@ -262,22 +309,24 @@ __device__ void box_cta(const uint8_t *__restrict__ plane, int pitch, const NccP
 /* The map's preparation in one launch of 256-thread CTAs: the first nbox sum the windows (the longer work, so they
  * start first), the rest convert the picture, and those also zero the cells' words the map merges into. The two jobs
  * are independent and run side by side. */
-template <int KIND>
+template <int KIND, bool FILTER>
 __global__ void __launch_bounds__(256) ncc_prep(const uint8_t *__restrict__ plane, int pitch, NccPrm p, int fw, int fpitch,
-                                                int btx, int bgx, int nbox, float *__restrict__ fac, int rows, int cpitch,
-                                                int cgx, uint16_t *__restrict__ conv, unsigned long long *__restrict__ cellw,
-                                                int cells)
+                                                int btx, int bgx, int nbox, float *__restrict__ fac,
+                                                uint16_t *__restrict__ tol, int rows, int cpitch, int cgx, uint16_t *__restrict__ conv, unsigned long long *__restrict__ cellw,
+                                                int cells, unsigned *__restrict__ ncand)
 {
     vtg_grid_launch_dependents(); /* the map may start its setup as this launch's last CTAs run */
     const int b = (int)blockIdx.x;
     if (b < nbox) {
-        box_cta(plane, pitch, p, fw, fpitch, btx, fac, b % bgx, b / bgx);
+        box_cta<FILTER>(plane, pitch, p, fw, fpitch, btx, fac, tol, b % bgx, b / bgx);
         return;
     }
     const int k = b - nbox, g = k * 256 + (int)threadIdx.x;
     if (g < cells)
         cellw[g] = 0ull;
-    conv_cta<KIND>(plane, pitch, p.w, p.h, p.x0, rows, cpitch, conv, k % cgx, k / cgx);
+    if (FILTER && g == 0)
+        *ncand = 0u;
+    conv_cta<KIND>(plane, pitch, p.w, p.h, p.x0, rows, cpitch, FILTER ? 128.0f : 0.0f, conv, k % cgx, k / cgx);
 }
 
 /* ---- PTX helpers ---- */
@@ -357,14 +406,6 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16])
                  : "r"(taddr));
 }
 
-/* A cell's candidate as one orderable word: higher score first, then the earlier corner in scan order. 0: none. */
-__device__ __forceinline__ unsigned long long cell_word(float v, int key)
-{
-    unsigned u = __float_as_uint(v);
-    u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-    return ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)key);
-}
-
 /* ---- the map ---- */
 
 /* Tensor-memory columns a CTA allocates: the issuers' accumulators (8 Q columns each), rounded up to a power of two
@@ -399,15 +440,23 @@ template <int Q> struct TcShape {
     static constexpr int chunks = Q / 2 / halves;
 };
 
-template <int KIND, int Q>
+/* FILTER: the F32 map's first half. Instead of a cell's best, the corners whose score may be it in F32 arithmetic go to
+ * cand: a corner's F32 score lies within its tol of its score here (vtg_ncc_filter_bound), so only corners with score + tol
+ * >= max over the cell's corners here of (score - tol) can be the cell's best or tie with it. (Of a cell over two tiles, Q
+ * = 8, each tile's part is taken by itself, which can only keep more.) On the blurred-noise frames 1.0 to 1.3 corners a cell
+ * are left of 256, at 64 x 64 (29 us for this map, where the F32 map took 728). A near-blank window scores exactly 0 either way: the
+ * earliest of them goes straight to the cell's word. */
+template <int KIND, int Q, bool FILTER>
 __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, const uint16_t *__restrict__ band, int krow, int tiles_x,
                                                      uint32_t a_bytes, uint32_t stage_bytes,
                                                      const uint16_t *__restrict__ conv, int cpitch,
                                                      const float *__restrict__ fac, int fpitch,
-                                                     unsigned long long *__restrict__ cellw, int *__restrict__ err)
+                                                     unsigned long long *__restrict__ cellw, int *__restrict__ err,
+                                                     const uint16_t *__restrict__ tol, unsigned *__restrict__ cand, unsigned *__restrict__ ncand)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    vtg_grid_launch_dependents(); /* the top-8 pass may take the SMs this launch leaves free and wait there */
+    if (!FILTER)
+        vtg_grid_launch_dependents(); /* the top-8 pass may take the SMs this launch leaves free and wait there */
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
     const int Y0 = p.y0 + ty * Q;
@@ -452,6 +501,7 @@ __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, c
     const int fh = p.y1 - p.y0 + 1;
     uint4 jr[2 * CH];
     float4 fr[4 * CH];
+    uint4 er[FILTER ? 2 * CH : 1];
 #pragma unroll
     for (int i = 0; i < 2 * CH; i++) {
         const int yr = ty * Q + 2 * c0 + i;
@@ -459,7 +509,11 @@ __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, c
             jr[i] = __ldca(reinterpret_cast<const uint4 *>(conv + (size_t)(p.y0 + yr) * cpitch + xr));
             fr[2 * i] = __ldca(reinterpret_cast<const float4 *>(fac + (size_t)yr * fpitch + xr));
             fr[2 * i + 1] = __ldca(reinterpret_cast<const float4 *>(fac + (size_t)yr * fpitch + xr + 4));
+            if constexpr (FILTER)
+                er[i] = __ldca(reinterpret_cast<const uint4 *>(tol + (size_t)yr * fpitch + xr));
         } else {
+            if constexpr (FILTER)
+                er[i] = make_uint4(0u, 0u, 0u, 0u);
             jr[i] = make_uint4(0u, 0u, 0u, 0u);
             fr[2 * i] = fr[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
@@ -546,63 +600,124 @@ __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, c
         for (int s = 0; s < 8; s++)
             if (xr + s <= p.x1 - p.x0 && ((8 * m + s) & (p.step - 1)) == 0)
                 xmask |= 1u << s;
-        float best = -2.0f;
-        int bkey = 1 << 30;
-#pragma unroll
-        for (int cc = 0; cc < CH; cc++) {
-            const int c = c0 + cc;
-            /* columns 16 c .. 16 c + 15 (y-corners 2 c, 2 c + 1) of every issuer's accumulator, summed in issuer order */
-            float v[16];
-            {
-                const uint32_t row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(16 * c);
-                uint32_t r[TC_ISSUERS][16];
-#pragma unroll
-                for (int i = 0; i < TC_ISSUERS; i++)
-                    tc_ld16(row + (uint32_t)(8 * Q * i), r[i]);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int e = 0; e < 16; e++) {
-                    v[e] = __uint_as_float(r[0][e]);
-#pragma unroll
-                    for (int i = 1; i < TC_ISSUERS; i++)
-                        if (i < nk) /* an issuer with no stage left its accumulator unwritten */
-                            v[e] += __uint_as_float(r[i][e]);
-                }
+        /* f(its number, q, s, score, factor, bound) over the thread's corners on the step grid */
+        auto tol_of = [&](int i, int s) {
+            if constexpr (FILTER) {
+                const uint32_t ew[4] = {er[i].x, er[i].y, er[i].z, er[i].w};
+                return __half2float(__ushort_as_half((uint16_t)(ew[s >> 1] >> (16 * (s & 1)))));
+            } else {
+                return 0.0f;
             }
+        };
+        auto corners = [&](auto f) {
 #pragma unroll
-            for (int qq = 0; qq < 2; qq++) {
-                const int q = 2 * c + qq, yr = ty * Q + q;
-                if (yr >= fh || (yr & (p.step - 1)))
-                    continue;
-                const int i = 2 * cc + qq;
-                const uint32_t jw[4] = {jr[i].x, jr[i].y, jr[i].z, jr[i].w};
-                const float fq[8] = {fr[2 * i].x, fr[2 * i].y, fr[2 * i].z, fr[2 * i].w,
-                                     fr[2 * i + 1].x, fr[2 * i + 1].y, fr[2 * i + 1].z, fr[2 * i + 1].w};
+            for (int cc = 0; cc < CH; cc++) {
+                const int c = c0 + cc;
+                /* columns 16 c .. 16 c + 15 (y-corners 2 c, 2 c + 1) of every issuer's accumulator, summed in issuer
+                 * order */
+                float v[16];
+                {
+                    const uint32_t row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(16 * c);
+                    uint32_t r[TC_ISSUERS][16];
 #pragma unroll
-                for (int s = 0; s < 8; s++) {
-                    if (!((xmask >> s) & 1u))
+                    for (int i = 0; i < TC_ISSUERS; i++)
+                        tc_ld16(row + (uint32_t)(8 * Q * i), r[i]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int e = 0; e < 16; e++) {
+                        v[e] = __uint_as_float(r[0][e]);
+#pragma unroll
+                        for (int i = 1; i < TC_ISSUERS; i++)
+                            if (i < nk) /* an issuer with no stage left its accumulator unwritten */
+                                v[e] += __uint_as_float(r[i][e]);
+                    }
+                }
+#pragma unroll
+                for (int qq = 0; qq < 2; qq++) {
+                    const int q = 2 * c + qq, yr = ty * Q + q;
+                    if (yr >= fh || (yr & (p.step - 1)))
                         continue;
-                    const float j0 = from16((uint16_t)(jw[s >> 1] >> (16 * (s & 1))), KIND);
-                    /* a near-blank window's factor is 0: + 0 makes its score +0 whatever the sign of the sum, the
-                     * reference's 0 (a -0 would order below the other cells' +0 in the top-8 keys) */
-                    const float score = (v[8 * qq + s] - j0 * p.sum_t) * fq[s] + 0.0f;
-                    const int key = ((ly0 + q) >> sh) * per + ((8 * (m & 1) + s) >> sh);
-                    if (score > best || (score == best && key < bkey)) {
-                        best = score;
-                        bkey = key;
+                    const int i = 2 * cc + qq;
+                    const uint32_t jw[4] = {jr[i].x, jr[i].y, jr[i].z, jr[i].w};
+                    const float fq[8] = {fr[2 * i].x, fr[2 * i].y, fr[2 * i].z, fr[2 * i].w,
+                                         fr[2 * i + 1].x, fr[2 * i + 1].y, fr[2 * i + 1].z, fr[2 * i + 1].w};
+#pragma unroll
+                    for (int s = 0; s < 8; s++) {
+                        if (!((xmask >> s) & 1u))
+                            continue;
+                        const float j0 = from16((uint16_t)(jw[s >> 1] >> (16 * (s & 1))), KIND);
+                        /* a near-blank window's factor is 0: + 0 makes its score +0 whatever the sign of the sum, the
+                         * reference's 0 (a -0 would order below the other cells' +0 in the top-8 keys) */
+                        f(8 * (2 * cc + qq) + s, q, s, (v[8 * qq + s] - j0 * p.sum_t) * fq[s] + 0.0f, fq[s], tol_of(i, s));
                     }
                 }
             }
-        }
-        const float ob = __shfl_xor_sync(VTG_FULL, best, 1);
-        const int okey = __shfl_xor_sync(VTG_FULL, bkey, 1);
-        if (ob > best || (ob == best && okey < bkey)) {
-            best = ob;
-            bkey = okey;
-        }
+        };
+        auto key_of = [&](int q, int s) { return ((ly0 + q) >> sh) * per + ((8 * (m & 1) + s) >> sh); };
         const int ccol = tx * (TC_XS / NCC_CELL) + (m >> 1), crow = (Y0 - p.y0) / NCC_CELL;
-        if ((m & 1) == 0 && ccol < p.ccols && crow < p.crows && bkey < (1 << 30))
-            atomicMax(cellw + (size_t)crow * p.ccols + ccol, cell_word(best, bkey));
+        const bool mine = ccol < p.ccols && crow < p.crows;
+        if constexpr (FILTER) {
+            float lb = -2.0f;
+            int zkey = 1 << 30;
+            corners([&](int, int q, int s, float score, float fac, float e) {
+                if (fac > 0.0f) {
+                    lb = fmaxf(lb, score - e);
+                } else {
+                    lb = fmaxf(lb, 0.0f);
+                    zkey = min(zkey, key_of(q, s));
+                }
+            });
+            lb = fmaxf(lb, __shfl_xor_sync(VTG_FULL, lb, 1));
+            zkey = min(zkey, __shfl_xor_sync(VTG_FULL, zkey, 1));
+            if constexpr (TcShape<Q>::halves == 2) { /* the cell's other eight rows: the pair warp's */
+                __shared__ float s_lb[2][128];
+                s_lb[warp >> 2][m] = lb;
+                __syncthreads();
+                lb = fmaxf(lb, s_lb[(warp >> 2) ^ 1][m]);
+            }
+            if ((m & 1) == 0 && mine && zkey < (1 << 30))
+                atomicMax(cellw + (size_t)crow * p.ccols + ccol, ncc_cell_word(0.0f, zkey));
+            unsigned long long keep = 0ull;
+            corners([&](int k, int, int, float score, float fac, float e) {
+                if (fac > 0.0f && score + e >= lb)
+                    keep |= 1ull << k;
+            });
+            /* the warp's corners take a run of the list */
+            const int cnt = __popcll(keep);
+            int inc = cnt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int u = __shfl_up_sync(VTG_FULL, inc, d);
+                inc += lane >= d ? u : 0;
+            }
+            unsigned at = 0u;
+            if (lane == 31 && inc > 0)
+                at = atomicAdd(ncand, (unsigned)inc);
+            at = __shfl_sync(VTG_FULL, at, 31) + (unsigned)(inc - cnt);
+            while (keep) {
+                const int k = __ffsll((long long)keep) - 1;
+                keep &= keep - 1ull;
+                cand[at++] = ((unsigned)(ty * Q + 2 * c0 + (k >> 3)) << 16) | (unsigned)(xr + (k & 7));
+            }
+        } else {
+            float best = -2.0f;
+            int bkey = 1 << 30;
+            corners([&](int, int q, int s, float score, float, float) {
+                const int key = key_of(q, s);
+                if (score > best || (score == best && key < bkey)) {
+                    best = score;
+                    bkey = key;
+                }
+            });
+            const float ob = __shfl_xor_sync(VTG_FULL, best, 1);
+            const int okey = __shfl_xor_sync(VTG_FULL, bkey, 1);
+            if (ob > best || (ob == best && okey < bkey)) {
+                best = ob;
+                bkey = okey;
+            }
+            if ((m & 1) == 0 && mine && bkey < (1 << 30))
+                atomicMax(cellw + (size_t)crow * p.ccols + ccol, ncc_cell_word(best, bkey));
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -612,66 +727,92 @@ __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, c
     }
 }
 
+/* A search's tiles and scratch sizes on the tensor-core map. */
+struct TcGrid {
+    int krow, q, fw, fh, tiles_x, tiles_y, cpitch, fpitch, rows;
+};
+
+static TcGrid tc_grid(const NccPrm &p)
+{
+    TcGrid g;
+    g.krow = tc_krow(p.tw);
+    g.q = tc_q(p.tw, p.th);
+    g.fw = p.x1 - p.x0 + 1;
+    g.fh = p.y1 - p.y0 + 1;
+    g.tiles_x = (g.fw + TC_XS - 1) / TC_XS;
+    g.tiles_y = (g.fh + g.q - 1) / g.q;
+    g.cpitch = g.tiles_x * TC_XS + TC_MAX_KROW;
+    g.fpitch = g.tiles_x * TC_XS;          /* every tile's 1,024 corners inside a factor row */
+    g.rows = p.y0 + g.tiles_y * g.q + p.th; /* every row a tile's band reads */
+    return g;
+}
+
+static bool tc_fits(const NccPrm &p, const NccScratch &s, const TcGrid &g)
+{
+    return s.band && s.conv && s.fac && s.cellw && p.tw <= 128 && (size_t)g.cpitch * g.rows <= s.conv_elems &&
+           (size_t)g.fpitch * g.fh <= s.fac_elems && !(p.step & (p.step - 1)) && NCC_CELL % p.step == 0 &&
+           /* the converting CTAs zero the cells' words */
+           (long long)((g.cpitch / 8 + 255) / 256) * g.rows * 256 >= (long long)p.ccols * p.crows;
+}
+
+bool vtg_ncc_filters(const NccPrm &p, const NccScratch &s)
+{
+    if (!s.cand || !s.tol || !(p.flt_a >= 0.0f) || (p.step != 1 && p.step != 2) || p.w < 64)
+        return false;
+    const TcGrid g = tc_grid(p);
+    /* The filter costs a preparation over the plane and two more launches; the map it replaces is one launch whose CTAs take
+     * their whole template's products in one chain. Measured (whole searches, filter against map, us): 64 x 64 over 201 x
+     * 201 corners 77 / 110, over a 1080p frame 94 / 748; 32 x 32 over 401 x 301 corners (1.2e8 products) 56 / 51, over a
+     * 640 x 480 frame (2.8e8) 57 / 64, over a 1080p frame 70 / 227; 16 x 16 over 1280 x 720 (2.3e8) 57 / 57. So it takes every
+     * template from 2,048 pixels on, and smaller ones from 2.5e8 products. */
+    const double products = (double)g.fw * g.fh * p.n / (p.step * p.step);
+    return (p.n >= 2048 || products >= 2.5e8) && tc_fits(p, s, g) && (size_t)g.fw * g.fh <= s.cand_elems &&
+           (size_t)g.fpitch * g.fh <= s.tol_elems;
+}
+
+/* The preparation and the map. The map (and the passes after it) start as programmatic dependents, their launch and
+ * setup overlapping the kernel before, except when events around the map time it alone. */
+template <int KIND, bool FILTER>
+static cudaError_t tc_launch(const uint8_t *plane, int pitch, const NccPrm &p, const NccScratch &s, const TcGrid &g,
+                             cudaStream_t st)
+{
+    const TcSmem sm = tc_smem(g.krow, g.q);
+    const int cells = p.ccols * p.crows;
+    const int btx = bp_tx(p.tw), bgx = (g.fw + btx - 1) / btx, nbox = bgx * ((g.fh + BP_TY - 1) / BP_TY);
+    const int cgx = (g.cpitch / 8 + 255) / 256, nconv = cgx * g.rows;
+    ncc_prep<KIND, FILTER><<<nbox + nconv, 256, 0, st>>>(plane, pitch, p, g.fw, g.fpitch, btx, bgx, nbox, s.fac, s.tol, g.rows,
+                                                         g.cpitch, cgx, s.conv, s.cellw, cells, s.ncand);
+    const bool pdl = !s.map_ev0;
+    auto run = [&](auto kernel, int threads) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm.total);
+        if (e == cudaSuccess && s.map_ev0)
+            e = cudaEventRecord(s.map_ev0, st);
+        if (e != cudaSuccess)
+            return e;
+        return vtg_launch_k(kernel, dim3(g.tiles_x * g.tiles_y), dim3(threads), sm.total, st, pdl, p,
+                            (const uint16_t *)s.band, g.krow, g.tiles_x, sm.a_bytes, sm.stage_bytes, (const uint16_t *)s.conv,
+                            g.cpitch, (const float *)s.fac, g.fpitch, s.cellw, s.err, (const uint16_t *)s.tol, s.cand, s.ncand);
+    };
+    return g.q == 8 ? run(ncc_map_tc<KIND, 8, FILTER>, TcShape<8>::threads) : run(ncc_map_tc<KIND, 16, FILTER>, TcShape<16>::threads);
+}
+
+cudaError_t vtg_launch_ncc_filter(const uint8_t *plane, int pitch, const NccPrm &p, const NccScratch &s, cudaStream_t st)
+{
+    return tc_launch<VTG_NCC_FP16, true>(plane, pitch, p, s, tc_grid(p), st);
+}
+
 cudaError_t vtg_launch_ncc_map_tc(const void *plane, int pitch, int elem_bytes, const NccPrm &p, const NccScratch &s,
                                   int kind, cudaStream_t st)
 {
-    if (elem_bytes != 1 || !s.band || !s.conv || !s.fac || !s.cellw || (kind != VTG_NCC_BF16 && kind != VTG_NCC_FP16) ||
-        p.tw > 128)
+    const TcGrid g = tc_grid(p);
+    if (elem_bytes != 1 || (kind != VTG_NCC_BF16 && kind != VTG_NCC_FP16) || !tc_fits(p, s, g))
         return cudaErrorInvalidValue;
-    const int krow = tc_krow(p.tw), q = tc_q(p.tw, p.th);
-    const TcSmem sm = tc_smem(krow, q);
-    const int fw = p.x1 - p.x0 + 1, fh = p.y1 - p.y0 + 1;
-    const int tiles_x = (fw + TC_XS - 1) / TC_XS, tiles_y = (fh + q - 1) / q;
-    const int cpitch = tiles_x * TC_XS + TC_MAX_KROW;
-    const int fpitch = tiles_x * TC_XS; /* every tile's 1,024 corners inside a factor row */
-    const int rows = p.y0 + tiles_y * q + p.th; /* every row a tile's band reads */
-    if ((size_t)cpitch * rows > s.conv_elems || (size_t)fpitch * fh > s.fac_elems || (p.step & (p.step - 1)) ||
-        NCC_CELL % p.step)
-        return cudaErrorInvalidValue;
-    const int cells = p.ccols * p.crows;
-    cudaError_t e = cudaSuccess;
-    const int btx = bp_tx(p.tw), bgx = (fw + btx - 1) / btx, nbox = bgx * ((fh + BP_TY - 1) / BP_TY);
-    const int cgx = (cpitch / 8 + 255) / 256, nconv = cgx * rows;
-    if ((long long)nconv * 256 < cells) /* the converting CTAs zero the cells' words */
-        return cudaErrorInvalidValue;
-    if (kind == VTG_NCC_BF16)
-        ncc_prep<VTG_NCC_BF16><<<nbox + nconv, 256, 0, st>>>((const uint8_t *)plane, pitch, p, fw, fpitch, btx, bgx, nbox,
-                                                             s.fac, rows, cpitch, cgx, s.conv, s.cellw, cells);
-    else
-        ncc_prep<VTG_NCC_FP16><<<nbox + nconv, 256, 0, st>>>((const uint8_t *)plane, pitch, p, fw, fpitch, btx, bgx, nbox,
-                                                             s.fac, rows, cpitch, cgx, s.conv, s.cellw, cells);
-    /* the map and the passes after it start as programmatic dependents (their launch and setup overlap the kernel
-     * before), except when events around the map time it alone */
-    const bool pdl = !s.map_ev0;
-#define MAP_TC(K, QQ)                                                                                                  \
-    do {                                                                                                               \
-        e = cudaFuncSetAttribute(ncc_map_tc<K, QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm.total);       \
-        if (e != cudaSuccess)                                                                                          \
-            return e;                                                                                                  \
-        if (s.map_ev0 && (e = cudaEventRecord(s.map_ev0, st)) != cudaSuccess)                                          \
-            return e;                                                                                                  \
-        e = vtg_launch_k(ncc_map_tc<K, QQ>, dim3(tiles_x * tiles_y), dim3(TcShape<QQ>::threads), sm.total, st, pdl,    \
-                         p, (const uint16_t *)s.band, krow, tiles_x, sm.a_bytes, sm.stage_bytes,                        \
-                         (const uint16_t *)s.conv, cpitch, (const float *)s.fac, fpitch, s.cellw, s.err);              \
-        if (e != cudaSuccess)                                                                                          \
-            return e;                                                                                                  \
-        if (s.map_ev1 && (e = cudaEventRecord(s.map_ev1, st)) != cudaSuccess)                                          \
-            return e;                                                                                                  \
-    } while (0)
-    if (kind == VTG_NCC_BF16) {
-        if (q == 8)
-            MAP_TC(VTG_NCC_BF16, 8);
-        else
-            MAP_TC(VTG_NCC_BF16, 16);
-    } else {
-        if (q == 8)
-            MAP_TC(VTG_NCC_FP16, 8);
-        else
-            MAP_TC(VTG_NCC_FP16, 16);
-    }
-#undef MAP_TC
-    if ((e = cudaGetLastError()) != cudaSuccess)
+    cudaError_t e = kind == VTG_NCC_BF16 ? tc_launch<VTG_NCC_BF16, false>((const uint8_t *)plane, pitch, p, s, g, st)
+                                         : tc_launch<VTG_NCC_FP16, false>((const uint8_t *)plane, pitch, p, s, g, st);
+    if (e == cudaSuccess && s.map_ev1)
+        e = cudaEventRecord(s.map_ev1, st);
+    if (e != cudaSuccess)
         return e;
     /* the cells from their words, and their best eight */
-    return vtg_launch_ncc_top(p, s, true, st, pdl);
+    return vtg_launch_ncc_top(p, s, true, st, !s.map_ev0);
 }

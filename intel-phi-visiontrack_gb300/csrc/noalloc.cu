@@ -146,6 +146,9 @@ extern "C" int vtg_search_run_noalloc(const void *plane, int w, int h, int pitch
     s.fac = nullptr;
     s.fac_elems = 0;
     s.cellw = nullptr;
+    s.cand = s.ncand = nullptr;
+    s.tol = nullptr;
+    s.cand_elems = s.tol_elems = 0;
     s.map_ev0 = s.map_ev1 = nullptr;
     e = vtg_launch_ncc(plane, pitch, plane_type, app, p, s, VTG_NCC_F32, found, st);
     const size_t cells = (size_t)p.ccols * p.crows;

@@ -22,6 +22,14 @@ struct NccPrm {
     /* the near-blank rule on exact integers: n var <= nthr, 16 n var <= nthr16 (half pixels) */
     long long nthr, nthr16;
     float rnorm; /* sqrt(n / norm): the tensor-core map's factor is rnorm / sqrt(n var) */
+    /* the F32 map by filter: how far a corner's FP16 tensor-core score may lie from its F32 score, flt_a + flt_m |its
+     * window's mean - 128| / sigma + flt_f |mean - first pixel| / sigma (vtg_ncc_filter_bound); flt_a < 0: no bound */
+    float flt_a, flt_m, flt_f;
+};
+
+/* What the 16-bit band loses of the template, summed in double (ncc_band_sum): h the rounded value, d = t - h. */
+struct NccBandStats {
+    float sum_h, sum_d, sum_dd, sum_tt; /* sum h, sum d, sum d^2, sum t^2 */
 };
 
 /* nthr = floor(n norm / 16) and nthr16 = floor(n norm): n norm is exact in double (n <= 2^14, norm an F32), so an
@@ -56,6 +64,12 @@ struct NccScratch {
     unsigned long long *topblk;
     int topblk_lists; /* lists topblk holds */
     unsigned *arrive;
+    /* the F32 map by filter: the corners to score exactly ((y - y0) << 16 | (x - x0)), in the integral images' place
+     * (that map uses none), room for every corner of the plane; and how many they are */
+    unsigned *cand, *ncand;
+    size_t cand_elems;
+    uint16_t *tol; /* that map's bound a corner (FP16, rounded up), rows as fac's; beside the list */
+    size_t tol_elems;
     /* vtg_search_profile: events recorded just before and just after the map kernel (NULL: none) */
     cudaEvent_t map_ev0, map_ev1;
 };
@@ -64,6 +78,14 @@ struct NccScratch {
 #define NCC_TOPB_THREADS 256
 #define NCC_TOPB_PER 4
 static inline int ncc_top_ctas(int cells) { return (cells + NCC_TOPB_THREADS * NCC_TOPB_PER - 1) / (NCC_TOPB_THREADS * NCC_TOPB_PER); }
+
+/* A cell's candidate as one orderable word: higher score first, then the earlier corner in scan order. 0: none. */
+__device__ __forceinline__ unsigned long long ncc_cell_word(float v, int key)
+{
+    unsigned u = __float_as_uint(v);
+    u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+    return ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)key);
+}
 
 /* A cell of the tensor-core map from its 64-bit word (ordered score, inverted scan index): value and corner, or -2 and
  * the cell's origin where no corner was scored (the F32 map's convention). */
@@ -180,8 +202,17 @@ cudaError_t vtg_launch_ncc_corners(const void *plane, int pitch, int plane_type,
 /* The tensor-core map (ncc_tc.cu): the same map_v / map_x / map_y as ncc_map_f32, products in BF16 or FP16. */
 cudaError_t vtg_launch_ncc_map_tc(const void *plane, int pitch, int elem_bytes, const NccPrm &p, const NccScratch &s,
                                   int kind, cudaStream_t st);
+/* The F32 map by filter (U8 planes), first half: the FP16 tensor-core map, which leaves in s.cand the corners whose F32
+ * score may be their cell's best and in s.cellw the near-blank corners' zeros. */
+cudaError_t vtg_launch_ncc_filter(const uint8_t *plane, int pitch, const NccPrm &p, const NccScratch &s, cudaStream_t st);
+/* Whether that map takes a search of these sizes: its scratch is there and large enough, the bound holds and the
+ * search is large enough to gain by it. */
+bool vtg_ncc_filters(const NccPrm &p, const NccScratch &s);
+/* The bound's parts from the FP16 band's statistics; flt_a = -1 where it would let too many corners through. */
+void vtg_ncc_filter_bound(NccPrm &p, const NccBandStats &b);
 /* Builds the template band for the tensor-core map from a zero-mean template. */
-cudaError_t vtg_launch_ncc_band(const float *app, int tw, int th, int kind, uint16_t *band, float *sum_t, cudaStream_t st);
+cudaError_t vtg_launch_ncc_band(const float *app, int tw, int th, int kind, uint16_t *band, NccBandStats *stats,
+                                cudaStream_t st);
 size_t vtg_ncc_band_bytes(int tw, int th);
 
 #endif
