@@ -12,15 +12,15 @@
  * except the search window's origin, which the reference clamps into its padding (that moves the offsets searched)
  * and which is clamped here the same way.
  *
- * One call, on one stream:
- *   fg_reduce_kernel      the field's pyramid of both frames: level 0 is the frames' half size (x(levels))
- *   fg_hist_kernel        64-bin histograms of nine sections of both frames' level 1 (8 CTAs a section); the last
- *                         CTA's verdict
- *   fg_search_kernel      a warp an 8 x 8 block: the 24 x 24 window in shared memory, a lane 8 of the 256 offsets
- *   fg_filter_kernel      a thread a block: the 3 x 3's vector nearest the others
- *   fg_upscale_kernel     a thread a finer block: of four coarse vectors, the least 4 x 4 SAD, doubled
- *   fg_mid_kernel         a warp a block: the vectors at the middle instant
- *   fg_blend_kernel       a CTA a 16 x 16 tile of the full-size frame: the frame (Q6) and its bytes */
+ * One call, on one stream; each launch after the first a programmatic dependent of the one before:
+ *   fg_reduce3_kernel     three levels of the field's pyramid of both frames at once: level 0 is the frames' half size
+ *                         (once more for each further three levels); beside the second, the scene test: 64-bin
+ *                         histograms of nine sections of both frames' level 1, the last CTA's verdict
+ *   fg_search_kernel      once a level, coarsest first: a warp an 8 x 8 block. Its estimate from the coarser level (the
+ *                         coarser fields' filter and the upscale, a few lanes' work each), then the 24 x 24 window in
+ *                         shared memory, a lane 8 of the 256 offsets
+ *   fg_mid_kernel         a warp a block: the finest field's filter, then the vectors at the middle instant
+ *   fg_blend_kernel       a warp a 16 x 16 tile of the full-size frame: the frame (Q6) and its bytes */
 #include <math.h>
 #include <stdint.h>
 
@@ -54,9 +54,10 @@ struct vtg_framegen {
     unsigned char *pic;
 };
 
+/* Coherent loads: what a launch before this one wrote was not read-only while this one, its dependent, ran. */
 __device__ __forceinline__ float fg_at(const float *p, int pitch, int w, int h, int x, int y)
 {
-    return __ldg(p + (size_t)min(max(y, 0), h - 1) * pitch + min(max(x, 0), w - 1));
+    return __ldca(p + (size_t)min(max(y, 0), h - 1) * pitch + min(max(x, 0), w - 1));
 }
 
 __device__ __forceinline__ float fg_warp_sum(float v)
@@ -67,65 +68,166 @@ __device__ __forceinline__ float fg_warp_sum(float v)
     return v;
 }
 
-/* One pyramid step of both frames (img_reduce, src/kern/img_ref.c:98-114): the 5 x 5 binomial, (sum + 128) >> 8,
- * clamped borders; blockIdx.z picks the frame. */
-__global__ void fg_reduce_kernel(const float *__restrict__ sa, const float *__restrict__ sb, int sw, int sh,
-                                 int spa, int spb, float *__restrict__ da, float *__restrict__ db, int dw, int dh,
-                                 int dp)
+/* Three pyramid steps of both frames (img_reduce, src/kern/img_ref.c:98-114: the 5 x 5 binomial, (sum + 128) >> 8, clamped
+ * borders) in one launch. A CTA owns a 64 x 32 block of the first level made and the 32 x 16 and 16 x 8 blocks under it. The
+ * first level's vertical sums come straight from the source, a thread a column and eleven rows of them (25 loads in
+ * flight), for the 73 x 41 values that the levels above need; the rest runs in shared memory. A level reads the one below at
+ * the reference's clamped indices, which always fall inside the computed halo. At 1080p, both frames, levels 0 to 2: FGR3 us
+ * where a launch a level took 12 + 6 + 4 (25 loads a value). */
+#define FR_X 64
+#define FR_Y 32
+#define FR_A_C 73 /* the first level computed: columns X0 - 6 .. X0 + 66, rows Y0 - 6 .. Y0 + 34 */
+#define FR_A_R 41
+#define FR_S_C (2 * FR_A_C + 3) /* its source columns, from 2 X0 - 14 */
+#define FR_B_C 35
+#define FR_B_R 19
+#define FR_C_C 16
+#define FR_C_R 8
+#define FR_SEG 11 /* rows of vertical sums a thread: four segments */
+
+struct FgReduce {
+    const float *s[2];
+    int sw, sh, sp[2];
+    int n; /* levels to make, 1 to 3 */
+    float *d[3][2];
+    int w[3], h[3], p[3];
+    int bx, by; /* blocks */
+};
+
+struct FgReduceSmem {
+    int v[FR_A_R][FR_S_C]; /* the first level's vertical sums */
+    int a[FR_A_R][FR_A_C];
+    int v2[FR_B_R][FR_A_C];
+    int b[FR_B_R][FR_B_C];
+    int v3[FR_C_R][FR_B_C];
+};
+
+__device__ __forceinline__ int fg_tap5(int a, int b, int c, int d, int e) { return a + e + 4 * (b + d) + 6 * c; }
+
+__device__ void fg_reduce_block(const FgReduce &q, int block, FgReduceSmem &S)
 {
-    const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), y = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    if (x >= dw || y >= dh)
-        return;
-    const float *s = blockIdx.z ? sb : sa;
-    const int sp = blockIdx.z ? spb : spa;
-    const int k[5] = {1, 4, 6, 4, 1};
-    int sum = 0;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int f = block / (q.bx * q.by), at = block - f * q.bx * q.by;
+    const int X0 = (at % q.bx) * FR_X, Y0 = (at / q.bx) * FR_Y;
+    const float *src = q.s[f];
+    for (int i = tid; i < 4 * FR_S_C; i += nt) {
+        const int g = i / FR_S_C, c = i - g * FR_S_C, r0 = g * FR_SEG;
+        const float *col = src + min(max(2 * X0 - 14 + c, 0), q.sw - 1);
+        int v[2 * FR_SEG + 3];
 #pragma unroll
-    for (int j = 0; j < 5; j++) {
-        int row = 0;
+        for (int k = 0; k < 2 * FR_SEG + 3; k++)
+            v[k] = (int)__ldca(col + (size_t)min(max(2 * (Y0 - 6 + r0) - 2 + k, 0), q.sh - 1) * q.sp[f]);
 #pragma unroll
-        for (int i = 0; i < 5; i++)
-            row += k[i] * (int)fg_at(s, sp, sw, sh, 2 * x + i - 2, 2 * y + j - 2);
-        sum += k[j] * row;
+        for (int r = 0; r < FR_SEG; r++)
+            if (r0 + r < FR_A_R)
+                S.v[r0 + r][c] = fg_tap5(v[2 * r], v[2 * r + 1], v[2 * r + 2], v[2 * r + 3], v[2 * r + 4]);
     }
-    (blockIdx.z ? db : da)[(size_t)y * dp + x] = (float)((sum + 128) >> 8);
+    __syncthreads();
+    for (int i = tid; i < FR_A_R * FR_A_C; i += nt) {
+        const int y = i / FR_A_C, x = i - y * FR_A_C;
+        const int *v = &S.v[y][2 * x];
+        const int o = (fg_tap5(v[0], v[1], v[2], v[3], v[4]) + 128) >> 8;
+        S.a[y][x] = o;
+        const int gy = Y0 - 6 + y, gx = X0 - 6 + x;
+        if (y >= 6 && y < 6 + FR_Y && x >= 6 && x < 6 + FR_X && gy < q.h[0] && gx < q.w[0])
+            q.d[0][f][(size_t)gy * q.p[0] + gx] = (float)o;
+    }
+    if (q.n < 2)
+        return;
+    __syncthreads();
+    for (int i = tid; i < FR_B_R * FR_A_C; i += nt) {
+        const int y = i / FR_A_C, x = i - y * FR_A_C;
+        int v[5];
+#pragma unroll
+        for (int t = 0; t < 5; t++)
+            v[t] = S.a[min(max(2 * (Y0 / 2 - 2 + y) - 2 + t, 0), q.h[0] - 1) - (Y0 - 6)][x];
+        S.v2[y][x] = fg_tap5(v[0], v[1], v[2], v[3], v[4]);
+    }
+    __syncthreads();
+    for (int i = tid; i < FR_B_R * FR_B_C; i += nt) {
+        const int y = i / FR_B_C, x = i - y * FR_B_C;
+        int v[5];
+#pragma unroll
+        for (int t = 0; t < 5; t++)
+            v[t] = S.v2[y][min(max(2 * (X0 / 2 - 2 + x) - 2 + t, 0), q.w[0] - 1) - (X0 - 6)];
+        const int o = (fg_tap5(v[0], v[1], v[2], v[3], v[4]) + 128) >> 8;
+        S.b[y][x] = o;
+        const int gy = Y0 / 2 - 2 + y, gx = X0 / 2 - 2 + x;
+        if (y >= 2 && y < 2 + FR_Y / 2 && x >= 2 && x < 2 + FR_X / 2 && gy < q.h[1] && gx < q.w[1])
+            q.d[1][f][(size_t)gy * q.p[1] + gx] = (float)o;
+    }
+    if (q.n < 3)
+        return;
+    __syncthreads();
+    for (int i = tid; i < FR_C_R * FR_B_C; i += nt) {
+        const int y = i / FR_B_C, x = i - y * FR_B_C;
+        int v[5];
+#pragma unroll
+        for (int t = 0; t < 5; t++)
+            v[t] = S.b[min(max(2 * (Y0 / 4 + y) - 2 + t, 0), q.h[1] - 1) - (Y0 / 2 - 2)][x];
+        S.v3[y][x] = fg_tap5(v[0], v[1], v[2], v[3], v[4]);
+    }
+    __syncthreads();
+    for (int i = tid; i < FR_C_R * FR_C_C; i += nt) {
+        const int y = i / FR_C_C, x = i - y * FR_C_C;
+        const int gy = Y0 / 4 + y, gx = X0 / 4 + x;
+        if (gy >= q.h[2] || gx >= q.w[2])
+            continue;
+        int v[5];
+#pragma unroll
+        for (int t = 0; t < 5; t++)
+            v[t] = S.v3[y][min(max(2 * gx - 2 + t, 0), q.w[1] - 1) - (X0 / 2 - 2)];
+        q.d[2][f][(size_t)gy * q.p[2] + gx] = (float)((fg_tap5(v[0], v[1], v[2], v[3], v[4]) + 128) >> 8);
+    }
 }
 
-/* fg_hist_section (framegen.c:85-101): section blockIdx.x % 9 of frame blockIdx.x / 9, its sampled rows split over
- * FG_HIST_SPLIT CTAs (blockIdx.y), added into the global counts; the last CTA compares the frames (fg_scene_verdict,
+/* fg_hist_section (framegen.c:85-101): part `part` of FG_HIST_SPLIT of the sampled rows of section s of frame f, counted
+ * a warp and added into the global counts; the last CTA of the test compares the frames (fg_scene_verdict,
  * framegen.c:103-113: more than half the samples in other bins, i.e. sum |a - b| > sum b) and zeroes the counts for
  * the next call. */
 #define FG_HIST_SPLIT 8
-__global__ void __launch_bounds__(256) fg_hist_kernel(FgLevel lv, unsigned *__restrict__ hist, int *scene)
+#define FG_HIST_CTAS (18 * FG_HIST_SPLIT)
+struct FgHistSmem {
+    unsigned h[8][64];
+    unsigned long long sum[8][2];
+    bool last;
+};
+
+__device__ void fg_hist_part(const FgLevel &lv, int k0, unsigned *__restrict__ hist, int *scene, FgHistSmem &S)
 {
-    __shared__ unsigned s_h[64];
-    __shared__ bool s_last;
-    const int tid = threadIdx.x, s = blockIdx.x % 9, f = blockIdx.x / 9;
-    if (tid < 64)
-        s_h[tid] = 0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int s = k0 % 9, f = (k0 / 9) % 2, part = k0 / 18;
+    for (int i = tid; i < 8 * 64; i += 256)
+        S.h[i >> 6][i & 63] = 0u;
     __syncthreads();
     const float *p = f ? lv.b : lv.a;
     const int sx = s % 3, sy = s / 3;
     const int x0 = (lv.w * sx / 3) & ~15, x1 = (lv.w * (sx + 1) / 3) & ~15;
     const int y0 = lv.h * sy / 3, y1 = lv.h * (sy + 1) / 3;
     const int cols = x1 - x0, rows = (y1 - y0 + 1) / 2;
-    for (int k = (int)blockIdx.y * blockDim.x + tid; k < cols * rows; k += FG_HIST_SPLIT * blockDim.x) {
+    for (int k = part * 256 + tid; k < cols * rows; k += FG_HIST_SPLIT * 256) {
         const int y = y0 + 2 * (k / cols), x = x0 + k % cols;
-        atomicAdd(&s_h[(int)(p[(size_t)y * lv.pitch + x] * (1.0f / 256.0f)) & 63], 1u);
+        atomicAdd(&S.h[warp][(int)(__ldca(p + (size_t)y * lv.pitch + x) * (1.0f / 256.0f)) & 63], 1u);
     }
     __syncthreads();
-    if (tid < 64 && s_h[tid])
-        atomicAdd(&hist[(f * 9 + s) * 64 + tid], s_h[tid]);
+    if (tid < 64) {
+        unsigned n = 0u;
+#pragma unroll
+        for (int w = 0; w < 8; w++)
+            n += S.h[w][tid];
+        if (n)
+            atomicAdd(&hist[(f * 9 + s) * 64 + tid], n);
+    }
     __threadfence();
     __syncthreads();
     if (tid == 0)
-        s_last = atomicAdd(&scene[1], 1) == (int)(gridDim.x * gridDim.y) - 1;
+        S.last = atomicAdd(&scene[1], 1) == FG_HIST_CTAS - 1;
     __syncthreads();
-    if (!s_last || tid >= 32)
+    if (!S.last)
         return;
     __threadfence();
     unsigned long long diff = 0, total = 0;
-    for (int i = tid; i < 9 * 64; i += 32) {
+    for (int i = tid; i < 9 * 64; i += 256) {
         const unsigned a = __ldcg(&hist[i]), b = __ldcg(&hist[9 * 64 + i]);
         diff += a > b ? a - b : b - a;
         total += b;
@@ -137,32 +239,170 @@ __global__ void __launch_bounds__(256) fg_hist_kernel(FgLevel lv, unsigned *__re
         diff += __shfl_xor_sync(VTG_FULL, diff, d);
         total += __shfl_xor_sync(VTG_FULL, total, d);
     }
+    if (lane == 0) {
+        S.sum[warp][0] = diff;
+        S.sum[warp][1] = total;
+    }
+    __syncthreads();
     if (tid == 0) {
+        diff = total = 0;
+        for (int w = 0; w < 8; w++) {
+            diff += S.sum[w][0];
+            total += S.sum[w][1];
+        }
         scene[0] = total && diff > total;
         scene[1] = 0;
     }
 }
 
-/* fg_search (framegen.c:117-214) at one level: a warp an 8 x 8 block. pred: the coarser level's estimate (NULL at the
+/* The levels' CTAs first, then (hist) the scene test's on level 1, which an earlier launch made. */
+__global__ void __launch_bounds__(256) fg_reduce3_kernel(FgReduce q, int reduces, FgLevel l1, unsigned *hist, int *scene)
+{
+    __shared__ union {
+        FgReduceSmem r;
+        FgHistSmem h;
+    } S;
+    vtg_grid_launch_dependents();
+    vtg_grid_dependency_wait();
+    if ((int)blockIdx.x < reduces)
+        fg_reduce_block(q, blockIdx.x, S.r);
+    else
+        fg_hist_part(l1, (int)blockIdx.x - reduces, hist, scene, S.h);
+}
+
+/* fg_filter (framegen.c:218-247) of the block at (bx, by): of the 3 x 3 around it (clamped, column by column), the vector
+ * with the least sum of squared differences from the nine; the first on a tie. `ways` lanes of a warp share a block, this
+ * one the `way`-th: candidates way, way + ways, ..; ways a power of two share by xor partners, 3 by the two lanes on. */
+template <int WAYS>
+__device__ __forceinline__ short2 fg_filtered(const FgLevel &lv, int bx, int by, int way)
+{
+    int mx[9], my[9];
+#pragma unroll
+    for (int xx = 0; xx < 3; xx++)
+#pragma unroll
+        for (int yy = 0; yy < 3; yy++) {
+            const int at = min(max(by + yy - 1, 0), lv.bh - 1) * lv.bw + min(max(bx + xx - 1, 0), lv.bw - 1);
+            const int v = __ldca(reinterpret_cast<const int *>(lv.raw) + at);
+            mx[xx * 3 + yy] = (short)(v & 0xffff);
+            my[xx * 3 + yy] = v >> 16;
+        }
+    unsigned least = ~0u;
+    int pick = 9, vx = 0, vy = 0;
+#pragma unroll
+    for (int k = 0; k < (9 + WAYS - 1) / WAYS; k++) {
+        const int a = way + k * WAYS;
+        int ax = mx[0], ay = my[0];
+#pragma unroll
+        for (int b = 1; b < 9; b++) {
+            ax = a == b ? mx[b] : ax;
+            ay = a == b ? my[b] : ay;
+        }
+        unsigned d = 0;
+#pragma unroll
+        for (int b = 0; b < 9; b++) {
+            const int dx = ax - mx[b], dy = ay - my[b];
+            d += (unsigned)(dx * dx + dy * dy);
+        }
+        if (a < 9 && (pick == 9 || d < least)) {
+            least = d;
+            pick = a;
+            vx = ax;
+            vy = ay;
+        }
+    }
+    auto meet = [&](unsigned ol, int op, int ox, int oy) {
+        if (ol < least || (ol == least && op < pick)) {
+            least = ol;
+            pick = op;
+            vx = ox;
+            vy = oy;
+        }
+    };
+    if constexpr (WAYS == 3) { /* lanes 3 k, 3 k + 1, 3 k + 2 of a block: the first one ends with its vector */
+        const int lane = threadIdx.x & 31;
+        const unsigned l1 = __shfl_sync(VTG_FULL, least, lane + 1), l2 = __shfl_sync(VTG_FULL, least, lane + 2);
+        const int p1 = __shfl_sync(VTG_FULL, pick, lane + 1), p2 = __shfl_sync(VTG_FULL, pick, lane + 2);
+        const int x1 = __shfl_sync(VTG_FULL, vx, lane + 1), x2 = __shfl_sync(VTG_FULL, vx, lane + 2);
+        const int y1 = __shfl_sync(VTG_FULL, vy, lane + 1), y2 = __shfl_sync(VTG_FULL, vy, lane + 2);
+        meet(l1, p1, x1, y1);
+        meet(l2, p2, x2, y2);
+    } else {
+#pragma unroll
+        for (int d = 1; d < WAYS; d <<= 1)
+            meet(__shfl_xor_sync(VTG_FULL, least, d), __shfl_xor_sync(VTG_FULL, pick, d), __shfl_xor_sync(VTG_FULL, vx, d),
+                 __shfl_xor_sync(VTG_FULL, vy, d));
+    }
+    return make_short2((short)vx, (short)vy);
+}
+
+/* fg_upscale (framegen.c:251-288) for block (gx, gy) of the level under `lv`, a warp: of the four nearest blocks' filtered
+ * vectors, the one with the least SAD over the 4 x 4 of lv that the block covers (the first on a tie), doubled. Eight lanes
+ * a candidate: its filter, then two pixels each. The block whose own coarse block is candidate 3 (both places even) stores
+ * that filtered vector: every coarse block has one. */
+__device__ __forceinline__ short2 fg_upscaled(const FgLevel &lv, int gx, int gy, int lane)
+{
+    const int n = lane >> 3;
+    const int cx = gx / 2 + n % 2 - 1 + gx % 2, cy = gy / 2 + n / 2 - 1 + gy % 2;
+    const int px = gx * 4 + (lane & 3), py = gy * 4 + ((lane >> 2) & 1);
+    const float c0 = fg_at(lv.b, lv.pitch, lv.w, lv.h, px, py), c1 = fg_at(lv.b, lv.pitch, lv.w, lv.h, px, py + 2);
+    const short2 v = fg_filtered<8>(lv, min(max(cx, 0), lv.bw - 1), min(max(cy, 0), lv.bh - 1), lane & 7);
+    if (lane == 24 && !(gx & 1) && !(gy & 1))
+        lv.fil[(gy / 2) * lv.bw + gx / 2] = v;
+    float s = fabsf(c0 - fg_at(lv.a, lv.pitch, lv.w, lv.h, px + v.x, py + v.y)) +
+              fabsf(c1 - fg_at(lv.a, lv.pitch, lv.w, lv.h, px + v.x, py + 2 + v.y));
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1)
+        s += __shfl_xor_sync(VTG_FULL, s, d);
+    int pick = n, vx = v.x, vy = v.y;
+#pragma unroll
+    for (int d = 8; d < 32; d <<= 1) {
+        const float os = __shfl_xor_sync(VTG_FULL, s, d);
+        const int op = __shfl_xor_sync(VTG_FULL, pick, d), ox = __shfl_xor_sync(VTG_FULL, vx, d), oy = __shfl_xor_sync(VTG_FULL, vy, d);
+        if (os < s || (os == s && op < pick)) {
+            s = os;
+            pick = op;
+            vx = ox;
+            vy = oy;
+        }
+    }
+    return make_short2((short)(2 * vx), (short)(2 * vy));
+}
+
+/* fg_search (framegen.c:117-214) at one level: a warp an 8 x 8 block, from the coarser level's estimate (lv.up; none at the
  * top). The 256 offsets x0 - px + dx, wy + dy - 8 (dx, dy < 16) cost |dx - 8| + |dy - 8| plus the block's SAD; the
  * first lowest in row order wins. On the finest level a block the estimate explains (SAD <= 8192) is not searched, and
  * no motion wins when its SAD is no more than the best cost. */
-__global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, const short2 *__restrict__ pred,
-                                                                  int level, const int *__restrict__ scene)
+__global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, FgLevel coarse, bool top, int level,
+                                                                  const int *__restrict__ scene)
 {
-    __shared__ float s_win[FG_WARPS][24][25];
-    __shared__ float s_blk[FG_WARPS][8][8];
+    /* rows of 28: a quarter warp's eight rows of 16 bytes fall in different banks */
+    __shared__ __align__(16) float s_win[FG_WARPS][24][28];
+    __shared__ __align__(16) float s_blk[FG_WARPS][8][8];
+    vtg_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = (int)blockIdx.x * FG_WARPS + warp;
+    vtg_grid_dependency_wait();
     if (i >= lv.bw * lv.bh)
         return;
-    if (*scene) {
-        if (lane == 0)
+    const int gx = i % lv.bw, gy = i / lv.bw;
+    if (__ldca(scene)) {
+        if (lane == 0) {
             lv.raw[i] = make_short2(0, 0);
+            if (!top) {
+                lv.up[i] = make_short2(0, 0);
+                if (!(gx & 1) && !(gy & 1))
+                    coarse.fil[(gy / 2) * coarse.bw + gx / 2] = make_short2(0, 0);
+            }
+        }
         return;
     }
-    const int px = (i % lv.bw) * 8, py = (i / lv.bw) * 8;
-    const short2 want = pred ? pred[i] : make_short2(0, 0);
+    const int px = gx * 8, py = gy * 8;
+    short2 want = make_short2(0, 0);
+    if (!top) {
+        want = fg_upscaled(coarse, gx, gy, lane);
+        if (lane == 0)
+            lv.up[i] = want;
+    }
     const int wx = want.x, wy = want.y;
     const int lanes = (lv.w + 15) & ~15;
     const int x0 = min(max(px + wx - 8, -32), lanes), y0 = py + wy - 8;
@@ -203,20 +443,20 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, co
             return;
         }
     }
-    const int dy = lane >> 1, dx0 = (lane & 1) * 8;
+    const int dy = lane & 15, dx0 = (lane >> 4) * 8;
     float c[8];
 #pragma unroll
     for (int k = 0; k < 8; k++)
         c[k] = (float)abs(dx0 + k - 8) + (float)abs(dy - 8); /* FG_TIE_UNIT */
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-        float wv[15], bv[8];
+        float wv[16], bv[8];
 #pragma unroll
-        for (int k = 0; k < 15; k++)
-            wv[k] = s_win[warp][dy + r][dx0 + k];
+        for (int k = 0; k < 4; k++)
+            *reinterpret_cast<float4 *>(&wv[4 * k]) = *reinterpret_cast<const float4 *>(&s_win[warp][dy + r][dx0 + 4 * k]);
 #pragma unroll
-        for (int n = 0; n < 8; n++)
-            bv[n] = s_blk[warp][r][n];
+        for (int k = 0; k < 2; k++)
+            *reinterpret_cast<float4 *>(&bv[4 * k]) = *reinterpret_cast<const float4 *>(&s_blk[warp][r][4 * k]);
 #pragma unroll
         for (int k = 0; k < 8; k++)
 #pragma unroll
@@ -253,92 +493,22 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, co
         lv.raw[i] = make_short2((short)vx, (short)vy);
 }
 
-/* fg_filter (framegen.c:218-247): of the 3 x 3 around a block (clamped, column by column), the vector with the least
- * sum of squared differences from the nine; the first on a tie. */
-__global__ void fg_filter_kernel(FgLevel lv)
-{
-    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= lv.bw * lv.bh)
-        return;
-    const int bx = i % lv.bw, by = i / lv.bw;
-    int mx[9], my[9];
-#pragma unroll
-    for (int xx = 0; xx < 3; xx++)
-#pragma unroll
-        for (int yy = 0; yy < 3; yy++) {
-            const short2 v = lv.raw[min(max(by + yy - 1, 0), lv.bh - 1) * lv.bw + min(max(bx + xx - 1, 0), lv.bw - 1)];
-            mx[xx * 3 + yy] = v.x;
-            my[xx * 3 + yy] = v.y;
-        }
-    int pick = 0;
-    unsigned least = 0;
-#pragma unroll
-    for (int a = 0; a < 9; a++) {
-        unsigned d = 0;
-#pragma unroll
-        for (int b = 0; b < 9; b++) {
-            const int dx = mx[a] - mx[b], dy = my[a] - my[b];
-            d += (unsigned)(dx * dx + dy * dy);
-        }
-        if (a == 0 || d < least) {
-            least = d;
-            pick = a;
-        }
-    }
-    lv.fil[i] = make_short2((short)mx[pick], (short)my[pick]);
-}
-
-/* fg_upscale (framegen.c:251-288): block (gx, gy) of the finer level (fine.bw x fine.bh) takes, of the four nearest
- * blocks of this level, the vector with the least SAD over the 4 x 4 of this level it covers (the first on a tie),
- * doubled. */
-__global__ void fg_upscale_kernel(FgLevel lv, short2 *__restrict__ up, int fbw, int fbh, const int *__restrict__ scene)
-{
-    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= fbw * fbh)
-        return;
-    if (*scene) {
-        up[i] = make_short2(0, 0);
-        return;
-    }
-    const int gx = i % fbw, gy = i / fbw;
-    /* the four candidates' SADs with all their loads in flight, then the first least */
-    short2 v[4];
-    float sad[4];
-#pragma unroll
-    for (int n = 0; n < 4; n++) {
-        const int xo = n % 2 - 1 + gx % 2, yo = n / 2 - 1 + gy % 2;
-        v[n] = lv.fil[min(max(gy / 2 + yo, 0), lv.bh - 1) * lv.bw + min(max(gx / 2 + xo, 0), lv.bw - 1)];
-    }
-    float cur[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++)
-        cur[k] = fg_at(lv.b, lv.pitch, lv.w, lv.h, gx * 4 + (k & 3), gy * 4 + (k >> 2));
-#pragma unroll
-    for (int n = 0; n < 4; n++) {
-        float s = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 16; k++)
-            s += fabsf(cur[k] - fg_at(lv.a, lv.pitch, lv.w, lv.h, gx * 4 + (k & 3) + v[n].x, gy * 4 + (k >> 2) + v[n].y));
-        sad[n] = s;
-    }
-    int pick = 0;
-#pragma unroll
-    for (int n = 1; n < 4; n++)
-        if (sad[n] < sad[pick])
-            pick = n;
-    up[i] = make_short2((short)(2 * v[pick].x), (short)(2 * v[pick].y));
-}
-
 /* fg_mid_vectors (framegen.c:292-328) on the finest level: no motion first, favoured by one grey level over the block
  * (FG_MID_FAVOUR_ZERO), then each vector of the 3 x 3 (row by row) that agrees better when each frame moves half way.
- * A warp a block, a lane two of its pixels. */
+ * A warp a block, a lane two of its pixels. The 3 x 3's filtered vectors first, three lanes each. */
 __global__ void __launch_bounds__(32 * FG_WARPS) fg_mid_kernel(FgLevel lv, short2 *__restrict__ mid)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = (int)blockIdx.x * FG_WARPS + warp;
+    vtg_grid_launch_dependents();
+    vtg_grid_dependency_wait();
     if (i >= lv.bw * lv.bh)
         return;
     const int bx = i % lv.bw, by = i / lv.bw, px = bx * 8, py = by * 8;
+    const int nb = min(lane / 3, 8); /* the 3 x 3's block of this lane, row by row */
+    const short2 fv = fg_filtered<3>(lv, min(max(bx + nb % 3 - 1, 0), lv.bw - 1), min(max(by + nb / 3 - 1, 0), lv.bh - 1), lane % 3);
+    if (lane == 12)
+        lv.fil[i] = fv;
     auto sad = [&](int vx, int vy) {
         const int ax = vx >> 1, ay = vy >> 1, qx = vx - ax, qy = vy - ay;
         float s = 0.0f;
@@ -351,71 +521,93 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_mid_kernel(FgLevel lv, short
     };
     float best = sad(0, 0) - 64.0f;
     int vx = 0, vy = 0;
-    for (int yy = 0; yy < 3; yy++)
-        for (int xx = 0; xx < 3; xx++) {
-            const short2 v = lv.fil[min(max(by + yy - 1, 0), lv.bh - 1) * lv.bw + min(max(bx + xx - 1, 0), lv.bw - 1)];
-            if ((v.x == vx && v.y == vy) || (v.x == 0 && v.y == 0))
-                continue;
-            const float s = sad(v.x, v.y);
-            if (s < best) {
-                best = s;
-                vx = v.x;
-                vy = v.y;
-            }
+    for (int k = 0; k < 9; k++) {
+        const int qx = __shfl_sync(VTG_FULL, (int)fv.x, 3 * k), qy = __shfl_sync(VTG_FULL, (int)fv.y, 3 * k);
+        if ((qx == vx && qy == vy) || (qx == 0 && qy == 0))
+            continue;
+        const float s = sad(qx, qy);
+        if (s < best) {
+            best = s;
+            vx = qx;
+            vy = qy;
         }
+    }
     if (lane == 0)
         mid[i] = make_short2((short)vx, (short)vy);
 }
 
-/* fg_blend (framegen.c:332-357) and img_q6_to_u8_vx: a CTA a 16 x 16 tile, a thread a pixel. */
-__global__ void __launch_bounds__(256) fg_blend_kernel(const float *__restrict__ a0, int pa, const float *__restrict__ b0,
-                                                       int pb, int w, int h, const short2 *__restrict__ mid, int bw,
-                                                       int bh, float *__restrict__ out, int po,
-                                                       unsigned char *__restrict__ pic)
+/* fg_blend (framegen.c:332-357) and img_q6_to_u8_vx: a warp a 16 x 16 tile, a lane eight of its pixels (a column's every
+ * second row), so that a lane has many loads in flight. */
+#define FG_BLEND_WARPS 8
+__global__ void __launch_bounds__(32 * FG_BLEND_WARPS) fg_blend_kernel(const float *__restrict__ a0, int pa,
+                                                                       const float *__restrict__ b0, int pb, int w, int h,
+                                                                       const short2 *mid, int bw, int bh,
+                                                                       float *__restrict__ out, int po,
+                                                                       unsigned char *__restrict__ pic)
 {
-    __shared__ short2 s_near[3][3];
-    __shared__ int s_same;
-    const int tid = threadIdx.x, tx = blockIdx.x, ty = blockIdx.y;
-    if (tid < 9)
-        s_near[tid / 3][tid % 3] = mid[min(max(ty + tid / 3 - 1, 0), bh - 1) * bw + min(max(tx + tid % 3 - 1, 0), bw - 1)];
-    __syncthreads();
-    if (tid == 0) {
-        int same = 1;
-        for (int k = 0; k < 9; k++)
-            same &= s_near[k / 3][k % 3].x == s_near[0][0].x && s_near[k / 3][k % 3].y == s_near[0][0].y;
-        s_same = same;
-    }
-    __syncthreads();
-    const int k = tid & 15, s = tid >> 4, x = tx * 16 + k, y = ty * 16 + s;
-    if (x >= w || y >= h)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tx = (int)blockIdx.x * FG_BLEND_WARPS + warp, ty = blockIdx.y;
+    vtg_grid_dependency_wait();
+    if (16 * tx >= w)
         return;
-    float v;
-    if (s_same) {
-        const int vx = s_near[0][0].x, vy = s_near[0][0].y;
-        v = rintf((fg_at(a0, pa, w, h, x + vx, y + vy) + fg_at(b0, pb, w, h, x - vx, y - vy)) * 0.5f);
-    } else {
-        /* in 32nds: across, the left, own and right blocks; down, the own row and the one above or below */
-        const float wl = k < 8 ? (float)(15 - 2 * k) : 0.0f, wr = k < 8 ? 0.0f : (float)(2 * k - 15);
-        const float ws = k < 8 ? (float)(17 + 2 * k) : (float)(47 - 2 * k);
-        const float wh[3] = {wl, ws, wr};
-        const int other = s < 8 ? 0 : 2, wo = s < 8 ? 15 - 2 * s : 2 * s - 15;
+    /* lane k < 9: the 3 x 3's vector k, row by row; the others the first one again */
+    const int nk = lane < 9 ? lane : 0;
+    const int near = __ldca(reinterpret_cast<const int *>(mid) + min(max(ty + nk / 3 - 1, 0), bh - 1) * bw +
+                            min(max(tx + nk % 3 - 1, 0), bw - 1));
+    const int first = __shfl_sync(VTG_FULL, near, 0);
+    const bool same = __all_sync(VTG_FULL, near == first);
+    const int k = lane & 15, x = tx * 16 + k;
+    auto store = [&](int y, float v) {
+        out[(size_t)y * po + x] = v;
+        if (pic) {
+            const float q = rintf(v * (1.0f / 64.0f));
+            pic[(size_t)y * w + x] = q <= 0.0f ? 0 : q >= 255.0f ? 255 : (unsigned char)q;
+        }
+    };
+    auto at = [&](const float *p, int pitch, int xx, int yy) {
+        return __ldg(p + (size_t)min(max(yy, 0), h - 1) * pitch + min(max(xx, 0), w - 1));
+    };
+    if (same) {
+        const int vx = (short)(first & 0xffff), vy = first >> 16;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int y = ty * 16 + 2 * j + (lane >> 4);
+            v[j] = rintf((at(a0, pa, x + vx, y + vy) + at(b0, pb, x - vx, y - vy)) * 0.5f);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int y = ty * 16 + 2 * j + (lane >> 4);
+            if (x < w && y < h)
+                store(y, v[j]);
+        }
+        return;
+    }
+    /* in 32nds: across, the left, own and right blocks; down, the own row and the one above or below */
+    const float wl = k < 8 ? (float)(15 - 2 * k) : 0.0f, wr = k < 8 ? 0.0f : (float)(2 * k - 15);
+    const float ws = k < 8 ? (float)(17 + 2 * k) : (float)(47 - 2 * k);
+    const float wh[3] = {wl, ws, wr};
+    int q[3][3];
+#pragma unroll
+    for (int n = 0; n < 9; n++)
+        q[n / 3][n % 3] = __shfl_sync(VTG_FULL, near, n);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int s = 2 * j + (lane >> 4), y = ty * 16 + s;
+        const int wo = s < 8 ? 15 - 2 * s : 2 * s - 15;
         const float vw[2] = {(float)(32 - wo), (float)wo};
-        const int rows[2] = {1, other};
         float acc = 0.0f;
 #pragma unroll
         for (int a = 0; a < 2; a++)
 #pragma unroll
             for (int b = 0; b < 3; b++) {
-                const short2 q = s_near[rows[a]][b];
-                const float sum = fg_at(a0, pa, w, h, x + q.x, y + q.y) + fg_at(b0, pb, w, h, x - q.x, y - q.y);
+                const int e = a == 0 ? q[1][b] : j < 4 ? q[0][b] : q[2][b]; /* s < 8: the row above */
+                const int ex = (short)(e & 0xffff), ey = e >> 16;
+                const float sum = at(a0, pa, x + ex, y + ey) + at(b0, pb, x - ex, y - ey);
                 acc = __fmaf_rn(sum, wh[b] * vw[a], acc);
             }
-        v = rintf(acc * (1.0f / 2048.0f));
-    }
-    out[(size_t)y * po + x] = v;
-    if (pic) {
-        const float q = rintf(v * (1.0f / 64.0f));
-        pic[(size_t)y * w + x] = q <= 0.0f ? 0 : q >= 255.0f ? 255 : (unsigned char)q;
+        if (x < w && y < h)
+            store(y, rintf(acc * (1.0f / 2048.0f)));
     }
 }
 
@@ -584,39 +776,57 @@ extern "C" int vtg_framegen_run(vtg_framegen *g, const float *older, int older_p
         return VTG_EINVAL;
     const cudaStream_t st = stream ? (cudaStream_t)stream : g->stream;
     CU(cudaSetDevice(vtg_ctx_device(g->ctx)));
-    /* the field's pyramid: level 0 from the frames, each next from the last */
-    const float *sa = older, *sb = newer;
-    int sw = g->w, sh = g->h, spa = older_pitch, spb = newer_pitch;
-    for (int L = 0; L < g->levels; L++) {
-        const FgLevel &v = g->L[L];
-        fg_reduce_kernel<<<dim3((v.w + 31) / 32, (v.h + 7) / 8, 2), dim3(32, 8), 0, st>>>(
-            sa, sb, sw, sh, spa, spb, g->pa[L], g->pb[L], v.w, v.h, v.pitch);
-        sa = g->pa[L];
-        sb = g->pb[L];
-        sw = v.w;
-        sh = v.h;
-        spa = spb = v.pitch;
-    }
-    fg_hist_kernel<<<dim3(18, FG_HIST_SPLIT), 256, 0, st>>>(g->L[1], g->hist, g->scene);
-    for (int L = g->levels - 1; L >= 0; L--) {
-        const FgLevel &v = g->L[L];
-        const int nb = v.bw * v.bh;
-        fg_search_kernel<<<(nb + FG_WARPS - 1) / FG_WARPS, 32 * FG_WARPS, 0, st>>>(
-            v, L == g->levels - 1 ? nullptr : v.up, L, g->scene);
-        fg_filter_kernel<<<(nb + 255) / 256, 256, 0, st>>>(v);
-        if (L > 0) {
-            const FgLevel &f = g->L[L - 1];
-            fg_upscale_kernel<<<(f.bw * f.bh + 255) / 256, 256, 0, st>>>(v, f.up, f.bw, f.bh, g->scene);
+    /* the field's pyramid: level 0 from the frames, each next from the last, three levels a launch; the scene test with the
+     * launch after level 1's */
+    FgReduce q = {};
+    q.s[0] = older;
+    q.s[1] = newer;
+    q.sw = g->w;
+    q.sh = g->h;
+    q.sp[0] = older_pitch;
+    q.sp[1] = newer_pitch;
+    bool hist = false;
+    for (int L = 0; L < g->levels || !hist; L += 3) {
+        q.n = min(3, g->levels - L);
+        int reduces = 0;
+        if (q.n > 0) {
+            for (int k = 0; k < q.n; k++) {
+                q.d[k][0] = g->pa[L + k];
+                q.d[k][1] = g->pb[L + k];
+                q.w[k] = g->L[L + k].w;
+                q.h[k] = g->L[L + k].h;
+                q.p[k] = g->L[L + k].pitch;
+            }
+            q.bx = (q.w[0] + FR_X - 1) / FR_X;
+            q.by = (q.h[0] + FR_Y - 1) / FR_Y;
+            reduces = 2 * q.bx * q.by;
+        }
+        const bool test = L > 0 && !hist;
+        CU(vtg_launch_k(fg_reduce3_kernel, dim3(reduces + (test ? FG_HIST_CTAS : 0)), dim3(256), 0, st, L > 0, q, reduces, g->L[1],
+                        g->hist, g->scene));
+        hist = hist || test;
+        if (q.n == 3) {
+            q.s[0] = g->pa[L + 2];
+            q.s[1] = g->pb[L + 2];
+            q.sw = q.w[2];
+            q.sh = q.h[2];
+            q.sp[0] = q.sp[1] = q.p[2];
         }
     }
+    for (int L = g->levels - 1; L >= 0; L--) {
+        const FgLevel &v = g->L[L];
+        const bool top = L == g->levels - 1;
+        CU(vtg_launch_k(fg_search_kernel, dim3((v.bw * v.bh + FG_WARPS - 1) / FG_WARPS), dim3(32 * FG_WARPS), 0, st, true, v,
+                        g->L[top ? L : L + 1], top, L, (const int *)g->scene));
+    }
     const FgLevel &z = g->L[0];
-    fg_mid_kernel<<<(z.bw * z.bh + FG_WARPS - 1) / FG_WARPS, 32 * FG_WARPS, 0, st>>>(z, g->mid);
+    CU(vtg_launch_k(fg_mid_kernel, dim3((z.bw * z.bh + FG_WARPS - 1) / FG_WARPS), dim3(32 * FG_WARPS), 0, st, true, z, g->mid));
     float *dst = out ? out : g->out;
     const int dp = out ? out_pitch : g->out_pitch;
     unsigned char *pd = pic ? (where == VTG_DEVICE ? (unsigned char *)pic : g->pic) : nullptr;
-    fg_blend_kernel<<<dim3((g->w + 15) / 16, (g->h + 15) / 16), 256, 0, st>>>(older, older_pitch, newer, newer_pitch,
-                                                                            g->w, g->h, g->mid, z.bw, z.bh, dst, dp,
-                                                                            pd);
+    CU(vtg_launch_k(fg_blend_kernel, dim3((g->w + 16 * FG_BLEND_WARPS - 1) / (16 * FG_BLEND_WARPS), (g->h + 15) / 16),
+                    dim3(32 * FG_BLEND_WARPS), 0, st, true, older, older_pitch, newer, newer_pitch, g->w, g->h,
+                    (const short2 *)g->mid, z.bw, z.bh, dst, dp, pd));
     CU(cudaGetLastError());
     if (pic && where == VTG_HOST) {
         CU(cudaMemcpyAsync(pic, g->pic, (size_t)g->w * (size_t)g->h, cudaMemcpyDeviceToHost, st));
