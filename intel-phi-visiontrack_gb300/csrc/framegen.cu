@@ -104,19 +104,20 @@ struct FgReduceSmem {
 
 __device__ __forceinline__ int fg_tap5(int a, int b, int c, int d, int e) { return a + e + 4 * (b + d) + 6 * c; }
 
-__device__ void fg_reduce_block(const FgReduce &q, int block, FgReduceSmem &S)
+/* EDGE: some index of the block's needs its clamp. */
+template <bool EDGE>
+__device__ __forceinline__ void fg_reduce_block(const FgReduce &q, int f, int X0, int Y0, FgReduceSmem &S)
 {
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int f = block / (q.bx * q.by), at = block - f * q.bx * q.by;
-    const int X0 = (at % q.bx) * FR_X, Y0 = (at / q.bx) * FR_Y;
     const float *src = q.s[f];
+    auto clamp = [](int v, int n) { return EDGE ? min(max(v, 0), n - 1) : v; };
     for (int i = tid; i < 4 * FR_S_C; i += nt) {
         const int g = i / FR_S_C, c = i - g * FR_S_C, r0 = g * FR_SEG;
-        const float *col = src + min(max(2 * X0 - 14 + c, 0), q.sw - 1);
+        const float *col = src + clamp(2 * X0 - 14 + c, q.sw);
         int v[2 * FR_SEG + 3];
 #pragma unroll
         for (int k = 0; k < 2 * FR_SEG + 3; k++)
-            v[k] = (int)__ldca(col + (size_t)min(max(2 * (Y0 - 6 + r0) - 2 + k, 0), q.sh - 1) * q.sp[f]);
+            v[k] = (int)__ldca(col + (size_t)clamp(2 * (Y0 - 6 + r0) - 2 + k, q.sh) * q.sp[f]);
 #pragma unroll
         for (int r = 0; r < FR_SEG; r++)
             if (r0 + r < FR_A_R)
@@ -129,7 +130,7 @@ __device__ void fg_reduce_block(const FgReduce &q, int block, FgReduceSmem &S)
         const int o = (fg_tap5(v[0], v[1], v[2], v[3], v[4]) + 128) >> 8;
         S.a[y][x] = o;
         const int gy = Y0 - 6 + y, gx = X0 - 6 + x;
-        if (y >= 6 && y < 6 + FR_Y && x >= 6 && x < 6 + FR_X && gy < q.h[0] && gx < q.w[0])
+        if (y >= 6 && y < 6 + FR_Y && x >= 6 && x < 6 + FR_X && (!EDGE || (gy < q.h[0] && gx < q.w[0])))
             q.d[0][f][(size_t)gy * q.p[0] + gx] = (float)o;
     }
     if (q.n < 2)
@@ -140,7 +141,7 @@ __device__ void fg_reduce_block(const FgReduce &q, int block, FgReduceSmem &S)
         int v[5];
 #pragma unroll
         for (int t = 0; t < 5; t++)
-            v[t] = S.a[min(max(2 * (Y0 / 2 - 2 + y) - 2 + t, 0), q.h[0] - 1) - (Y0 - 6)][x];
+            v[t] = S.a[clamp(2 * (Y0 / 2 - 2 + y) - 2 + t, q.h[0]) - (Y0 - 6)][x];
         S.v2[y][x] = fg_tap5(v[0], v[1], v[2], v[3], v[4]);
     }
     __syncthreads();
@@ -149,11 +150,11 @@ __device__ void fg_reduce_block(const FgReduce &q, int block, FgReduceSmem &S)
         int v[5];
 #pragma unroll
         for (int t = 0; t < 5; t++)
-            v[t] = S.v2[y][min(max(2 * (X0 / 2 - 2 + x) - 2 + t, 0), q.w[0] - 1) - (X0 - 6)];
+            v[t] = S.v2[y][clamp(2 * (X0 / 2 - 2 + x) - 2 + t, q.w[0]) - (X0 - 6)];
         const int o = (fg_tap5(v[0], v[1], v[2], v[3], v[4]) + 128) >> 8;
         S.b[y][x] = o;
         const int gy = Y0 / 2 - 2 + y, gx = X0 / 2 - 2 + x;
-        if (y >= 2 && y < 2 + FR_Y / 2 && x >= 2 && x < 2 + FR_X / 2 && gy < q.h[1] && gx < q.w[1])
+        if (y >= 2 && y < 2 + FR_Y / 2 && x >= 2 && x < 2 + FR_X / 2 && (!EDGE || (gy < q.h[1] && gx < q.w[1])))
             q.d[1][f][(size_t)gy * q.p[1] + gx] = (float)o;
     }
     if (q.n < 3)
@@ -164,21 +165,32 @@ __device__ void fg_reduce_block(const FgReduce &q, int block, FgReduceSmem &S)
         int v[5];
 #pragma unroll
         for (int t = 0; t < 5; t++)
-            v[t] = S.b[min(max(2 * (Y0 / 4 + y) - 2 + t, 0), q.h[1] - 1) - (Y0 / 2 - 2)][x];
+            v[t] = S.b[clamp(2 * (Y0 / 4 + y) - 2 + t, q.h[1]) - (Y0 / 2 - 2)][x];
         S.v3[y][x] = fg_tap5(v[0], v[1], v[2], v[3], v[4]);
     }
     __syncthreads();
     for (int i = tid; i < FR_C_R * FR_C_C; i += nt) {
         const int y = i / FR_C_C, x = i - y * FR_C_C;
         const int gy = Y0 / 4 + y, gx = X0 / 4 + x;
-        if (gy >= q.h[2] || gx >= q.w[2])
+        if (EDGE && (gy >= q.h[2] || gx >= q.w[2]))
             continue;
         int v[5];
 #pragma unroll
         for (int t = 0; t < 5; t++)
-            v[t] = S.v3[y][min(max(2 * gx - 2 + t, 0), q.w[1] - 1) - (X0 / 2 - 2)];
+            v[t] = S.v3[y][clamp(2 * gx - 2 + t, q.w[1]) - (X0 / 2 - 2)];
         q.d[2][f][(size_t)gy * q.p[2] + gx] = (float)((fg_tap5(v[0], v[1], v[2], v[3], v[4]) + 128) >> 8);
     }
+}
+
+__device__ void fg_reduce_any(const FgReduce &q, int block, FgReduceSmem &S)
+{
+    const int f = block / (q.bx * q.by), at = block - f * q.bx * q.by;
+    const int X0 = (at % q.bx) * FR_X, Y0 = (at / q.bx) * FR_Y;
+    /* every source row and column that the block reads lies inside the source: rows 2 Y0 - 14 .. + 4 FR_SEG x 2 + 2 */
+    if (X0 > 0 && Y0 > 0 && 2 * X0 - 14 + FR_S_C <= q.sw && 2 * Y0 - 14 + 8 * FR_SEG + 3 <= q.sh)
+        fg_reduce_block<false>(q, f, X0, Y0, S);
+    else
+        fg_reduce_block<true>(q, f, X0, Y0, S);
 }
 
 /* fg_hist_section (framegen.c:85-101): part `part` of FG_HIST_SPLIT of the sampled rows of section s of frame f, counted
@@ -265,7 +277,7 @@ __global__ void __launch_bounds__(256) fg_reduce3_kernel(FgReduce q, int reduces
     vtg_grid_launch_dependents();
     vtg_grid_dependency_wait();
     if ((int)blockIdx.x < reduces)
-        fg_reduce_block(q, blockIdx.x, S.r);
+        fg_reduce_any(q, blockIdx.x, S.r);
     else
         fg_hist_part(l1, (int)blockIdx.x - reduces, hist, scene, S.h);
 }
@@ -407,28 +419,22 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, Fg
     const int lanes = (lv.w + 15) & ~15;
     const int x0 = min(max(px + wx - 8, -32), lanes), y0 = py + wy - 8;
     {
-        /* every load of the window and the block in flight before the first store */
-        float wv[18], bv[2];
+        /* every load of the window (a lane a column) and of the block in flight before the first store */
+        float wv[24], bv[2];
+        const float *col = lv.a + min(max(x0 + min(lane, 23), 0), lv.w - 1);
 #pragma unroll
-        for (int j = 0; j < 18; j++) {
-            const int k = lane + 32 * j;
-            wv[j] = fg_at(lv.a, lv.pitch, lv.w, lv.h, x0 + k % 24, y0 + k / 24);
-        }
+        for (int r = 0; r < 24; r++)
+            wv[r] = __ldca(col + (size_t)(min(max(y0 + r, 0), lv.h - 1) * lv.pitch));
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int k = lane + 32 * j;
-            bv[j] = fg_at(lv.b, lv.pitch, lv.w, lv.h, px + (k & 7), py + (k >> 3));
-        }
+        for (int j = 0; j < 2; j++)
+            bv[j] = fg_at(lv.b, lv.pitch, lv.w, lv.h, px + (lane & 7), py + (lane >> 3) + 4 * j);
+        if (lane < 24)
 #pragma unroll
-        for (int j = 0; j < 18; j++) {
-            const int k = lane + 32 * j;
-            s_win[warp][k / 24][k % 24] = wv[j];
-        }
+            for (int r = 0; r < 24; r++)
+                s_win[warp][r][lane] = wv[r];
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int k = lane + 32 * j;
-            s_blk[warp][k >> 3][k & 7] = bv[j];
-        }
+        for (int j = 0; j < 2; j++)
+            s_blk[warp][(lane >> 3) + 4 * j][lane & 7] = bv[j];
     }
     __syncwarp();
     if (level == 0) {
@@ -587,27 +593,47 @@ __global__ void __launch_bounds__(32 * FG_BLEND_WARPS) fg_blend_kernel(const flo
     const float wl = k < 8 ? (float)(15 - 2 * k) : 0.0f, wr = k < 8 ? 0.0f : (float)(2 * k - 15);
     const float ws = k < 8 ? (float)(17 + 2 * k) : (float)(47 - 2 * k);
     const float wh[3] = {wl, ws, wr};
-    int q[3][3];
+    /* a tile whose every read lies inside the frame takes them without clamps: six places of each frame, a column's rows
+     * two rows apart */
+    const int reach_x = (int)__reduce_max_sync(VTG_FULL, (unsigned)abs((int)(short)(near & 0xffff)));
+    const int reach_y = (int)__reduce_max_sync(VTG_FULL, (unsigned)abs(near >> 16));
+    const bool inside = tx * 16 >= reach_x && tx * 16 + 16 + reach_x <= w && ty * 16 >= reach_y && ty * 16 + 16 + reach_y <= h;
 #pragma unroll
-    for (int n = 0; n < 9; n++)
-        q[n / 3][n % 3] = __shfl_sync(VTG_FULL, near, n);
+    for (int half = 0; half < 2; half++) { /* the tile's upper rows blend with the row of blocks above, the lower below */
+        int q[2][3];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int s = 2 * j + (lane >> 4), y = ty * 16 + s;
-        const int wo = s < 8 ? 15 - 2 * s : 2 * s - 15;
-        const float vw[2] = {(float)(32 - wo), (float)wo};
-        float acc = 0.0f;
+        for (int b = 0; b < 3; b++) {
+            q[0][b] = __shfl_sync(VTG_FULL, near, 3 + b);
+            q[1][b] = __shfl_sync(VTG_FULL, near, 6 * half + b);
+        }
+        const int s0 = 8 * half + (lane >> 4), y0 = ty * 16 + s0;
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int a = 0; a < 2; a++)
 #pragma unroll
             for (int b = 0; b < 3; b++) {
-                const int e = a == 0 ? q[1][b] : j < 4 ? q[0][b] : q[2][b]; /* s < 8: the row above */
-                const int ex = (short)(e & 0xffff), ey = e >> 16;
-                const float sum = at(a0, pa, x + ex, y + ey) + at(b0, pb, x - ex, y - ey);
-                acc = __fmaf_rn(sum, wh[b] * vw[a], acc);
+                const int ex = (short)(q[a][b] & 0xffff), ey = q[a][b] >> 16;
+                float sum[4];
+                if (inside) {
+                    const float *fa = a0 + (ptrdiff_t)(y0 + ey) * pa + (x + ex), *fb = b0 + (ptrdiff_t)(y0 - ey) * pb + (x - ex);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        sum[j] = __ldg(fa + 2 * j * pa) + __ldg(fb + 2 * j * pb);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        sum[j] = at(a0, pa, x + ex, y0 + 2 * j + ey) + at(b0, pb, x - ex, y0 + 2 * j - ey);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int s = s0 + 2 * j, wo = s < 8 ? 15 - 2 * s : 2 * s - 15;
+                    acc[j] = __fmaf_rn(sum[j], wh[b] * (float)(a == 0 ? 32 - wo : wo), acc[j]);
+                }
             }
-        if (x < w && y < h)
-            store(y, rintf(acc * (1.0f / 2048.0f)));
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (x < w && y0 + 2 * j < h)
+                store(y0 + 2 * j, rintf(acc[j] * (1.0f / 2048.0f)));
     }
 }
 
