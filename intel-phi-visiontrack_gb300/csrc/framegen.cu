@@ -72,13 +72,14 @@ __device__ __forceinline__ float fg_warp_sum(float v)
  * borders) in one launch. A CTA owns a 64 x 32 block of the first level made and the 32 x 16 and 16 x 8 blocks under it. The
  * first level's vertical sums come straight from the source, a thread a column and eleven rows of them (25 loads in
  * flight), for the 73 x 41 values that the levels above need; the rest runs in shared memory. A level reads the one below at
- * the reference's clamped indices, which always fall inside the computed halo. At 1080p, both frames, levels 0 to 2: FGR3 us
- * where a launch a level took 12 + 6 + 4 (25 loads a value). */
+ * the reference's clamped indices, which always fall inside the computed halo. At 1080p, both frames, levels 0 to 2: 14 us
+ * where a launch a level took 12 + 6 + 4 (25 loads a value); issue at half, between barriers, bounds it. */
 #define FR_X 64
 #define FR_Y 32
 #define FR_A_C 73 /* the first level computed: columns X0 - 6 .. X0 + 66, rows Y0 - 6 .. Y0 + 34 */
 #define FR_A_R 41
 #define FR_S_C (2 * FR_A_C + 3) /* its source columns, from 2 X0 - 14 */
+#define FR_S_P 152              /* 16-byte rows, and the last pair's eight values */
 #define FR_B_C 35
 #define FR_B_R 19
 #define FR_C_C 16
@@ -95,8 +96,8 @@ struct FgReduce {
 };
 
 struct FgReduceSmem {
-    int v[FR_A_R][FR_S_C]; /* the first level's vertical sums */
-    int a[FR_A_R][FR_A_C];
+    __align__(16) int v[FR_A_R][FR_S_P]; /* the first level's vertical sums */
+    int a[FR_A_R][FR_A_C + 1];
     int v2[FR_B_R][FR_A_C];
     int b[FR_B_R][FR_B_C];
     int v3[FR_C_R][FR_B_C];
@@ -124,14 +125,21 @@ __device__ __forceinline__ void fg_reduce_block(const FgReduce &q, int f, int X0
                 S.v[r0 + r][c] = fg_tap5(v[2 * r], v[2 * r + 1], v[2 * r + 2], v[2 * r + 3], v[2 * r + 4]);
     }
     __syncthreads();
-    for (int i = tid; i < FR_A_R * FR_A_C; i += nt) {
-        const int y = i / FR_A_C, x = i - y * FR_A_C;
-        const int *v = &S.v[y][2 * x];
-        const int o = (fg_tap5(v[0], v[1], v[2], v[3], v[4]) + 128) >> 8;
-        S.a[y][x] = o;
-        const int gy = Y0 - 6 + y, gx = X0 - 6 + x;
-        if (y >= 6 && y < 6 + FR_Y && x >= 6 && x < 6 + FR_X && (!EDGE || (gy < q.h[0] && gx < q.w[0])))
-            q.d[0][f][(size_t)gy * q.p[0] + gx] = (float)o;
+    /* two columns a thread, from eight vertical sums (column 73, past the last, is computed and not used) */
+    for (int i = tid; i < FR_A_R * ((FR_A_C + 1) / 2); i += nt) {
+        const int y = i / ((FR_A_C + 1) / 2), x = 2 * (i - y * ((FR_A_C + 1) / 2));
+        const int4 u = *reinterpret_cast<const int4 *>(&S.v[y][2 * x]), t = *reinterpret_cast<const int4 *>(&S.v[y][2 * x + 4]);
+        const int o0 = (fg_tap5(u.x, u.y, u.z, u.w, t.x) + 128) >> 8, o1 = (fg_tap5(u.z, u.w, t.x, t.y, t.z) + 128) >> 8;
+        S.a[y][x] = o0;
+        S.a[y][x + 1] = o1;
+        const int gy = Y0 - 6 + y, gx = X0 - 6 + x; /* x and the block's edges are even */
+        if (y >= 6 && y < 6 + FR_Y && x >= 6 && x < 6 + FR_X && (!EDGE || (gy < q.h[0] && gx < q.w[0]))) {
+            float *d = q.d[0][f] + (size_t)gy * q.p[0] + gx;
+            if (!EDGE || gx + 1 < q.w[0])
+                *reinterpret_cast<float2 *>(d) = make_float2((float)o0, (float)o1);
+            else
+                *d = (float)o0;
+        }
     }
     if (q.n < 2)
         return;
@@ -282,69 +290,86 @@ __global__ void __launch_bounds__(256) fg_reduce3_kernel(FgReduce q, int reduces
         fg_hist_part(l1, (int)blockIdx.x - reduces, hist, scene, S.h);
 }
 
-/* fg_filter (framegen.c:218-247) of the block at (bx, by): of the 3 x 3 around it (clamped, column by column), the vector
- * with the least sum of squared differences from the nine; the first on a tie. `ways` lanes of a warp share a block, this
- * one the `way`-th: candidates way, way + ways, ..; ways a power of two share by xor partners, 3 by the two lanes on. */
-template <int WAYS>
-__device__ __forceinline__ short2 fg_filtered(const FgLevel &lv, int bx, int by, int way)
+/* fg_filter (framegen.c:218-247) of the block at (bx, by): of the 3 x 3 around it (clamped; candidate 3 column + row), the
+ * vector with the least sum of squared differences from the nine; the first on a tie. A lane reads all nine, and again, by
+ * its own index, those it sums for. */
+struct FgNine {
+    int v[9]; /* packed short2 */
+};
+
+__device__ __forceinline__ int fg_raw_at(const FgLevel &lv, int bx, int by, int a)
 {
-    int mx[9], my[9];
+    const int xx = a / 3, yy = a - 3 * xx;
+    return __ldca(reinterpret_cast<const int *>(lv.raw) + min(max(by + yy - 1, 0), lv.bh - 1) * lv.bw +
+                  min(max(bx + xx - 1, 0), lv.bw - 1));
+}
+__device__ __forceinline__ FgNine fg_nine(const FgLevel &lv, int bx, int by)
+{
+    FgNine n;
+    const int *raw = reinterpret_cast<const int *>(lv.raw);
+    int row[3], col[3];
 #pragma unroll
-    for (int xx = 0; xx < 3; xx++)
-#pragma unroll
-        for (int yy = 0; yy < 3; yy++) {
-            const int at = min(max(by + yy - 1, 0), lv.bh - 1) * lv.bw + min(max(bx + xx - 1, 0), lv.bw - 1);
-            const int v = __ldca(reinterpret_cast<const int *>(lv.raw) + at);
-            mx[xx * 3 + yy] = (short)(v & 0xffff);
-            my[xx * 3 + yy] = v >> 16;
-        }
-    unsigned least = ~0u;
-    int pick = 9, vx = 0, vy = 0;
-#pragma unroll
-    for (int k = 0; k < (9 + WAYS - 1) / WAYS; k++) {
-        const int a = way + k * WAYS;
-        int ax = mx[0], ay = my[0];
-#pragma unroll
-        for (int b = 1; b < 9; b++) {
-            ax = a == b ? mx[b] : ax;
-            ay = a == b ? my[b] : ay;
-        }
-        unsigned d = 0;
-#pragma unroll
-        for (int b = 0; b < 9; b++) {
-            const int dx = ax - mx[b], dy = ay - my[b];
-            d += (unsigned)(dx * dx + dy * dy);
-        }
-        if (a < 9 && (pick == 9 || d < least)) {
-            least = d;
-            pick = a;
-            vx = ax;
-            vy = ay;
-        }
+    for (int k = 0; k < 3; k++) {
+        row[k] = min(max(by + k - 1, 0), lv.bh - 1) * lv.bw;
+        col[k] = min(max(bx + k - 1, 0), lv.bw - 1);
     }
-    auto meet = [&](unsigned ol, int op, int ox, int oy) {
-        if (ol < least || (ol == least && op < pick)) {
-            least = ol;
-            pick = op;
-            vx = ox;
-            vy = oy;
-        }
-    };
-    if constexpr (WAYS == 3) { /* lanes 3 k, 3 k + 1, 3 k + 2 of a block: the first one ends with its vector */
-        const int lane = threadIdx.x & 31;
-        const unsigned l1 = __shfl_sync(VTG_FULL, least, lane + 1), l2 = __shfl_sync(VTG_FULL, least, lane + 2);
-        const int p1 = __shfl_sync(VTG_FULL, pick, lane + 1), p2 = __shfl_sync(VTG_FULL, pick, lane + 2);
-        const int x1 = __shfl_sync(VTG_FULL, vx, lane + 1), x2 = __shfl_sync(VTG_FULL, vx, lane + 2);
-        const int y1 = __shfl_sync(VTG_FULL, vy, lane + 1), y2 = __shfl_sync(VTG_FULL, vy, lane + 2);
-        meet(l1, p1, x1, y1);
-        meet(l2, p2, x2, y2);
-    } else {
 #pragma unroll
-        for (int d = 1; d < WAYS; d <<= 1)
-            meet(__shfl_xor_sync(VTG_FULL, least, d), __shfl_xor_sync(VTG_FULL, pick, d), __shfl_xor_sync(VTG_FULL, vx, d),
-                 __shfl_xor_sync(VTG_FULL, vy, d));
+    for (int a = 0; a < 9; a++)
+        n.v[a] = __ldca(raw + row[a % 3] + col[a / 3]);
+    return n;
+}
+__device__ __forceinline__ unsigned fg_apart(int a, int b)
+{
+    const int dx = (short)(a & 0xffff) - (short)(b & 0xffff), dy = (a >> 16) - (b >> 16);
+    return (unsigned)(dx * dx + dy * dy);
+}
+__device__ __forceinline__ unsigned fg_sum_apart(const FgNine &n, int me)
+{
+    unsigned d = 0u;
+#pragma unroll
+    for (int b = 0; b < 9; b++)
+        d += fg_apart(me, n.v[b]);
+    return d;
+}
+/* the lesser of two (sum, candidate) with their vectors */
+__device__ __forceinline__ void fg_lesser(unsigned &d, int &a, int &v, unsigned od, int oa, int ov)
+{
+    const bool o = od < d || (od == d && oa < a);
+    d = o ? od : d;
+    a = o ? oa : a;
+    v = o ? ov : v;
+}
+/* Eight lanes a block, lane j candidate j. Candidate 8's sum is that of the eight lanes' distances from it. */
+__device__ __forceinline__ int fg_filtered8(const FgLevel &lv, int bx, int by, int j)
+{
+    const FgNine n = fg_nine(lv, bx, by);
+    int v = fg_raw_at(lv, bx, by, j), a = j;
+    unsigned d = fg_sum_apart(n, v), d8 = fg_apart(v, n.v[8]);
+#pragma unroll
+    for (int k = 1; k < 8; k <<= 1) {
+        d8 += __shfl_xor_sync(VTG_FULL, d8, k);
+        fg_lesser(d, a, v, __shfl_xor_sync(VTG_FULL, d, k), __shfl_xor_sync(VTG_FULL, a, k), __shfl_xor_sync(VTG_FULL, v, k));
     }
-    return make_short2((short)vx, (short)vy);
+    return d8 < d ? n.v[8] : v;
+}
+/* Three lanes a block (lanes 3 k, 3 k + 1, 3 k + 2), lane j candidates 3 j .. 3 j + 2; the first lane ends with the vector. */
+__device__ __forceinline__ int fg_filtered3(const FgLevel &lv, int bx, int by, int j)
+{
+    const FgNine n = fg_nine(lv, bx, by);
+    int v = fg_raw_at(lv, bx, by, 3 * j), a = 3 * j;
+    unsigned d = fg_sum_apart(n, v);
+#pragma unroll
+    for (int k = 1; k < 3; k++) {
+        const int u = fg_raw_at(lv, bx, by, 3 * j + k);
+        fg_lesser(d, a, v, fg_sum_apart(n, u), 3 * j + k, u);
+    }
+    const int lane = threadIdx.x & 31;
+    const unsigned d1 = __shfl_sync(VTG_FULL, d, lane + 1), d2 = __shfl_sync(VTG_FULL, d, lane + 2);
+    const int a1 = __shfl_sync(VTG_FULL, a, lane + 1), a2 = __shfl_sync(VTG_FULL, a, lane + 2);
+    const int v1 = __shfl_sync(VTG_FULL, v, lane + 1), v2 = __shfl_sync(VTG_FULL, v, lane + 2);
+    fg_lesser(d, a, v, d1, a1, v1);
+    fg_lesser(d, a, v, d2, a2, v2);
+    return v;
 }
 
 /* fg_upscale (framegen.c:251-288) for block (gx, gy) of the level under `lv`, a warp: of the four nearest blocks' filtered
@@ -357,7 +382,8 @@ __device__ __forceinline__ short2 fg_upscaled(const FgLevel &lv, int gx, int gy,
     const int cx = gx / 2 + n % 2 - 1 + gx % 2, cy = gy / 2 + n / 2 - 1 + gy % 2;
     const int px = gx * 4 + (lane & 3), py = gy * 4 + ((lane >> 2) & 1);
     const float c0 = fg_at(lv.b, lv.pitch, lv.w, lv.h, px, py), c1 = fg_at(lv.b, lv.pitch, lv.w, lv.h, px, py + 2);
-    const short2 v = fg_filtered<8>(lv, min(max(cx, 0), lv.bw - 1), min(max(cy, 0), lv.bh - 1), lane & 7);
+    const int f = fg_filtered8(lv, min(max(cx, 0), lv.bw - 1), min(max(cy, 0), lv.bh - 1), lane & 7);
+    const short2 v = make_short2((short)(f & 0xffff), (short)(f >> 16));
     if (lane == 24 && !(gx & 1) && !(gy & 1))
         lv.fil[(gy / 2) * lv.bw + gx / 2] = v;
     float s = fabsf(c0 - fg_at(lv.a, lv.pitch, lv.w, lv.h, px + v.x, py + v.y)) +
@@ -365,25 +391,25 @@ __device__ __forceinline__ short2 fg_upscaled(const FgLevel &lv, int gx, int gy,
 #pragma unroll
     for (int d = 1; d < 8; d <<= 1)
         s += __shfl_xor_sync(VTG_FULL, s, d);
-    int pick = n, vx = v.x, vy = v.y;
+    int pick = n, at = f;
 #pragma unroll
     for (int d = 8; d < 32; d <<= 1) {
         const float os = __shfl_xor_sync(VTG_FULL, s, d);
-        const int op = __shfl_xor_sync(VTG_FULL, pick, d), ox = __shfl_xor_sync(VTG_FULL, vx, d), oy = __shfl_xor_sync(VTG_FULL, vy, d);
-        if (os < s || (os == s && op < pick)) {
-            s = os;
-            pick = op;
-            vx = ox;
-            vy = oy;
-        }
+        const int op = __shfl_xor_sync(VTG_FULL, pick, d), oa = __shfl_xor_sync(VTG_FULL, at, d);
+        const bool o = os < s || (os == s && op < pick);
+        s = o ? os : s;
+        pick = o ? op : pick;
+        at = o ? oa : at;
     }
-    return make_short2((short)(2 * vx), (short)(2 * vy));
+    return make_short2((short)(2 * (short)(at & 0xffff)), (short)(2 * (at >> 16)));
 }
 
 /* fg_search (framegen.c:117-214) at one level: a warp an 8 x 8 block, from the coarser level's estimate (lv.up; none at the
  * top). The 256 offsets x0 - px + dx, wy + dy - 8 (dx, dy < 16) cost |dx - 8| + |dy - 8| plus the block's SAD; the
  * first lowest in row order wins. On the finest level a block the estimate explains (SAD <= 8192) is not searched, and
  * no motion wins when its SAD is no more than the best cost. */
+#define FG_BIAS 12582912.0f /* 1.5 x 2^23: whole numbers below 2^22 of either sign keep one exponent with it */
+#define FG_INT 5 /* of a row's eight differences, those taken as integers */
 __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, FgLevel coarse, bool top, int level,
                                                                   const int *__restrict__ scene)
 {
@@ -431,10 +457,10 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, Fg
         if (lane < 24)
 #pragma unroll
             for (int r = 0; r < 24; r++)
-                s_win[warp][r][lane] = wv[r];
+                s_win[warp][r][lane] = wv[r] + FG_BIAS;
 #pragma unroll
         for (int j = 0; j < 2; j++)
-            s_blk[warp][(lane >> 3) + 4 * j][lane & 7] = bv[j];
+            s_blk[warp][(lane >> 3) + 4 * j][lane & 7] = bv[j] + FG_BIAS;
     }
     __syncwarp();
     if (level == 0) {
@@ -449,11 +475,18 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, Fg
             return;
         }
     }
+    /* The staged values carry FG_BIAS, so their bits as integers differ by the values' difference: five of a row's eight
+     * absolute differences take one integer instruction each (sum of absolute differences, on the ALU pipe), three take two
+     * F32 ones (on the FMA pipe), which keeps both pipes and the issue busy. A generated 1080p frame with 0, 3, 4, 5, 6, 8 of
+     * them as integers: 46.0, 43.5, 42.5, 42.2, 42.5, 43.5 us. */
     const int dy = lane & 15, dx0 = (lane >> 4) * 8;
     float c[8];
+    unsigned ci[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++)
-        c[k] = (float)abs(dx0 + k - 8) + (float)abs(dy - 8); /* FG_TIE_UNIT */
+    for (int k = 0; k < 8; k++) {
+        c[k] = 0.0f;
+        ci[k] = (unsigned)(abs(dx0 + k - 8) + abs(dy - 8)); /* FG_TIE_UNIT */
+    }
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         float wv[16], bv[8];
@@ -467,8 +500,14 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, Fg
         for (int k = 0; k < 8; k++)
 #pragma unroll
             for (int n = 0; n < 8; n++)
-                c[k] += fabsf(wv[k + n] - bv[n]);
+                if (n < FG_INT)
+                    ci[k] = __usad(__float_as_uint(wv[k + n]), __float_as_uint(bv[n]), ci[k]);
+                else
+                    c[k] += fabsf(wv[k + n] - bv[n]);
     }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        c[k] += (float)ci[k];
     float best = c[0];
     int bi = dy * 16 + dx0;
 #pragma unroll
@@ -490,7 +529,8 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_search_kernel(FgLevel lv, Fg
     if (level == 0) {
         float s = 0.0f;
         for (int k = lane; k < 64; k += 32)
-            s += fabsf(s_blk[warp][k >> 3][k & 7] - fg_at(lv.a, lv.pitch, lv.w, lv.h, px + (k & 7), py + (k >> 3)));
+            s += fabsf(s_blk[warp][k >> 3][k & 7] -
+                       (fg_at(lv.a, lv.pitch, lv.w, lv.h, px + (k & 7), py + (k >> 3)) + FG_BIAS));
         s = fg_warp_sum(s);
         if (s <= best)
             vx = vy = 0;
@@ -512,9 +552,9 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_mid_kernel(FgLevel lv, short
         return;
     const int bx = i % lv.bw, by = i / lv.bw, px = bx * 8, py = by * 8;
     const int nb = min(lane / 3, 8); /* the 3 x 3's block of this lane, row by row */
-    const short2 fv = fg_filtered<3>(lv, min(max(bx + nb % 3 - 1, 0), lv.bw - 1), min(max(by + nb / 3 - 1, 0), lv.bh - 1), lane % 3);
+    const int fv = fg_filtered3(lv, min(max(bx + nb % 3 - 1, 0), lv.bw - 1), min(max(by + nb / 3 - 1, 0), lv.bh - 1), lane % 3);
     if (lane == 12)
-        lv.fil[i] = fv;
+        lv.fil[i] = make_short2((short)(fv & 0xffff), (short)(fv >> 16));
     auto sad = [&](int vx, int vy) {
         const int ax = vx >> 1, ay = vy >> 1, qx = vx - ax, qy = vy - ay;
         float s = 0.0f;
@@ -528,7 +568,7 @@ __global__ void __launch_bounds__(32 * FG_WARPS) fg_mid_kernel(FgLevel lv, short
     float best = sad(0, 0) - 64.0f;
     int vx = 0, vy = 0;
     for (int k = 0; k < 9; k++) {
-        const int qx = __shfl_sync(VTG_FULL, (int)fv.x, 3 * k), qy = __shfl_sync(VTG_FULL, (int)fv.y, 3 * k);
+        const int q = __shfl_sync(VTG_FULL, fv, 3 * k), qx = (short)(q & 0xffff), qy = q >> 16;
         if ((qx == vx && qy == vy) || (qx == 0 && qy == 0))
             continue;
         const float s = sad(qx, qy);
