@@ -10,20 +10,20 @@
  * to bottom, the box as (v + (v_-1 + v_+1)) + (v_-2 + v_+2) with the columns outside the region's 16-column groups
  * reading 0, and det - 0.04 trace^2 as two fused multiply-subtracts). No sqrt or division, so no arithmetic differs.
  *
- * Pipeline, one stream, no host round trip:
+ * Pipeline, one stream, no host round trip, four launches, each after the first a programmatic dependent:
  *   det_response  a CTA a tile of 16 rows x 64 columns: the plane tile, the tensor, the row sums and the box in
- *                 shared memory; the response out, and the four cells' strongest (floored at 0)
- *   det_near      each cell's 3 x 3 neighbourhood strongest, a thread a cell, and the best cell
- *   det_count     a warp an eighth of a row: the local maxima above max(quality x neighbourhood, 2500), counted
- *   det_scan      the segments' counts scanned: each segment's first place in scan order
- *   det_collect   a warp a segment: the candidates in scan order, the first 8,192 kept (DETECT_MAX_CANDIDATES), each
+ *                 shared memory; the response out, the four cells' strongest (floored at 0)
+ *   det_count     the best cell; a CTA a row, a warp an eighth of it: the local maxima above max(quality x the strongest of their 3 x 3
+ *                 cells, 2500), counted
+ *   det_collect   a CTA a row: its first place in scan order from the rows' counts (tall regions: det_scan, a launch of
+ *                 its own), then the candidates in scan order, the first 8,192 kept (DETECT_MAX_CANDIDATES), each
  *                 scored v / local + 0.001 v / best in FP64 and rounded to F32 (the reference's long double rounds to
  *                 the same F32 but where the sum lies within 2^-53 of a rounding boundary)
- *   det_select    one CTA: the candidates sorted by (score descending, scan order) -- a stable radix sort of the 32-bit
- *                 score keys in shared memory, four 8-bit passes -- their places gathered, then the greedy spacing
- *                 in blocks of 1,024 candidates, a thread each, settled in parallel passes with the in-order result,
- *                 up to max corners. The corners taken and the block's candidates sit in grids of linked lists (cells
- *                 at least the spacing wide), so a candidate looks at its 3 x 3 grid cells only.
+ *   det_select    one CTA: the greedy spacing over the candidates by (score descending, scan order), in blocks of the best
+ *                 up to 256 left: a block's members by a histogram of their keys, its order by counting the lesser keys, its
+ *                 conflicts as bit masks, settled 32 at a time by one warp with the in-order result, until max corners are
+ *                 taken. The corners taken sit in a grid of linked lists (cells at least the spacing wide), so a candidate
+ *                 looks at 3 x 3 grid cells only.
  * The threshold needs no long double: local x quality is an exact product of two F32s, so its F32 rounding is the
  * reference's (float)(rel) and max(fl(rel), 2500) equals its (float)(rel > 2500 ? rel : 2500). */
 #include <math.h>
@@ -39,13 +39,11 @@
 #define DET_TY 16           /* ... and one cell row high */
 #define DET_SELECT_THREADS 1024
 #define DET_SEGS 8          /* a row's candidate columns in this many segments, a warp each */
-#define DET_GRID_MAX 16384  /* the taken corners' grid: at most this many cells (their list heads fill the keys' space) */
-#define DET_RADIX 256       /* the sort's digit: 8 bits, four passes over the 32-bit score key */
-#define DET_HIST_PITCH 257  /* a warp's digit counts: one word of padding against bank conflicts */
-static_assert(DET_SELECT_THREADS / 32 * 256 == DET_MAX_CAND, "the sort: a warp 256 candidates, 8 a lane");
-static_assert(DET_GRID_MAX <= 2 * DET_MAX_CAND, "grid heads in the spare keys' and places' space");
-static_assert(DET_SELECT_THREADS * 2 <= DET_MAX_CAND, "a block's places in the keys' space");
-static_assert(DET_GRID_MAX <= 2 * DET_HIST_PITCH * 32, "block grid heads in the counts' space");
+#define DET_GRID_MAX 16384  /* the taken corners' grid: at most this many cells */
+#define DET_BLOCK 256       /* candidates a block of the selection, at most */
+#define DET_BINS 2048       /* of its histogram: two a thread */
+#define DET_SCAN_ROWS 2048  /* regions of more rows scan the rows' counts in a launch of their own */
+static_assert(DET_BINS == 2 * DET_SELECT_THREADS, "two bins a thread");
 
 struct DetGeo {
     int x0, y0, x1, y1, ax, cols, rows, nv, cell_rows;
@@ -67,8 +65,8 @@ struct vtg_detector {
     char *mem;
     size_t bytes;
     int max_w, max_h, max_cols, max_cells;
-    float *resp, *cell, *near, *best;
-    int *rowcount, *rowbase, *ncand;
+    float *resp, *cell, *best;
+    int *rowcount, *rowbase, *ncand; /* counts a segment; counts a row, or (tall regions) first places a segment */
     unsigned *keys;
     int2 *cxy;
     float *xs, *ys;
@@ -87,8 +85,12 @@ __global__ void __launch_bounds__(256) det_response(DetPrm q, float *__restrict_
     const DetGeo &g = q.g;
     const int tid = threadIdx.x;
     const int r0 = blockIdx.y * DET_TY, c0 = blockIdx.x * DET_TX;
+    vtg_grid_launch_dependents();
     if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0)
-        *best = 0.0f; /* det_near's maximum starts here */
+        *best = 0.0f; /* det_count's maximum starts here */
+    /* a whole number of cell rows leaves one more, empty, at the region's foot */
+    if (g.rows % DET_TY == 0 && blockIdx.y == gridDim.y - 1 && tid < 4 && 4 * (int)blockIdx.x + tid < g.nv)
+        cell[gridDim.y * g.nv + 4 * blockIdx.x + tid] = 0.0f;
     for (int i = tid; i < (DET_TY + 6) * (DET_TX + 6); i += blockDim.x) {
         const int a = i / (DET_TX + 6), b = i - a * (DET_TX + 6);
         const int y = min(max(g.y0 - 3 + r0 + a, 0), q.h - 1), x = min(max(g.ax + c0 - 3 + b, 0), q.w - 1);
@@ -161,51 +163,41 @@ __global__ void __launch_bounds__(256) det_response(DetPrm q, float *__restrict_
 
 /* ---- the selection ---- */
 
-/* Each cell's 3 x 3 neighbourhood strongest, a thread a cell, and the best cell over the CTAs: an integer atomicMax
- * on the F32 bits orders them as the floats, all being >= 0 (det_response zeroes the best first). */
-__global__ void __launch_bounds__(256) det_near(DetGeo g, const float *__restrict__ cell, float *__restrict__ near,
-                                                float *__restrict__ best)
+/* The strongest response of the 3 x 3 cells around region row r, column c (detect_finish's neighbourhood). */
+__device__ __forceinline__ float det_near(const DetGeo &g, const float *cell, int r, int c)
 {
-    __shared__ float s_w[8];
-    const int n = g.nv * g.cell_rows, i = (int)(blockIdx.x * blockDim.x + threadIdx.x), tid = threadIdx.x;
+    const int cr = r >> 4, k = c >> 4;
     float m = 0.0f;
-    if (i < n) {
-        const int cr = i / g.nv, k = i - cr * g.nv;
-        for (int a = cr > 0 ? cr - 1 : 0; a <= cr + 1 && a < g.cell_rows; a++)
-            for (int b = k > 0 ? k - 1 : 0; b <= k + 1 && b < g.nv; b++)
-                m = fmaxf(m, cell[a * g.nv + b]);
-        near[i] = m;
-    }
 #pragma unroll
-    for (int s = 16; s >= 1; s >>= 1)
-        m = fmaxf(m, __shfl_xor_sync(VTG_FULL, m, s));
-    if ((tid & 31) == 0)
-        s_w[tid >> 5] = m;
-    __syncthreads();
-    if (tid == 0) {
-        float b = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++)
-            b = fmaxf(b, s_w[w]);
-        if (b > 0.0f)
-            atomicMax(reinterpret_cast<int *>(best), __float_as_int(b));
-    }
+    for (int a = -1; a <= 1; a++)
+#pragma unroll
+        for (int b = -1; b <= 1; b++)
+            if (cr + a >= 0 && cr + a < g.cell_rows && k + b >= 0 && k + b < g.nv)
+                m = fmaxf(m, __ldca(cell + (cr + a) * g.nv + k + b));
+    return m;
 }
 
-/* A corner candidate: inside the rectangle's lanes, above its threshold, and no smaller than any of its 8 neighbours
- * (those past the region's columns read 0). */
-__device__ __forceinline__ bool det_candidate(const DetPrm &q, const float *__restrict__ resp,
-                                              const float *__restrict__ near, int r, int c)
+/* A corner candidate: inside the rectangle's lanes, above its threshold (at least 2500: tried first), and no smaller than
+ * any of its 8 neighbours (those past the region's columns read 0). near: its neighbourhood's strongest, when it is one. */
+__device__ __forceinline__ bool det_candidate(const DetPrm &q, const float *resp, const float *cell, int r, int c, float &near)
 {
     const DetGeo &g = q.g;
-    const float *me = resp + (size_t)r * g.cols;
-    const float v = me[c];
-    const float thresh = fmaxf(near[(r >> 4) * g.nv + (c >> 4)] * q.quality, 2500.0f);
-    if (!(thresh < v))
+    const float *me = resp + (size_t)r * g.cols + c;
+    const float v = __ldca(me);
+    if (!(2500.0f < v))
         return false;
     const float *up = me - g.cols, *dn = me + g.cols;
     const bool lo = c > 0, hi = c + 1 < g.cols;
-    return (lo ? up[c - 1] : 0.0f) <= v && up[c] <= v && (hi ? up[c + 1] : 0.0f) <= v && (lo ? me[c - 1] : 0.0f) <= v &&
-           (hi ? me[c + 1] : 0.0f) <= v && (lo ? dn[c - 1] : 0.0f) <= v && dn[c] <= v && (hi ? dn[c + 1] : 0.0f) <= v;
+    const float n[8] = {lo ? __ldca(up - 1) : 0.0f, __ldca(up), hi ? __ldca(up + 1) : 0.0f, lo ? __ldca(me - 1) : 0.0f,
+                        hi ? __ldca(me + 1) : 0.0f, lo ? __ldca(dn - 1) : 0.0f, __ldca(dn), hi ? __ldca(dn + 1) : 0.0f};
+    bool top = true;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        top = top && n[k] <= v;
+    if (!top)
+        return false;
+    near = det_near(g, cell, r, c);
+    return fmaxf(near * q.quality, 2500.0f) < v;
 }
 
 __device__ __forceinline__ void det_lanes(const DetGeo &g, int &lo, int &hi)
@@ -224,36 +216,57 @@ __device__ __forceinline__ void det_segment(const DetGeo &g, int s, int &a, int 
     b = min(a + per, lo + len);
 }
 
-__global__ void __launch_bounds__(256) det_count(DetPrm q, const float *__restrict__ resp,
-                                                 const float *__restrict__ near, const float *__restrict__ best,
-                                                 int *__restrict__ rowcount)
+/* A CTA a row; rowtotal (regions up to DET_SCAN_ROWS) gets the row's count, rowcount its segments'. The first row of each cell
+ * row finds its best cell too: an integer atomicMax on the F32 bits orders them as the floats, all being >= 0. */
+__global__ void __launch_bounds__(32 * DET_SEGS) det_count(DetPrm q, const float *resp, const float *cell, float *best,
+                                                        int *rowcount, int *rowtotal)
 {
-    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    const int r = w / DET_SEGS, sg = w - r * DET_SEGS;
-    if (r >= q.g.rows)
-        return;
+    __shared__ int s_n[DET_SEGS];
+    const int r = blockIdx.x, sg = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    vtg_grid_launch_dependents();
+    vtg_grid_dependency_wait();
+    if (r % 16 == 0 && sg == 0) {
+        unsigned m = 0u;
+        for (int k = lane; k < q.g.nv; k += 32)
+            m = max(m, __float_as_uint(__ldca(cell + (r >> 4) * q.g.nv + k)));
+        m = __reduce_max_sync(VTG_FULL, m);
+        if (lane == 0 && m > 0u)
+            atomicMax(reinterpret_cast<int *>(best), (int)m);
+    }
     int cnt = 0;
-    if (*best > 0.0f && r >= 1 && r < q.g.rows - 1) {
+    if (r >= 1 && r < q.g.rows - 1) {
         int a, b;
+        float near;
         det_segment(q.g, sg, a, b);
         for (int c0 = a; c0 < b; c0 += 32) {
             const int c = c0 + lane;
-            cnt += __popc(__ballot_sync(VTG_FULL, c < b && det_candidate(q, resp, near, r, c)));
+            cnt += __popc(__ballot_sync(VTG_FULL, c < b && det_candidate(q, resp, cell, r, c, near)));
         }
     }
     if (lane == 0)
-        rowcount[w] = cnt;
+        rowcount[r * DET_SEGS + sg] = s_n[sg] = cnt;
+    if (!rowtotal)
+        return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int n = 0;
+        for (int k = 0; k < DET_SEGS; k++)
+            n += s_n[k];
+        rowtotal[r] = n;
+    }
 }
 
-/* Each row's first place in scan order (exclusive scan over rows), and the candidates kept: at most 8,192. */
-__global__ void __launch_bounds__(1024) det_scan(int rows, const int *__restrict__ rowcount, int *__restrict__ rowbase,
+/* Tall regions: each segment's first place in scan order (an exclusive scan), and the candidates kept: at most 8,192. */
+__global__ void __launch_bounds__(1024) det_scan(int rows, const int *rowcount, int *__restrict__ rowbase,
                                                  int *__restrict__ ncand)
 {
     __shared__ int s[1024];
     const int tid = threadIdx.x, per = (rows + 1023) / 1024, a = tid * per, b = min(a + per, rows);
+    vtg_grid_launch_dependents();
+    vtg_grid_dependency_wait();
     int sum = 0;
     for (int r = a; r < b; r++)
-        sum += rowcount[r];
+        sum += __ldca(rowcount + r);
     s[tid] = sum;
     __syncthreads();
     for (int d = 1; d < 1024; d <<= 1) {
@@ -265,35 +278,60 @@ __global__ void __launch_bounds__(1024) det_scan(int rows, const int *__restrict
     int run = s[tid] - sum;
     for (int r = a; r < b; r++) {
         rowbase[r] = run;
-        run += rowcount[r];
+        run += __ldca(rowcount + r);
     }
     if (tid == 1023)
         *ncand = min(s[1023], DET_MAX_CAND);
 }
 
-__global__ void __launch_bounds__(256) det_collect(DetPrm q, const float *__restrict__ resp,
-                                                   const float *__restrict__ near, const float *__restrict__ best,
-                                                   const int *__restrict__ rowbase, unsigned *__restrict__ keys,
-                                                   int2 *__restrict__ cxy)
+/* A CTA a row: the candidates of its segments from their first places on. scanned: rowbase holds the segments' places
+ * (det_scan); otherwise it holds the rows' counts, and the row's place is the sum of those before it (a regular load a
+ * thread for every 256 rows; at 2,048 rows this costs less than the launch it saves), the last row's CTA then knowing the
+ * number kept. */
+__global__ void __launch_bounds__(32 * DET_SEGS) det_collect(DetPrm q, const float *resp, const float *cell, const float *best,
+                                                          const int *rowcount, const int *rowbase, bool scanned,
+                                                          unsigned *__restrict__ keys, int2 *__restrict__ cxy,
+                                                          int *__restrict__ ncand)
 {
-    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    const int r = w / DET_SEGS, sg = w - r * DET_SEGS;
-    if (r < 1 || r >= q.g.rows - 1 || !(*best > 0.0f))
+    __shared__ int s_n[DET_SEGS];
+    const int r = blockIdx.x, sg = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    vtg_grid_launch_dependents();
+    vtg_grid_dependency_wait();
+    int pos;
+    if (scanned) {
+        pos = __ldca(rowbase + r * DET_SEGS + sg);
+    } else {
+        int sum = 0;
+        for (int k = threadIdx.x; k < r; k += 32 * DET_SEGS)
+            sum += __ldca(rowbase + k);
+        sum = __reduce_add_sync(VTG_FULL, sum);
+        if (lane == 0)
+            s_n[sg] = sum;
+        __syncthreads();
+        pos = 0;
+#pragma unroll
+        for (int k = 0; k < DET_SEGS; k++)
+            pos += s_n[k];
+        if (r == q.g.rows - 1 && threadIdx.x == 0)
+            *ncand = min(pos + __ldca(rowbase + r), DET_MAX_CAND);
+#pragma unroll
+        for (int k = 0; k < DET_SEGS; k++)
+            pos += k < sg ? __ldca(rowcount + r * DET_SEGS + k) : 0;
+    }
+    if (r < 1 || r >= q.g.rows - 1 || pos >= DET_MAX_CAND)
         return;
-    int pos = rowbase[w];
-    if (pos >= DET_MAX_CAND)
-        return;
-    const double bst = (double)*best;
+    const double bst = (double)__ldca(best);
     int a, b;
     det_segment(q.g, sg, a, b);
     for (int c0 = a; c0 < b && pos < DET_MAX_CAND; c0 += 32) {
         const int c = c0 + lane;
-        const bool f = c < b && det_candidate(q, resp, near, r, c);
+        float near = 0.0f;
+        const bool f = c < b && det_candidate(q, resp, cell, r, c, near);
         const unsigned m = __ballot_sync(VTG_FULL, f);
         const int p = pos + __popc(m & ((1u << lane) - 1u));
         if (f && p < DET_MAX_CAND) {
-            const double v = (double)resp[(size_t)r * q.g.cols + c];
-            const double local = (double)near[(r >> 4) * q.g.nv + (c >> 4)];
+            const double v = (double)__ldca(resp + (size_t)r * q.g.cols + c);
+            const double local = (double)near;
             const float score = (float)(v / local + 0.001 * v / bst);
             keys[p] = ~__float_as_uint(score); /* ascending: the best first; the place is the index */
             cxy[p] = make_int2(q.g.ax + c, q.g.y0 + r);
@@ -324,219 +362,203 @@ __device__ __forceinline__ bool det_far(const DetPrm &q, const int *s_head, cons
     return true;
 }
 
-#define DET_OPEN 0
-#define DET_TAKEN 1
-#define DET_OUT 2
+struct DetSelectSmem {
+    int head[DET_GRID_MAX]; /* the taken corners' grid: the newest of each cell */
+    int tx[512], ty[512], next[512];
+    int hist[DET_BINS];
+    unsigned long long list[DET_BLOCK]; /* a block's members: key << 13 | place in scan order */
+    int2 xy[DET_BLOCK];                 /* in order */
+    unsigned mask[DET_BLOCK / 32][DET_BLOCK]; /* [k][i]: which of candidates 32 k .. 32 k + 31 before i are too close to i */
+    unsigned far[DET_BLOCK / 32], got[DET_BLOCK / 32];
+    int wsum[32], cut, below, upto, members;
+    unsigned lo, hi;
+};
 
-/* A block candidate's earlier neighbours within the spacing (the block grid's 3 x 3 cells around it): DET_OUT when
- * one of them is taken, DET_OPEN when none is but one is still open, else DET_TAKEN. The states are read while other
- * threads set theirs: a state once set never changes, so a stale read only defers the answer to the next pass. */
-__device__ __forceinline__ int det_earlier(const DetPrm &q, const int *s_bhead, const int *s_bnext, const int2 *xy,
-                                           const unsigned char *s_st, int me, int x, int y)
+/* The greedy spacing. The reference sorts the candidates by (score descending, scan order) and takes each that keeps the
+ * spacing from every corner taken; the result of walking them in blocks, in that order, is the same. A key is ~score bits << 13
+ * | place in scan order: 45 bits, all different. Eight keys a thread stay in registers. A block is the keys below a limit,
+ * found by a histogram over the range of those left (2,048 bins; a range whose first bin holds more than a block is zoomed
+ * into, which ends as keys differ), so nothing is sorted that the walk never reaches: a walk takes 1.1 to 2 candidates a
+ * corner. Whatever of a block is too close to a corner taken before it is out; the rest is settled by conflict masks, 32
+ * candidates at a time: a candidate is taken once no earlier one in conflict with it is taken or open, out once one is taken. */
+__global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, const int *ncand, const float *best, const unsigned *keys,
+                                                                 const int2 *cxy, float *__restrict__ xs,
+                                                                 float *__restrict__ ys, int *__restrict__ count)
 {
-    const volatile unsigned char *st = s_st;
-    const int gx = (x - q.g.ax) / q.gs, gy = (y - q.g.y0) / q.gs;
-    bool pending = false;
-    for (int j = 0; j < 9; j++) {
-        const int a = gx + j % 3 - 1, b = gy + j / 3 - 1;
-        if (a < 0 || a >= q.gw || b < 0 || b >= q.gh)
-            continue;
-        for (int u = s_bhead[b * q.gw + a]; u >= 0; u = s_bnext[u]) {
-            if (u >= me)
-                continue;
-            const int dx = xy[u].x - x, dy = xy[u].y - y;
-            if (dx * dx + dy * dy >= q.need)
-                continue;
-            const int su = st[u];
-            if (su == DET_TAKEN)
-                return DET_OUT;
-            pending = pending || su == DET_OPEN;
-        }
-    }
-    return pending ? DET_OPEN : DET_TAKEN;
-}
-
-/* One pass of the stable LSD radix sort over the candidates' score keys in shared memory: the 8-bit digit at shift,
- * from (ka, va) to (kb, vb). Warp w holds elements 256 w + 32 k + lane (k = 0..7), ranked in that order within the
- * warp (the lanes with the same digit found by eight ballots); the per-(digit, warp) counts, scanned in digit-major
- * order, place them. The counts sit at warp * DET_HIST_PITCH + digit: a warp's lanes and a scan step's lanes fall in
- * different banks. Two count buffers alternate: this pass counts in hist (zeroed by the pass before) and zeroes
- * next. Warps past the candidates (256 w >= n) count nothing. */
-__device__ __forceinline__ void det_radix_pass(const unsigned *ka, const unsigned *va, unsigned *kb, unsigned *vb,
-                                               int *hist, int *next, int *s_wsum, int n, int shift, bool first)
-{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    DetSelectSmem &S = *reinterpret_cast<DetSelectSmem *>(s_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < DET_HIST_PITCH * 32; i += blockDim.x)
-        next[i] = 0;
-    const bool active = 256 * warp < n;
-    unsigned key[8], val[8];
-    int rank[8];
-    if (active) {
+    for (int i = tid; i < q.gw * q.gh; i += DET_SELECT_THREADS)
+        S.head[i] = -1;
+    vtg_grid_dependency_wait();
+    const int n = __ldca(best) > 0.0f ? __ldca(ncand) : 0;
+    unsigned key[DET_MAX_CAND / DET_SELECT_THREADS];
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int i = 256 * warp + 32 * k + lane;
-            key[k] = ka[i];
-            val[k] = first ? (unsigned)i : va[i];
-            const unsigned dig = (key[k] >> shift) & (DET_RADIX - 1);
-            unsigned peers = VTG_FULL;
-#pragma unroll
-            for (int b = 0; b < 8; b++) {
-                const unsigned m = __ballot_sync(VTG_FULL, (dig >> b) & 1u);
-                peers &= ((dig >> b) & 1u) ? m : ~m;
-            }
-            const int lt = __popc(peers & ((1u << lane) - 1u));
-            int *h = hist + warp * DET_HIST_PITCH + dig;
-            const int base = *h;
-            rank[k] = base + lt;
-            __syncwarp();
-            if (lt == 0)
-                *h = base + __popc(peers);
-            __syncwarp();
-        }
+    for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++) {
+        const int i = tid + k * DET_SELECT_THREADS;
+        key[k] = i < n ? __ldca(keys + i) : 0u;
     }
-    __syncthreads();
-    /* exclusive scan of the 8,192 counts: 8 a thread, across a warp, then across the warps (each warp scans the 32
-     * warp totals itself) */
-    int c[8], sum = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int e = 8 * tid + j; /* digit e / 32, warp e % 32 */
-        c[j] = hist[(e & 31) * DET_HIST_PITCH + (e >> 5)];
-        sum += c[j];
-    }
-    int inc = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(VTG_FULL, inc, d);
-        if (lane >= d)
-            inc += v;
-    }
-    if (lane == 31)
-        s_wsum[warp] = inc;
-    __syncthreads();
-    const int t = s_wsum[lane];
-    int ti = t;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(VTG_FULL, ti, d);
-        if (lane >= d)
-            ti += v;
-    }
-    int run = __shfl_sync(VTG_FULL, ti - t, warp) + inc - sum;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int e = 8 * tid + j;
-        hist[(e & 31) * DET_HIST_PITCH + (e >> 5)] = run;
-        run += c[j];
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const unsigned dig = (key[k] >> shift) & (DET_RADIX - 1);
-            const int dst = hist[warp * DET_HIST_PITCH + dig] + rank[k];
-            kb[dst] = key[k];
-            vb[dst] = val[k];
-        }
-    }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, const int *__restrict__ ncand,
-                                                                 const float *__restrict__ best,
-                                                                 const unsigned *__restrict__ keys,
-                                                                 const int2 *__restrict__ cxy,
-                                                                 float *__restrict__ xs, float *__restrict__ ys,
-                                                                 int *__restrict__ count)
-{
-    /* two buffers of keys and places (DET_MAX_CAND each), then two of radix counts. Once sorted (places in v0),
-     * k1 and v1 hold the taken corners' grid heads, the counts the block grid's, and k0 a block's (x, y). */
-    extern __shared__ unsigned s_buf[];
-    __shared__ int s_tx[512], s_ty[512], s_next[512], s_wsum[32];
-    __shared__ int s_bnext[DET_SELECT_THREADS];
-    __shared__ unsigned char s_st[DET_SELECT_THREADS];
-    unsigned *k0 = s_buf, *v0 = s_buf + DET_MAX_CAND, *k1 = s_buf + 2 * DET_MAX_CAND, *v1 = s_buf + 3 * DET_MAX_CAND;
-    int *h0 = reinterpret_cast<int *>(s_buf + 4 * DET_MAX_CAND), *h1 = h0 + DET_HIST_PITCH * 32;
-    int2 *s_xy = reinterpret_cast<int2 *>(k0);
-    int *s_head = reinterpret_cast<int *>(k1);
-    int *s_bhead = h0;
-    const int tid = threadIdx.x;
-    const int n = *best > 0.0f ? *ncand : 0;
-    const int n256 = (n + 255) & ~255;
-    for (int i = tid; i < n256; i += blockDim.x)
-        k0[i] = i < n ? keys[i] : ~0u; /* past the candidates: after every score, and stable behind them */
-    for (int i = tid; i < DET_HIST_PITCH * 32; i += blockDim.x)
-        h0[i] = 0;
-    __syncthreads();
-    /* ascending ~score bits, ties in scan order: the order detect_finish's qsort gives (score descending, then order) */
-    det_radix_pass(k0, v0, k1, v1, h0, h1, s_wsum, n, 0, true);
-    det_radix_pass(k1, v1, k0, v0, h1, h0, s_wsum, n, 8, false);
-    det_radix_pass(k0, v0, k1, v1, h0, h1, s_wsum, n, 16, false);
-    det_radix_pass(k1, v1, k0, v0, h1, h0, s_wsum, n, 24, false);
-    for (int i = tid; i < q.gw * q.gh; i += blockDim.x) {
-        s_head[i] = -1;
-        s_bhead[i] = -1;
-    }
-    __syncthreads();
-    /* The greedy spacing in blocks of up to 1,024 candidates, a thread a candidate; the result is the one-by-one
-     * order's. A candidate too close to a corner taken in an earlier block is out. Within the block the candidates
-     * sit in a grid of their own, and each open one looks at its earlier neighbours within the spacing: out once one
-     * of them is taken, taken once all of them are out. Every pass settles at least the earliest open one, so a block ends
-     * within as many passes as it has candidates. The taken ones past max are dropped in order. */
-    const int lane = tid & 31, warp = tid >> 5;
-    int taken = 0;
-    for (int base = 0, B = 0; base < n && taken < q.max; base += B) {
-        /* twice the corners still wanted, 64 to 1,024: the greedy rarely looks further, and a shorter block settles
-         * in fewer passes */
-        B = min(n - base, min(DET_SELECT_THREADS, max(64, 2 * (q.max - taken))));
-        int2 me = make_int2(0, 0);
-        int cell = 0;
-        if (tid < B) {
-            me = cxy[v0[base + tid]]; /* the block's places, gathered as it starts */
-            s_xy[tid] = me;
-            cell = ((me.y - q.g.y0) / q.gs) * q.gw + (me.x - q.g.ax) / q.gs;
-            s_st[tid] = det_far(q, s_head, s_next, s_tx, s_ty, me.x, me.y) ? DET_OPEN : DET_OUT;
-            s_bnext[tid] = atomicExch(&s_bhead[cell], tid);
+    auto whole = [&](int k) { return ((unsigned long long)key[k] << 13) | (unsigned)(tid + k * DET_SELECT_THREADS); };
+    unsigned long long from = 0ull; /* keys below are done with */
+    int taken = 0, left = n;
+    while (left > 0 && taken < q.max) {
+        /* the range of the keys left */
+        if (tid == 0) {
+            S.lo = ~0u;
+            S.hi = 0u;
+            S.members = 0;
         }
         __syncthreads();
-        bool open = tid < B && s_st[tid] == DET_OPEN;
-        while (__syncthreads_or(open)) {
-            if (open) {
-                const int r = det_earlier(q, s_bhead, s_bnext, s_xy, s_st, tid, me.x, me.y);
-                if (r != DET_OPEN) {
-                    s_st[tid] = (unsigned char)r;
-                    open = false;
+        unsigned lo = ~0u, hi = 0u;
+#pragma unroll
+        for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++)
+            if (tid + k * DET_SELECT_THREADS < n && whole(k) >= from) {
+                lo = min(lo, key[k]);
+                hi = max(hi, key[k]);
+            }
+        lo = __reduce_min_sync(VTG_FULL, lo);
+        hi = __reduce_max_sync(VTG_FULL, hi);
+        if (lane == 0) {
+            atomicMin(&S.lo, lo);
+            atomicMax(&S.hi, hi);
+        }
+        __syncthreads();
+        unsigned long long a = (unsigned long long)S.lo << 13, b = ((unsigned long long)S.hi << 13) | 8191ull, limit;
+        a = a > from ? a : from;
+        /* twice the corners still wanted: the greedy rarely looks further */
+        const int want = min(left, min(DET_BLOCK, max(64, 2 * (q.max - taken))));
+        for (;;) {
+            const int shift = max(0, 64 - __clzll((long long)(b - a)) - 11);
+            S.hist[2 * tid] = 0;
+            S.hist[2 * tid + 1] = 0;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++)
+                if (tid + k * DET_SELECT_THREADS < n && whole(k) >= a && whole(k) <= b)
+                    atomicAdd(&S.hist[(int)((whole(k) - a) >> shift)], 1);
+            __syncthreads();
+            const int h0 = S.hist[2 * tid], h1 = S.hist[2 * tid + 1];
+            int inc = h0 + h1;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int v = __shfl_up_sync(VTG_FULL, inc, d);
+                inc += lane >= d ? v : 0;
+            }
+            if (lane == 31)
+                S.wsum[warp] = inc;
+            __syncthreads();
+            const int w = S.wsum[lane];
+            const int base = __reduce_add_sync(VTG_FULL, lane < warp ? w : 0);
+            const int e1 = base + inc, e0 = e1 - h1, s0 = e0 - h0; /* up to and with the thread's bins; before them */
+            /* the bin where the count reaches what is wanted: one thread has it, unless fewer are left in the range */
+            if (s0 < want && want <= e1) {
+                const bool first = want <= e0;
+                S.cut = 2 * tid + (first ? 0 : 1);
+                S.below = first ? s0 : e0;
+                S.upto = first ? e0 : e1;
+            }
+            if (tid == DET_SELECT_THREADS - 1 && e1 < want) {
+                S.cut = DET_BINS - 1;
+                S.below = S.upto = e1;
+            }
+            __syncthreads();
+            const int cut = S.cut, below = S.below, upto = S.upto;
+            __syncthreads();
+            if (upto <= DET_BLOCK) {
+                limit = a + ((unsigned long long)(cut + 1) << shift);
+                break;
+            }
+            if (below > 0) {
+                limit = a + ((unsigned long long)cut << shift);
+                break;
+            }
+            b = a + ((unsigned long long)(cut + 1) << shift) - 1ull;
+            a += (unsigned long long)cut << shift;
+        }
+        /* the members, in any order, then in theirs: a thread a member counts the lesser ones */
+#pragma unroll
+        for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++)
+            if (tid + k * DET_SELECT_THREADS < n && whole(k) >= from && whole(k) < limit)
+                S.list[atomicAdd(&S.members, 1)] = whole(k);
+        if (tid < DET_BLOCK / 32)
+            S.far[tid] = 0u;
+        __syncthreads();
+        const int M = S.members; /* 1 .. DET_BLOCK */
+        from = limit;
+        left -= M;
+        int2 me = make_int2(0, 0);
+        int at = 0, cell = 0;
+        if (tid < M) {
+            const unsigned long long mine = S.list[tid];
+            me = __ldca(cxy + (int)(mine & 8191ull));
+            for (int j = 0; j < M; j++)
+                at += S.list[j] < mine;
+            S.xy[at] = me;
+            cell = ((me.y - q.g.y0) / q.gs) * q.gw + (me.x - q.g.ax) / q.gs;
+            if (!det_far(q, S.head, S.next, S.tx, S.ty, me.x, me.y))
+                atomicOr(&S.far[at >> 5], 1u << (at & 31));
+        }
+        __syncthreads();
+        /* the conflicts: thread (i, part) compares candidate i with 64 of those before it */
+        {
+            const int i = tid % DET_BLOCK, part = tid / DET_BLOCK;
+            unsigned m0 = 0u, m1 = 0u;
+            if (64 * part <= (i | 31) && 64 * part < M) { /* uniform in a warp */
+                const int2 p = S.xy[min(i, M - 1)];
+#pragma unroll 4
+                for (int j = 0; j < 32; j++) {
+                    const int2 u = S.xy[64 * part + j], v = S.xy[64 * part + 32 + j];
+                    const int ux = u.x - p.x, uy = u.y - p.y, vx = v.x - p.x, vy = v.y - p.y;
+                    m0 |= ux * ux + uy * uy < q.need ? 1u << j : 0u;
+                    m1 |= vx * vx + vy * vy < q.need ? 1u << j : 0u;
                 }
             }
+            /* only those before i */
+            auto before = [&](int k) { return k > (i >> 5) ? 0u : k < (i >> 5) ? ~0u : (1u << (i & 31)) - 1u; };
+            S.mask[2 * part][i] = m0 & before(2 * part);
+            S.mask[2 * part + 1][i] = m1 & before(2 * part + 1);
         }
-        /* the taken ones in order: their places in the list of corners */
-        const bool yes = tid < B && s_st[tid] == DET_TAKEN;
-        const unsigned bal = __ballot_sync(VTG_FULL, yes);
-        if (lane == 0)
-            s_wsum[warp] = __popc(bal);
         __syncthreads();
-        const int wt = s_wsum[lane];
-        int wi = wt;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int v = __shfl_up_sync(VTG_FULL, wi, d);
-            if (lane >= d)
-                wi += v;
+        if (warp == 0) {
+            unsigned got = 0u; /* lane k: the taken ones of word k */
+            for (int k = 0; 32 * k < M; k++) {
+                const int i = 32 * k + lane;
+                unsigned hit = 0u;
+                for (int e = 0; e < k; e++)
+                    hit |= S.mask[e][i] & __shfl_sync(VTG_FULL, got, e);
+                const unsigned own = S.mask[k][i];
+                unsigned open = __ballot_sync(VTG_FULL, i < M && !hit && !((S.far[k] >> lane) & 1u)), yes = 0u;
+                while (open) {
+                    const bool mine = (open >> lane) & 1u;
+                    const bool now = mine && !(own & (open | yes));
+                    const bool out = mine && (own & yes);
+                    yes |= __ballot_sync(VTG_FULL, now);
+                    open &= ~__ballot_sync(VTG_FULL, now || out);
+                }
+                got = lane == k ? yes : got;
+            }
+            if (lane < DET_BLOCK / 32)
+                S.got[lane] = got;
         }
-        const int rank = __shfl_sync(VTG_FULL, wi - wt, warp) + __popc(bal & ((1u << lane) - 1u));
-        const int total = __shfl_sync(VTG_FULL, wi, 31);
-        if (yes && taken + rank < q.max) {
-            const int at = taken + rank;
-            s_tx[at] = me.x;
-            s_ty[at] = me.y;
-            xs[at] = (float)me.x;
-            ys[at] = (float)me.y;
-            s_next[at] = atomicExch(&s_head[cell], at);
+        __syncthreads();
+        /* the taken ones in order, those past max dropped */
+        int total = 0, rank = 0;
+#pragma unroll
+        for (int k = 0; k < DET_BLOCK / 32; k++) {
+            const int c = __popc(S.got[k]);
+            rank += k < (at >> 5) ? c : 0;
+            total += c;
+        }
+        rank += __popc(S.got[at >> 5] & ((1u << (at & 31)) - 1u));
+        if (tid < M && ((S.got[at >> 5] >> (at & 31)) & 1u) && taken + rank < q.max) {
+            const int t = taken + rank;
+            S.tx[t] = me.x;
+            S.ty[t] = me.y;
+            xs[t] = (float)me.x;
+            ys[t] = (float)me.y;
+            S.next[t] = atomicExch(&S.head[cell], t);
         }
         taken = min(taken + total, q.max);
-        __syncthreads();
-        if (tid < B)
-            s_bhead[cell] = -1;
         __syncthreads();
     }
     if (tid == 0)
@@ -583,7 +605,7 @@ static bool det_geometry(int w, int h, float rx, float ry, float rw, float rh, i
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 struct DetLayout {
-    size_t resp, cell, near, best, rowcount, rowbase, ncand, keys, cxy, xs, ys, count, bytes;
+    size_t resp, cell, best, rowcount, rowbase, ncand, keys, cxy, xs, ys, count, bytes;
 };
 
 static DetLayout det_layout(int max_w, int max_h, int &max_cols, int &max_cells)
@@ -595,8 +617,6 @@ static DetLayout det_layout(int max_w, int max_h, int &max_cols, int &max_cells)
     L.resp = b;
     b += up256(sizeof(float) * (size_t)max_cols * max_h);
     L.cell = b;
-    b += up256(sizeof(float) * (size_t)max_cells);
-    L.near = b;
     b += up256(sizeof(float) * (size_t)max_cells);
     L.best = b;
     b += 256;
@@ -668,7 +688,6 @@ extern "C" int vtg_detector_create(vtg_ctx *ctx, int max_w, int max_h, vtg_detec
     }
     d->resp = (float *)(d->mem + L.resp);
     d->cell = (float *)(d->mem + L.cell);
-    d->near = (float *)(d->mem + L.near);
     d->best = (float *)(d->mem + L.best);
     d->rowcount = (int *)(d->mem + L.rowcount);
     d->rowbase = (int *)(d->mem + L.rowbase);
@@ -742,19 +761,24 @@ extern "C" int vtg_detect(vtg_detector *d, const float *plane, int w, int h, int
         return VTG_OK;
     }
     const DetGeo &g = q.g;
-    CU(cudaMemsetAsync(d->cell, 0, sizeof(float) * (size_t)g.nv * g.cell_rows, st));
-    det_response<<<dim3((g.cols + DET_TX - 1) / DET_TX, (g.rows + DET_TY - 1) / DET_TY), 256, 0, st>>>(q, d->resp,
-                                                                                                   d->cell, d->best);
-    det_near<<<(g.nv * g.cell_rows + 255) / 256, 256, 0, st>>>(g, d->cell, d->near, d->best);
-    const int rblocks = (g.rows * DET_SEGS * 32 + 255) / 256;
-    det_count<<<rblocks, 256, 0, st>>>(q, d->resp, d->near, d->best, d->rowcount);
-    det_scan<<<1, 1024, 0, st>>>(g.rows * DET_SEGS, d->rowcount, d->rowbase, d->ncand);
-    det_collect<<<rblocks, 256, 0, st>>>(q, d->resp, d->near, d->best, d->rowbase, d->keys, d->cxy);
-    const int smem = (int)(4 * sizeof(unsigned) * DET_MAX_CAND + 2 * sizeof(int) * DET_HIST_PITCH * 32);
-    CU(cudaFuncSetAttribute(det_select, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     float *oxs = where == VTG_DEVICE ? xs : d->xs, *oys = where == VTG_DEVICE ? ys : d->ys;
     int *ocount = where == VTG_DEVICE ? count : d->count;
-    det_select<<<1, DET_SELECT_THREADS, smem, st>>>(q, d->ncand, d->best, d->keys, d->cxy, oxs, oys, ocount);
+    const bool scan = g.rows > DET_SCAN_ROWS;
+    const dim3 rows(g.rows), threads(32 * DET_SEGS);
+    const float *resp = d->resp, *cell = d->cell, *best = d->best;
+    const int *rowcount = d->rowcount, *rowbase = d->rowbase;
+    det_response<<<dim3((g.cols + DET_TX - 1) / DET_TX, (g.rows + DET_TY - 1) / DET_TY), 256, 0, st>>>(q, d->resp,
+                                                                                                   d->cell, d->best);
+    CU(vtg_launch_k(det_count, rows, threads, 0, st, true, q, resp, cell, d->best, d->rowcount,
+                    scan ? (int *)nullptr : d->rowbase));
+    if (scan)
+        CU(vtg_launch_k(det_scan, dim3(1), dim3(1024), 0, st, true, g.rows * DET_SEGS, rowcount, d->rowbase, d->ncand));
+    CU(vtg_launch_k(det_collect, rows, threads, 0, st, true, q, resp, cell, best, rowcount, rowbase, scan, d->keys, d->cxy,
+                    d->ncand));
+    const int smem = (int)sizeof(DetSelectSmem);
+    CU(cudaFuncSetAttribute(det_select, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CU(vtg_launch_k(det_select, dim3(1), dim3(DET_SELECT_THREADS), smem, st, true, q, (const int *)d->ncand, best,
+                    (const unsigned *)d->keys, (const int2 *)d->cxy, oxs, oys, ocount));
     CU(cudaGetLastError());
     if (where == VTG_HOST) {
         CU(cudaMemcpyAsync(count, d->count, sizeof(int), cudaMemcpyDeviceToHost, st));
