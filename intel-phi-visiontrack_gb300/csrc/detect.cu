@@ -284,6 +284,28 @@ __global__ void __launch_bounds__(1024) det_scan(int rows, const int *rowcount, 
         *ncand = min(s[1023], DET_MAX_CAND);
 }
 
+/* v / local + 0.001 v / best in FP64, rounded to F32. GB300's FP64 rate is a small fraction of its F32 rate (8,192 scores
+ * bound the kernel by it: 22 us over a 1080p frame), so the sum is formed in pairs of F32s first (each quotient and its
+ * remainder's, 0.001 as two F32s: within 2^-44), which decides the rounding unless it lies within 2^-40 of halfway between two
+ * F32s; only then, or where a value is out of the pairs' range, are the FP64 divisions made. */
+__device__ __forceinline__ float det_score(float v, float local, float best)
+{
+    const float rl = __frcp_rn(local), rb = __frcp_rn(best);
+    const float q = v * rl, q1 = __fmaf_rn(-q, local, v) * rl;
+    const float C0 = 0.001f, C1 = (float)(0.001 - (double)0.001f);
+    const float p = C0 * v, p1 = __fmaf_rn(C0, v, -p) + C1 * v;
+    const float t = p * rb, t1 = (__fmaf_rn(-t, best, p) + p1) * rb;
+    /* q + t (q is the larger: local <= best), then everything below it */
+    const float s = q + t, e = (t - (s - q)) + (q1 + t1);
+    const float hi = s + e, lo = e - (hi - s);
+    /* how far hi + lo is from halfway to hi's neighbour on lo's side */
+    const float step = fabsf(__int_as_float(__float_as_int(hi) + (lo < 0.0f ? -1 : 1)) - hi);
+    if (v < 1e30f && best < 1e30f && fabsf(fabsf(lo) - 0.5f * step) > 1e-12f * hi)
+        return hi;
+    const double x = (double)v;
+    return (float)(x / (double)local + 0.001 * x / (double)best);
+}
+
 /* A CTA a row: the candidates of its segments from their first places on. scanned: rowbase holds the segments' places
  * (det_scan); otherwise it holds the rows' counts, and the row's place is the sum of those before it (a regular load a
  * thread for every 256 rows; at 2,048 rows this costs less than the launch it saves), the last row's CTA then knowing the
@@ -320,7 +342,7 @@ __global__ void __launch_bounds__(32 * DET_SEGS) det_collect(DetPrm q, const flo
     }
     if (r < 1 || r >= q.g.rows - 1 || pos >= DET_MAX_CAND)
         return;
-    const double bst = (double)__ldca(best);
+    const float bst = __ldca(best);
     int a, b;
     det_segment(q.g, sg, a, b);
     for (int c0 = a; c0 < b && pos < DET_MAX_CAND; c0 += 32) {
@@ -330,9 +352,7 @@ __global__ void __launch_bounds__(32 * DET_SEGS) det_collect(DetPrm q, const flo
         const unsigned m = __ballot_sync(VTG_FULL, f);
         const int p = pos + __popc(m & ((1u << lane) - 1u));
         if (f && p < DET_MAX_CAND) {
-            const double v = (double)__ldca(resp + (size_t)r * q.g.cols + c);
-            const double local = (double)near;
-            const float score = (float)(v / local + 0.001 * v / bst);
+            const float score = det_score(__ldca(resp + (size_t)r * q.g.cols + c), near, bst);
             keys[p] = ~__float_as_uint(score); /* ascending: the best first; the place is the index */
             cxy[p] = make_int2(q.g.ax + c, q.g.y0 + r);
         }
@@ -366,11 +386,12 @@ struct DetSelectSmem {
     int head[DET_GRID_MAX]; /* the taken corners' grid: the newest of each cell */
     int tx[512], ty[512], next[512];
     int hist[DET_BINS];
-    unsigned long long list[DET_BLOCK]; /* a block's members: key << 13 | place in scan order */
-    int2 xy[DET_BLOCK];                 /* in order */
+    unsigned long long list[DET_SELECT_THREADS]; /* a block's members: key << 13 | place in scan order */
+    unsigned long long order[DET_SELECT_THREADS];
+    int2 xy[DET_BLOCK]; /* those of them that keep the spacing from every corner taken before it, in order */
     unsigned mask[DET_BLOCK / 32][DET_BLOCK]; /* [k][i]: which of candidates 32 k .. 32 k + 31 before i are too close to i */
-    unsigned far[DET_BLOCK / 32], got[DET_BLOCK / 32];
-    int wsum[32], cut, below, upto, members;
+    unsigned got[DET_BLOCK / 32];
+    int wsum[32], cut, below, upto;
     unsigned lo, hi;
 };
 
@@ -378,62 +399,65 @@ struct DetSelectSmem {
  * spacing from every corner taken; the result of walking them in blocks, in that order, is the same. A key is ~score bits << 13
  * | place in scan order: 45 bits, all different. Eight keys a thread stay in registers. A block is the keys below a limit,
  * found by a histogram over the range of those left (2,048 bins; a range whose first bin holds more than a block is zoomed
- * into, which ends as keys differ), so nothing is sorted that the walk never reaches: a walk takes 1.1 to 2 candidates a
- * corner. Whatever of a block is too close to a corner taken before it is out; the rest is settled by conflict masks, 32
- * candidates at a time: a candidate is taken once no earlier one in conflict with it is taken or open, out once one is taken. */
+ * into, which ends as keys differ), so nothing is ordered that the walk never reaches; the histogram's prefix sums also place
+ * the members, a bin's few among themselves by counting. Whatever of it is too close to a corner
+ * taken before it is out at once, a thread a member; up to 256 may be left (a block with more is tried again with fewer
+ * members; the share left sets the next block's size). Those are settled by conflict masks, 32 candidates at a time by one warp: a candidate is taken once no earlier one in conflict with it is taken or open, out once
+ * one is taken. 128 corners of a 384 x 307 box (2,673 candidates): 13 us, where four radix passes over the candidates and
+ * blocks settled in passes took 32. Latency of one SM's barriers and shared memory bounds it. */
 __global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, const int *ncand, const float *best, const unsigned *keys,
                                                                  const int2 *cxy, float *__restrict__ xs,
                                                                  float *__restrict__ ys, int *__restrict__ count)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     DetSelectSmem &S = *reinterpret_cast<DetSelectSmem *>(s_raw);
+    constexpr int KEYS = DET_MAX_CAND / DET_SELECT_THREADS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < q.gw * q.gh; i += DET_SELECT_THREADS)
         S.head[i] = -1;
+    if (tid == 0) {
+        S.lo = ~0u;
+        S.hi = 0u;
+    }
     vtg_grid_dependency_wait();
     const int n = __ldca(best) > 0.0f ? __ldca(ncand) : 0;
-    unsigned key[DET_MAX_CAND / DET_SELECT_THREADS];
+    unsigned key[KEYS], lo = ~0u, hi = 0u;
 #pragma unroll
-    for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++) {
+    for (int k = 0; k < KEYS; k++) {
         const int i = tid + k * DET_SELECT_THREADS;
         key[k] = i < n ? __ldca(keys + i) : 0u;
     }
-    auto whole = [&](int k) { return ((unsigned long long)key[k] << 13) | (unsigned)(tid + k * DET_SELECT_THREADS); };
-    unsigned long long from = 0ull; /* keys below are done with */
-    int taken = 0, left = n;
-    while (left > 0 && taken < q.max) {
-        /* the range of the keys left */
-        if (tid == 0) {
-            S.lo = ~0u;
-            S.hi = 0u;
-            S.members = 0;
-        }
-        __syncthreads();
-        unsigned lo = ~0u, hi = 0u;
+    __syncthreads();
 #pragma unroll
-        for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++)
-            if (tid + k * DET_SELECT_THREADS < n && whole(k) >= from) {
-                lo = min(lo, key[k]);
-                hi = max(hi, key[k]);
-            }
-        lo = __reduce_min_sync(VTG_FULL, lo);
-        hi = __reduce_max_sync(VTG_FULL, hi);
-        if (lane == 0) {
-            atomicMin(&S.lo, lo);
-            atomicMax(&S.hi, hi);
+    for (int k = 0; k < KEYS; k++)
+        if (tid + k * DET_SELECT_THREADS < n) {
+            lo = min(lo, key[k]);
+            hi = max(hi, key[k]);
         }
-        __syncthreads();
-        unsigned long long a = (unsigned long long)S.lo << 13, b = ((unsigned long long)S.hi << 13) | 8191ull, limit;
-        a = a > from ? a : from;
-        /* twice the corners still wanted: the greedy rarely looks further */
-        const int want = min(left, min(DET_BLOCK, max(64, 2 * (q.max - taken))));
+    lo = __reduce_min_sync(VTG_FULL, lo);
+    hi = __reduce_max_sync(VTG_FULL, hi);
+    if (lane == 0) {
+        atomicMin(&S.lo, lo);
+        atomicMax(&S.hi, hi);
+    }
+    __syncthreads();
+    auto whole = [&](int k) { return ((unsigned long long)key[k] << 13) | (unsigned)(tid + k * DET_SELECT_THREADS); };
+    /* keys below `from` are done with; the last one */
+    unsigned long long from = (unsigned long long)S.lo << 13;
+    const unsigned long long last = ((unsigned long long)S.hi << 13) | 8191ull;
+    int taken = 0, left = n;
+    int size = min(DET_BLOCK, max(64, 2 * q.max)); /* members of the next block: the greedy rarely looks further */
+    while (left > 0 && taken < q.max) {
+        const int cap = size <= DET_BLOCK ? DET_BLOCK : DET_SELECT_THREADS, want = min(left, size);
+        unsigned long long a = from, b = last, limit;
+        int shift, members;
         for (;;) {
-            const int shift = max(0, 64 - __clzll((long long)(b - a)) - 11);
+            shift = max(0, 64 - __clzll((long long)(b - a)) - 11);
             S.hist[2 * tid] = 0;
             S.hist[2 * tid + 1] = 0;
             __syncthreads();
 #pragma unroll
-            for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++)
+            for (int k = 0; k < KEYS; k++)
                 if (tid + k * DET_SELECT_THREADS < n && whole(k) >= a && whole(k) <= b)
                     atomicAdd(&S.hist[(int)((whole(k) - a) >> shift)], 1);
             __syncthreads();
@@ -450,54 +474,71 @@ __global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, co
             const int w = S.wsum[lane];
             const int base = __reduce_add_sync(VTG_FULL, lane < warp ? w : 0);
             const int e1 = base + inc, e0 = e1 - h1, s0 = e0 - h0; /* up to and with the thread's bins; before them */
-            /* the bin where the count reaches what is wanted: one thread has it, unless fewer are left in the range */
+            /* the bin where the count reaches what is wanted: one thread has it (the range holds as many) */
             if (s0 < want && want <= e1) {
                 const bool first = want <= e0;
                 S.cut = 2 * tid + (first ? 0 : 1);
                 S.below = first ? s0 : e0;
                 S.upto = first ? e0 : e1;
             }
-            if (tid == DET_SELECT_THREADS - 1 && e1 < want) {
-                S.cut = DET_BINS - 1;
-                S.below = S.upto = e1;
-            }
             __syncthreads();
             const int cut = S.cut, below = S.below, upto = S.upto;
+            S.hist[2 * tid] = s0; /* where each bin's members go */
+            S.hist[2 * tid + 1] = e0;
             __syncthreads();
-            if (upto <= DET_BLOCK) {
+            if (upto <= cap) {
                 limit = a + ((unsigned long long)(cut + 1) << shift);
+                members = upto;
                 break;
             }
             if (below > 0) {
                 limit = a + ((unsigned long long)cut << shift);
+                members = below;
                 break;
             }
             b = a + ((unsigned long long)(cut + 1) << shift) - 1ull;
             a += (unsigned long long)cut << shift;
         }
-        /* the members, in any order, then in theirs: a thread a member counts the lesser ones */
+        /* the members (none lies before a) by their bins, then in order: bin k's end where the next one's began */
 #pragma unroll
-        for (int k = 0; k < DET_MAX_CAND / DET_SELECT_THREADS; k++)
-            if (tid + k * DET_SELECT_THREADS < n && whole(k) >= from && whole(k) < limit)
-                S.list[atomicAdd(&S.members, 1)] = whole(k);
-        if (tid < DET_BLOCK / 32)
-            S.far[tid] = 0u;
+        for (int k = 0; k < KEYS; k++)
+            if (tid + k * DET_SELECT_THREADS < n && whole(k) >= a && whole(k) < limit)
+                S.list[atomicAdd(&S.hist[(int)((whole(k) - a) >> shift)], 1)] = whole(k);
         __syncthreads();
-        const int M = S.members; /* 1 .. DET_BLOCK */
-        from = limit;
-        left -= M;
-        int2 me = make_int2(0, 0);
-        int at = 0, cell = 0;
-        if (tid < M) {
-            const unsigned long long mine = S.list[tid];
-            me = __ldca(cxy + (int)(mine & 8191ull));
-            for (int j = 0; j < M; j++)
-                at += S.list[j] < mine;
-            S.xy[at] = me;
-            cell = ((me.y - q.g.y0) / q.gs) * q.gw + (me.x - q.g.ax) / q.gs;
-            if (!det_far(q, S.head, S.next, S.tx, S.ty, me.x, me.y))
-                atomicOr(&S.far[at >> 5], 1u << (at & 31));
+        if (tid < members) {
+            const unsigned long long k = S.list[tid];
+            const int bin = (int)((k - a) >> shift), end = S.hist[bin];
+            int at = bin ? S.hist[bin - 1] : 0;
+            for (int j = at, e = end; j < e; j++)
+                at += S.list[j] < k;
+            S.order[at] = k;
         }
+        __syncthreads();
+        /* of them, those clear of every corner taken */
+        int2 me = make_int2(0, 0);
+        bool clear = false;
+        if (tid < members) {
+            me = __ldca(cxy + (int)(S.order[tid] & 8191ull));
+            clear = det_far(q, S.head, S.next, S.tx, S.ty, me.x, me.y);
+        }
+        const unsigned bal = __ballot_sync(VTG_FULL, clear);
+        if (lane == 0)
+            S.wsum[warp] = __popc(bal);
+        __syncthreads();
+        const int wc = S.wsum[lane];
+        const int M = __reduce_add_sync(VTG_FULL, wc), slot = __reduce_add_sync(VTG_FULL, lane < warp ? wc : 0) +
+                                                              __popc(bal & ((1u << lane) - 1u));
+        __syncthreads();
+        if (M > DET_BLOCK) { /* only when size > DET_BLOCK */
+            size = max(DET_BLOCK, size / 2);
+            continue;
+        }
+        from = limit;
+        left -= members;
+        /* the next block: three quarters of a full one clear, by this one's share */
+        size = min(DET_SELECT_THREADS, max(DET_BLOCK, DET_BLOCK * 3 / 4 * members / max(M, 1)));
+        if (clear)
+            S.xy[slot] = me;
         __syncthreads();
         /* the conflicts: thread (i, part) compares candidate i with 64 of those before it */
         {
@@ -527,11 +568,11 @@ __global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, co
                 for (int e = 0; e < k; e++)
                     hit |= S.mask[e][i] & __shfl_sync(VTG_FULL, got, e);
                 const unsigned own = S.mask[k][i];
-                unsigned open = __ballot_sync(VTG_FULL, i < M && !hit && !((S.far[k] >> lane) & 1u)), yes = 0u;
+                unsigned open = __ballot_sync(VTG_FULL, i < M && !hit), yes = 0u;
                 while (open) {
-                    const bool mine = (open >> lane) & 1u;
-                    const bool now = mine && !(own & (open | yes));
-                    const bool out = mine && (own & yes);
+                    const bool here = (open >> lane) & 1u;
+                    const bool now = here && !(own & (open | yes));
+                    const bool out = here && (own & yes);
                     yes |= __ballot_sync(VTG_FULL, now);
                     open &= ~__ballot_sync(VTG_FULL, now || out);
                 }
@@ -546,17 +587,20 @@ __global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, co
 #pragma unroll
         for (int k = 0; k < DET_BLOCK / 32; k++) {
             const int c = __popc(S.got[k]);
-            rank += k < (at >> 5) ? c : 0;
+            rank += k < (tid >> 5) ? c : 0;
             total += c;
         }
-        rank += __popc(S.got[at >> 5] & ((1u << (at & 31)) - 1u));
-        if (tid < M && ((S.got[at >> 5] >> (at & 31)) & 1u) && taken + rank < q.max) {
-            const int t = taken + rank;
-            S.tx[t] = me.x;
-            S.ty[t] = me.y;
-            xs[t] = (float)me.x;
-            ys[t] = (float)me.y;
-            S.next[t] = atomicExch(&S.head[cell], t);
+        if (tid < M) {
+            rank += __popc(S.got[tid >> 5] & ((1u << lane) - 1u));
+            if (((S.got[tid >> 5] >> lane) & 1u) && taken + rank < q.max) {
+                const int t = taken + rank;
+                const int2 c = S.xy[tid];
+                S.tx[t] = c.x;
+                S.ty[t] = c.y;
+                xs[t] = (float)c.x;
+                ys[t] = (float)c.y;
+                S.next[t] = atomicExch(&S.head[((c.y - q.g.y0) / q.gs) * q.gw + (c.x - q.g.ax) / q.gs], t);
+            }
         }
         taken = min(taken + total, q.max);
         __syncthreads();
