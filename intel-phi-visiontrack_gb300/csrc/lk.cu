@@ -661,30 +661,32 @@ __device__ __forceinline__ void lk_track(const DevPyr &I, const DevPyr &J, int t
         const float lo_x = (float)(mx - bx), lo_y = (float)(my - by);
         const float hi_x = (float)(JL.w - mx - 1 - bx), hi_y = (float)(JL.h - my - 1 - by);
         float vx = 0.0f, vy = 0.0f;
-        /* the correlation at the last whole pixel sampled (none yet on this level) */
+        /* the correlation at the last whole pixel sampled, (bx + cfx, by + cfy); none yet on this level */
         float X[8];
-        int cjx = INT_MIN, cjy = INT_MIN;
+        float cfx = __int_as_float(0x7fffffff), cfy = cfx;
         for (int it = 0; it < p.max_iter; it++) {
             const float qx = (rx + gx) + vx, qy = (ry + gy) + vy; /* offsets from (bx, by) */
-            if (!(qx >= lo_x && qy >= lo_y && qx < hi_x && qy < hi_y)) { /* NaN fails it too (a NaN guess) */
-                if (L == 0) {
-                    status |= VTG_LK_OUT;
-                    valid0 = false;
+            /* A position in that pixel needs no floor, and no test of the bounds, which are whole numbers that its first
+             * position passed: its phase is q - floor, exact, in [0, 1). (A phase that rounds to 1, from just below the next
+             * pixel, takes the long way to the same sums.) */
+            float fx = qx - cfx, fy = qy - cfy;
+            if (!(fx >= 0.0f && fy >= 0.0f && fx < 1.0f && fy < 1.0f)) { /* NaN fails it: no pixel yet, or no position */
+                if (!(qx >= lo_x && qy >= lo_y && qx < hi_x && qy < hi_y)) { /* NaN fails it too (a NaN guess) */
+                    if (L == 0) {
+                        status |= VTG_LK_OUT;
+                        valid0 = false;
+                    }
+                    break;
                 }
-                break;
-            }
-            int jx, jy;
-            float fx, fy;
-            split(bx, qx, jx, fx);
-            split(by, qy, jy, fy);
-            if (jx != cjx || jy != cjy) {
-                lk_correlate<MAXH, EXACT, TS>(JL, jx, jy + dy, W, H, lane, P, tc, X);
+                cfx = floorf(qx);
+                cfy = floorf(qy);
+                fx = qx - cfx;
+                fy = qy - cfy;
+                lk_correlate<MAXH, EXACT, TS>(JL, bx + (int)cfx, by + (int)cfy + dy, W, H, lane, P, tc, X);
                 if constexpr (NW == 2)
                     pair_add(X, q, lane);
                 lk_phase_diffs(X);
                 work += LK_WORK_PASS;
-                cjx = jx;
-                cjy = jy;
             }
             const float sx = lk_at_phase(X, cx, fx, fy), sy = lk_at_phase(X + 4, cy, fx, fy);
             const float ex = __fmaf_rn(ia, sx, ib * sy), ey = __fmaf_rn(ib, sx, ic * sy);
