@@ -888,7 +888,7 @@ __device__ __forceinline__ int lk_tile_cell(const CellGrid &g, int w)
     return (col < g.cols && row < g.rows) ? row * g.cols + col : -1;
 }
 
-template <int MAXH, bool EXACT, bool PERSISTENT, int WARPS, int MINB, bool TS>
+template <int MAXH, bool EXACT, bool PERSISTENT, int WARPS, int MINB, bool TS, bool COUNT = false>
 __global__ void __launch_bounds__(WARPS * 32, MINB) lk_batch_kernel(const LkJob *__restrict__ jobs,
                                                                     const int *__restrict__ item_start, int njobs,
                                                                     int items, int chunk, LkPrm p,
@@ -945,7 +945,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) lk_batch_kernel(const LkJob 
             const int cell = tiled ? lk_tile_cell(jb.g, c) : (c < jb.g.n ? c : -1);
             if (cell >= 0)
                 lk_cell<MAXH, EXACT, TS>(*jb.I, *jb.J, jb.top, p, jb.g, jb.base_w, jb.base_h, cell, lane, jb.out,
-                                         jb.cells, ts, count);
+                                         jb.cells, ts, COUNT ? count : nullptr);
         }
         if (!PERSISTENT)
             break;
@@ -982,6 +982,15 @@ static cudaError_t lk_batch_launch(const LkJob *jobs, const int *item_start, int
         if (e2 != cudaSuccess)                                                                                         \
             return e2;                                                                                                 \
     } while (0)
+    if (count) {
+        /* counting: one shape for every tuning (a cell's work does not depend on it), so that the others carry no counters */
+        const size_t smem = sizeof(f2_t) * 16 * (MAXH / 2) * 32;
+        auto kernel = lk_batch_kernel<MAXH, EXACT, true, 16, 1, true, true>;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return e != cudaSuccess ? e
+                                : vtg_launch_k(kernel, sms, 16 * 32, smem, s, pdl, jobs, item_start, njobs, items, t.chunk, p,
+                                               counter, count, t.tiled);
+    }
     if (t.tsmem) {
         /* the template's T in shared memory: fewer registers, or more warps an SM */
         if (t.block_warps == 4)
