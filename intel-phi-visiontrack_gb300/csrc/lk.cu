@@ -850,17 +850,23 @@ __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int to
     }
 }
 
+/* A warp a cell, 2 x 2 cells a CTA: neighbours' windows overlap in L1, and a CTA of few warps leaves its place as soon as its
+ * few cells are done. A 1080p pair (build and cells, 16,200 cells), by cells a CTA: 8 x 1 0.243 ms, 4 x 2 0.242, 4 x 4 0.249,
+ * 4 x 1 0.240, 2 x 2 0.236, 2 x 1 0.240, one 0.242. */
+#define LK_CTA_CELLS 4
 template <int MAXH, bool EXACT>
-__global__ void __launch_bounds__(256, 2) lk_cells_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp,
+__global__ void __launch_bounds__(32 * LK_CTA_CELLS, 16 / LK_CTA_CELLS) lk_cells_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp,
                                                           int top, LkPrm p, CellGrid g, int base_w, int base_h,
                                                           vtg_lk_out *__restrict__ out, vtg_cell *__restrict__ cells)
 {
-    extern __shared__ f2_t s_tc[]; /* the template's T: 8 warps x (MAXH / 2) x 32 pairs */
-    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (i >= g.n)
+    extern __shared__ f2_t s_tc[]; /* the template's T: 4 warps x (MAXH / 2) x 32 pairs */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, across = (g.cols + 1) / 2;
+    const int col = 2 * ((int)blockIdx.x % across) + (warp & 1), row = 2 * ((int)blockIdx.x / across) + (warp >> 1);
+    vtg_grid_dependency_wait(); /* the pyramid, when its kernel is the one before on the stream */
+    if (col >= g.cols || row >= g.rows)
         return;
-    lk_cell<MAXH, EXACT, true>(*Ip, *Jp, top, p, g, base_w, base_h, i, lane, out, cells,
-                               s_tc + (size_t)(threadIdx.x >> 5) * (MAXH / 2) * 32);
+    lk_cell<MAXH, EXACT, true>(*Ip, *Jp, top, p, g, base_w, base_h, row * g.cols + col, lane, out, cells,
+                               s_tc + (size_t)warp * (MAXH / 2) * 32);
 }
 
 /* Many streams' cells in one launch. Work items are runs of `chunk` cells of one job; job j's items start at
@@ -1080,20 +1086,20 @@ __global__ void __launch_bounds__(256, 2) lk_points_pair_kernel(const DevPyr *__
         store_out(out + i, o, lane);
 }
 
-/* shared memory of a 256-thread single-stream CTA: its 8 warps' template intensities (at most 30 KB) */
-static constexpr size_t lk_t_bytes(int maxh) { return sizeof(f2_t) * 8 * (size_t)(maxh / 2) * 32; }
+/* shared memory of a single-stream CTA: its warps' template intensities (at most 30 KB) */
+static constexpr size_t lk_t_bytes(int maxh, int warps) { return sizeof(f2_t) * (size_t)warps * (size_t)(maxh / 2) * 32; }
 
 cudaError_t vtg_launch_cells(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, const CellGrid &g, int base_w,
                              int base_h, vtg_lk_out *out, vtg_cell *cells, cudaStream_t s)
 {
-    const int blocks = (g.n + 7) / 8;
-    if (p.H == 21)
-        lk_cells_kernel<21, true><<<blocks, 256, lk_t_bytes(21), s>>>(I, J, top, p, g, base_w, base_h, out, cells);
-    else if (p.H == 15)
-        lk_cells_kernel<15, true><<<blocks, 256, lk_t_bytes(15), s>>>(I, J, top, p, g, base_w, base_h, out, cells);
-    else
-        lk_cells_kernel<31, false><<<blocks, 256, lk_t_bytes(31), s>>>(I, J, top, p, g, base_w, base_h, out, cells);
-    return cudaGetLastError();
+    const dim3 blocks((unsigned)((g.cols + 1) / 2) * (unsigned)((g.rows + 1) / 2)), threads(32 * LK_CTA_CELLS);
+    auto launch = [&](auto kernel, int maxh) {
+        return vtg_launch_k(kernel, blocks, threads, lk_t_bytes(maxh, LK_CTA_CELLS), s, true, I, J, top, p, g, base_w, base_h, out,
+                            cells);
+    };
+    return p.H == 21   ? launch(lk_cells_kernel<21, true>, 21)
+           : p.H == 15 ? launch(lk_cells_kernel<15, true>, 15)
+                       : launch(lk_cells_kernel<31, false>, 31);
 }
 
 cudaError_t vtg_launch_points(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, int n, const float *xs,
@@ -1107,17 +1113,17 @@ cudaError_t vtg_launch_points(const DevPyr *I, const DevPyr *J, int top, const L
     if (vtg_points_pair(n, warps)) {
         const int pblocks = (n + 3) / 4;
         if (p.H <= 22)
-            lk_points_pair_kernel<11><<<pblocks, 256, lk_t_bytes(11), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
+            lk_points_pair_kernel<11><<<pblocks, 256, lk_t_bytes(11, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
         else
-            lk_points_pair_kernel<16><<<pblocks, 256, lk_t_bytes(16), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
+            lk_points_pair_kernel<16><<<pblocks, 256, lk_t_bytes(16, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
         return cudaGetLastError();
     }
     const int blocks = (n + 7) / 8;
     if (p.H == 21)
-        lk_points_kernel<21, true><<<blocks, 256, lk_t_bytes(21), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
+        lk_points_kernel<21, true><<<blocks, 256, lk_t_bytes(21, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
     else if (p.H == 15)
-        lk_points_kernel<15, true><<<blocks, 256, lk_t_bytes(15), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
+        lk_points_kernel<15, true><<<blocks, 256, lk_t_bytes(15, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
     else
-        lk_points_kernel<31, false><<<blocks, 256, lk_t_bytes(31), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
+        lk_points_kernel<31, false><<<blocks, 256, lk_t_bytes(31, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
     return cudaGetLastError();
 }
