@@ -820,7 +820,8 @@ __device__ __forceinline__ void lk_count(unsigned long long *count, unsigned wor
 template <int MAXH, bool EXACT, bool TS>
 __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int top, const LkPrm &p, const CellGrid &g,
                                         int base_w, int base_h, int i, int lane, vtg_lk_out *__restrict__ out,
-                                        vtg_cell *__restrict__ cells, f2_t *ts, unsigned long long *count = nullptr)
+                                        vtg_cell *__restrict__ cells, f2_t *ts, unsigned long long *count = nullptr,
+                                        int *hist = nullptr)
 {
     const int col = i % g.cols, row = i / g.cols;
     const float mx = (float)(p.W / 2 + 2), my = (float)(p.H / 2 + 2);
@@ -846,6 +847,8 @@ __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int to
             c.sigma = o.status ? 0.0f : sqrtf(o.cov_xx + o.cov_yy);
             c.pad = 0.0f;
             cells[i] = c;
+            if (hist)
+                atomicAdd(hist + vtg_still_bin(diff), 1);
         }
     }
 }
@@ -1038,6 +1041,39 @@ cudaError_t vtg_launch_lk_batch(const LkJob *jobs, const int *item_start, int nj
     return lk_batch_launch<31, false>(jobs, item_start, njobs, items, p, tune, sms, counter, s, pdl, count);
 }
 
+/* shared memory of a single-stream CTA: its warps' template intensities (at most 30 KB) */
+static constexpr size_t lk_t_bytes(int maxh, int warps) { return sizeof(f2_t) * (size_t)warps * (size_t)(maxh / 2) * 32; }
+
+/* The still picture's vectors (still.cu): one level, its descriptors by value, and the cells' differences counted. */
+__global__ void __launch_bounds__(32 * LK_CTA_CELLS, 16 / LK_CTA_CELLS) lk_still_kernel(DevLevel I, DevLevel J, LkPrm p, CellGrid g,
+                                                                                     vtg_cell *__restrict__ cells, int *hist)
+{
+    extern __shared__ f2_t s_tc[]; /* the template's T: 4 warps x 7 x 32 pairs */
+    __shared__ DevPyr s_pyr[2];    /* the walk indexes its levels */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, across = (g.cols + 1) / 2;
+    const int col = 2 * ((int)blockIdx.x % across) + (warp & 1), row = 2 * ((int)blockIdx.x / across) + (warp >> 1);
+    if (threadIdx.x == 0) {
+        s_pyr[0].l[0] = I;
+        s_pyr[1].l[0] = J;
+    }
+    __syncthreads();
+    vtg_grid_launch_dependents();
+    vtg_grid_dependency_wait(); /* the mean, when its kernel is the one before on the stream */
+    if (col >= g.cols || row >= g.rows)
+        return;
+    lk_cell<15, true, true>(s_pyr[0], s_pyr[1], 0, p, g, I.w, I.h, row * g.cols + col, lane, nullptr, cells,
+                            s_tc + (size_t)warp * 7 * 32, nullptr, hist);
+}
+
+cudaError_t vtg_launch_still_cells(const DevLevel &I, const DevLevel &J, const LkPrm &p, const CellGrid &g, vtg_cell *cells,
+                                   int *hist, cudaStream_t s)
+{
+    const unsigned blocks = (unsigned)((g.cols + 1) / 2) * (unsigned)((g.rows + 1) / 2);
+    return p.H == 15 ? vtg_launch_k(lk_still_kernel, dim3(blocks), dim3(32 * LK_CTA_CELLS), lk_t_bytes(15, LK_CTA_CELLS), s, true, I, J,
+                                    p, g, cells, hist)
+                     : cudaErrorInvalidValue;
+}
+
 template <int MAXH, bool EXACT>
 __global__ void __launch_bounds__(256, 2) lk_points_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp,
                                                         int top, LkPrm p, int n, const float *__restrict__ xs,
@@ -1086,8 +1122,6 @@ __global__ void __launch_bounds__(256, 2) lk_points_pair_kernel(const DevPyr *__
         store_out(out + i, o, lane);
 }
 
-/* shared memory of a single-stream CTA: its warps' template intensities (at most 30 KB) */
-static constexpr size_t lk_t_bytes(int maxh, int warps) { return sizeof(f2_t) * (size_t)warps * (size_t)(maxh / 2) * 32; }
 
 cudaError_t vtg_launch_cells(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, const CellGrid &g, int base_w,
                              int base_h, vtg_lk_out *out, vtg_cell *cells, cudaStream_t s)

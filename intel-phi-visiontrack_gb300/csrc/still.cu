@@ -4,14 +4,15 @@
  * Reference: still_vectors, still_decide, still_update and still_finish (src/kern/still.c:116-251), run in that order
  * once a frame (src/kern/still.h:11; src/host/m3_ref.c:272-277), the vectors skipped on the first frame.
  *
- * A frame is five launches on one stream, no host round trip:
+ * A frame is two launches on one stream, no host round trip:
  *   vectors   lk.cu's per-cell kernel: LK from the mean to the frame at every cell's centre, one level, a 15 x 15
- *             patch, 6 iterations, forward-backward 0.25 px (still.c:14-19), the cell's mean |frame - mean|;
- *   decide    three launches a thread a cell (still_decide, still.c:143-222): the noise median (a histogram of the
- *             cells' differences in 1/16 grey) and the scalars; each cell's evidence; the 3 x 3 vote, the counts,
- *             weights and states, and the drift statistics. Their FP64 work (below) is spread over every SM: GB300's
- *             FP64 rate is a small fraction of its FP32 rate, and one SM took 0.42 ms over 16,200 cells;
- *   update    a thread a pixel: m + w (f - m) as one fused multiply-add, or f where the weight is 1 (still.c:224-246).
+ *             patch, 6 iterations, forward-backward 0.25 px (still.c:14-19), the cell's mean |frame - mean|, counted in a
+ *             histogram in 1/16 grey (the caller's own cells, and the first frame's, are counted by still_hist_kernel);
+ *   decide    a CTA 8 x 4 cells: the noise median from the histogram, the limits (every CTA for itself), the evidence of
+ *             its cells and the ring around them, the 3 x 3 vote, the counts, weights and states, the mean under its cells
+ *             (still_decide, still_update: still.c:143-246), and its share of the drift statistics; the last CTA (an atomic
+ *             ticket) finishes those and the state. FP64, a small fraction of F32's rate on GB300, is left to the cells that F32
+ *             cannot decide and to that one thread.
  *
  * Exactness against the reference's long double:
  *   - the histogram, the median, the noise and its limit, the votes, the counts and the mean are exact;
@@ -32,32 +33,25 @@
 #include "vtg_ctx.h"
 #include "vtg_internal.cuh"
 
-#define STILL_BLOCK 256     /* threads a CTA, a cell each */
 #define STILL_MAX_SIDE 4096 /* up to 256 x 512 cells */
-#define STILL_HIST 256      /* HIST_BINS, src/kern/still.c:30 */
-#define STILL_MAX_BLOCKS ((STILL_MAX_SIDE / 16) * (STILL_MAX_SIDE / 8) / STILL_BLOCK)
-static_assert(STILL_BLOCK == STILL_HIST, "a thread a histogram bin");
+#define STILL_HIST VTG_STILL_BINS
+#define STILL_TX 8 /* cells a CTA of the decision */
+#define STILL_TY 4
 
 /* The decision's state across frames, its newest statistics and the launches' hand-offs, in device memory. */
 struct StillScal {
     double noise_usual;
     vtg_still_motion motion;
-    double limit;      /* this frame's difference limit */
-    int all;           /* this frame: everything moved */
-    unsigned ticket;   /* CTAs done in the current launch; 0 between launches */
+    unsigned ticket;   /* CTAs done in the decision; 0 between frames, like the sums below */
+    int tracked, moving, good;
+    unsigned long long counts;
+    unsigned long long sums[3][3]; /* the drift sums' 42-bit pieces (StillFix) added up */
     int hist[STILL_HIST];
 };
 
 /* a double-double: hi + lo, |lo| at most half an ulp of hi */
 struct DD {
     double hi, lo;
-};
-
-/* A CTA's share of the statistics: the drift sums as exact fixed-point integers, units of 2^-60. */
-struct StillPart {
-    int tracked, moving, good, pad;
-    long long counts, pad2;
-    __int128 su, sv, suu;
 };
 
 struct vtg_still {
@@ -70,12 +64,7 @@ struct vtg_still {
     float *mean;
     vtg_cell *cells;
     unsigned *count;
-    float *weight;
     StillScal *scal;
-    unsigned char *raw; /* (cols + 2) x (rows + 2): each cell's evidence, a zero border */
-    StillPart *part;
-    DevPyr *dpyr; /* [0] the mean, [1] the frame: one level each */
-    DevPyr hpyr[2];
     unsigned long long frames;
 };
 
@@ -126,7 +115,7 @@ __device__ __forceinline__ DD dd_neg(DD a) { return DD{-a.hi, -a.lo}; }
 /* Whether a good vector moved (still.c:178-182): u^2 + v^2, rounded to a 64-bit significand as the x87 rounds the
  * long double sum, greater than need = max((12 sigma)^2, px^2), which is exact (56 bits at most). Both sides are
  * canonical double-doubles (head = the double nearest the sum), so they compare as (head, tail) pairs. */
-__device__ bool still_longer(float u, float v, float sigma, float px)
+__device__ __noinline__ bool still_longer_exact(float u, float v, float sigma, float px)
 {
     const double a = (double)u * (double)u, b = (double)v * (double)v; /* exact: 48-bit products */
     double s = a + b, t = two_sum_err(a, b, s);
@@ -151,24 +140,18 @@ __device__ bool still_longer(float u, float v, float sigma, float px)
     return s > np || (s == np && t > ne);
 }
 
-__device__ __forceinline__ int warp_sum_i(int v)
+/* The same, by F32 where the two sides differ by more than F32's rounding of them (a few parts in 2^24; no square under- or
+ * overflows there). */
+__device__ __forceinline__ bool still_longer(float u, float v, float sigma, float px)
 {
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1)
-        v += __shfl_xor_sync(VTG_FULL, v, d);
-    return v;
-}
-
-__device__ __forceinline__ DD warp_sum_dd(DD v)
-{
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        DD o;
-        o.hi = __shfl_xor_sync(VTG_FULL, v.hi, d);
-        o.lo = __shfl_xor_sync(VTG_FULL, v.lo, d);
-        v = dd_add(v, o);
+    const float s = __fmaf_rn(u, u, v * v), sg = sigma * 12.0f, need = fmaxf(sg * sg, px * px);
+    if (s > 1e-30f && s < 1e30f && need > 1e-30f && need < 1e30f) {
+        if (s > need * 1.000002f)
+            return true;
+        if (s < need * 0.999998f)
+            return false;
     }
-    return v;
+    return still_longer_exact(u, v, sigma, px);
 }
 
 /* The drift sums (su += u, sv += v, suu += u^2 + v^2, still.c:206-211) exactly: each F32 u, and its square (exact
@@ -216,236 +199,228 @@ __device__ DD dd_of_fix60(__int128 v)
     const unsigned long long k = (1ull << 42) - 1ull;
     const double c0 = (double)(unsigned long long)(a & k), c1 = (double)(unsigned long long)((a >> 42) & k);
     const double c2 = (double)(unsigned long long)(a >> 84);
-    DD r = dd_add(dd_add(dd_of(ldexp(c2, 24)), dd_of(ldexp(c1, -18))), dd_of(ldexp(c0, -60)));
+    DD r = dd_add(dd_add(dd_of(c2 * 0x1p24), dd_of(c1 * 0x1p-18)), dd_of(c0 * 0x1p-60));
     return neg ? dd_neg(r) : r;
 }
 
-/* still_decide (still.c:143-222) over the whole GPU in three launches, a thread a cell; the first and the last finish
- * in whichever CTA ends last (a ticket counter, no waiting): the histogram and then the scalars, the evidence, the
- * vote with the counts, weights and states and then the statistics. */
+/* A CTA's 128-bit sum into the frame's: its 42-bit pieces, the top one signed, each added up by a 64-bit atomic (at most
+ * 131,072 cells' worth: 17 bits more). */
+__device__ __forceinline__ void still_add(unsigned long long *to, __int128 v)
+{
+    const unsigned long long k = (1ull << 42) - 1ull;
+    if (v) {
+        atomicAdd(to + 0, (unsigned long long)v & k);
+        atomicAdd(to + 1, (unsigned long long)(v >> 42) & k);
+        atomicAdd(to + 2, (unsigned long long)(long long)(v >> 84));
+    }
+}
+__device__ __forceinline__ __int128 still_sum(unsigned long long *from)
+{
+    const __int128 v = (__int128)__ldcg(from) + ((__int128)__ldcg(from + 1) << 42) + ((__int128)(long long)__ldcg(from + 2) << 84);
+    from[0] = from[1] = from[2] = 0ull; /* ready for the next frame */
+    return v;
+}
 
-/* the camera's noise: the median cell difference, in 1/16 grey (HIST_PER_GREY); then, in the last CTA, the noise,
- * its limit, the usual noise and whether everything moved */
-__global__ void __launch_bounds__(STILL_BLOCK) still_hist_kernel(StillPrm q, const vtg_cell *__restrict__ cells,
-                                                                 StillScal *sc)
+/* The cells' differences counted, where lk_still_kernel did not. */
+__global__ void __launch_bounds__(256) still_hist_kernel(int n, const vtg_cell *cells, int *hist)
 {
     __shared__ int s_hist[STILL_HIST];
-    __shared__ bool s_last;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    s_hist[tid] = 0; /* STILL_BLOCK == STILL_HIST */
+    const int i = (int)(blockIdx.x * 256 + threadIdx.x);
+    s_hist[threadIdx.x] = 0;
     __syncthreads();
-    const int i = (int)(blockIdx.x * blockDim.x) + tid;
-    if (i < q.n) {
-        const int b = (int)(cells[i].diff * 16.0f); /* diff >= 0; x 16 is exact; the cast truncates as (long) does */
-        atomicAdd(&s_hist[b < STILL_HIST - 1 ? b : STILL_HIST - 1], 1);
-    }
+    if (i < n)
+        atomicAdd(&s_hist[vtg_still_bin(cells[i].diff)], 1);
     __syncthreads();
-    if (s_hist[tid])
-        atomicAdd(&sc->hist[tid], s_hist[tid]);
-    __threadfence();
-    __syncthreads();
-    if (tid == 0)
-        s_last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last || warp != 0)
-        return;
-    __threadfence();
-    /* med = the first bin whose running count reaches n / 2, at most 255 (the reference's walk) */
-    const int half = q.n / 2;
-    int c[8], sum = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        c[j] = __ldcg(&sc->hist[8 * lane + j]);
-        sum += c[j];
-    }
-    int inc = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(VTG_FULL, inc, d);
-        if (lane >= d)
-            inc += v;
-    }
-    int run = inc - sum, first = STILL_HIST - 1;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        run += c[j];
-        if (run >= half && 8 * lane + j < first)
-            first = 8 * lane + j;
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1)
-        first = min(first, __shfl_xor_sync(VTG_FULL, first, d));
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-        sc->hist[8 * lane + j] = 0; /* ready for the next frame */
-    if (lane == 0) {
-        const double noise = (double)first / 16.0, three = noise * 3.0; /* DIFF_OVER_NOISE */
-        const double grey = (double)q.motion_grey;
-        const double limit = three > grey ? three : grey;
-        const double nu = sc->noise_usual, usual3 = nu * 3.0;
-        const double usual = usual3 > grey ? usual3 : grey;
-        const int all = q.frames >= 2 && noise > usual;
-        if (!all && q.frames >= 1)
-            sc->noise_usual = q.frames == 1 ? noise : nu + (noise - nu) / 32.0; /* NOISE_FRAMES */
-        sc->motion.diff_median = (float)noise;
-        sc->motion.diff_limit = (float)limit;
-        sc->limit = limit;
-        sc->all = all;
-        sc->ticket = 0;
-    }
+    if (s_hist[threadIdx.x])
+        atomicAdd(hist + threadIdx.x, s_hist[threadIdx.x]);
 }
 
-/* each cell's own evidence: a good vector that moved, a lost patch (LK_RESIDUAL), or a difference past the limit;
- * raw is (cols + 2) x (rows + 2) bytes whose border stays 0 */
-__global__ void __launch_bounds__(STILL_BLOCK) still_evidence_kernel(StillPrm q, const vtg_cell *__restrict__ cells,
-                                                                     const StillScal *__restrict__ sc,
-                                                                     unsigned char *__restrict__ raw)
+/* The decision and the mean (above). wide: the frame's rows may be read 16 bytes at a time. */
+__global__ void __launch_bounds__(256) still_decide_kernel(StillPrm q, vtg_cell *cells, unsigned *__restrict__ count,
+                                                           StillScal *sc, float *__restrict__ mean, int mpitch,
+                                                           const float *__restrict__ cur, int cpitch, int w, int h, bool wide)
 {
-    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= q.n)
-        return;
-    const vtg_cell c = cells[i];
-    const unsigned lk = c.state & 0xffu;
-    const bool moved = lk == 0 && still_longer(c.u, c.v, c.sigma, q.motion_px);
-    const bool failed = (lk & 4u) != 0;
-    const bool changed = (double)c.diff > sc->limit;
-    raw[(i / q.cols + 1) * (q.cols + 2) + i % q.cols + 1] = (unsigned char)(moved || failed || changed);
-}
-
-/* a cell moves when two cells of its 3 x 3 have evidence (EVIDENCE_MIN) or everything moved: its mean restarts;
- * otherwise its count grows to avg. Then the statistics, in the last CTA. */
-__global__ void __launch_bounds__(STILL_BLOCK) still_vote_kernel(StillPrm q, vtg_cell *__restrict__ cells,
-                                                                 const unsigned char *__restrict__ raw,
-                                                                 unsigned *__restrict__ count,
-                                                                 float *__restrict__ weight, StillScal *sc,
-                                                                 StillPart *__restrict__ part)
-{
-    __shared__ int s_wi[STILL_BLOCK / 32][3];
-    __shared__ long long s_cnt[STILL_BLOCK / 32];
-    __shared__ __int128 s_ws[STILL_BLOCK / 32][3];
-    __shared__ bool s_last;
+    __shared__ float s_limit, s_noise; /* exact: 16ths of grey, three times as many, or the caller's F32 */
+    __shared__ int s_all;
+    __shared__ unsigned char s_raw[STILL_TY + 2][STILL_TX + 2];
+    __shared__ float s_w[STILL_TY][STILL_TX];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int i = (int)(blockIdx.x * blockDim.x) + tid;
-    const bool all = sc->all != 0;
-    int tracked = 0, moving = 0, good = 0;
-    long long counts = 0;
-    __int128 su = 0, sv = 0, suu = 0;
-    if (i < q.n) {
-        const int wide = q.cols + 2, r = i / q.cols, col = i - r * q.cols;
-        const unsigned char *a = raw + r * wide + col;
-        const int votes = a[0] + a[1] + a[2] + a[wide] + a[wide + 1] + a[wide + 2] + a[2 * wide] + a[2 * wide + 1] +
-                          a[2 * wide + 2];
-        const bool any = votes >= 2 || all;
-        const bool own = a[wide + 1] != 0;
-        const unsigned grown = count[i] + 1u;
-        const unsigned n = any ? 1u : grown < (unsigned)q.avg ? grown : (unsigned)q.avg;
-        count[i] = n;
-        weight[i] = __fdiv_rn(1.0f, (float)n);
-        const vtg_cell c = cells[i];
-        const unsigned lk = c.state & 0xffu;
-        cells[i].state = lk | (own ? 0x100u : 0u) | (any ? 0x200u : 0u) | (n << 16);
-        tracked = lk == 0;
-        moving = any;
-        counts = n;
-        if (lk == 0 && !any) {
-            su = fix60(c.u);
-            sv = fix60(c.v);
-            suu = fix60_sq(c.u) + fix60_sq(c.v);
-            good = 1;
+    const int tiles_x = (q.cols + STILL_TX - 1) / STILL_TX;
+    const int c0 = (int)(blockIdx.x % tiles_x) * STILL_TX, r0 = (int)(blockIdx.x / tiles_x) * STILL_TY;
+    vtg_grid_dependency_wait();
+    /* the frame's and the mean's pixels on their way while the decision is made: four rows of four a thread */
+    const int x = c0 * 16 + 4 * lane;
+    const bool quad = wide && x + 4 <= w;
+    float4 fv[4], mv[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int y = r0 * 8 + 8 * k + warp;
+        if (quad && y < h) {
+            fv[k] = __ldg(reinterpret_cast<const float4 *>(cur + (size_t)y * cpitch + x));
+            mv[k] = *reinterpret_cast<const float4 *>(mean + (size_t)y * mpitch + x);
         }
     }
-    /* the CTA's share, then (in the CTA that ends last) every share: the same reduction twice */
-    for (int pass = 0; pass < 2; pass++) {
-        tracked = warp_sum_i(tracked);
-        moving = warp_sum_i(moving);
-        good = warp_sum_i(good);
+    if (warp == 0) {
+        /* med = the first bin whose running count reaches n / 2, at most 255 (the reference's walk) */
+        const int half = q.n / 2;
+        int c[8], sum = 0;
 #pragma unroll
-        for (int d = 16; d >= 1; d >>= 1)
-            counts += __shfl_xor_sync(VTG_FULL, counts, d);
+        for (int j = 0; j < 8; j++) {
+            c[j] = __ldcg(&sc->hist[8 * lane + j]);
+            sum += c[j];
+        }
+        int inc = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(VTG_FULL, inc, d);
+            inc += lane >= d ? v : 0;
+        }
+        int run = inc - sum, first = STILL_HIST - 1;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            run += c[j];
+            if (run >= half && 8 * lane + j < first)
+                first = 8 * lane + j;
+        }
+        first = __reduce_min_sync(VTG_FULL, first);
+        if (lane == 0) {
+            const float noise = (float)first * 0.0625f, three = noise * 3.0f, grey = q.motion_grey; /* DIFF_OVER_NOISE */
+            const double usual3 = sc->noise_usual * 3.0;
+            s_noise = noise;
+            s_limit = three > grey ? three : grey;
+            s_all = q.frames >= 2 && noise > grey && (double)noise > usual3; /* above the larger of the two */
+        }
+    }
+    __syncthreads();
+    /* each cell's own evidence, the ring around the CTA's cells too (outside the grid: none): a good vector that moved, a lost
+     * patch (LK_RESIDUAL), or a difference past the limit */
+    if (tid < (STILL_TY + 2) * (STILL_TX + 2)) {
+        const int a = tid / (STILL_TX + 2), b = tid - a * (STILL_TX + 2), r = r0 - 1 + a, c = c0 - 1 + b;
+        bool e = false;
+        if (r >= 0 && r < q.rows && c >= 0 && c < q.cols) {
+            const vtg_cell *p = cells + r * q.cols + c;
+            /* another CTA may store this cell's state now: its low byte stays */
+            const unsigned lk = __ldcg(&p->state) & 0xffu;
+            const bool moved = lk == 0 && still_longer(__ldcg(&p->u), __ldcg(&p->v), __ldcg(&p->sigma), q.motion_px);
+            e = moved || (lk & 4u) != 0 || __ldcg(&p->diff) > s_limit;
+        }
+        s_raw[a][b] = (unsigned char)e;
+    }
+    __syncthreads();
+    /* a cell moves when two cells of its 3 x 3 have evidence (EVIDENCE_MIN) or everything moved: its mean restarts;
+     * otherwise its count grows to avg */
+    int tracked = 0, moving = 0, good = 0, counts = 0, ci = 0;
+    if (warp == 0) {
+        const int a = lane / STILL_TX, b = lane % STILL_TX, r = r0 + a, c = c0 + b;
+        if (r < q.rows && c < q.cols) {
+            ci = r * q.cols + c;
+            int votes = 0;
+#pragma unroll
+            for (int k = 0; k < 9; k++)
+                votes += s_raw[a + k / 3][b + k % 3];
+            const bool any = votes >= 2 || s_all, own = s_raw[a + 1][b + 1] != 0;
+            const unsigned grown = count[ci] + 1u, n = any ? 1u : grown < (unsigned)q.avg ? grown : (unsigned)q.avg;
+            count[ci] = n;
+            s_w[a][b] = __fdiv_rn(1.0f, (float)n);
+            const unsigned lk = __ldcg(&cells[ci].state) & 0xffu;
+            cells[ci].state = lk | (own ? 0x100u : 0u) | (any ? 0x200u : 0u) | (n << 16);
+            tracked = lk == 0;
+            moving = any;
+            counts = (int)n;
+            good = lk == 0 && !any;
+        }
+    }
+    __syncthreads();
+    /* the mean: f where the weight is 1, else m + weight (f - m) as one fused multiply-add */
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int y = r0 * 8 + 8 * k + warp;
+        if (y >= h || x >= w)
+            continue;
+        const float wt = s_w[k][lane >> 2];
+        float *m = mean + (size_t)y * mpitch + x;
+        auto mix = [&](float f, float o) { return wt == 1.0f ? f : __fmaf_rn(f - o, wt, o); };
+        if (quad) {
+            *reinterpret_cast<float4 *>(m) = make_float4(mix(fv[k].x, mv[k].x), mix(fv[k].y, mv[k].y), mix(fv[k].z, mv[k].z),
+                                                         mix(fv[k].w, mv[k].w));
+        } else {
+            const float *f = cur + (size_t)y * cpitch + x;
+            for (int e = 0; e < 4 && x + e < w; e++)
+                m[e] = mix(__ldg(f + e), m[e]);
+        }
+    }
+    if (warp != 0)
+        return;
+    /* the CTA's share of the statistics */
+    {
+        __int128 su = 0, sv = 0, suu = 0;
+        if (good) {
+            const float u = __ldcg(&cells[ci].u), v = __ldcg(&cells[ci].v);
+            su = fix60(u);
+            sv = fix60(v);
+            suu = fix60_sq(u) + fix60_sq(v);
+        }
+        tracked = __reduce_add_sync(VTG_FULL, tracked);
+        moving = __reduce_add_sync(VTG_FULL, moving);
+        good = __reduce_add_sync(VTG_FULL, good);
+        counts = __reduce_add_sync(VTG_FULL, counts); /* 32 x 65,535 at most */
         su = warp_sum_i128(su);
         sv = warp_sum_i128(sv);
         suu = warp_sum_i128(suu);
+        if (lane < 3)
+            still_add(sc->sums[lane], lane == 0 ? su : lane == 1 ? sv : suu);
         if (lane == 0) {
-            s_wi[warp][0] = tracked;
-            s_wi[warp][1] = moving;
-            s_wi[warp][2] = good;
-            s_cnt[warp] = counts;
-            s_ws[warp][0] = su;
-            s_ws[warp][1] = sv;
-            s_ws[warp][2] = suu;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            StillPart P{};
-            for (int w = 0; w < STILL_BLOCK / 32; w++) {
-                P.tracked += s_wi[w][0];
-                P.moving += s_wi[w][1];
-                P.good += s_wi[w][2];
-                P.counts += s_cnt[w];
-                P.su += s_ws[w][0];
-                P.sv += s_ws[w][1];
-                P.suu += s_ws[w][2];
-            }
-            if (pass == 0) {
-                part[blockIdx.x] = P;
-                __threadfence();
-                s_last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
-            } else {
-                vtg_still_motion &m = sc->motion;
-                m.cols = (uint32_t)q.cols;
-                m.rows = (uint32_t)q.rows;
-                m.tracked = (uint32_t)P.tracked;
-                m.moving = (uint32_t)P.moving;
-                m.count_mean = (float)((double)P.counts / (double)q.n);
-                if (P.good > 0) {
-                    const double G = (double)P.good;
-                    const DD mu = dd_div(dd_of_fix60(P.su), G), mv = dd_div(dd_of_fix60(P.sv), G);
-                    const DD var =
-                        dd_add(dd_add(dd_div(dd_of_fix60(P.suu), G), dd_neg(dd_sqr(mu))), dd_neg(dd_sqr(mv)));
-                    m.drift_u = (float)(mu.hi + mu.lo);
-                    m.drift_v = (float)(mv.hi + mv.lo);
-                    const double vv = var.hi + var.lo;
-                    m.drift_rms = vv > 0.0 ? (float)sqrt(vv) : 0.0f;
-                } else {
-                    m.drift_u = m.drift_v = m.drift_rms = 0.0f;
-                }
-                m.frames = q.frames + 1;
-                sc->ticket = 0;
-            }
-        }
-        __syncthreads();
-        if (pass == 1 || !s_last)
-            return;
-        /* the last CTA: every CTA's share, a thread a share (read through L2, where the others' stores are) */
-        __threadfence();
-        tracked = moving = good = 0;
-        counts = 0;
-        su = sv = suu = 0;
-        for (int b = tid; b < (int)gridDim.x; b += blockDim.x) {
-            const StillPart *pb = part + b;
-            tracked += __ldcg(&pb->tracked);
-            moving += __ldcg(&pb->moving);
-            good += __ldcg(&pb->good);
-            counts += __ldcg(&pb->counts);
-            const long long *w = reinterpret_cast<const long long *>(&pb->su);
-            su += ((__int128)__ldcg(w + 1) << 64) | (__int128)(unsigned long long)__ldcg(w);
-            sv += ((__int128)__ldcg(w + 3) << 64) | (__int128)(unsigned long long)__ldcg(w + 2);
-            suu += ((__int128)__ldcg(w + 5) << 64) | (__int128)(unsigned long long)__ldcg(w + 4);
+            atomicAdd(&sc->tracked, tracked);
+            atomicAdd(&sc->moving, moving);
+            atomicAdd(&sc->good, good);
+            atomicAdd(&sc->counts, (unsigned long long)counts);
         }
     }
-}
-
-/* still_update (still.c:224-246): a thread a pixel of row blockIdx.y. */
-__global__ void still_update_kernel(float *__restrict__ mean, int mpitch, const float *__restrict__ cur, int cpitch,
-                                    const float *__restrict__ weight, int w, int cols)
-{
-    const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x), y = (int)blockIdx.y;
-    if (x >= w)
+    /* the last CTA: the frame's statistics and state. A CTA takes its ticket when its share is added and it has read the
+     * state that this changes. */
+    unsigned last = 0u;
+    __threadfence();
+    __syncwarp();
+    if (lane == 0)
+        last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
+    if (!__shfl_sync(VTG_FULL, last, 0))
         return;
-    const float wt = weight[(y >> 3) * cols + (x >> 4)];
-    const float f = cur[(size_t)y * cpitch + x];
-    float *m = mean + (size_t)y * mpitch + x;
-    *m = wt == 1.0f ? f : __fmaf_rn(f - *m, wt, *m);
+    __threadfence();
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        sc->hist[8 * lane + j] = 0; /* ready for the next frame, like the sums and the ticket */
+    /* lane k: the k-th sum's mean over the good cells */
+    const int all_good = __ldcg(&sc->good);
+    const DD mine = all_good > 0 && lane < 3 ? dd_div(dd_of_fix60(still_sum(sc->sums[lane])), (double)all_good) : DD{0.0, 0.0};
+    if (all_good <= 0 && lane < 3)
+        still_sum(sc->sums[lane]);
+    const DD mv2{__shfl_sync(VTG_FULL, mine.hi, 1), __shfl_sync(VTG_FULL, mine.lo, 1)};
+    const DD muu{__shfl_sync(VTG_FULL, mine.hi, 2), __shfl_sync(VTG_FULL, mine.lo, 2)};
+    if (lane != 0)
+        return;
+    vtg_still_motion &m = sc->motion;
+    m.cols = (uint32_t)q.cols;
+    m.rows = (uint32_t)q.rows;
+    m.tracked = (uint32_t)__ldcg(&sc->tracked);
+    m.moving = (uint32_t)__ldcg(&sc->moving);
+    m.count_mean = (float)((double)__ldcg(&sc->counts) / (double)q.n);
+    m.drift_u = m.drift_v = m.drift_rms = 0.0f;
+    if (all_good > 0) {
+        const DD var = dd_add(dd_add(muu, dd_neg(dd_sqr(mine))), dd_neg(dd_sqr(mv2)));
+        m.drift_u = (float)(mine.hi + mine.lo);
+        m.drift_v = (float)(mv2.hi + mv2.lo);
+        const double vv = var.hi + var.lo;
+        m.drift_rms = vv > 0.0 ? (float)sqrt(vv) : 0.0f;
+    }
+    m.diff_median = s_noise;
+    m.diff_limit = s_limit;
+    m.frames = q.frames + 1;
+    const double nu = sc->noise_usual, noise = (double)s_noise;
+    if (!s_all && q.frames >= 1)
+        sc->noise_usual = q.frames == 1 ? noise : nu + (noise - nu) / 32.0; /* NOISE_FRAMES */
+    sc->tracked = sc->moving = sc->good = 0;
+    sc->counts = 0ull;
+    sc->ticket = 0u;
 }
 
 /* ---- the C ABI ---- */
@@ -462,7 +437,7 @@ __global__ void still_update_kernel(float *__restrict__ mean, int mpitch, const 
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 struct StillLayout {
-    size_t mean, cells, count, weight, scal, raw, part, dpyr, bytes;
+    size_t mean, cells, count, scal, bytes;
 };
 
 static bool still_cfg_ok(const vtg_still_config *c)
@@ -482,16 +457,8 @@ static StillLayout still_layout(const vtg_still_config *c)
     b += up256(sizeof(vtg_cell) * (size_t)n);
     L.count = b;
     b += up256(sizeof(unsigned) * (size_t)n);
-    L.weight = b;
-    b += up256(sizeof(float) * (size_t)n);
     L.scal = b;
     b += up256(sizeof(StillScal));
-    L.raw = b;
-    b += up256((size_t)(cols + 2) * (size_t)(rows + 2));
-    L.part = b;
-    b += up256(sizeof(StillPart) * (size_t)((n + STILL_BLOCK - 1) / STILL_BLOCK));
-    L.dpyr = b;
-    b += up256(2 * sizeof(DevPyr));
     L.bytes = b;
     return L;
 }
@@ -550,19 +517,7 @@ extern "C" int vtg_still_create(vtg_ctx *ctx, const struct vtg_still_config *c, 
     s->mean = (float *)(s->mem + L.mean);
     s->cells = (vtg_cell *)(s->mem + L.cells);
     s->count = (unsigned *)(s->mem + L.count);
-    s->weight = (float *)(s->mem + L.weight);
     s->scal = (StillScal *)(s->mem + L.scal);
-    s->raw = (unsigned char *)(s->mem + L.raw);
-    s->part = (StillPart *)(s->mem + L.part);
-    s->dpyr = (DevPyr *)(s->mem + L.dpyr);
-    for (int k = 0; k < 2; k++) {
-        s->hpyr[k] = DevPyr{};
-        s->hpyr[k].levels = 1;
-        s->hpyr[k].l[0].w = c->w;
-        s->hpyr[k].l[0].h = c->h;
-    }
-    s->hpyr[0].l[0].p = s->mean;
-    s->hpyr[0].l[0].pitch = s->pitch;
     vtg_ctx_track(ctx, s->stream, true);
     *out = s;
     return VTG_OK;
@@ -591,15 +546,13 @@ extern "C" int vtg_still_frame(vtg_still *s, const float *cur, int pitch, const 
     const cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
     CU(cudaSetDevice(vtg_ctx_device(s->ctx)));
     const int w = s->c.w, h = s->c.h;
-    if (cells_in) {
+    const bool vectors = !cells_in && s->frames > 0;
+    if (cells_in)
         CU(cudaMemcpyAsync(s->cells, cells_in, sizeof(vtg_cell) * (size_t)s->n,
                            where == VTG_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
-    } else if (s->frames > 0) {
+    if (vectors) {
         /* still_vectors (still.c:116-141): the mean to the frame, one level; PATCH, LK_ITER, LK_EPS, LK_MIN_EIG,
          * LK_MAX_RESIDUAL, FB_MAX (still.c:14-19) */
-        s->hpyr[1].l[0].p = cur;
-        s->hpyr[1].l[0].pitch = pitch;
-        CU(cudaMemcpyAsync(s->dpyr, s->hpyr, sizeof(s->hpyr), cudaMemcpyHostToDevice, st));
         LkPrm p;
         p.W = 15;
         p.H = 15;
@@ -615,7 +568,10 @@ extern "C" int vtg_still_frame(vtg_still *s, const float *cur, int pitch, const 
         g.cols = s->cols;
         g.rows = s->rows;
         g.n = s->n;
-        CU(vtg_launch_cells(s->dpyr, s->dpyr + 1, 0, p, g, w, h, nullptr, s->cells, st));
+        CU(vtg_launch_still_cells(DevLevel{s->mean, w, h, s->pitch}, DevLevel{cur, w, h, pitch}, p, g, s->cells, s->scal->hist, st));
+    } else {
+        still_hist_kernel<<<(s->n + 255) / 256, 256, 0, st>>>(s->n, s->cells, s->scal->hist);
+        CU(cudaGetLastError());
     }
     StillPrm q;
     q.cols = s->cols;
@@ -625,12 +581,10 @@ extern "C" int vtg_still_frame(vtg_still *s, const float *cur, int pitch, const 
     q.motion_px = s->c.motion_px;
     q.motion_grey = s->c.motion_grey;
     q.frames = s->frames;
-    const int nb = (s->n + STILL_BLOCK - 1) / STILL_BLOCK;
-    still_hist_kernel<<<nb, STILL_BLOCK, 0, st>>>(q, s->cells, s->scal);
-    still_evidence_kernel<<<nb, STILL_BLOCK, 0, st>>>(q, s->cells, s->scal, s->raw);
-    still_vote_kernel<<<nb, STILL_BLOCK, 0, st>>>(q, s->cells, s->raw, s->count, s->weight, s->scal, s->part);
-    still_update_kernel<<<dim3((w + 255) / 256, h), 256, 0, st>>>(s->mean, s->pitch, cur, pitch, s->weight, w,
-                                                                  s->cols);
+    const bool wide = (((uintptr_t)cur | (sizeof(float) * (uintptr_t)pitch)) & 15) == 0;
+    const int tiles = ((s->cols + STILL_TX - 1) / STILL_TX) * ((s->rows + STILL_TY - 1) / STILL_TY);
+    CU(vtg_launch_k(still_decide_kernel, dim3(tiles), dim3(256), 0, st, true, q, s->cells, s->count, s->scal, s->mean, s->pitch, cur,
+                    pitch, w, h, wide));
     CU(cudaGetLastError());
     s->frames++; /* still_finish (still.c:248-251) */
     return VTG_OK;

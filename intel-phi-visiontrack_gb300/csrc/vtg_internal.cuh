@@ -97,6 +97,16 @@ cudaError_t vtg_launch_pyramid_opts(const uint8_t *frame, int stride, int w, int
                                     const int *pitches, int nlevels, int opts, uint32_t *mm, cudaStream_t s);
 cudaError_t vtg_launch_cells(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, const CellGrid &g, int base_w,
                              int base_h, vtg_lk_out *out, vtg_cell *cells, cudaStream_t s);
+/* The still picture's vectors: per-cell flow over one level (15 x 15 patch), each cell's difference counted in hist (256
+ * bins of 1/16 grey). Lets the next launch start early: it runs griddepcontrol.wait before it reads the cells. */
+#define VTG_STILL_BINS 256 /* HIST_BINS, src/kern/still.c:30 */
+__device__ __forceinline__ int vtg_still_bin(float diff)
+{
+    const int b = (int)(diff * 16.0f); /* diff >= 0; x 16 is exact; the cast truncates as (long) does */
+    return min(max(b, 0), VTG_STILL_BINS - 1);
+}
+cudaError_t vtg_launch_still_cells(const DevLevel &I, const DevLevel &J, const LkPrm &p, const CellGrid &g, vtg_cell *cells,
+                                   int *hist, cudaStream_t s);
 int vtg_pyr_tiles(int w, int h, int level);
 /* Blocks of the fused launch that makes levels 0 .. 3 of a w x h frame at once. */
 int vtg_pyr_fused_tiles(int w, int h);
