@@ -2,7 +2,8 @@
  *
  * A batch step takes one new frame for each of n trackers (uneven sizes and cell counts) and runs, on one CUDA
  * stream:
- *   - the pyramids of all n frames, one launch per level for all of them (pyr_batch_kernel, a tile table per level);
+ *   - the pyramids of all n frames: levels 0 to 3 in one launch (pyr_fused_batch_kernel), then one per level for all of
+ *     them (pyr_batch_kernel), a tile table per launch;
  *   - the per-cell flow of all n streams in one LK launch (lk_batch_kernel): work items of `chunk` cells of one
  *     stream, taken from a device counter by a persistent grid of warps, so short and long streams balance.
  * The step's tables (per-frame level pointers, tile offsets, per-stream cell grids, item offsets) are prepared once
@@ -44,13 +45,14 @@ struct BatchSlot {
     std::vector<uint8_t *> h_dst;
     std::vector<int> h_stride, h_w, h_h;
     std::string key; /* the size mix, for the tuning cache */
-    /* frames under build options: their level 0 is made by launches of their own before the batched pyramid */
+    /* frames under build options: their levels 0 to 3 are made by launches of their own before the batched pyramid */
     struct Input {
         const uint8_t *src;
         int stride, w, h, opts;
         uint32_t *mm;
-        float *l0;
-        int pitch0;
+        int levels;
+        float *lv[4];
+        int pitch[4];
     };
     std::vector<Input> inputs;
     cudaGraphExec_t graph;
@@ -223,14 +225,19 @@ extern "C" int vtg_batch_prepare(vtg_batch *b, int slot, int n, vtg_tracker *con
         p.h = h;
         p.levels = t->levels;
         p.opts = t->build_opts;
-        if (p.opts)
-            sl.inputs.push_back({p.src, p.stride, w, h, p.opts, t->d_mm + (size_t)cur * VTG_MM_WORDS,
-                                 t->sets[cur] + t->loff[0], t->lpitch[0]});
         for (int L = 0; L < VTG_MAX_LEVELS; L++) {
             p.lv[L] = L < t->levels ? t->sets[cur] + t->loff[L] : nullptr;
             p.pitch[L] = t->lpitch[L];
             p.lw[L] = t->lw[L];
             p.lh[L] = t->lh[L];
+        }
+        if (p.opts) {
+            BatchSlot::Input in = {p.src, p.stride, w, h, p.opts, t->d_mm + (size_t)cur * VTG_MM_WORDS, t->levels, {}, {}};
+            for (int L = 0; L < 4; L++) {
+                in.lv[L] = p.lv[L];
+                in.pitch[L] = p.pitch[L];
+            }
+            sl.inputs.push_back(in);
         }
         max_levels = std::max(max_levels, t->levels);
         const int fl = (int)t->cfg.flow_level;
@@ -321,11 +328,10 @@ static int launch_slot(vtg_batch *b, BatchSlot &sl, cudaStream_t s, int nwait = 
     for (int k = 0; k < nwait; k++)
         CU(cudaStreamWaitEvent(s, (cudaEvent_t)wait[k], 0));
     for (const BatchSlot::Input &in : sl.inputs)
-        CU(vtg_launch_build_input(in.src, in.stride, in.w, in.h, in.opts, in.mm, in.l0, in.pitch0, s));
+        CU(vtg_launch_build_input(in.src, in.stride, in.w, in.h, in.opts, in.mm, in.lv, in.pitch, in.levels, s));
     /* the pyramid's levels and the LK launch as a chain of programmatic dependents: each starts as the one before
      * drains; the last pyramid launch zeroes the LK launch's work counter */
-    CU(vtg_launch_pyramid_batch(sl.d_pyr, sl.d_tiles, sl.tiles, sl.njobs, sl.max_levels, s, sl.d_counter, true,
-                                sl.inputs.empty()));
+    CU(vtg_launch_pyramid_batch(sl.d_pyr, sl.d_tiles, sl.tiles, sl.njobs, sl.max_levels, s, sl.d_counter, true));
     /* what only the LK launch must wait for (earlier reads of the result buffers it writes) */
     for (int k = 0; k < nwait_lk; k++)
         CU(cudaStreamWaitEvent(s, (cudaEvent_t)wait_lk[k], 0));
@@ -575,9 +581,8 @@ extern "C" int vtg_batch_profile(vtg_batch *b, int slot, int reps, float *pyr_ms
             CU(cudaMemcpy2DAsync(sl.h_dst[k], (size_t)sl.h_w[k], sl.h_src[k], (size_t)sl.h_stride[k], (size_t)sl.h_w[k],
                                  (size_t)sl.h_h[k], cudaMemcpyHostToDevice, b->stream));
         for (const BatchSlot::Input &in : sl.inputs)
-            CU(vtg_launch_build_input(in.src, in.stride, in.w, in.h, in.opts, in.mm, in.l0, in.pitch0, b->stream));
-        CU(vtg_launch_pyramid_batch(sl.d_pyr, sl.d_tiles, sl.tiles, sl.njobs, sl.max_levels, b->stream, nullptr, false,
-                                    sl.inputs.empty()));
+            CU(vtg_launch_build_input(in.src, in.stride, in.w, in.h, in.opts, in.mm, in.lv, in.pitch, in.levels, b->stream));
+        CU(vtg_launch_pyramid_batch(sl.d_pyr, sl.d_tiles, sl.tiles, sl.njobs, sl.max_levels, b->stream));
         CU(cudaMemsetAsync(sl.d_counter, 0, sizeof(int), b->stream));
         CU(cudaEventRecord(e[1], b->stream));
         CU(vtg_launch_lk_batch(sl.d_lk, sl.d_items, sl.njobs, sl.items, sl.prm, t, b->sms, sl.d_counter, b->stream));

@@ -6,12 +6,13 @@
  * reading a replicated border. Every value is a whole number below 2^24, so the reference's F32 sums are exact; here
  * they are int32 sums, the border is a clamped index, and the results are the same bits.
  *
- * Levels 0 to 3 in one launch (pyr_fused_kernel, pyr_fused_batch_kernel): a CTA reads its block's bytes once and
- * reduces level by level in shared memory, halos included (below). Levels from 4 on, and level 1 when level 0 came
- * from tk_build's input steps, take one launch per level (pyr_reduce_kernel, pyr_batch_kernel): a CTA of 256 threads
- * makes a 64 x 16 tile of its output level from a 132 x 36 source tile staged in shared memory, the vertical pass over
- * the staged rows, the horizontal pass over the vertical sums, as the reference's vert5 / shift8 do. */
+ * Levels 0 to 3 in one launch (pyr_fused_kernel, pyr_fused_batch_kernel; pyr_input_kernel where tk_build's input steps make
+ * level 0): a CTA reads its block's bytes once and reduces level by level in shared memory, halos included (below). Levels
+ * from 4 on take one launch per level (pyr_reduce_kernel, pyr_batch_kernel): a CTA of 256 threads makes a 64 x 16 tile of
+ * its output level from a 136 x 36 source tile staged in shared memory, the vertical pass over the staged rows, the
+ * horizontal pass over the vertical sums, as the reference's vert5 / shift8 do. */
 #include <math.h>
+#include <stddef.h>
 
 #include "vtg_internal.cuh"
 #include "x87.cuh"
@@ -19,13 +20,10 @@
 #define RT_X 64 /* output tile */
 #define RT_Y 16
 #define RS_Y (2 * RT_Y + 4) /* source rows of a tile: two each side */
-/* Staged columns. A tile's source columns are 2 ox - 2 .. 2 ox + 129; staging starts 16-byte aligned before them:
- * bytes from 2 ox - 16 (160 of them), F32 values from 2 ox - 4 (136). Column k of the vertical sums is source column
- * 2 ox - 4 + k in both. */
-#define SB_X 160
+/* Staged columns: a tile's source columns are 2 ox - 2 .. 2 ox + 129; staging starts 16-byte aligned before them, at 2 ox - 4
+ * (136 values). Column k of the vertical sums is source column 2 ox - 4 + k. */
 #define SF_X 136
-#define SF_P 140 /* int row pitch of staged F32 values and of the vertical sums: 16-byte aligned rows */
-#define PK_G (SF_X / 4) /* four-column groups of vertical sums in a row (the byte path's packed words) */
+#define SF_P 140 /* row pitch of staged values and of the vertical sums: 16-byte aligned rows */
 
 /* A whole number 0 <= v < 2^23 as a float without a conversion instruction: the bits of 2^23 + v, less 2^23. */
 __device__ __forceinline__ float small_int_to_float(int v)
@@ -40,144 +38,42 @@ __device__ __forceinline__ float q6_of(uint32_t w, int e)
     return __fmaf_rn(__int_as_float((int)__byte_perm(w, 0x4Bu, 0x4550u + (unsigned)e)), 64.0f, -536870912.0f);
 }
 
-/* One 64 x 16 tile of the output level at (ox, oy). With FROM_U8 the source is the frame's bytes (rows `spitch`
- * bytes apart), level 0 (byte x 64) is written from the same staged bytes, and the sums run on the bytes:
- * (64 h + 128) >> 8 = (h + 2) >> 2 exactly. Otherwise the source is level L - 1 (F32 Q6, whole numbers) and the result
- * is (h + 128) >> 8. vec: the source rows may be read 16 bytes at a time (base and pitch 16-byte aligned). dst may be
- * NULL (level 0 only). Staging reads whole 16-byte chunks inside the row and clamps the chunks that reach past an
- * edge element by element, so every read is inside the plane and the border is the reference's replicated edge. */
-template <bool FROM_U8>
-__device__ __forceinline__ void reduce_tile(const void *__restrict__ src_, int sw, int sh, int spitch, bool vec,
-                                            float *__restrict__ l0, int l0pitch, float *__restrict__ dst, int dw, int dh,
-                                            int dpitch, int ox, int oy, uint8_t (*s_b)[SB_X], int (*s_f)[SF_P],
-                                            int (*s_v)[SF_P])
+/* One 64 x 16 tile of the output level at (ox, oy) from level L - 1 (F32 Q6, whole numbers), (h + 128) >> 8. The source's base and
+ * pitch are 16-byte aligned. Staging reads whole 16-byte chunks inside the row and clamps the chunks that reach past an edge
+ * element by element, so every read is inside the plane and the border is the reference's replicated edge. */
+__device__ __forceinline__ void reduce_tile(const float *src, int sw, int sh, int spitch, float *__restrict__ dst, int dw, int dh,
+                                            int dpitch, int ox, int oy, float (*s_f)[SF_P], float (*s_v)[SF_P])
 {
     const int tid = threadIdx.x;
     const int sy0 = 2 * oy - 2;
-    if (FROM_U8) {
-        const uint8_t *src = (const uint8_t *)src_;
-        const int gx0 = 2 * ox - 16;
-        for (int i = tid; i < RS_Y * (SB_X / 16); i += blockDim.x) {
-            const int r = i / (SB_X / 16), k = i - r * (SB_X / 16);
-            const int gy = min(max(sy0 + r, 0), sh - 1), gx = gx0 + 16 * k;
-            const uint8_t *row = src + (size_t)gy * spitch;
-            uint4 v;
-            if (vec && gx >= 0 && gx + 16 <= sw) {
-                v = __ldg(reinterpret_cast<const uint4 *>(row + gx));
-            } else {
-                uint32_t w[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    uint32_t x = 0;
-#pragma unroll
-                    for (int e = 0; e < 4; e++)
-                        x |= (uint32_t)__ldg(row + min(max(gx + 4 * q + e, 0), sw - 1)) << (8 * e);
-                    w[q] = x;
-                }
-                v = make_uint4(w[0], w[1], w[2], w[3]);
+                    const int gx0 = 2 * ox - 4;
+            for (int i = tid; i < RS_Y * (SF_X / 4); i += blockDim.x) {
+                const int r = i / (SF_X / 4), k = i - r * (SF_X / 4);
+                const int gy = min(max(sy0 + r, 0), sh - 1), gx = gx0 + 4 * k;
+                const float *row = src + (size_t)gy * spitch;
+                float4 v;
+                if (gx >= 0 && gx + 4 <= sw)
+                    v = __ldg(reinterpret_cast<const float4 *>(row + gx));
+                else
+                    v = make_float4(__ldg(row + min(max(gx, 0), sw - 1)), __ldg(row + min(max(gx + 1, 0), sw - 1)),
+                                    __ldg(row + min(max(gx + 2, 0), sw - 1)), __ldg(row + min(max(gx + 3, 0), sw - 1)));
+                *reinterpret_cast<float4 *>(&s_f[r][4 * k]) = v;
             }
-            *reinterpret_cast<uint4 *>(&s_b[r][16 * k]) = v;
-        }
-        __syncthreads();
-        /* level 0: rows 2 oy .. 2 oy + 31, columns 2 ox .. 2 ox + 127 (staged columns 16 .. 143), four a thread */
-        for (int i = tid; i < 2 * RT_Y * (2 * RT_X / 4); i += blockDim.x) {
-            const int r = i / (2 * RT_X / 4), g = i - r * (2 * RT_X / 4);
-            const int gy = 2 * oy + r, gx = 2 * ox + 4 * g;
-            if (gy >= sh || gx >= sw)
-                continue;
-            const uint32_t w = *reinterpret_cast<const uint32_t *>(&s_b[r + 2][16 + 4 * g]);
-            const float4 f = make_float4(q6_of(w, 0), q6_of(w, 1), q6_of(w, 2), q6_of(w, 3));
-            float *d = l0 + (size_t)gy * l0pitch + gx;
-            if (gx + 4 <= sw) {
-                *reinterpret_cast<float4 *>(d) = f;
-            } else {
-                d[0] = f.x;
-                if (gx + 1 < sw)
-                    d[1] = f.y;
-                if (gx + 2 < sw)
-                    d[2] = f.z;
+            __syncthreads();
+            for (int i = tid; i < RT_Y * (SF_X / 4); i += blockDim.x) {
+                const int r = i / (SF_X / 4), g = i - r * (SF_X / 4);
+                /* F32 as the reference sums: whole numbers below 2^24, so every sum is exact */
+                float4 t[5];
+    #pragma unroll
+                for (int q = 0; q < 5; q++)
+                    t[q] = *reinterpret_cast<const float4 *>(&s_f[2 * r + q][4 * g]);
+                float4 o;
+                o.x = t[0].x + t[4].x + 4.0f * (t[1].x + t[3].x) + 6.0f * t[2].x;
+                o.y = t[0].y + t[4].y + 4.0f * (t[1].y + t[3].y) + 6.0f * t[2].y;
+                o.z = t[0].z + t[4].z + 4.0f * (t[1].z + t[3].z) + 6.0f * t[2].z;
+                o.w = t[0].w + t[4].w + 4.0f * (t[1].w + t[3].w) + 6.0f * t[2].w;
+                *reinterpret_cast<float4 *>(&s_v[r][4 * g]) = o;
             }
-        }
-        if (!dst)
-            return;
-        /* vertical sums of staged byte columns 12 .. 147 (source 2 ox - 4 ..), four columns a thread, two to a word:
-         * group g's even columns in the 16-bit halves of E_g, its odd columns in O_g. A sum is at most 16 x 255 =
-         * 4080, so whole-word adds never carry from one half into the other. */
-        uint32_t *s_e = reinterpret_cast<uint32_t *>(&s_v[0][0]), *s_o = s_e + RT_Y * PK_G;
-        for (int i = tid; i < RT_Y * PK_G; i += blockDim.x) {
-            const int r = i / PK_G, g = i - r * PK_G;
-            uint32_t e[5], o[5];
-#pragma unroll
-            for (int t = 0; t < 5; t++) {
-                const uint32_t w = *reinterpret_cast<const uint32_t *>(&s_b[2 * r + t][12 + 4 * g]);
-                e[t] = w & 0x00FF00FFu;
-                o[t] = (w >> 8) & 0x00FF00FFu;
-            }
-            s_e[i] = e[0] + e[4] + 4u * (e[1] + e[3]) + 6u * e[2];
-            s_o[i] = o[0] + o[4] + 4u * (o[1] + o[3]) + 6u * o[2];
-        }
-        __syncthreads();
-        /* horizontal, two outputs a word: outputs 2m and 2m + 1 take vertical sums 4m + 2 .. 4m + 6 and 4m + 4 ..
-         * 4m + 8, i.e. the pairs (E_m hi, E_m+1 lo), (O_m hi, O_m+1 lo), E_m+1, O_m+1, (E_m+1 hi, E_m+2 lo) with
-         * weights 1, 4, 6, 4, 1. A sum is at most 16 x 4080 = 65280 in each half; (h + 2) >> 2 is at most 16320, so
-         * the mask drops exactly the bits the high half shifts into the low one. Four outputs a thread. */
-        for (int i = tid; i < RT_Y * (RT_X / 4); i += blockDim.x) {
-            const int r = i / (RT_X / 4), q = i - r * (RT_X / 4);
-            const int gy = oy + r, gx = ox + 4 * q;
-            if (gy >= dh || gx >= dw)
-                continue;
-            const uint32_t *E = s_e + r * PK_G + 2 * q, *O = s_o + r * PK_G + 2 * q;
-            uint32_t res[2];
-#pragma unroll
-            for (int p = 0; p < 2; p++) {
-                const uint32_t e1 = E[p + 1], o1 = O[p + 1];
-                const uint32_t A = __byte_perm(E[p], e1, 0x5432), B = __byte_perm(O[p], o1, 0x5432);
-                const uint32_t F = __byte_perm(e1, E[p + 2], 0x5432);
-                const uint32_t h = A + F + 4u * (B + o1) + 6u * e1;
-                res[p] = ((h + 0x00020002u) >> 2) & 0x3FFF3FFFu;
-            }
-            const float o[4] = {small_int_to_float((int)(res[0] & 0xFFFFu)), small_int_to_float((int)(res[0] >> 16)),
-                                small_int_to_float((int)(res[1] & 0xFFFFu)), small_int_to_float((int)(res[1] >> 16))};
-            float *d = dst + (size_t)gy * dpitch + gx;
-            if (gx + 4 <= dw) {
-                *reinterpret_cast<float4 *>(d) = make_float4(o[0], o[1], o[2], o[3]);
-            } else {
-                for (int e = 0; e < 4 && gx + e < dw; e++)
-                    d[e] = o[e];
-            }
-        }
-        return;
-    } else {
-        const float *src = (const float *)src_;
-        const int gx0 = 2 * ox - 4;
-        for (int i = tid; i < RS_Y * (SF_X / 4); i += blockDim.x) {
-            const int r = i / (SF_X / 4), k = i - r * (SF_X / 4);
-            const int gy = min(max(sy0 + r, 0), sh - 1), gx = gx0 + 4 * k;
-            const float *row = src + (size_t)gy * spitch;
-            float4 v;
-            if (vec && gx >= 0 && gx + 4 <= sw) /* vec: the plane and its pitch are 16-byte aligned */
-                v = __ldg(reinterpret_cast<const float4 *>(row + gx));
-            else
-                v = make_float4(__ldg(row + min(max(gx, 0), sw - 1)), __ldg(row + min(max(gx + 1, 0), sw - 1)),
-                                __ldg(row + min(max(gx + 2, 0), sw - 1)), __ldg(row + min(max(gx + 3, 0), sw - 1)));
-            *reinterpret_cast<float4 *>(&s_f[r][4 * k]) = v;
-        }
-        __syncthreads();
-        for (int i = tid; i < RT_Y * (SF_X / 4); i += blockDim.x) {
-            const int r = i / (SF_X / 4), g = i - r * (SF_X / 4);
-            /* F32 as the reference sums: whole numbers below 2^24, so every sum is exact */
-            float4 t[5];
-#pragma unroll
-            for (int q = 0; q < 5; q++)
-                t[q] = *reinterpret_cast<const float4 *>(&s_f[2 * r + q][4 * g]);
-            float4 o;
-            o.x = t[0].x + t[4].x + 4.0f * (t[1].x + t[3].x) + 6.0f * t[2].x;
-            o.y = t[0].y + t[4].y + 4.0f * (t[1].y + t[3].y) + 6.0f * t[2].y;
-            o.z = t[0].z + t[4].z + 4.0f * (t[1].z + t[3].z) + 6.0f * t[2].z;
-            o.w = t[0].w + t[4].w + 4.0f * (t[1].w + t[3].w) + 6.0f * t[2].w;
-            *reinterpret_cast<float4 *>(&s_v[r][4 * g]) = o;
-        }
-    }
     __syncthreads();
     /* horizontal: output x takes vertical sums 2 x + 2 .. 2 x + 6; four outputs a thread (sums 8 g .. 8 g + 15) */
     for (int i = tid; i < RT_Y * (RT_X / 4); i += blockDim.x) {
@@ -185,15 +81,14 @@ __device__ __forceinline__ void reduce_tile(const void *__restrict__ src_, int s
         const int gy = oy + r, gx = ox + 4 * g;
         if (gy >= dh || gx >= dw)
             continue;
-        int v[16];
+        float f[16];
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            *reinterpret_cast<int4 *>(&v[4 * q]) = *reinterpret_cast<const int4 *>(&s_v[r][8 * g + 4 * q]);
+            *reinterpret_cast<float4 *>(&f[4 * q]) = *reinterpret_cast<const float4 *>(&s_v[r][8 * g + 4 * q]);
         float o[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int c = 2 * e + 4;
-            const float *f = reinterpret_cast<const float *>(v);
             const float h = f[c - 2] + f[c + 2] + 4.0f * (f[c - 1] + f[c + 1]) + 6.0f * f[c];
             o[e] = floorf((h + 128.0f) * (1.0f / 256.0f)); /* (h + 128) >> 8, exact */
         }
@@ -207,36 +102,24 @@ __device__ __forceinline__ void reduce_tile(const void *__restrict__ src_, int s
     }
 }
 
-/* The staged source: bytes for the first launch, ints (F32 values) for the others. */
-union TileSmem {
-    __align__(16) uint8_t b[RS_Y][SB_X];
-    __align__(16) int f[RS_Y][SF_P];
+struct ReduceSmem {
+    __align__(16) float f[RS_Y][SF_P], v[RT_Y][SF_P];
 };
 
-static __device__ __forceinline__ bool aligned16(const void *p, int pitch_bytes)
-{
-    return (((uintptr_t)p | (uintptr_t)pitch_bytes) & 15) == 0;
-}
-
-template <bool FROM_U8>
-__global__ void __launch_bounds__(256) pyr_reduce_kernel(const void *__restrict__ src_, int sw, int sh, int spitch,
-                                                         float *__restrict__ l0, int l0pitch, float *__restrict__ dst,
+__global__ void __launch_bounds__(256) pyr_reduce_kernel(const float *src, int sw, int sh, int spitch, float *__restrict__ dst,
                                                          int dw, int dh, int dpitch)
 {
-    __shared__ TileSmem s_t;
-    __shared__ __align__(16) int s_v[RT_Y][SF_P];
-    reduce_tile<FROM_U8>(src_, sw, sh, spitch, aligned16(src_, FROM_U8 ? spitch : spitch * 4), l0, l0pitch, dst, dw, dh, dpitch,
-                         blockIdx.x * RT_X, blockIdx.y * RT_Y, s_t.b, s_t.f, s_v);
+    __shared__ ReduceSmem S;
+    vtg_grid_dependency_wait(); /* the level below, when launched as a dependent of its launch */
+    reduce_tile(src, sw, sh, spitch, dst, dw, dh, dpitch, blockIdx.x * RT_X, blockIdx.y * RT_Y, S.f, S.v);
 }
 
 /* Many frames at once: the launch's tiles are every job's tiles of this level, back to back; a block finds its job by
- * binary search over the tile offsets. Level 1 (with level 0) from each job's bytes, or level L from level L - 1. */
-template <bool FROM_U8>
+ * binary search over the tile offsets. */
 __global__ void __launch_bounds__(256) pyr_batch_kernel(const PyrJob *__restrict__ jobs, const int *__restrict__ start,
                                                         int njobs, int level, int *__restrict__ reset)
 {
-    __shared__ TileSmem s_t;
-    __shared__ __align__(16) int s_v[RT_Y][SF_P];
+    __shared__ ReduceSmem S;
     vtg_grid_dependency_wait(); /* the level below, when launched as a dependent of its launch */
     if (reset && blockIdx.x == 0 && threadIdx.x == 0)
         *reset = 0;
@@ -251,21 +134,10 @@ __global__ void __launch_bounds__(256) pyr_batch_kernel(const PyrJob *__restrict
     }
     const PyrJob &j = jobs[lo];
     const int t = b - __ldg(start + lo);
-    const int sw = FROM_U8 ? j.w : j.lw[level - 1], sh = FROM_U8 ? j.h : j.lh[level - 1];
-    const int dw = (sw + 1) / 2, dh = (sh + 1) / 2;
+    const int dw = j.lw[level], dh = j.lh[level];
     const int tiles_x = (dw + RT_X - 1) / RT_X;
-    const int ox = (t % tiles_x) * RT_X, oy = (t / tiles_x) * RT_Y;
-    if (FROM_U8 && j.opts) {
-        /* level 0 came from the build options' launches: level 1 reduces it like any other level */
-        if (j.levels > 1)
-            reduce_tile<false>(j.lv[0], j.w, j.h, j.pitch[0], true, nullptr, 0, j.lv[1], dw, dh, j.pitch[1], ox, oy,
-                               s_t.b, s_t.f, s_v);
-    } else if (FROM_U8)
-        reduce_tile<true>(j.src, j.w, j.h, j.stride, aligned16(j.src, j.stride), j.lv[0], j.pitch[0],
-                          j.levels > 1 ? j.lv[1] : nullptr, dw, dh, j.pitch[1], ox, oy, s_t.b, s_t.f, s_v);
-    else
-        reduce_tile<false>(j.lv[level - 1], sw, sh, j.pitch[level - 1], true, nullptr, 0, j.lv[level], dw, dh,
-                           j.pitch[level], ox, oy, s_t.b, s_t.f, s_v);
+    reduce_tile(j.lv[level - 1], j.lw[level - 1], j.lh[level - 1], j.pitch[level - 1], j.lv[level], dw, dh, j.pitch[level],
+                (t % tiles_x) * RT_X, (t / tiles_x) * RT_Y, S.f, S.v);
 }
 
 /* ---- levels 0 to 3 from the bytes in one launch ----
@@ -291,13 +163,17 @@ __global__ void __launch_bounds__(256) pyr_batch_kernel(const PyrJob *__restrict
 #define F3_R 8   /* level 3: the block, rows Y0 / 8 .. + 7 */
 #define F3_C 16  /*          columns X0 / 8 .. + 15 */
 
-struct FusedSmem {
-    __align__(16) uint8_t b[FB_R][FB_C];   /* the bytes */
-    __align__(16) uint16_t v1[F1_R][FB_C]; /* level 1's vertical sums of the bytes (at most 16 x 255) */
+struct FusedUpper {
     __align__(16) uint16_t l1[F1_R][F1_P]; /* level 1 (at most 16320) */
     __align__(16) int v2[F2_R][F1_P];      /* level 2's vertical sums of level 1 */
     __align__(16) uint16_t l2[F2_R][F2_P]; /* level 2 */
     __align__(16) int v3[F3_R][F2_P];      /* level 3's vertical sums of level 2 */
+};
+
+struct FusedSmem {
+    __align__(16) uint8_t b[FB_R][FB_C];   /* the bytes */
+    __align__(16) uint16_t v1[F1_R][FB_C]; /* level 1's vertical sums of the bytes (at most 16 x 255) */
+    FusedUpper u;
 };
 
 /* One frame of a fused launch: the bytes (rows `stride` apart), and levels 0 .. min(levels, 4) - 1. */
@@ -317,89 +193,13 @@ __device__ __forceinline__ bool fused_interior(const FusedFrame &f, int X0, int 
     return X0 >= 16 && X0 + 144 <= f.w && Y0 >= 14 && Y0 + 71 <= f.h;
 }
 
+/* Levels 1 to 3 of a block from level 1 in S.l1. */
 template <bool EDGE>
-__device__ void fused_block(const FusedFrame &f, int X0, int Y0, FusedSmem &S)
+__device__ __forceinline__ void fused_upper(const FusedFrame &f, int X0, int Y0, FusedUpper &S)
 {
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int w = f.w, h = f.h;
-    const int w1 = (w + 1) / 2, h1 = (h + 1) / 2, w2 = (w1 + 1) / 2, h2 = (h1 + 1) / 2, w3 = (w2 + 1) / 2,
+    const int w1 = (f.w + 1) / 2, h1 = (f.h + 1) / 2, w2 = (w1 + 1) / 2, h2 = (h1 + 1) / 2, w3 = (w2 + 1) / 2,
               h3 = (h2 + 1) / 2;
-    const bool vec = (((uintptr_t)f.src | (uintptr_t)f.stride) & 15) == 0;
-    /* the bytes: staged row r is frame row Y0 - 14 + r, staged column c frame column X0 - 16 + c, both clamped */
-    for (int i = tid; i < FB_R * (FB_C / 16); i += nt) {
-        const int r = i / (FB_C / 16), k = i - r * (FB_C / 16);
-        const int gy = EDGE ? min(max(Y0 - 14 + r, 0), h - 1) : Y0 - 14 + r, gx = X0 - 16 + 16 * k;
-        const uint8_t *row = f.src + (size_t)gy * f.stride;
-        uint4 v;
-        if (vec && (!EDGE || (gx >= 0 && gx + 16 <= w))) {
-            v = __ldg(reinterpret_cast<const uint4 *>(row + gx));
-        } else {
-            uint32_t q[4];
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                uint32_t x = 0;
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                    x |= (uint32_t)__ldg(row + min(max(gx + 4 * a + e, 0), w - 1)) << (8 * e);
-                q[a] = x;
-            }
-            v = make_uint4(q[0], q[1], q[2], q[3]);
-        }
-        *reinterpret_cast<uint4 *>(&S.b[r][16 * k]) = v;
-    }
-    __syncthreads();
-    /* level 0: the block's rows (staged 14 ..) and columns (staged 16 ..), four a thread */
-    for (int i = tid; i < FP_Y * (FP_X / 4); i += nt) {
-        const int r = i / (FP_X / 4), g = i - r * (FP_X / 4);
-        const int gy = Y0 + r, gx = X0 + 4 * g;
-        if (EDGE && (gy >= h || gx >= w))
-            continue;
-        const uint32_t q = *reinterpret_cast<const uint32_t *>(&S.b[r + 14][16 + 4 * g]);
-        const float4 o = make_float4(q6_of(q, 0), q6_of(q, 1), q6_of(q, 2), q6_of(q, 3));
-        float *d = f.lv[0] + (size_t)gy * f.pitch[0] + gx;
-        if (!EDGE || gx + 4 <= w) {
-            *reinterpret_cast<float4 *>(d) = o;
-        } else {
-            d[0] = o.x;
-            if (gx + 1 < w)
-                d[1] = o.y;
-            if (gx + 2 < w)
-                d[2] = o.z;
-        }
-    }
-    if (f.levels < 2)
-        return;
-    /* level 1's vertical sums: local row y (frame row of level 1 Y0 / 2 - 6 + y) takes staged rows 2 y .. 2 y + 4;
-     * four columns a thread, even and odd bytes in the 16-bit halves of two words (no half carries: at most 4080) */
-    for (int i = tid; i < F1_R * (FB_C / 4); i += nt) {
-        const int y = i / (FB_C / 4), g = i - y * (FB_C / 4);
-        uint32_t e[5], o[5];
-#pragma unroll
-        for (int t = 0; t < 5; t++) {
-            const uint32_t q = *reinterpret_cast<const uint32_t *>(&S.b[2 * y + t][4 * g]);
-            e[t] = q & 0x00FF00FFu;
-            o[t] = (q >> 8) & 0x00FF00FFu;
-        }
-        const uint32_t E = e[0] + e[4] + 4u * (e[1] + e[3]) + 6u * e[2];
-        const uint32_t O = o[0] + o[4] + 4u * (o[1] + o[3]) + 6u * o[2];
-        *reinterpret_cast<uint2 *>(&S.v1[y][4 * g]) = make_uint2((E & 0xFFFFu) | (O << 16), (E >> 16) | (O & 0xFFFF0000u));
-    }
-    __syncthreads();
-    /* level 1: local column x (frame column X0 / 2 - 6 + x) centres on staged column 2 x + 4. Two columns a thread in
-     * the halves of one word: with w_k = v1 columns 2 x + 2 + 2 k and 2 x + 3 + 2 k, column x takes (w_0 lo, w_0 hi,
-     * w_1 lo, w_1 hi, w_2 lo) and column x + 1 the same one word on. A sum is at most 16 x 4080 = 65280 a half, and
-     * (h + 2) >> 2 at most 16320, so the mask drops exactly what the high half shifts into the low one. */
-    for (int i = tid; i < F1_R * ((F1_C + 1) / 2); i += nt) {
-        const int y = i / ((F1_C + 1) / 2), x = 2 * (i - y * ((F1_C + 1) / 2));
-        const uint32_t *v = reinterpret_cast<const uint32_t *>(&S.v1[y][2 * x + 2]);
-        const uint32_t w0 = v[0], w1 = v[1], w2 = v[2], w3 = v[3];
-        const uint32_t L0 = __byte_perm(w0, w1, 0x5410), H0 = __byte_perm(w0, w1, 0x7632);
-        const uint32_t L1 = __byte_perm(w1, w2, 0x5410), H1 = __byte_perm(w1, w2, 0x7632);
-        const uint32_t L2 = __byte_perm(w2, w3, 0x5410);
-        const uint32_t hs = L0 + L2 + 4u * (H0 + H1) + 6u * L1;
-        *reinterpret_cast<uint32_t *>(&S.l1[y][x]) = ((hs + 0x00020002u) >> 2) & 0x3FFF3FFFu;
-    }
-    __syncthreads();
     /* level 1's block (local rows and columns 6 ..), four columns a thread */
     const int o1x = X0 / 2 - 6, o1y = Y0 / 2 - 6; /* level 1's local origin */
     for (int i = tid; i < (FP_Y / 2) * (FP_X / 8); i += nt) {
@@ -474,6 +274,90 @@ __device__ void fused_block(const FusedFrame &f, int X0, int Y0, FusedSmem &S)
     }
 }
 
+template <bool EDGE>
+__device__ void fused_block(const FusedFrame &f, int X0, int Y0, FusedSmem &S)
+{
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int w = f.w, h = f.h;
+    const bool vec = (((uintptr_t)f.src | (uintptr_t)f.stride) & 15) == 0;
+    /* the bytes: staged row r is frame row Y0 - 14 + r, staged column c frame column X0 - 16 + c, both clamped */
+    for (int i = tid; i < FB_R * (FB_C / 16); i += nt) {
+        const int r = i / (FB_C / 16), k = i - r * (FB_C / 16);
+        const int gy = EDGE ? min(max(Y0 - 14 + r, 0), h - 1) : Y0 - 14 + r, gx = X0 - 16 + 16 * k;
+        const uint8_t *row = f.src + (size_t)gy * f.stride;
+        uint4 v;
+        if (vec && (!EDGE || (gx >= 0 && gx + 16 <= w))) {
+            v = __ldg(reinterpret_cast<const uint4 *>(row + gx));
+        } else {
+            uint32_t q[4];
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                uint32_t x = 0;
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    x |= (uint32_t)__ldg(row + min(max(gx + 4 * a + e, 0), w - 1)) << (8 * e);
+                q[a] = x;
+            }
+            v = make_uint4(q[0], q[1], q[2], q[3]);
+        }
+        *reinterpret_cast<uint4 *>(&S.b[r][16 * k]) = v;
+    }
+    __syncthreads();
+    /* level 0: the block's rows (staged 14 ..) and columns (staged 16 ..), four a thread */
+    for (int i = tid; i < FP_Y * (FP_X / 4); i += nt) {
+        const int r = i / (FP_X / 4), g = i - r * (FP_X / 4);
+        const int gy = Y0 + r, gx = X0 + 4 * g;
+        if (EDGE && (gy >= h || gx >= w))
+            continue;
+        const uint32_t q = *reinterpret_cast<const uint32_t *>(&S.b[r + 14][16 + 4 * g]);
+        const float4 o = make_float4(q6_of(q, 0), q6_of(q, 1), q6_of(q, 2), q6_of(q, 3));
+        float *d = f.lv[0] + (size_t)gy * f.pitch[0] + gx;
+        if (!EDGE || gx + 4 <= w) {
+            *reinterpret_cast<float4 *>(d) = o;
+        } else {
+            d[0] = o.x;
+            if (gx + 1 < w)
+                d[1] = o.y;
+            if (gx + 2 < w)
+                d[2] = o.z;
+        }
+    }
+    if (f.levels < 2)
+        return;
+    /* level 1's vertical sums: local row y (frame row of level 1 Y0 / 2 - 6 + y) takes staged rows 2 y .. 2 y + 4;
+     * four columns a thread, even and odd bytes in the 16-bit halves of two words (no half carries: at most 4080) */
+    for (int i = tid; i < F1_R * (FB_C / 4); i += nt) {
+        const int y = i / (FB_C / 4), g = i - y * (FB_C / 4);
+        uint32_t e[5], o[5];
+#pragma unroll
+        for (int t = 0; t < 5; t++) {
+            const uint32_t q = *reinterpret_cast<const uint32_t *>(&S.b[2 * y + t][4 * g]);
+            e[t] = q & 0x00FF00FFu;
+            o[t] = (q >> 8) & 0x00FF00FFu;
+        }
+        const uint32_t E = e[0] + e[4] + 4u * (e[1] + e[3]) + 6u * e[2];
+        const uint32_t O = o[0] + o[4] + 4u * (o[1] + o[3]) + 6u * o[2];
+        *reinterpret_cast<uint2 *>(&S.v1[y][4 * g]) = make_uint2((E & 0xFFFFu) | (O << 16), (E >> 16) | (O & 0xFFFF0000u));
+    }
+    __syncthreads();
+    /* level 1: local column x (frame column X0 / 2 - 6 + x) centres on staged column 2 x + 4. Two columns a thread in
+     * the halves of one word: with w_k = v1 columns 2 x + 2 + 2 k and 2 x + 3 + 2 k, column x takes (w_0 lo, w_0 hi,
+     * w_1 lo, w_1 hi, w_2 lo) and column x + 1 the same one word on. A sum is at most 16 x 4080 = 65280 a half, and
+     * (h + 2) >> 2 at most 16320, so the mask drops exactly what the high half shifts into the low one. */
+    for (int i = tid; i < F1_R * ((F1_C + 1) / 2); i += nt) {
+        const int y = i / ((F1_C + 1) / 2), x = 2 * (i - y * ((F1_C + 1) / 2));
+        const uint32_t *v = reinterpret_cast<const uint32_t *>(&S.v1[y][2 * x + 2]);
+        const uint32_t w0 = v[0], w1 = v[1], w2 = v[2], w3 = v[3];
+        const uint32_t L0 = __byte_perm(w0, w1, 0x5410), H0 = __byte_perm(w0, w1, 0x7632);
+        const uint32_t L1 = __byte_perm(w1, w2, 0x5410), H1 = __byte_perm(w1, w2, 0x7632);
+        const uint32_t L2 = __byte_perm(w2, w3, 0x5410);
+        const uint32_t hs = L0 + L2 + 4u * (H0 + H1) + 6u * L1;
+        *reinterpret_cast<uint32_t *>(&S.u.l1[y][x]) = ((hs + 0x00020002u) >> 2) & 0x3FFF3FFFu;
+    }
+    __syncthreads();
+    fused_upper<EDGE>(f, X0, Y0, S.u);
+}
+
 __device__ __forceinline__ void fused_any(const FusedFrame &f, int bx, int by, FusedSmem &S)
 {
     const int X0 = bx * FP_X, Y0 = by * FP_Y;
@@ -506,6 +390,8 @@ __global__ void __launch_bounds__(256) pyr_fused_batch_kernel(const PyrJob *__re
             hi = mid;
     }
     const PyrJob &j = jobs[lo];
+    if (j.opts) /* vtg_launch_build_input made these levels */
+        return;
     FusedFrame f;
     f.src = j.src;
     f.stride = j.stride;
@@ -641,87 +527,218 @@ __global__ void __launch_bounds__(256) pyr_minmax_kernel(const uint8_t *__restri
     }
 }
 
-#define PT_X 64 /* level-0 tile of the input steps */
-#define PT_Y 16
+/* Levels 0 to 3 under the input steps in one launch, blocks as above. The bytes (rows Y0 - 16 .. Y0 + 72, columns X0 - 16 ..
+ * X0 + 143, clamped into the frame) are staged through the stretch's table (or x 64) as whole numbers; GAUSS then makes level 0
+ * over the block and the halo that level 1 needs (rows Y0 - 14 .. Y0 + 70, columns X0 - 14 .. X0 + 134) by the binomial's two
+ * passes, else the staged values are level 0. Past the frame's edge the levels read the clamped index, never the halo's own
+ * value there. A value's bit 15 keeps the table's -0, which a level-0 store without GAUSS must (the sums mask it).
+ * A 1281 x 719 frame with both steps: 13 us for this launch, where level 0 and each level above took
+ * one (27 us). */
+#define PI_R 89
+#define PI_C 160
+#define P0_R 85 /* level 0 as level 1 reads it */
+#define P0_C 149
+#define P0_P 152
+#define PI_T 512
 
-/* Level 0 under the build options, one 64 x 16 tile a CTA: the bytes mapped through the stretch's table (or x 64),
- * staged with a two-pixel clamped border, then the binomial's vertical and horizontal passes on whole numbers
- * (at most 16320 x 256, exact in int) when GAUSS. */
-template <bool CONTRAST, bool GAUSS>
-__global__ void __launch_bounds__(256) pyr_input_kernel(const uint8_t *__restrict__ src, int w, int h, int stride,
-                                                        const uint32_t *__restrict__ mm, float *__restrict__ l0,
-                                                        int pitch)
+struct InputSmem {
+    uint32_t lut[256]; /* a byte's value; bit 15: it is -0 */
+    union {
+        __align__(16) uint16_t n[PI_R][PI_C]; /* the mapped bytes */
+        FusedUpper u;                         /* once they are not needed */
+    };
+    union {
+        int v0[P0_R][P0_P + 4]; /* GAUSS: vertical sums, columns X0 - 16 .. X0 + 139 */
+        int v1[F1_R][P0_P];     /* level 1's vertical sums, columns X0 - 14 .. */
+    };
+    __align__(16) uint16_t l0[P0_R][P0_P]; /* GAUSS: level 0 (must stay last) */
+};
+
+template <bool GAUSS, bool EDGE>
+__device__ __forceinline__ void input_block(const FusedFrame &f, int X0, int Y0, InputSmem &S)
 {
-    __shared__ float s_lut[256];
-    __shared__ __align__(16) int s_n[PT_Y + 4][PT_X + 4];
-    __shared__ __align__(16) int s_v[PT_Y][PT_X + 4];
-    const int tid = threadIdx.x;
-    const int ox = blockIdx.x * PT_X, oy = blockIdx.y * PT_Y;
-    if (CONTRAST) {
-        const float g = __ldcg(reinterpret_cast<const float *>(mm) + VTG_MM_BLOCKS + 1);
-        const float o = __ldcg(reinterpret_cast<const float *>(mm) + VTG_MM_BLOCKS + 2);
-        /* the reference's x87 form rounds Q6 x gain + offset to F32 from an exact extended sum (the product has 38
-         * bits, the sum's lowest bit is at least 2^-23 and its size below 2^23); one fused multiply-add rounds the
-         * same exact value once */
-        const float v = rintf(__fmaf_rn((float)(64 * tid), g, o));
-        /* the reference's select, which keeps the -0 that rint gives a small negative value (the level's bits) */
-        s_lut[tid] = v < 0.0f ? 0.0f : v > 16320.0f ? 16320.0f : v;
-    } else {
-        s_lut[tid] = (float)(64 * tid);
-    }
-    __syncthreads();
-    if (GAUSS) {
-        for (int i = tid; i < (PT_Y + 4) * (PT_X + 4); i += blockDim.x) {
-            const int r = i / (PT_X + 4), c = i - r * (PT_X + 4);
-            const int gy = min(max(oy - 2 + r, 0), h - 1), gx = min(max(ox - 2 + c, 0), w - 1);
-            s_n[r][c] = (int)s_lut[__ldg(src + (size_t)gy * stride + gx)];
-        }
-        __syncthreads();
-        for (int i = tid; i < PT_Y * (PT_X + 4); i += blockDim.x) {
-            const int r = i / (PT_X + 4), c = i - r * (PT_X + 4);
-            s_v[r][c] = s_n[r][c] + s_n[r + 4][c] + 4 * (s_n[r + 1][c] + s_n[r + 3][c]) + 6 * s_n[r + 2][c];
-        }
-        __syncthreads();
-    }
-    for (int i = tid; i < PT_Y * (PT_X / 4); i += blockDim.x) {
-        const int r = i / (PT_X / 4), g = i - r * (PT_X / 4);
-        const int gy = oy + r, gx = ox + 4 * g;
-        if (gy >= h || gx >= w)
-            continue;
-        float o[4];
+    const int tid = threadIdx.x, w = f.w, h = f.h;
+    const bool vec = (((uintptr_t)f.src | (uintptr_t)f.stride) & 15) == 0;
+    for (int i = tid; i < PI_R * (PI_C / 16); i += PI_T) {
+        const int r = i / (PI_C / 16), k = i - r * (PI_C / 16);
+        const int gy = EDGE ? min(max(Y0 - 16 + r, 0), h - 1) : Y0 - 16 + r, gx = X0 - 16 + 16 * k;
+        const uint8_t *row = f.src + (size_t)gy * f.stride;
+        uint32_t q[4];
+        if (vec && (!EDGE || (gx >= 0 && gx + 16 <= w))) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + gx));
+            q[0] = v.x;
+            q[1] = v.y;
+            q[2] = v.z;
+            q[3] = v.w;
+        } else {
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            if (GAUSS) {
-                const int c = 4 * g + e; /* vertical sums c .. c + 4 around output column c + 2 of the staged tile */
-                const int hs = s_v[r][c] + s_v[r][c + 4] + 4 * (s_v[r][c + 1] + s_v[r][c + 3]) + 6 * s_v[r][c + 2];
-                o[e] = small_int_to_float((hs + 128) >> 8);
-            } else {
-                o[e] = s_lut[__ldg(src + (size_t)gy * stride + min(gx + e, w - 1))];
+            for (int a = 0; a < 4; a++) {
+                q[a] = 0u;
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    q[a] |= (uint32_t)__ldg(row + (EDGE ? min(max(gx + 4 * a + e, 0), w - 1) : gx + 4 * a + e)) << (8 * e);
             }
         }
-        float *d = l0 + (size_t)gy * pitch + gx;
-        if (gx + 4 <= w) {
-            *reinterpret_cast<float4 *>(d) = make_float4(o[0], o[1], o[2], o[3]);
-        } else {
-            for (int e = 0; e < 4 && gx + e < w; e++)
-                d[e] = o[e];
+        uint32_t o[8];
+#pragma unroll
+        for (int a = 0; a < 8; a++) {
+            const uint32_t two = q[a >> 1] >> (16 * (a & 1));
+            o[a] = S.lut[two & 255u] | S.lut[(two >> 8) & 255u] << 16;
         }
+        *reinterpret_cast<uint4 *>(&S.n[r][16 * k]) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4 *>(&S.n[r][16 * k + 8]) = make_uint4(o[4], o[5], o[6], o[7]);
     }
+    __syncthreads();
+    /* two columns of a row of level 0's staged values, low and high half */
+    auto l0_pair = [&](int r, int c) {
+        return GAUSS ? *reinterpret_cast<const uint32_t *>(&S.l0[r][c]) :
+                       *reinterpret_cast<const uint32_t *>(&S.n[r + 2][c + 2]) & 0x7fff7fffu;
+    };
+    if (GAUSS) {
+        for (int i = tid; i < P0_R * (P0_P + 4) / 2; i += PI_T) {
+            const int r = i / ((P0_P + 4) / 2), c = 2 * (i - r * ((P0_P + 4) / 2));
+            int a[5], b[5];
+#pragma unroll
+            for (int t = 0; t < 5; t++) {
+                const uint32_t q = *reinterpret_cast<const uint32_t *>(&S.n[r + t][c]);
+                a[t] = (int)(q & 0x7fffu);
+                b[t] = (int)((q >> 16) & 0x7fffu);
+            }
+            *reinterpret_cast<int2 *>(&S.v0[r][c]) = make_int2(tap5(a[0], a[1], a[2], a[3], a[4]), tap5(b[0], b[1], b[2], b[3], b[4]));
+        }
+        __syncthreads();
+        /* level 0's column c (frame column X0 - 14 + c) centres on vertical sum c + 2 */
+        for (int i = tid; i < P0_R * P0_P / 2; i += PI_T) {
+            const int r = i / (P0_P / 2), c = 2 * (i - r * (P0_P / 2));
+            const int2 q0 = *reinterpret_cast<const int2 *>(&S.v0[r][c]), q1 = *reinterpret_cast<const int2 *>(&S.v0[r][c + 2]),
+                       q2 = *reinterpret_cast<const int2 *>(&S.v0[r][c + 4]);
+            const int o0 = (tap5(q0.x, q0.y, q1.x, q1.y, q2.x) + 128) >> 8, o1 = (tap5(q0.y, q1.x, q1.y, q2.x, q2.y) + 128) >> 8;
+            *reinterpret_cast<uint32_t *>(&S.l0[r][c]) = (uint32_t)o0 | (uint32_t)o1 << 16;
+        }
+        __syncthreads();
+    }
+    /* level 0's block: its local rows and columns 14 .., two columns a thread */
+    for (int i = tid; i < FP_Y * (FP_X / 2); i += PI_T) {
+        const int r = i / (FP_X / 2), c = 2 * (i - r * (FP_X / 2));
+        const int gy = Y0 + r, gx = X0 + c;
+        if (EDGE && (gy >= h || gx >= w))
+            continue;
+        const uint32_t q = GAUSS ? *reinterpret_cast<const uint32_t *>(&S.l0[r + 14][c + 14])
+                                 : *reinterpret_cast<const uint32_t *>(&S.n[r + 16][c + 16]);
+        auto value = [](uint32_t u) { return __int_as_float(__float_as_int(small_int_to_float((int)(u & 0x7fffu))) | (int)((u >> 15 & 1u) << 31)); };
+        float *d = f.lv[0] + (size_t)gy * f.pitch[0] + gx;
+        if (!EDGE || gx + 2 <= w)
+            *reinterpret_cast<float2 *>(d) = make_float2(value(q & 0xffffu), value(q >> 16));
+        else
+            *d = value(q & 0xffffu);
+    }
+    if (f.levels < 2)
+        return;
+    /* level 1: its local origin is X0 / 2 - 6, Y0 / 2 - 6, level 0's X0 - 14, Y0 - 14 */
+    /* (v1 takes v0's place: nothing of v0 is read after the barrier above) */
+    for (int i = tid; i < F1_R * (P0_P / 2); i += PI_T) {
+        const int y = i / (P0_P / 2), c = 2 * (i - y * (P0_P / 2));
+        int a[5], b[5];
+#pragma unroll
+        for (int t = 0; t < 5; t++) {
+            const int r = EDGE ? min(max(2 * (Y0 / 2 - 6 + y) - 2 + t, 0), h - 1) - (Y0 - 14) : 2 * y + t;
+            const uint32_t q = l0_pair(EDGE ? min(max(r, 0), P0_R - 1) : r, c);
+            a[t] = (int)(q & 0xffffu);
+            b[t] = (int)(q >> 16);
+        }
+        *reinterpret_cast<int2 *>(&S.v1[y][c]) = make_int2(tap5(a[0], a[1], a[2], a[3], a[4]), tap5(b[0], b[1], b[2], b[3], b[4]));
+    }
+    __syncthreads();
+    for (int i = tid; i < F1_R * F1_C; i += PI_T) {
+        const int y = i / F1_C, x = i - y * F1_C;
+        int a[5];
+#pragma unroll
+        for (int t = 0; t < 5; t++) {
+            const int c = EDGE ? min(max(2 * (X0 / 2 - 6 + x) - 2 + t, 0), w - 1) - (X0 - 14) : 2 * x + t;
+            a[t] = S.v1[y][EDGE ? min(max(c, 0), P0_C - 1) : c];
+        }
+        S.u.l1[y][x] = (uint16_t)((tap5(a[0], a[1], a[2], a[3], a[4]) + 128) >> 8);
+    }
+    __syncthreads();
+    fused_upper<EDGE>(f, X0, Y0, S.u);
 }
 
-cudaError_t vtg_launch_build_input(const uint8_t *frame, int stride, int w, int h, int opts, uint32_t *mm, float *l0,
-                                   int pitch0, cudaStream_t s)
+template <bool GAUSS>
+__global__ void __launch_bounds__(PI_T) pyr_input_kernel(FusedFrame f, bool contrast, const uint32_t *mm)
+{
+    extern __shared__ __align__(16) unsigned char s_input[];
+    InputSmem &S = *reinterpret_cast<InputSmem *>(s_input);
+    const int tid = threadIdx.x;
+    vtg_grid_dependency_wait(); /* the gain and offset, when launched as the minimum and maximum's dependent */
+    if (tid < 256) {
+        float v = (float)(64 * tid);
+        if (contrast) {
+            const float g = __ldcg(reinterpret_cast<const float *>(mm) + VTG_MM_BLOCKS + 1);
+            const float o = __ldcg(reinterpret_cast<const float *>(mm) + VTG_MM_BLOCKS + 2);
+            /* the reference's x87 form rounds Q6 x gain + offset to F32 from an exact extended sum (the product has 38
+             * bits, the sum's lowest bit is at least 2^-23 and its size below 2^23); one fused multiply-add rounds the
+             * same exact value once */
+            v = rintf(__fmaf_rn(v, g, o));
+            /* the reference's select, which keeps the -0 that rint gives a small negative value (the level's bits) */
+            v = v < 0.0f ? 0.0f : v > 16320.0f ? 16320.0f : v;
+        }
+        S.lut[tid] = (uint32_t)fabsf(v) | (__float_as_uint(v) >> 31 << 15);
+    }
+    __syncthreads();
+    const int X0 = blockIdx.x * FP_X, Y0 = blockIdx.y * FP_Y;
+    if (X0 >= 16 && X0 + 144 <= f.w && Y0 >= 16 && Y0 + 73 <= f.h)
+        input_block<GAUSS, false>(f, X0, Y0, S);
+    else
+        input_block<GAUSS, true>(f, X0, Y0, S);
+}
+
+static FusedFrame fused_frame(const uint8_t *frame, int stride, int w, int h, float *const *levels, const int *pitches, int nlevels)
+{
+    FusedFrame f;
+    f.src = frame;
+    f.stride = stride;
+    f.w = w;
+    f.h = h;
+    f.levels = nlevels;
+    for (int L = 0; L < 4; L++) {
+        f.lv[L] = L < nlevels ? levels[L] : nullptr;
+        f.pitch[L] = L < nlevels ? pitches[L] : 0;
+    }
+    return f;
+}
+
+cudaError_t vtg_launch_build_input(const uint8_t *frame, int stride, int w, int h, int opts, uint32_t *mm, float *const *levels,
+                                   const int *pitches, int nlevels, cudaStream_t s)
 {
     const bool contrast = (opts & VTG_BUILD_CONTRAST) != 0, gauss = (opts & VTG_BUILD_PRE_GAUSS) != 0;
     if (contrast)
         pyr_minmax_kernel<<<min(h, VTG_MM_BLOCKS), 256, 0, s>>>(frame, w, h, stride, mm);
-    const dim3 grid((w + PT_X - 1) / PT_X, (h + PT_Y - 1) / PT_Y);
-    if (contrast && gauss)
-        pyr_input_kernel<true, true><<<grid, 256, 0, s>>>(frame, w, h, stride, mm, l0, pitch0);
-    else if (contrast)
-        pyr_input_kernel<true, false><<<grid, 256, 0, s>>>(frame, w, h, stride, mm, l0, pitch0);
-    else if (gauss)
-        pyr_input_kernel<false, true><<<grid, 256, 0, s>>>(frame, w, h, stride, mm, l0, pitch0);
+    const dim3 grid((w + FP_X - 1) / FP_X, (h + FP_Y - 1) / FP_Y);
+    auto kernel = gauss ? pyr_input_kernel<true> : pyr_input_kernel<false>;
+    const size_t smem = gauss ? sizeof(InputSmem) : offsetof(InputSmem, v1) + sizeof(InputSmem::v1);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+        e = vtg_launch_k(kernel, grid, dim3(PI_T), smem, s, contrast, fused_frame(frame, stride, w, h, levels, pitches, nlevels),
+                         contrast, (const uint32_t *)mm);
+    return e;
+}
+
+/* Levels 4 on, a launch each, as dependents of the one before. */
+static cudaError_t launch_upper_levels(int w, int h, float *const *levels, const int *pitches, int nlevels, cudaStream_t s)
+{
+    int sw = w, sh = h;
+    for (int L = 1; L < nlevels; L++) {
+        const int dw = (sw + 1) / 2, dh = (sh + 1) / 2;
+        if (L >= 4) {
+            const cudaError_t e = vtg_launch_k(pyr_reduce_kernel, dim3((dw + RT_X - 1) / RT_X, (dh + RT_Y - 1) / RT_Y), dim3(256), 0, s,
+                                               true, (const float *)levels[L - 1], sw, sh, pitches[L - 1], levels[L], dw, dh,
+                                               pitches[L]);
+            if (e != cudaSuccess)
+                return e;
+        }
+        sw = dw;
+        sh = dh;
+    }
     return cudaGetLastError();
 }
 
@@ -730,18 +747,8 @@ cudaError_t vtg_launch_pyramid_opts(const uint8_t *frame, int stride, int w, int
 {
     if (!(opts & (VTG_BUILD_CONTRAST | VTG_BUILD_PRE_GAUSS)))
         return vtg_launch_pyramid(frame, stride, w, h, levels, pitches, nlevels, s);
-    cudaError_t e = vtg_launch_build_input(frame, stride, w, h, opts, mm, levels[0], pitches[0], s);
-    int sw = w, sh = h;
-    for (int L = 1; L < nlevels && e == cudaSuccess; L++) {
-        const int dw = (sw + 1) / 2, dh = (sh + 1) / 2;
-        const dim3 grid((dw + RT_X - 1) / RT_X, (dh + RT_Y - 1) / RT_Y);
-        pyr_reduce_kernel<false><<<grid, 256, 0, s>>>(levels[L - 1], sw, sh, pitches[L - 1], nullptr, 0, levels[L], dw,
-                                                      dh, pitches[L]);
-        e = cudaGetLastError();
-        sw = dw;
-        sh = dh;
-    }
-    return e;
+    const cudaError_t e = vtg_launch_build_input(frame, stride, w, h, opts, mm, levels, pitches, nlevels, s);
+    return e != cudaSuccess ? e : launch_upper_levels(w, h, levels, pitches, nlevels, s);
 }
 
 int vtg_pyr_tiles(int w, int h, int level)
@@ -757,62 +764,28 @@ int vtg_pyr_tiles(int w, int h, int level)
 }
 
 cudaError_t vtg_launch_pyramid_batch(const PyrJob *jobs, const int *starts, const int *tiles_total, int njobs,
-                                     int max_levels, cudaStream_t s, int *reset, bool pdl, bool fused)
+                                     int max_levels, cudaStream_t s, int *reset, bool pdl)
 {
-    const int top = max_levels > 1 ? max_levels : 2;
-    int last = 1; /* the last level launched (level 1's launch always has tiles) */
-    for (int L = fused ? 4 : 1; L < top; L++)
+    int last = 3; /* the last level launched */
+    for (int L = 4; L < max_levels; L++)
         if (tiles_total[L - 1] > 0)
             last = L;
-    if (fused) {
-        /* levels 0 .. 3 of every job in one launch (row VTG_MAX_LEVELS - 1 of the tables), then levels 4 .. */
-        const cudaError_t e = vtg_launch_k(pyr_fused_batch_kernel, tiles_total[VTG_MAX_LEVELS - 1], 256, 0, s, false,
-                                           jobs, (const int *)(starts + (size_t)(VTG_MAX_LEVELS - 1) * (njobs + 1)),
-                                           njobs, last < 4 ? reset : (int *)nullptr);
-        if (e != cudaSuccess)
-            return e;
-    }
-    for (int L = fused ? 4 : 1; L < top; L++) {
-        const int tiles = tiles_total[L - 1];
-        if (tiles <= 0)
-            continue;
-        const int *st = starts + (size_t)(L - 1) * (njobs + 1);
-        int *r = L == last ? reset : nullptr;
-        const cudaError_t e = L == 1 ? vtg_launch_k(pyr_batch_kernel<true>, tiles, 256, 0, s, false, jobs, st, njobs, L, r)
-                                     : vtg_launch_k(pyr_batch_kernel<false>, tiles, 256, 0, s, pdl, jobs, st, njobs, L, r);
-        if (e != cudaSuccess)
-            return e;
-    }
-    return cudaGetLastError();
+    /* levels 0 .. 3 of every job in one launch (row VTG_MAX_LEVELS - 1 of the tables), then levels 4 .. */
+    cudaError_t e = vtg_launch_k(pyr_fused_batch_kernel, tiles_total[VTG_MAX_LEVELS - 1], 256, 0, s, false, jobs,
+                                 (const int *)(starts + (size_t)(VTG_MAX_LEVELS - 1) * (njobs + 1)), njobs,
+                                 last < 4 ? reset : (int *)nullptr);
+    for (int L = 4; L < max_levels && e == cudaSuccess; L++)
+        if (tiles_total[L - 1] > 0)
+            e = vtg_launch_k(pyr_batch_kernel, tiles_total[L - 1], 256, 0, s, pdl, jobs, (const int *)(starts + (size_t)(L - 1) * (njobs + 1)),
+                             njobs, L, L == last ? reset : (int *)nullptr);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t vtg_launch_pyramid(const uint8_t *frame, int stride, int w, int h, float *const *levels, const int *pitches,
                                int nlevels, cudaStream_t s)
 {
     /* Levels 0 .. 3 from the bytes in one launch, then one launch per further level. */
-    FusedFrame f;
-    f.src = frame;
-    f.stride = stride;
-    f.w = w;
-    f.h = h;
-    f.levels = nlevels;
-    for (int L = 0; L < 4; L++) {
-        f.lv[L] = L < nlevels ? levels[L] : nullptr;
-        f.pitch[L] = L < nlevels ? pitches[L] : 0;
-    }
-    pyr_fused_kernel<<<dim3((w + FP_X - 1) / FP_X, (h + FP_Y - 1) / FP_Y), 256, 0, s>>>(f);
-    int sw = w, sh = h;
-    for (int L = 1; L < 4 && L < nlevels; L++) {
-        sw = (sw + 1) / 2;
-        sh = (sh + 1) / 2;
-    }
-    for (int L = 4; L < nlevels; L++) {
-        const int dw = (sw + 1) / 2, dh = (sh + 1) / 2;
-        const dim3 grid((dw + RT_X - 1) / RT_X, (dh + RT_Y - 1) / RT_Y);
-        pyr_reduce_kernel<false><<<grid, 256, 0, s>>>(levels[L - 1], sw, sh, pitches[L - 1], nullptr, 0, levels[L], dw, dh,
-                                                      pitches[L]);
-        sw = dw;
-        sh = dh;
-    }
-    return cudaGetLastError();
+    pyr_fused_kernel<<<dim3((w + FP_X - 1) / FP_X, (h + FP_Y - 1) / FP_Y), 256, 0, s>>>(
+        fused_frame(frame, stride, w, h, levels, pitches, nlevels));
+    return launch_upper_levels(w, h, levels, pitches, nlevels, s);
 }

@@ -49,7 +49,7 @@ static inline int vtg_pitch(int w) { return (w + 31) & ~31; }
 #define VTG_MM_WORDS (VTG_MM_BLOCKS + 4)
 
 /* One frame's pyramid in a batched build: its bytes and its set's level planes. lw / lh: level sizes. opts: build
- * options; a job with options has its level 0 written by vtg_launch_build_input before the batched launches. */
+ * options; a job with options has its levels 0 to 3 written by vtg_launch_build_input before the batched launches. */
 struct PyrJob {
     const uint8_t *src;
     int stride, w, h, levels, opts;
@@ -88,11 +88,11 @@ static inline int vtg_lk_items(int cols, int rows, int chunk, int tiled)
 /* Launchers (pyramid.cu, lk.cu). All asynchronous on `s`; each returns a cudaError_t. */
 cudaError_t vtg_launch_pyramid(const uint8_t *frame, int stride, int w, int h, float *const *levels, const int *pitches,
                                int nlevels, cudaStream_t s);
-/* Level 0 of a frame under build options (the contrast stretch and / or the 5 x 5 binomial); `mm`: VTG_MM_WORDS words
+/* Levels 0 to 3 of a frame under build options (the contrast stretch and / or the 5 x 5 binomial); `mm`: VTG_MM_WORDS words
  * of device memory whose ticket word (mm[VTG_MM_BLOCKS]) is 0. */
-cudaError_t vtg_launch_build_input(const uint8_t *frame, int stride, int w, int h, int opts, uint32_t *mm, float *l0,
-                                   int pitch0, cudaStream_t s);
-/* The whole pyramid under build options: level 0 as above, then the reduce per level. */
+cudaError_t vtg_launch_build_input(const uint8_t *frame, int stride, int w, int h, int opts, uint32_t *mm, float *const *levels,
+                                   const int *pitches, int nlevels, cudaStream_t s);
+/* The whole pyramid under build options: levels 0 to 3 as above, then the reduce per level. */
 cudaError_t vtg_launch_pyramid_opts(const uint8_t *frame, int stride, int w, int h, float *const *levels,
                                     const int *pitches, int nlevels, int opts, uint32_t *mm, cudaStream_t s);
 cudaError_t vtg_launch_cells(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, const CellGrid &g, int base_w,
@@ -110,15 +110,13 @@ cudaError_t vtg_launch_still_cells(const DevLevel &I, const DevLevel &J, const L
 int vtg_pyr_tiles(int w, int h, int level);
 /* Blocks of the fused launch that makes levels 0 .. 3 of a w x h frame at once. */
 int vtg_pyr_fused_tiles(int w, int h);
-/* The batched pyramid: one launch per level for all jobs. With pdl, each level after the first is launched as a
- * programmatic dependent of the one before (it starts as the previous level drains and waits in griddepcontrol.wait
- * until that level's writes are visible). reset (may be NULL): a device int the last launch sets to 0, for a
- * programmatic dependent launched after it (the LK launch's work counter). fused (no job with build options): levels 0
- * .. 3 of every job in one launch, whose tiles are row VTG_MAX_LEVELS - 1 of starts / tiles_total, then a launch per
- * further level. */
+/* The batched pyramid: levels 0 to 3 of every job without build options in one launch, whose tiles are row VTG_MAX_LEVELS - 1 of
+ * starts / tiles_total, then one launch per further level for all jobs. With pdl, those are launched as programmatic
+ * dependents of the one before (each starts as the previous drains and waits in griddepcontrol.wait until that level's
+ * writes are visible). reset (may be NULL): a device int the last launch sets to 0, for a programmatic dependent launched
+ * after it (the LK launch's work counter). */
 cudaError_t vtg_launch_pyramid_batch(const PyrJob *jobs, const int *starts, const int *tiles_total, int njobs,
-                                     int max_levels, cudaStream_t s, int *reset = nullptr, bool pdl = false,
-                                     bool fused = false);
+                                     int max_levels, cudaStream_t s, int *reset = nullptr, bool pdl = false);
 /* Batched LK over jobs: items of `chunk` cells, job j's items from item_start[j]; `counter` must be 0 at launch.
  * count (NULL, or four device words): adds the launch's template builds, residual passes, window passes and
  * iterations, both walks of every cell, for the algorithmic operation count. */

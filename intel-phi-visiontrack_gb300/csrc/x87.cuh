@@ -17,7 +17,7 @@ struct X87 {
     int e;
 };
 
-/* num / den rounded to a 64-bit significand; 0 < num, den < 2^31. Long division, one quotient bit a step. */
+/* num / den rounded to a 64-bit significand; 0 < num, den < 2^31. Long division in two 32-bit digits. */
 __host__ __device__ static inline X87 x87_div(uint32_t num, uint32_t den)
 {
     uint64_t R = num, D = den;
@@ -30,20 +30,13 @@ __host__ __device__ static inline X87 x87_div(uint32_t num, uint32_t den)
         R <<= 1;
         s--;
     }
-    uint64_t m = 0;
-    for (int i = 0; i < 64; i++) { /* R < 2 D throughout */
-        m <<= 1;
-        if (R >= D) {
-            m |= 1;
-            R -= D;
-        }
-        R <<= 1;
-    }
-    const bool guard = R >= D;
-    if (guard)
-        R -= D;
+    /* floor(2^63 R / D), and its remainder: R, D < 2^32 */
+    const uint64_t q1 = (R << 31) / D, r1 = (R << 31) - q1 * D;
+    const uint64_t q0 = (r1 << 32) / D, r0 = (r1 << 32) - q0 * D;
+    const uint64_t m = (q1 << 32) + q0;
+    const bool guard = 2 * r0 >= D;
     X87 r = {m, s - 63};
-    if (guard && (R != 0 || (m & 1))) {
+    if (guard && (2 * r0 != D || (m & 1))) {
         r.m++;
         if (r.m == 0) {
             r.m = 1ull << 63;
