@@ -258,14 +258,14 @@ __global__ void __launch_bounds__(256) ncc_map_f32(const T *__restrict__ plane, 
  * row's T_w column sums, and slides ST columns to the next corner. The integers are the integral images' box sums, so
  * the scores are those of ncc_map_f32 bit for bit, and the search needs no integral images. Without SUMS they come from
  * the integral images (ncc_sums_in_map decides). */
-#define NMQ_K 4       /* corners a thread */
-#define NMQ_CORNERS 32 /* corners a CTA's side */
+#define NMQ_K 4        /* corners a thread */
+#define NMQ_CORNERS 32 /* corners a CTA across; CY (32, or 16: nmq_narrow) down */
 
 /* The window a CTA of ncc_map_f32q<ST> stages: columns (with the two values the sliding window reads past the last
  * corner's row on its last column pair), its odd pitch, and rows. */
 __host__ __device__ inline int nmq_cols(int st, int tw) { return (NMQ_CORNERS - 1) * st + tw + 2; }
 __host__ __device__ inline int nmq_pitch(int st, int tw) { return nmq_cols(st, tw) | 1; }
-__host__ __device__ inline int nmq_rows(int st, int th) { return (NMQ_CORNERS - 1) * st + th; }
+__host__ __device__ inline int nmq_rows(int st, int th, int cy) { return (cy - 1) * st + th; }
 /* the columns a CTA's corners' windows cover, and the floats of shared memory before the window: the template, later
  * eight corner rows of column sums (two int64 tables) in the same place */
 __host__ __device__ inline int nmq_sum_cols(int st, int tw) { return (NMQ_CORNERS - 1) * st + tw; }
@@ -317,36 +317,62 @@ __device__ __forceinline__ void nmq_col_slide(const float *s_img, int ip, int th
 /* With SUMS, six CTAs an SM: the sums' phase would otherwise take the registers to 48 and small templates to five CTAs
  * an SM. Without it no bound: the integral images' variant runs large templates, which shared memory already holds to
  * one or two CTAs an SM, and the bound slowed it (96 x 96 by 4 %). */
-template <typename T, int ST, bool SUMS>
-__global__ void __launch_bounds__(256, SUMS ? 6 : 1) ncc_map_f32q(const T *__restrict__ plane, int pitch, const float *__restrict__ app,
+template <typename T, int ST, bool SUMS, int CY>
+__global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q(const T *__restrict__ plane, int pitch, const float *__restrict__ app,
                                                     NccPrm p, const long long *__restrict__ S1,
                                                     const long long *__restrict__ S2, int tp, int bcols,
                                                     float *__restrict__ map_v, int *__restrict__ map_x,
                                                     int *__restrict__ map_y)
 {
-    constexpr int BC = NMQ_CORNERS * ST / NCC_CELL; /* cells a CTA's side */
+    constexpr int BC = NMQ_CORNERS * ST / NCC_CELL, BR = CY * ST / NCC_CELL; /* cells a CTA's sides */
     constexpr int PER = NCC_CELL / ST;             /* corners a cell's side */
     constexpr int M = (NMQ_K - 1) * ST + 2;        /* the sliding window */
     extern __shared__ __align__(16) float sm[];
-    __shared__ unsigned long long s_best[BC * BC];
+    __shared__ unsigned long long s_best[BC * BR];
     const int bx = blockIdx.x % bcols, by = blockIdx.x / bcols;
-    const int ccx0 = BC * bx, ccy0 = BC * by; /* the CTA's first cell column and row */
+    const int ccx0 = BC * bx, ccy0 = BR * by; /* the CTA's first cell column and row */
     const int X0 = p.x0 + ccx0 * NCC_CELL, Y0 = p.y0 + ccy0 * NCC_CELL;
-    const int iw = nmq_cols(ST, p.tw), ip = nmq_pitch(ST, p.tw), ih = nmq_rows(ST, p.th);
+    const int iw = nmq_cols(ST, p.tw), ip = nmq_pitch(ST, p.tw), ih = nmq_rows(ST, p.th, CY);
     /* a multiple of 8 floats either way: s_img stays 16-byte aligned. Without SUMS nothing takes the template's place, and
      * the launch sizes the head by the template alone (shorter than the column sums for a wide, low template). */
     float *s_app = sm, *s_img = sm + (SUMS ? nmq_head(ST, p.tw, p.th) : p.tw * p.th);
     for (int i = threadIdx.x; i < p.tw * p.th; i += blockDim.x)
         s_app[i] = app[i];
     bool small = true; /* every value this thread staged converts to the same integer in 32 bits */
-    for (int i = threadIdx.x; i < iw * ih; i += blockDim.x) {
-        const int r = i / iw, c = i - r * iw;
-        const int yy = min(Y0 + r, p.h - 1), xx = min(X0 + c, p.w - 1);
-        const float v = (float)__ldg(plane + (size_t)yy * pitch + xx);
-        s_img[r * ip + c] = v;
-        small = small && fabsf(v) < 2147483648.0f;
+    if constexpr (CY == 32) {
+        for (int i = threadIdx.x; i < iw * ih; i += blockDim.x) {
+            const int r = i / iw, c = i - r * iw;
+            const int yy = min(Y0 + r, p.h - 1), xx = min(X0 + c, p.w - 1);
+            const float v = (float)__ldg(plane + (size_t)yy * pitch + xx);
+            s_img[r * ip + c] = v;
+            small = small && fabsf(v) < 2147483648.0f;
+        }
+    } else {
+        /* few CTAs, whose wait for the picture nothing hides: a warp two rows at a time, both rows' loads in flight */
+        constexpr int CH = 4; /* 32-column chunks: nmq_narrow's windows have at most 130 columns */
+        const int lane = threadIdx.x & 31;
+        for (int r = threadIdx.x >> 5; r < ih; r += 2 * (8 * CY / 32)) {
+            T v[2][CH + 1];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const T *row = plane + (size_t)min(Y0 + r + k * (8 * CY / 32), p.h - 1) * pitch;
+#pragma unroll
+                for (int u = 0; u <= CH; u++)
+                    if (32 * u < iw)
+                        v[k][u] = __ldg(row + min(X0 + lane + 32 * u, p.w - 1));
+            }
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+#pragma unroll
+                for (int u = 0; u <= CH; u++)
+                    if (lane + 32 * u < iw && r + k * (8 * CY / 32) < ih) {
+                        const float f = (float)v[k][u];
+                        s_img[(r + k * (8 * CY / 32)) * ip + lane + 32 * u] = f;
+                        small = small && fabsf(f) < 2147483648.0f;
+                    }
+        }
     }
-    if (threadIdx.x < BC * BC)
+    if (threadIdx.x < BC * BR)
         s_best[threadIdx.x] = 0ull;
     const bool w32 = __syncthreads_and(small ? 1 : 0) != 0 || sizeof(T) == 1;
     constexpr int GROUPS = NMQ_CORNERS / NMQ_K;
@@ -406,21 +432,30 @@ __global__ void __launch_bounds__(256, SUMS ? 6 : 1) ncc_map_f32q(const T *__res
                 nmq_col_first<false>(s_img, ip, p.th, t, r1, r2);
         }
 #pragma unroll 1
-        for (int q = 0; q < NMQ_CORNERS / 8; q++) {
-            if (t < ncols)
-                for (int k = 0; k < 8; k++) {
-                    const int rb = 8 * q + k;
-                    if (rb > 0)
+        for (int q = 0; q < CY / 8; q++) {
+            auto column = [&](int k) {
+                const int rb = 8 * q + k;
+                if (rb > 0)
 #pragma unroll
-                        for (int u = 0; u < ST; u++) {
-                            if (w32)
-                                nmq_col_slide<true>(s_img, ip, p.th, t, (rb - 1) * ST + u, r1, r2);
-                            else
-                                nmq_col_slide<false>(s_img, ip, p.th, t, (rb - 1) * ST + u, r1, r2);
-                        }
-                    cs1[k * ncols + t] = r1;
-                    cs2[k * ncols + t] = r2;
+                    for (int u = 0; u < ST; u++) {
+                        if (w32)
+                            nmq_col_slide<true>(s_img, ip, p.th, t, (rb - 1) * ST + u, r1, r2);
+                        else
+                            nmq_col_slide<false>(s_img, ip, p.th, t, (rb - 1) * ST + u, r1, r2);
+                    }
+                cs1[k * ncols + t] = r1;
+                cs2[k * ncols + t] = r2;
+            };
+            if (t < ncols) {
+                if constexpr (CY == 32) {
+                    for (int k = 0; k < 8; k++)
+                        column(k);
+                } else { /* unrolled: the next rows' values on their way */
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        column(k);
                 }
+            }
             __syncthreads();
             if (b / 8 == q) {
                 const long long *c1 = cs1 + (b % 8) * ncols + a0 * ST, *c2 = cs2 + (b % 8) * ncols + a0 * ST;
@@ -460,7 +495,7 @@ __global__ void __launch_bounds__(256, SUMS ? 6 : 1) ncc_map_f32q(const T *__res
         atomicMax(&s_best[(b / PER) * BC + a / PER], ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)key));
     }
     __syncthreads();
-    if (t < BC * BC) {
+    if (t < BC * BR) {
         const int ccx = ccx0 + t % BC, ccy = ccy0 + t / BC;
         if (ccx < p.ccols && ccy < p.crows) {
             const int cell = ccy * p.ccols + ccx;
@@ -485,18 +520,28 @@ __global__ void __launch_bounds__(256, SUMS ? 6 : 1) ncc_map_f32q(const T *__res
     }
 }
 
-template <typename T, int ST, bool SUMS>
+/* Whether a search's F32 map at steps 1 and 2 takes CTAs of 16 corner rows: up to four CTAs of 32 rows an SM, whose barriers and
+ * loads little hides (a CTA of 32 x 32 corners of a 32 x 21 template at step 2 takes 36 us by itself), and a window with a
+ * thread a column. Measured, 16 rows against 32, us by the CTAs that 32 would take: 32 x 21 at step 2, 20 CTAs 23 / 36, 135
+ * 27 / 36, 510 64 / 71; at step 1, 285 33 / 36, 493 53 / 56, 858 84 / 76; 64 x 64 at step 2, 112 85 / 95, 464 253 / 281. */
+static bool nmq_narrow(const NccPrm &p)
+{
+    const int bc = NMQ_CORNERS * p.step / NCC_CELL;
+    return nmq_cols(p.step, p.tw) <= 130 && (long long)((p.ccols + bc - 1) / bc) * ((p.crows + bc - 1) / bc) <= 608;
+}
+
+template <typename T, int ST, bool SUMS, int CY>
 static cudaError_t launch_map_f32q(const T *plane, int pitch, const float *app, const NccPrm &p, const NccScratch &s,
                                    cudaStream_t st)
 {
-    constexpr int BC = NMQ_CORNERS * ST / NCC_CELL;
+    constexpr int BC = NMQ_CORNERS * ST / NCC_CELL, BR = CY * ST / NCC_CELL;
     const int head = SUMS ? nmq_head(ST, p.tw, p.th) : p.tw * p.th;
-    const size_t smem = sizeof(float) * ((size_t)head + (size_t)nmq_pitch(ST, p.tw) * nmq_rows(ST, p.th));
-    cudaError_t e = cudaFuncSetAttribute(ncc_map_f32q<T, ST, SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = sizeof(float) * ((size_t)head + (size_t)nmq_pitch(ST, p.tw) * nmq_rows(ST, p.th, CY));
+    cudaError_t e = cudaFuncSetAttribute(ncc_map_f32q<T, ST, SUMS, CY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
-    const int bcols = (p.ccols + BC - 1) / BC, brows = (p.crows + BC - 1) / BC;
-    ncc_map_f32q<T, ST, SUMS><<<bcols * brows, NMQ_CORNERS * NMQ_CORNERS / NMQ_K, smem, st>>>(
+    const int bcols = (p.ccols + BC - 1) / BC, brows = (p.crows + BR - 1) / BR;
+    ncc_map_f32q<T, ST, SUMS, CY><<<bcols * brows, NMQ_CORNERS * CY / NMQ_K, smem, st>>>(
         plane, pitch, app, p, s.S1, s.S2, s.tp, bcols, s.map_v, s.map_x, s.map_y);
     return cudaGetLastError();
 }
@@ -689,8 +734,8 @@ static cudaError_t launch_rescore(const uint8_t *plane, int pitch, const float *
 
 /* ---- the eight best cells ---- */
 
-/* The eight best cells. Each CTA takes NCC_TOPB_PER x NCC_TOPB_THREADS cells (a thread keeps its best eight in
- * registers; the lists merge across each warp, then across the CTA's warps) and writes its eight to blk. The CTA that
+/* The eight best cells. Each CTA takes NCC_TOPB_PER x NCC_TOPB_THREADS cells (each warp's best eight, then the best of those)
+ * and writes its eight to blk. The CTA that
  * arrives last merges every CTA's list into top / ntop and resets the counter, so the pass is one launch. WORDS: the
  * cells come as the tensor-core map's 64-bit words, which this pass also decodes into map_v / map_x / map_y. */
 template <bool WORDS>
@@ -705,10 +750,7 @@ __global__ void __launch_bounds__(NCC_TOPB_THREADS) ncc_top_ctas(NccPrm p, const
     __shared__ bool s_last;
     vtg_grid_launch_dependents(); /* the half-pixel pass may start its CTAs and wait */
     vtg_grid_dependency_wait();   /* the map's cells, when launched as its programmatic dependent */
-    unsigned long long t[NCC_TOP];
-#pragma unroll
-    for (int k = 0; k < NCC_TOP; k++)
-        t[k] = 0ull;
+    unsigned long long t[NCC_TOPB_PER];
     float v[NCC_TOPB_PER];
     const int i0 = blockIdx.x * NCC_TOPB_THREADS * NCC_TOPB_PER + threadIdx.x;
 #pragma unroll
@@ -731,27 +773,25 @@ __global__ void __launch_bounds__(NCC_TOPB_THREADS) ncc_top_ctas(NccPrm p, const
     }
 #pragma unroll
     for (int u = 0; u < NCC_TOPB_PER; u++)
-        top_insert(t, top_key(v[u], i0 + u * NCC_TOPB_THREADS));
+        t[u] = top_key(v[u], i0 + u * NCC_TOPB_THREADS);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    top_warp_merge(t);
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NCC_TOP; k++)
-            s[warp][k] = t[k];
+    const unsigned long long mine = top_of_warp(t);
+    if (lane < NCC_TOP)
+        s[warp][lane] = mine;
     __syncthreads();
     if (warp == 0) {
+        unsigned long long w[NCC_TOPB_THREADS / 32 * NCC_TOP / 32];
 #pragma unroll
-        for (int k = 0; k < NCC_TOP; k++)
-            t[k] = lane < NCC_TOPB_THREADS / 32 ? s[lane][k] : 0ull;
-        top_warp_merge(t);
-        /* every lane holds the list: lane 0 publishes it, then counts it */
-        if (lane == 0) {
-#pragma unroll
-            for (int k = 0; k < NCC_TOP; k++)
-                blk[(size_t)blockIdx.x * NCC_TOP + k] = t[k];
-            __threadfence();
+        for (int k = 0; k < NCC_TOPB_THREADS / 32 * NCC_TOP / 32; k++)
+            w[k] = (&s[0][0])[32 * k + lane];
+        const unsigned long long best = top_of_warp(w);
+        /* eight lanes publish the list, then one counts it */
+        if (lane < NCC_TOP)
+            blk[(size_t)blockIdx.x * NCC_TOP + lane] = best;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0)
             s_last = atomicAdd(arrive, 1u) == gridDim.x - 1;
-        }
     }
     __syncthreads();
     if (!s_last || warp != 0)
@@ -793,28 +833,56 @@ __device__ float half_score_cta(const T *__restrict__ plane, int pitch, const fl
     const float first = (float)__ldg(plane + (size_t)y * pitch + x);
     float st = 0.0f;
     Q a1 = 0, a2 = 0; /* in quarters */
-    /* the columns of a row as four unrolled, predicated steps (T_w <= 128) and two rows at a time, so a thread's loads
-     * are in flight together; the order of its sums is still rows, then columns, ascending */
-#pragma unroll 2
-    for (int i = warp; i < p.th; i += 8) {
-        const T *r0 = plane + (size_t)(y + i) * pitch + x, *r1 = r0 + pitch;
-        const float *ar = app + (size_t)i * p.tw;
+    /* A warp's rows four at a time (two past 32 columns), a lane's columns of them (four at most, T_w <= 128) all loaded before
+     * they are summed: one wait for memory for all of them. The order of its sums is still rows, then columns, ascending. */
+    auto rows = [&](auto columns, int i0) {
+        constexpr int C = decltype(columns)::value, R = 4 / C > 2 ? 4 / C : 2;
+        T a[R][C], b[R][C], c[R][C], d[R][C];
+        float t[R][C];
 #pragma unroll
-        for (int u = 0; u < VTG_NCC_MAX_T / 32; u++) {
-            const int j = lane + 32 * u;
-            if (j >= p.tw)
-                break;
-            const Q a = (Q)__ldg(r0 + j), b = ox ? (Q)__ldg(r0 + j + 1) : a;
-            Q q = 2 * (a + b);
-            if (oy) {
-                const Q c = (Q)__ldg(r1 + j), d = ox ? (Q)__ldg(r1 + j + 1) : c;
-                q = (q + 2 * (c + d)) / 2;
+        for (int k = 0; k < R; k++) {
+            const int i = min(i0 + 8 * k, p.th - 1);
+            const T *r0 = plane + (size_t)(y + i) * pitch + x, *r1 = r0 + pitch;
+#pragma unroll
+            for (int u = 0; u < C; u++) {
+                const int j = min(lane + 32 * u, p.tw - 1);
+                a[k][u] = __ldg(r0 + j);
+                t[k][u] = __ldg(app + i * p.tw + j);
+                if (ox)
+                    b[k][u] = __ldg(r0 + j + 1);
+                if (oy) {
+                    c[k][u] = __ldg(r1 + j);
+                    if (ox)
+                        d[k][u] = __ldg(r1 + j + 1);
+                }
             }
-            a1 += q;
-            a2 += q * q;
-            st = __fmaf_rn((float)q * 0.25f - first, __ldg(ar + j), st);
         }
-    }
+#pragma unroll
+        for (int k = 0; k < R; k++)
+#pragma unroll
+            for (int u = 0; u < C; u++) {
+                if (i0 + 8 * k >= p.th || lane + 32 * u >= p.tw)
+                    continue;
+                const Q qa = (Q)a[k][u];
+                Q q = 2 * (qa + (ox ? (Q)b[k][u] : qa));
+                if (oy) {
+                    const Q qc = (Q)c[k][u];
+                    q = (q + 2 * (qc + (ox ? (Q)d[k][u] : qc))) / 2;
+                }
+                a1 += q;
+                a2 += q * q;
+                st = __fmaf_rn((float)q * 0.25f - first, t[k][u], st);
+            }
+    };
+    if (p.tw > 64)
+        for (int i = warp; i < p.th; i += 16)
+            rows(std::integral_constant<int, 4>(), i);
+    else if (p.tw > 32)
+        for (int i = warp; i < p.th; i += 16)
+            rows(std::integral_constant<int, 2>(), i);
+    else
+        for (int i = warp; i < p.th; i += 32)
+            rows(std::integral_constant<int, 1>(), i);
     long long q1 = a1, q2 = a2;
 #pragma unroll
     for (int s = 16; s >= 1; s >>= 1) {
@@ -934,7 +1002,7 @@ __device__ void ncc_pick(const NccPrm &p, const int *__restrict__ map_x, const i
  * to hs[candidate][(around + 1 + dy) ring + around + 1 + dx], ring = 2 around + 3. The CTA that arrives last (every
  * CTA counts, those past the candidates too) makes the pick and resets the counter. */
 template <typename T>
-__global__ void __launch_bounds__(NCC_TOP * 32) ncc_half_all(const T *__restrict__ plane, int pitch,
+__global__ void __launch_bounds__(NCC_TOP * 32, 4) ncc_half_all(const T *__restrict__ plane, int pitch,
                                                              const float *__restrict__ app, NccPrm p,
                                                              const int *__restrict__ map_x, const int *__restrict__ map_y,
                                                              const int *__restrict__ top, const int *__restrict__ ntop,
@@ -1044,11 +1112,14 @@ static cudaError_t launch_all(const T *plane, int pitch, const float *app, const
             return e;
         if (s.map_ev0 && (e = cudaEventRecord(s.map_ev0, st)) != cudaSuccess)
             return e;
+        const bool narrow = sums && nmq_narrow(p);
         if (quad)
-            e = p.step == 1 ? (sums ? launch_map_f32q<T, 1, true>(plane, pitch, app, p, s, st)
-                                    : launch_map_f32q<T, 1, false>(plane, pitch, app, p, s, st))
-                            : (sums ? launch_map_f32q<T, 2, true>(plane, pitch, app, p, s, st)
-                                    : launch_map_f32q<T, 2, false>(plane, pitch, app, p, s, st));
+            e = p.step == 1 ? (narrow ? launch_map_f32q<T, 1, true, 16>(plane, pitch, app, p, s, st)
+                               : sums ? launch_map_f32q<T, 1, true, 32>(plane, pitch, app, p, s, st)
+                                      : launch_map_f32q<T, 1, false, 32>(plane, pitch, app, p, s, st))
+                            : (narrow ? launch_map_f32q<T, 2, true, 16>(plane, pitch, app, p, s, st)
+                               : sums ? launch_map_f32q<T, 2, true, 32>(plane, pitch, app, p, s, st)
+                                      : launch_map_f32q<T, 2, false, 32>(plane, pitch, app, p, s, st));
         else
             ncc_map_f32<T><<<cells, 256, smem, st>>>(plane, pitch, app, p, s.S1, s.S2, s.tp, s.map_v, s.map_x, s.map_y);
         if (e != cudaSuccess)

@@ -169,9 +169,29 @@ void vtg_ncc_filter_bound(NccPrm &p, const NccBandStats &b)
 
 /* ---- per-search preparation ---- */
 
-/* conv[r][i] = 16-bit J[r][x0 + i] - centre (minus the centre past the picture), for rows 0 .. rows - 1 and columns 0 .. cpitch - 1: the
- * CTA (bx, by) of 256 threads converts row by, eight elements a thread and one 16-byte store (cpitch is a multiple of 8
- * and rows start 16-byte aligned: 2 cpitch = 2048 tiles_x + 288 bytes). */
+/* A word's four bytes less `centre`, as 16-bit values in two words. */
+template <int KIND>
+__device__ __forceinline__ uint2 conv4(uint32_t w, float centre)
+{
+    if (KIND == VTG_NCC_FP16) { /* 0x6400 | b is 1024 + b */
+        const __half2 off = __float2half2_rn(1024.0f + centre);
+        const uint32_t a = __byte_perm(w, 0x64646464u, 0x4140u), b = __byte_perm(w, 0x64646464u, 0x4342u);
+        const __half2 x = __hsub2(*reinterpret_cast<const __half2 *>(&a), off), y = __hsub2(*reinterpret_cast<const __half2 *>(&b), off);
+        return make_uint2(*reinterpret_cast<const uint32_t *>(&x), *reinterpret_cast<const uint32_t *>(&y));
+    }
+    /* bytes are BF16 values: the upper half of the F32, from 2^23 + b */
+    const float off = 8388608.0f + centre;
+    uint32_t f[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        f[k] = __float_as_uint(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + k)) - off);
+    return make_uint2(__byte_perm(f[0], f[1], 0x7632u), __byte_perm(f[2], f[3], 0x7632u));
+}
+
+/* conv[r][i] = 16-bit J[r][x0 + i] - centre (minus the centre past the picture), for rows 0 .. rows - 1 and columns 0 .. cpitch - 1:
+ * the CTA (bx, by) of 256 threads converts row by, eight elements a thread and one 16-byte store (cpitch is a multiple of 8
+ * and rows start 16-byte aligned: 2 cpitch = 2048 tiles_x + 288 bytes). Inside the row the bytes come as three aligned words,
+ * shifted: the first starts up to three bytes before, the third ends up to twelve after. */
 template <int KIND>
 __device__ __forceinline__ void conv_cta(const uint8_t *__restrict__ plane, int pitch, int w, int h, int x0, int rows,
                                          int cpitch, float centre, uint16_t *__restrict__ conv, int bx, int by)
@@ -179,130 +199,140 @@ __device__ __forceinline__ void conv_cta(const uint8_t *__restrict__ plane, int 
     const int r = by, i0 = 8 * (bx * 256 + (int)threadIdx.x);
     if (r >= rows || i0 >= cpitch)
         return;
-    uint32_t o[4];
+    uint32_t v[2] = {0u, 0u};
+    const int x = x0 + i0;
+    const uint8_t *src = plane + (size_t)r * pitch + x;
+    const bool whole = r < h && x >= 3 && x + 12 <= w;
+    if (whole) {
+        const uint32_t *q = reinterpret_cast<const uint32_t *>((uintptr_t)src & ~(uintptr_t)3);
+        const int sh = 8 * (int)((uintptr_t)src & 3);
+        const uint32_t q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
+        v[0] = __funnelshift_r(q0, q1, sh);
+        v[1] = __funnelshift_r(q1, q2, sh);
+    } else if (r < h) {
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        uint32_t pr = 0;
-#pragma unroll
-        for (int f = 0; f < 2; f++) {
-            const int x = x0 + i0 + 2 * e + f;
-            const float v = (r < h && x < w) ? (float)__ldg(plane + (size_t)r * pitch + x) - centre : -centre;
-            pr |= (uint32_t)to16(v, KIND) << (16 * f);
-        }
-        o[e] = pr;
+        for (int e = 0; e < 8; e++)
+            if (x + e < w)
+                v[e >> 2] |= (uint32_t)__ldg(src + e) << (8 * (e & 3));
     }
-    *reinterpret_cast<uint4 *>(conv + (size_t)r * cpitch + i0) = make_uint4(o[0], o[1], o[2], o[3]);
+    const uint2 a = conv4<KIND>(v[0], centre), b = conv4<KIND>(v[1], centre);
+    *reinterpret_cast<uint4 *>(conv + (size_t)r * cpitch + i0) = make_uint4(a.x, a.y, b.x, b.y);
 }
 
 /* fac[(y - y0) fpitch + (x - x0)] = 1 / sqrt(norm var) from the corner's exact window sums; 0 for a near-blank window
  * (n var <= n norm / 16) or norm <= 0 -- the reference's rule (src/kern/track.c:203-205) on exact integers.
- * The sums come straight from the bytes, a tile of btx x BP_TY corners a CTA (btx = bp_tx(T_w)), one thread a column
- * of the tile:
- *   - down its column, running sums over the template's T_h rows for the tile's BP_TY corner rows (registers);
- *   - across the columns, each row's prefix sums: a shuffle scan in the warp, the earlier warps' totals added from
- *     shared memory;
- *   - a corner's window sums are then P(x + T_w) - P(x), consecutive lanes on consecutive corners.
+ * The sums come straight from the bytes, a tile of btx x BP_TY corners a CTA (btx = bp_tx(T_w)):
+ *   - a thread a column of the tile, down its column: running sums over the template's T_h rows for the tile's BP_TY corner
+ *     rows, into shared memory;
+ *   - a thread 16 columns of a row: its prefix sums, the row's 16 threads' totals scanned by shuffles;
+ *   - a corner's window sums are then P(x + T_w) - P(x), four consecutive corners a thread by 16-byte reads.
  * Bytes keep every window sum in 32 bits (sum J^2 <= 255^2 x 128^2 < 2^31). A row's prefix of J^2 may pass 2^32, so
- * the prefixes are unsigned and wrap: their differences are still exact. n var is formed in 64 bits. */
-#ifndef BP_TY
-#define BP_TY 16 /* corner rows a CTA: a multiple of the 8 warps, each warp writing rows warp, warp + 8, .. */
-#endif
+ * the prefixes are unsigned and wrap: their differences are still exact. n var is formed in 64 bits. The kernel is bound by
+ * issue and by its loads' latency: 18 us over a 1080p frame at 64 x 64; a shuffle scan of every row by every warp, and a
+ * corner a thread, took 13M instructions where this takes 8M, and 23 us. */
+#define BP_TY 16 /* corner rows a CTA: 16 threads each in the scan */
+#define BP_P 260 /* words of a row of prefixes: 0 .. 256, rows 16-byte aligned */
 /* corners a CTA across: the most, a multiple of 32, whose columns (+ T_w - 1) fit the CTA's 256 threads */
 static inline int bp_tx(int tw) { return ((257 - tw) / 32) * 32; }
+
+struct BoxSmem {
+    __align__(16) unsigned p[2][BP_TY][BP_P]; /* P[r][c]: columns 0 .. c - 1 of row r; of J and of J^2 */
+};
+
 template <bool TOL>
 __device__ void box_cta(const uint8_t *__restrict__ plane, int pitch, const NccPrm &p, int fw, int fpitch, int btx,
-                        float *__restrict__ fac, uint16_t *__restrict__ tol, int bx, int by)
+                        float *__restrict__ fac, uint16_t *__restrict__ tol, int bx, int by, BoxSmem &S)
 {
-    __shared__ unsigned P1[BP_TY][257], P2[BP_TY][257]; /* P[r][c]: columns 0 .. c - 1 of row r */
-    __shared__ unsigned t1[8][BP_TY], t2[8][BP_TY];     /* each warp's column totals, then the earlier warps' */
     const int fh = p.y1 - p.y0 + 1;
     const int tx0 = bx * btx, ty0 = by * BP_TY;
     const int nx = min(btx, fw - tx0), ny = min(BP_TY, fh - ty0);
-    const int c = threadIdx.x, lane = c & 31, warp = c >> 5;
+    const int tid = threadIdx.x;
     const int ncol = nx + p.tw - 1; /* <= 256 */
-    unsigned a[BP_TY], b[BP_TY];
-    if (c < ncol) {
-        const uint8_t *col = plane + (size_t)(p.y0 + ty0) * pitch + (p.x0 + tx0 + c);
+    {
+        /* column tid's sums (0 past the tile's columns); every load of the sliding part in flight, before the first window's
+         * rows are added */
+        const bool in = tid < ncol;
+        const uint8_t *col = plane + (size_t)(p.y0 + ty0) * pitch + (p.x0 + tx0 + min(tid, ncol - 1));
+        unsigned leave[BP_TY], enter[BP_TY];
+#pragma unroll
+        for (int r = 1; r < BP_TY; r++) {
+            const int k = min(r, ny - 1) - (ny > 1 ? 1 : 0);
+            leave[r] = __ldg(col + (size_t)k * pitch);
+            enter[r] = __ldg(col + (size_t)(k + p.th) * pitch);
+        }
         unsigned sa = 0, sb = 0;
-#pragma unroll 8
+#pragma unroll 16
         for (int i = 0; i < p.th; i++) {
             const unsigned v = __ldg(col + (size_t)i * pitch);
             sa += v;
             sb += v * v;
         }
-        a[0] = sa;
-        b[0] = sb;
+        S.p[0][0][tid] = in ? sa : 0u;
+        S.p[1][0][tid] = in ? sb : 0u;
 #pragma unroll
         for (int r = 1; r < BP_TY; r++) {
-            if (r < ny) {
-                const unsigned o = __ldg(col + (size_t)(r - 1) * pitch), n = __ldg(col + (size_t)(r - 1 + p.th) * pitch);
-                sa += n - o;
-                sb += n * n - o * o;
-            }
-            a[r] = sa;
-            b[r] = sb;
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r < BP_TY; r++)
-            a[r] = b[r] = 0u;
-    }
-    /* inclusive scans across the warp's 32 columns */
-#pragma unroll
-    for (int sh = 1; sh < 32; sh <<= 1)
-#pragma unroll
-        for (int r = 0; r < BP_TY; r++) {
-            const unsigned ua = __shfl_up_sync(VTG_FULL, a[r], sh), ub = __shfl_up_sync(VTG_FULL, b[r], sh);
-            if (lane >= sh) {
-                a[r] += ua;
-                b[r] += ub;
-            }
-        }
-    if (lane == 31)
-#pragma unroll
-        for (int r = 0; r < BP_TY; r++) {
-            t1[warp][r] = a[r];
-            t2[warp][r] = b[r];
-        }
-    __syncthreads();
-    if (c < 2 * BP_TY) { /* each (row, table): the totals of the warps before, in place */
-        unsigned(*t)[BP_TY] = c < BP_TY ? t1 : t2;
-        const int r = c % BP_TY;
-        unsigned run = 0;
-        for (int w = 0; w < 8; w++) {
-            const unsigned v = t[w][r];
-            t[w][r] = run;
-            run += v;
+            sa += enter[r] - leave[r];
+            sb += enter[r] * enter[r] - leave[r] * leave[r];
+            S.p[0][r][tid] = in ? sa : 0u;
+            S.p[1][r][tid] = in ? sb : 0u;
         }
     }
     __syncthreads();
+    /* row tid / 16, columns 16 (tid % 16) ..: read, scanned, and (after a barrier) written one place on */
+    const int row = tid >> 4, seg = tid & 15;
 #pragma unroll
-    for (int r = 0; r < BP_TY; r++) {
-        P1[r][c + 1] = t1[warp][r] + a[r];
-        P2[r][c + 1] = t2[warp][r] + b[r];
-        if (c == 0) {
-            P1[r][0] = 0u;
-            P2[r][0] = 0u;
+    for (int t = 0; t < 2; t++) {
+        unsigned v[16];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            *reinterpret_cast<uint4 *>(&v[4 * k]) = *reinterpret_cast<const uint4 *>(&S.p[t][row][16 * seg + 4 * k]);
+#pragma unroll
+        for (int k = 1; k < 16; k++)
+            v[k] += v[k - 1];
+        unsigned before = v[15];
+#pragma unroll
+        for (int d = 1; d < 16; d <<= 1) {
+            const unsigned u = __shfl_up_sync(VTG_FULL, before, d, 16);
+            before += seg >= d ? u : 0u;
         }
+        before -= v[15];
+        __syncwarp(); /* a row lies in one half of a warp */
+        /* P[16 seg] = before, P[16 seg + 1 ..] = before + v[0] ..: the 16 places from 16 seg on, and 256 */
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            *reinterpret_cast<uint4 *>(&S.p[t][row][16 * seg + 4 * k]) =
+                make_uint4(k ? before + v[4 * k - 1] : before, before + v[4 * k], before + v[4 * k + 1], before + v[4 * k + 2]);
+        if (seg == 15)
+            S.p[t][row][256] = before + v[15];
     }
     __syncthreads();
-    /* warp w writes corner rows w, w + 8, ..; its lanes consecutive corners (btx is a multiple of 32) */
-    for (int r = warp; r < ny; r += 8) {
-        float *frow = fac + (size_t)(ty0 + r) * fpitch + tx0;
-#pragma unroll 1
-        for (int x = lane; x < nx; x += 32) {
-            const long long s1 = (long long)(P1[r][x + p.tw] - P1[r][x]), s2 = (long long)(P2[r][x + p.tw] - P2[r][x]);
-            const long long nvar = (long long)p.n * s2 - s1 * s1;
+    /* four corners a thread of a row (tw is a multiple of 8: both ends 16-byte aligned); fac's rows hold whole tiles, so a
+     * group's store stays inside, past the window's last corner too */
+    const int groups = (nx + 3) / 4;
+    for (int i = tid; i < ny * groups; i += 256) {
+        const int r = i / groups, x = 4 * (i - r * groups);
+        const uint4 l1 = *reinterpret_cast<const uint4 *>(&S.p[0][r][x]), h1 = *reinterpret_cast<const uint4 *>(&S.p[0][r][x + p.tw]);
+        const uint4 l2 = *reinterpret_cast<const uint4 *>(&S.p[1][r][x]), h2 = *reinterpret_cast<const uint4 *>(&S.p[1][r][x + p.tw]);
+        const unsigned w1[4] = {h1.x - l1.x, h1.y - l1.y, h1.z - l1.z, h1.w - l1.w};
+        const unsigned w2[4] = {h2.x - l2.x, h2.y - l2.y, h2.z - l2.z, h2.w - l2.w};
+        float f[4];
+        uint32_t e[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const long long nvar = (long long)p.n * (long long)w2[k] - (long long)w1[k] * (long long)w1[k];
             /* 1 / sqrt(norm var) = sqrt(n / norm) / sqrt(n var) */
             const float rs = rsqrtf((float)nvar);
-            frow[x] = (nvar <= p.nthr || p.norm <= 0.0f) ? 0.0f : p.rnorm * rs;
+            f[k] = (nvar <= p.nthr || p.norm <= 0.0f) ? 0.0f : p.rnorm * rs;
             if constexpr (TOL) { /* |mean - c| / sigma = |sum J - n c| / sqrt(n var); rounded up */
-                const int f = __ldg(plane + (size_t)(p.y0 + ty0 + r) * pitch + (p.x0 + tx0 + x));
-                const float zm = fabsf((float)(s1 - 128 * p.n)) * rs, zf = fabsf((float)(s1 - (long long)f * p.n)) * rs;
-                tol[(size_t)(ty0 + r) * fpitch + tx0 + x] =
-                    __half_as_ushort(__float2half_ru(p.flt_a + p.flt_m * zm + p.flt_f * zf));
+                const int j = x + k < nx ? __ldg(plane + (size_t)(p.y0 + ty0 + r) * pitch + (p.x0 + tx0 + x + k)) : 0;
+                const float zm = fabsf((float)((int)w1[k] - 128 * p.n)) * rs, zf = fabsf((float)((int)w1[k] - j * p.n)) * rs;
+                e[k] = __half_as_ushort(__float2half_ru(p.flt_a + p.flt_m * zm + p.flt_f * zf));
             }
         }
+        const size_t at = (size_t)(ty0 + r) * fpitch + tx0 + x;
+        *reinterpret_cast<float4 *>(fac + at) = make_float4(f[0], f[1], f[2], f[3]);
+        if constexpr (TOL)
+            *reinterpret_cast<uint2 *>(tol + at) = make_uint2(e[0] | e[1] << 16, e[2] | e[3] << 16);
     }
 }
 
@@ -315,10 +345,11 @@ __global__ void __launch_bounds__(256) ncc_prep(const uint8_t *__restrict__ plan
                                                 uint16_t *__restrict__ tol, int rows, int cpitch, int cgx, uint16_t *__restrict__ conv, unsigned long long *__restrict__ cellw,
                                                 int cells, unsigned *__restrict__ ncand)
 {
+    __shared__ BoxSmem S;
     vtg_grid_launch_dependents(); /* the map may start its setup as this launch's last CTAs run */
     const int b = (int)blockIdx.x;
     if (b < nbox) {
-        box_cta<FILTER>(plane, pitch, p, fw, fpitch, btx, fac, tol, b % bgx, b / bgx);
+        box_cta<FILTER>(plane, pitch, p, fw, fpitch, btx, fac, tol, b % bgx, b / bgx, S);
         return;
     }
     const int k = b - nbox, g = k * 256 + (int)threadIdx.x;
@@ -762,11 +793,11 @@ bool vtg_ncc_filters(const NccPrm &p, const NccScratch &s)
     const TcGrid g = tc_grid(p);
     /* The filter costs a preparation over the plane and two more launches; the map it replaces is one launch whose CTAs take
      * their whole template's products in one chain. Measured (whole searches, filter against map, us): 64 x 64 over 201 x
-     * 201 corners 77 / 110, over a 1080p frame 94 / 748; 32 x 32 over 401 x 301 corners (1.2e8 products) 56 / 51, over a
-     * 640 x 480 frame (2.8e8) 57 / 64, over a 1080p frame 70 / 227; 16 x 16 over 1280 x 720 (2.3e8) 57 / 57. So it takes every
-     * template from 2,048 pixels on, and smaller ones from 2.5e8 products. */
+     * 201 corners 64 / 67, over a 1080p frame 80 / 748; 48 x 48 over 201 x 201 corners (9e7 products) 56 / 48, over 401 x 301
+     * (2.8e8) 57 / 61; 32 x 21 over a 640 x 480 frame (1.9e8) 45 / 44, over 960 x 540 (3.2e8) 48 / 64; 16 x 16 over 960 x 540
+     * (1.3e8) 47 / 43. So it takes every template from 4,096 pixels on, and smaller ones from 2e8 products. */
     const double products = (double)g.fw * g.fh * p.n / (p.step * p.step);
-    return (p.n >= 2048 || products >= 2.5e8) && tc_fits(p, s, g) && (size_t)g.fw * g.fh <= s.cand_elems &&
+    return (p.n >= 4096 || products >= 2.0e8) && tc_fits(p, s, g) && (size_t)g.fw * g.fh <= s.cand_elems &&
            (size_t)g.fpitch * g.fh <= s.tol_elems;
 }
 

@@ -107,7 +107,7 @@ __device__ __forceinline__ void ncc_cell_decode(const NccPrm &p, int cell, unsig
     y = cy0 + (key / per) * p.step;
 }
 
-/* ---- the eight best cells: keys, a register list, a warp's merge ---- */
+/* ---- the eight best cells: keys, a warp's best ---- */
 
 /* A cell's key: its value in ascending float order as unsigned, then the inverted cell index (the earlier cell first
  * among equal values); 0 for no value (-2). */
@@ -120,46 +120,29 @@ __device__ __forceinline__ unsigned long long top_key(float v, int i)
     return ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)i);
 }
 
-/* k into the descending list t, keeping its NCC_TOP largest: one compare-exchange a place, unrolled, so t stays in
- * registers. Keys are distinct (the cell index is in their low bits). */
-__device__ __forceinline__ void top_insert(unsigned long long (&t)[NCC_TOP], unsigned long long k)
+/* The NCC_TOP largest of a warp's keys, N a lane, best first: lane k (and k + 8, ..) ends with the k-th, 0 where there are fewer.
+ * Each turn takes the largest by two 32-bit maxima over the warp and strikes it from its lane: about 60 cycles a turn, where
+ * merging sorted lists by shuffles took six times that. Keys are distinct (the cell index is in their low bits). */
+template <int N>
+__device__ __forceinline__ unsigned long long top_of_warp(unsigned long long (&t)[N])
 {
-    if (k <= t[NCC_TOP - 1])
-        return;
+    unsigned long long mine = 0ull;
 #pragma unroll
-    for (int j = 0; j < NCC_TOP; j++) {
-        const unsigned long long hi = t[j] > k ? t[j] : k;
-        k = t[j] > k ? k : t[j];
-        t[j] = hi;
+    for (int k = 0; k < NCC_TOP; k++) {
+        unsigned long long m = t[0];
+#pragma unroll
+        for (int j = 1; j < N; j++)
+            m = t[j] > m ? t[j] : m;
+        const unsigned hi = __reduce_max_sync(VTG_FULL, (unsigned)(m >> 32));
+        const unsigned lo = __reduce_max_sync(VTG_FULL, (unsigned)(m >> 32) == hi ? (unsigned)m : 0u);
+        const unsigned long long best = ((unsigned long long)hi << 32) | lo;
+        if (((threadIdx.x & 31) % NCC_TOP) == k)
+            mine = best;
+#pragma unroll
+        for (int j = 0; j < N; j++)
+            t[j] = t[j] == best ? 0ull : t[j];
     }
-}
-
-/* Two descending lists' best eight: max(a_k, b_(7 - k)) is their top eight as a bitonic sequence, which three
- * compare-exchange layers sort. Across the warp by xor partners, so every lane ends with the warp's best eight. */
-__device__ __forceinline__ void top_warp_merge(unsigned long long (&t)[NCC_TOP])
-{
-#pragma unroll 1
-    for (int sh = 1; sh < 32; sh <<= 1) {
-        unsigned long long c[NCC_TOP];
-#pragma unroll
-        for (int k = 0; k < NCC_TOP; k++) {
-            const unsigned long long o = __shfl_xor_sync(VTG_FULL, t[NCC_TOP - 1 - k], sh);
-            c[k] = t[k] > o ? t[k] : o;
-        }
-#pragma unroll
-        for (int d = NCC_TOP / 2; d >= 1; d >>= 1)
-#pragma unroll
-            for (int k = 0; k < NCC_TOP; k++)
-                if ((k & d) == 0) {
-                    const unsigned long long hi = c[k] > c[k + d] ? c[k] : c[k + d];
-                    const unsigned long long lo = c[k] > c[k + d] ? c[k + d] : c[k];
-                    c[k] = hi;
-                    c[k + d] = lo;
-                }
-#pragma unroll
-        for (int k = 0; k < NCC_TOP; k++)
-            t[k] = c[k];
-    }
+    return mine;
 }
 
 /* The last CTA of a top-8 pass, its warp 0: the best eight of the n CTAs' lists in blk (read through L2) into top /
@@ -167,23 +150,19 @@ __device__ __forceinline__ void top_warp_merge(unsigned long long (&t)[NCC_TOP])
 __device__ __forceinline__ void ncc_top_final(const unsigned long long *blk, int n, unsigned *arrive, int *top, int *ntop)
 {
     const int lane = threadIdx.x & 31;
-    unsigned long long t[NCC_TOP];
+    unsigned long long t[5] = {0ull, 0ull, 0ull, 0ull, 0ull}; /* [0]: the best so far, on lanes 0 .. 7 */
+    for (int b = 0; b < n * NCC_TOP; b += 4 * 32) {
 #pragma unroll
-    for (int k = 0; k < NCC_TOP; k++)
-        t[k] = 0ull;
-    for (int b = lane; b < n; b += 32)
-#pragma unroll
-        for (int k = 0; k < NCC_TOP; k++)
-            top_insert(t, __ldcg(blk + (size_t)b * NCC_TOP + k));
-    top_warp_merge(t);
+        for (int k = 0; k < 4; k++)
+            t[1 + k] = b + 32 * k + lane < n * NCC_TOP ? __ldcg(blk + b + 32 * k + lane) : 0ull;
+        const unsigned long long best = top_of_warp(t);
+        t[0] = lane < NCC_TOP ? best : 0ull;
+    }
+    const unsigned found = __ballot_sync(VTG_FULL, lane < NCC_TOP && t[0] != 0ull);
+    if (lane < NCC_TOP && t[0] != 0ull)
+        top[lane] = (int)(0xFFFFFFFFu - (unsigned)(t[0] & 0xFFFFFFFFull));
     if (lane == 0) {
-        int c = 0;
-        for (int k = 0; k < NCC_TOP; k++) {
-            if (t[k] == 0ull)
-                break;
-            top[c++] = (int)(0xFFFFFFFFu - (unsigned)(t[k] & 0xFFFFFFFFull));
-        }
-        *ntop = c;
+        *ntop = __popc(found);
         *arrive = 0u;
     }
 }

@@ -58,6 +58,8 @@ def _picture(kind, w, h):
     (190, 170, 64, 33, 1, (60, 60, 20, 20)),    # one corner
     (641, 481, 24, 40, 1, None),                # a small template over a large window
     (64, 140, 48, 48, 1, None),                 # the narrowest plane
+    (1300, 800, 16, 16, 1, None),               # the F32 plane's map in CTAs of 32 corner rows (over 608 of them)
+    (330, 250, 72, 40, 2, None),                # and where a window is wider than its CTA's threads
 ])
 def test_bytes_and_floats_have_one_map(vtg_lib, ctx, kind, w, h, tw, th, step, win):
     import torch
