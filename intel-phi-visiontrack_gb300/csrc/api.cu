@@ -30,6 +30,8 @@ void vtg_set_cuda_error(cudaError_t e) { g_last_cuda = (int)e; }
         }                                                                                                              \
     } while (0)
 
+#define POINTS_KEPT 16384 /* points of a list whose scratch a tracker keeps: 1.5 MB at most */
+
 struct vtg_ctx {
     int device;
     size_t budget, used;
@@ -139,7 +141,11 @@ extern "C" int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms)
         for (cudaStream_t s : ctx->streams)
             streams.push_back(s);
     }
-    const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(timeout_ms < 0 ? 0 : timeout_ms);
+    /* the first 300 us by asking again at once, since a frame's work is shorter and a sleep of 50 us takes up to 110; then
+     * asleep in between */
+    const auto start = std::chrono::steady_clock::now();
+    const auto deadline = start + std::chrono::milliseconds(timeout_ms < 0 ? 0 : timeout_ms);
+    const auto patient = start + std::chrono::microseconds(300);
     for (cudaStream_t s : streams) {
         for (;;) {
             const cudaError_t e = cudaStreamQuery(s);
@@ -149,9 +155,13 @@ extern "C" int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms)
                 g_last_cuda = (int)e;
                 return VTG_ECUDA;
             }
-            if (std::chrono::steady_clock::now() > deadline)
+            const auto now = std::chrono::steady_clock::now();
+            if (now > deadline)
                 return VTG_ETIMEOUT;
-            std::this_thread::sleep_for(std::chrono::microseconds(50));
+            if (now < patient)
+                std::this_thread::yield();
+            else
+                std::this_thread::sleep_for(std::chrono::microseconds(50));
         }
     }
     return VTG_OK;
@@ -305,6 +315,8 @@ extern "C" int vtg_tracker_create(vtg_ctx *ctx, const vtg_config *cfg, vtg_track
     t->d_cells = (vtg_cell *)(t->mem + L.cells_off);
     t->d_mm = (uint32_t *)(t->mem + L.mm_off);
     t->d_app = (float *)(t->mem + L.app_off);
+    t->points = nullptr;
+    t->points_bytes = 0;
     t->build_opts = 0;
     t->point_warps = 0;
     DevPyr d[4] = {pyr_from(t, 0, 0), pyr_from(t, 0, (int)cfg->flow_level), pyr_from(t, 1, 0),
@@ -348,6 +360,7 @@ extern "C" void vtg_tracker_destroy(vtg_tracker *t)
     cudaStreamSynchronize(t->stream);
     cudaStreamDestroy(t->stream);
     cudaFree(t->mem);
+    cudaFree(t->points);
     {
         std::lock_guard<std::mutex> g(ctx->mu);
         ctx->used -= t->bytes;
@@ -471,10 +484,36 @@ extern "C" int vtg_points(vtg_tracker *t, int prev, int cur, int top, int n, con
                              t->point_warps));
         return VTG_OK;
     }
-    /* Host arrays: one stream-ordered scratch allocation for the call. */
-    const size_t fbytes = (size_t)n * sizeof(float);
+    /* Host arrays go through device scratch: on the tracker's own stream, which orders the calls, its own (kept, grown to the
+     * longest list up to POINTS_KEPT); on another stream, for longer lists and in a capture, where nothing may be allocated
+     * otherwise, a stream-ordered allocation of the call's. The pool gives its memory back at every device-wide wait, so an
+     * allocation a call can take longer than the call's work (200 us of 270 for 512 points). */
+    const size_t fbytes = (size_t)n * sizeof(float), need = 4 * fbytes + (size_t)n * sizeof(vtg_lk_out);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(s, &cap));
+    std::unique_lock<std::mutex> own(t->points_mu, std::defer_lock);
     char *d = nullptr;
-    CU(cudaMallocAsync((void **)&d, 4 * fbytes + (size_t)n * sizeof(vtg_lk_out), s));
+    bool kept = s == t->stream && n <= POINTS_KEPT && cap == cudaStreamCaptureStatusNone;
+    if (kept) {
+        own.lock(); /* to the end of the call: its copies and kernel follow each other on the stream */
+        if (t->points_bytes < need) {
+            CU(cudaSetDevice(t->ctx->device));
+            char *more = nullptr;
+            if (cudaMalloc(&more, 2 * need) == cudaSuccess) {
+                cudaFree(t->points); /* waits for the work that reads it */
+                t->points = more;
+                t->points_bytes = 2 * need;
+            } else {
+                cudaGetLastError();
+                kept = false;
+                own.unlock();
+            }
+        }
+    }
+    if (kept)
+        d = t->points;
+    else
+        CU(cudaMallocAsync((void **)&d, need, s));
     float *dx = (float *)d, *dy = dx + n, *dgx = gx ? dy + n : nullptr, *dgy = gy ? dy + 2 * (size_t)n : nullptr;
     vtg_lk_out *dout = (vtg_lk_out *)(d + 4 * fbytes);
     CU(cudaMemcpyAsync(dx, xs, fbytes, cudaMemcpyHostToDevice, s));
@@ -486,7 +525,8 @@ extern "C" int vtg_points(vtg_tracker *t, int prev, int cur, int top, int n, con
     CU(vtg_launch_points(t->desc + 2 * prev, t->desc + 2 * cur, top, t->prm, n, dx, dy, dgx, dgy, dout, s,
                          t->point_warps));
     CU(cudaMemcpyAsync(out, dout, (size_t)n * sizeof(vtg_lk_out), cudaMemcpyDeviceToHost, s));
-    CU(cudaFreeAsync(d, s));
+    if (!kept)
+        CU(cudaFreeAsync(d, s));
     return VTG_OK;
 }
 

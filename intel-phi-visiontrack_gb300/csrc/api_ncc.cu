@@ -18,7 +18,11 @@ struct vtg_search {
     NccBandStats *stats; /* [0]: the BF16 band's, [1]: the FP16 band's (device) */
     NccScratch sc;
     uint16_t *band[2]; /* BF16 and FP16 bands */
-    vtg_found *found;  /* device result slot for host callers */
+    vtg_found *found;  /* device result slot (vtg_search_profile) */
+    struct Host {
+        vtg_found found;
+        int err; /* the tensor-core map's status word */
+    } *host, *host_dev; /* pinned host memory that the kernels write: a host caller's result needs no copy */
     int *xy;           /* corners for vtg_correlate from the host */
     float *vals;
     int tw, th;
@@ -30,7 +34,7 @@ struct vtg_search {
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 struct SearchLayout {
-    size_t app, sum, S1, S2, map_v, map_x, map_y, top, ntop, err, half, band0, band1, found, conv, fac, cellw, topblk,
+    size_t app, sum, S1, S2, map_v, map_x, map_y, top, ntop, half, band0, band1, found, conv, fac, cellw, topblk,
         arrive, bytes;
     size_t conv_elems, fac_elems;
     int tp, cells, lists;
@@ -65,8 +69,6 @@ static SearchLayout search_layout(int max_w, int max_h, int max_tw, int max_th)
     L.top = b;
     b += 256;
     L.ntop = b;
-    b += 256;
-    L.err = b;
     b += 256;
     L.half = b;
     b += up256(sizeof(float) * NCC_HALF_MAX);
@@ -135,13 +137,20 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
         e = cudaMemsetAsync(s->mem, 0, L.bytes, s->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s->stream);
+    s->host = nullptr;
+    if (e == cudaSuccess)
+        e = cudaHostAlloc(&s->host, sizeof *s->host, cudaHostAllocMapped);
+    if (e == cudaSuccess)
+        e = cudaHostGetDevicePointer(&s->host_dev, s->host, 0);
     if (e != cudaSuccess) {
         vtg_set_cuda_error(e);
+        cudaFreeHost(s->host);
         cudaFree(s->mem);
         vtg_ctx_release(ctx, L.bytes);
         delete s;
         return VTG_ECUDA;
     }
+    s->host->err = 0;
     s->app = (float *)(s->mem + L.app);
     s->stats = (NccBandStats *)(s->mem + L.sum);
     s->sc.S1 = (long long *)(s->mem + L.S1);
@@ -152,7 +161,7 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
     s->sc.map_y = (int *)(s->mem + L.map_y);
     s->sc.top = (int *)(s->mem + L.top);
     s->sc.ntop = (int *)(s->mem + L.ntop);
-    s->sc.err = (int *)(s->mem + L.err);
+    s->sc.err = &s->host_dev->err;
     s->sc.half = (float *)(s->mem + L.half);
     s->band[0] = (uint16_t *)(s->mem + L.band0);
     s->band[1] = (uint16_t *)(s->mem + L.band1);
@@ -188,6 +197,7 @@ extern "C" void vtg_search_destroy(vtg_search *s)
     vtg_ctx_track(s->ctx, s->stream, false);
     cudaStreamDestroy(s->stream);
     cudaFree(s->mem);
+    cudaFreeHost(s->host);
     vtg_ctx_release(s->ctx, s->bytes);
     delete s;
 }
@@ -266,7 +276,7 @@ extern "C" int vtg_search_run(vtg_search *s, const void *plane, int w, int h, in
     if (chk != VTG_OK)
         return chk;
     const cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
-    vtg_found *dst = where == VTG_DEVICE ? found : s->found;
+    vtg_found *dst = where == VTG_DEVICE ? found : &s->host_dev->found;
     if (empty) {
         vtg_found f = {0, 0, -2.0f, -2.0f, 0.0f, 0.0f, 0, 0};
         if (where == VTG_HOST)
@@ -287,12 +297,10 @@ extern "C" int vtg_search_run(vtg_search *s, const void *plane, int w, int h, in
     if (map_y)
         CU(cudaMemcpyAsync(map_y, sc.map_y, cells * sizeof(int), k, st));
     if (where == VTG_HOST) {
-        CU(cudaMemcpyAsync(found, dst, sizeof(vtg_found), cudaMemcpyDeviceToHost, st));
-        int err = 0;
-        CU(cudaMemcpyAsync(&err, sc.err, sizeof(int), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
-        if (err) {
-            CU(cudaMemsetAsync(sc.err, 0, sizeof(int), st));
+        *found = s->host->found;
+        if (s->host->err) {
+            s->host->err = 0;
             return VTG_ETIMEOUT;
         }
     }

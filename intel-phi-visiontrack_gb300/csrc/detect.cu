@@ -28,6 +28,7 @@
  * reference's (float)(rel) and max(fl(rel), 2500) equals its (float)(rel > 2500 ? rel : 2500). */
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <new>
 
@@ -69,8 +70,10 @@ struct vtg_detector {
     int *rowcount, *rowbase, *ncand; /* counts a segment; counts a row, or (tall regions) first places a segment */
     unsigned *keys;
     int2 *cxy;
-    float *xs, *ys;
-    int *count;
+    struct Host {
+        int count;
+        float xs[512], ys[512];
+    } *host, *host_dev; /* pinned host memory that det_select writes: a host caller's corners need no copy */
 };
 
 /* ---- the response and the cells ---- */
@@ -649,7 +652,7 @@ static bool det_geometry(int w, int h, float rx, float ry, float rw, float rh, i
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 struct DetLayout {
-    size_t resp, cell, best, rowcount, rowbase, ncand, keys, cxy, xs, ys, count, bytes;
+    size_t resp, cell, best, rowcount, rowbase, ncand, keys, cxy, bytes;
 };
 
 static DetLayout det_layout(int max_w, int max_h, int &max_cols, int &max_cells)
@@ -674,12 +677,6 @@ static DetLayout det_layout(int max_w, int max_h, int &max_cols, int &max_cells)
     b += up256(sizeof(unsigned) * DET_MAX_CAND);
     L.cxy = b;
     b += up256(sizeof(int2) * DET_MAX_CAND);
-    L.xs = b;
-    b += up256(sizeof(float) * 512);
-    L.ys = b;
-    b += up256(sizeof(float) * 512);
-    L.count = b;
-    b += 256;
     L.bytes = b;
     return L;
 }
@@ -722,9 +719,15 @@ extern "C" int vtg_detector_create(vtg_ctx *ctx, int max_w, int max_h, vtg_detec
         delete d;
         return VTG_ENOMEM;
     }
-    e = cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking);
+    d->host = nullptr;
+    e = cudaHostAlloc(&d->host, sizeof *d->host, cudaHostAllocMapped);
+    if (e == cudaSuccess)
+        e = cudaHostGetDevicePointer(&d->host_dev, d->host, 0);
+    if (e == cudaSuccess)
+        e = cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         vtg_set_cuda_error(e);
+        cudaFreeHost(d->host);
         cudaFree(d->mem);
         vtg_ctx_release(ctx, L.bytes);
         delete d;
@@ -738,9 +741,6 @@ extern "C" int vtg_detector_create(vtg_ctx *ctx, int max_w, int max_h, vtg_detec
     d->ncand = (int *)(d->mem + L.ncand);
     d->keys = (unsigned *)(d->mem + L.keys);
     d->cxy = (int2 *)(d->mem + L.cxy);
-    d->xs = (float *)(d->mem + L.xs);
-    d->ys = (float *)(d->mem + L.ys);
-    d->count = (int *)(d->mem + L.count);
     vtg_ctx_track(ctx, d->stream, true);
     *out = d;
     return VTG_OK;
@@ -755,6 +755,7 @@ extern "C" void vtg_detector_destroy(vtg_detector *d)
     vtg_ctx_track(d->ctx, d->stream, false);
     cudaStreamDestroy(d->stream);
     cudaFree(d->mem);
+    cudaFreeHost(d->host);
     vtg_ctx_release(d->ctx, d->bytes);
     delete d;
 }
@@ -805,8 +806,8 @@ extern "C" int vtg_detect(vtg_detector *d, const float *plane, int w, int h, int
         return VTG_OK;
     }
     const DetGeo &g = q.g;
-    float *oxs = where == VTG_DEVICE ? xs : d->xs, *oys = where == VTG_DEVICE ? ys : d->ys;
-    int *ocount = where == VTG_DEVICE ? count : d->count;
+    float *oxs = where == VTG_DEVICE ? xs : d->host_dev->xs, *oys = where == VTG_DEVICE ? ys : d->host_dev->ys;
+    int *ocount = where == VTG_DEVICE ? count : &d->host_dev->count;
     const bool scan = g.rows > DET_SCAN_ROWS;
     const dim3 rows(g.rows), threads(32 * DET_SEGS);
     const float *resp = d->resp, *cell = d->cell, *best = d->best;
@@ -825,10 +826,10 @@ extern "C" int vtg_detect(vtg_detector *d, const float *plane, int w, int h, int
                     (const unsigned *)d->keys, (const int2 *)d->cxy, oxs, oys, ocount));
     CU(cudaGetLastError());
     if (where == VTG_HOST) {
-        CU(cudaMemcpyAsync(count, d->count, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CU(cudaMemcpyAsync(xs, d->xs, sizeof(float) * (size_t)max, cudaMemcpyDeviceToHost, st));
-        CU(cudaMemcpyAsync(ys, d->ys, sizeof(float) * (size_t)max, cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
+        *count = d->host->count;
+        memcpy(xs, d->host->xs, sizeof(float) * (size_t)*count);
+        memcpy(ys, d->host->ys, sizeof(float) * (size_t)*count);
     }
     return VTG_OK;
 }

@@ -7,6 +7,8 @@
 #ifndef VTG_TRACKER_H
 #define VTG_TRACKER_H
 
+#include <mutex>
+
 #include "vtg_internal.cuh"
 
 struct vtg_tracker {
@@ -28,6 +30,9 @@ struct vtg_tracker {
     uint32_t *d_mm;       /* the build options' VTG_MM_WORDS words a set (min / max partials, ticket, gain / offset) */
     int build_opts;       /* VTG_BUILD_CONTRAST | VTG_BUILD_PRE_GAUSS */
     float *d_app;         /* an appearance template and its norm (VTG_APP_W x VTG_APP_H + 1 floats), for host reads */
+    char *points; /* the host point lists' scratch, allocated at the first one, and the calls that use it in turn */
+    size_t points_bytes;
+    std::mutex points_mu;
     LkPrm prm;
     int point_warps; /* warps a point of the point list: 0 by the list's length, 1 or 2 */
 };
