@@ -853,18 +853,33 @@ __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int to
     }
 }
 
-/* A warp a cell, 2 x 2 cells a CTA: neighbours' windows overlap in L1, and a CTA of few warps leaves its place as soon as its
- * few cells are done. A 1080p pair (build and cells, 16,200 cells), by cells a CTA: 8 x 1 0.243 ms, 4 x 2 0.242, 4 x 4 0.249,
- * 4 x 1 0.240, 2 x 2 0.236, 2 x 1 0.240, one 0.242. */
-#define LK_CTA_CELLS 4
-template <int MAXH, bool EXACT>
-__global__ void __launch_bounds__(32 * LK_CTA_CELLS, 16 / LK_CTA_CELLS) lk_cells_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp,
-                                                          int top, LkPrm p, CellGrid g, int base_w, int base_h,
-                                                          vtg_lk_out *__restrict__ out, vtg_cell *__restrict__ cells)
+/* How a single stream's cells and a point list launch. Many: 128 registers a thread, 16 warps an SM. Few: as many points as
+ * the chip has places for two-warp CTAs at eight warps an SM; then nothing but a point's own latency counts, and with 256
+ * registers a thread it spills nothing and keeps more loads in flight. Measured, us, few against many: 512 points at 1920 x
+ * 1080 28 / 33, 128 at 640 x 480 22 / 24, 1,024 at 1080p 34 / 38; past one wave, 2,048 at 1080p, 55 / 46. A whole 640 x 480 pair
+ * from host memory (1,200 cells) 64.4 / 66.7. The shape before both, for point lists of any length, was 8 warps a CTA of 128
+ * registers and no launch ahead of the kernel before: 28, 37 and 39 for the three lists above. */
+#define LK_SMS 152
+template <bool FEW>
+struct LkShape {
+    static constexpr int cell_rows = FEW ? 1 : 2, cells = 2 * cell_rows; /* a CTA's cells, two across */
+    static constexpr int cell_ctas = FEW ? 4 : 16 / cells;                /* CTAs an SM */
+    static constexpr int points = FEW ? 2 : 1, point_ctas = FEW ? 4 : 16;
+};
+static bool lk_few(int n) { return n <= 8 * LK_SMS; }
+
+/* A warp a cell. Many: 2 x 2 cells a CTA, as neighbours' windows overlap in L1, and a CTA of few warps leaves its place as soon
+ * as its few cells are done. A 1080p pair (build and cells, 16,200 cells), by cells a CTA: 8 x 1 0.243 ms, 4 x 2 0.242, 4 x 4
+ * 0.249, 4 x 1 0.240, 2 x 2 0.236, 2 x 1 0.240, one 0.242. */
+template <int MAXH, bool EXACT, bool FEW>
+__global__ void __launch_bounds__(32 * LkShape<FEW>::cells, LkShape<FEW>::cell_ctas)
+    lk_cells_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp, int top, LkPrm p, CellGrid g, int base_w, int base_h,
+                    vtg_lk_out *__restrict__ out, vtg_cell *__restrict__ cells)
 {
-    extern __shared__ f2_t s_tc[]; /* the template's T: 4 warps x (MAXH / 2) x 32 pairs */
+    extern __shared__ f2_t s_tc[]; /* the template's T: a warp (MAXH / 2) x 32 pairs */
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, across = (g.cols + 1) / 2;
-    const int col = 2 * ((int)blockIdx.x % across) + (warp & 1), row = 2 * ((int)blockIdx.x / across) + (warp >> 1);
+    const int col = 2 * ((int)blockIdx.x % across) + (warp & 1);
+    const int row = LkShape<FEW>::cell_rows * ((int)blockIdx.x / across) + (warp >> 1);
     vtg_grid_dependency_wait(); /* the pyramid, when its kernel is the one before on the stream */
     if (col >= g.cols || row >= g.rows)
         return;
@@ -1044,7 +1059,9 @@ cudaError_t vtg_launch_lk_batch(const LkJob *jobs, const int *item_start, int nj
 /* shared memory of a single-stream CTA: its warps' template intensities (at most 30 KB) */
 static constexpr size_t lk_t_bytes(int maxh, int warps) { return sizeof(f2_t) * (size_t)warps * (size_t)(maxh / 2) * 32; }
 
-/* The still picture's vectors (still.cu): one level, its descriptors by value, and the cells' differences counted. */
+/* The still picture's vectors (still.cu): one level, its descriptors by value, and the cells' differences counted. Its 15 x 15
+ * patch spills nothing at 128 registers. */
+#define LK_CTA_CELLS LkShape<false>::cells
 __global__ void __launch_bounds__(32 * LK_CTA_CELLS, 16 / LK_CTA_CELLS) lk_still_kernel(DevLevel I, DevLevel J, LkPrm p, CellGrid g,
                                                                                      vtg_cell *__restrict__ cells, int *hist)
 {
@@ -1074,14 +1091,15 @@ cudaError_t vtg_launch_still_cells(const DevLevel &I, const DevLevel &J, const L
                      : cudaErrorInvalidValue;
 }
 
-template <int MAXH, bool EXACT>
-__global__ void __launch_bounds__(256, 2) lk_points_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp,
-                                                        int top, LkPrm p, int n, const float *__restrict__ xs,
-                                                        const float *__restrict__ ys, const float *__restrict__ gxs,
-                                                        const float *__restrict__ gys, vtg_lk_out *__restrict__ out)
+template <int MAXH, bool EXACT, bool FEW>
+__global__ void __launch_bounds__(32 * LkShape<FEW>::points, LkShape<FEW>::point_ctas)
+    lk_points_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp, int top, LkPrm p, int n, const float *__restrict__ xs,
+                     const float *__restrict__ ys, const float *__restrict__ gxs, const float *__restrict__ gys,
+                     vtg_lk_out *__restrict__ out)
 {
-    extern __shared__ f2_t s_tp[]; /* the template's T: 8 warps x (MAXH / 2) x 32 pairs */
+    extern __shared__ f2_t s_tp[]; /* the template's T: a warp (MAXH / 2) x 32 pairs */
     const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    vtg_grid_dependency_wait(); /* the pyramid or the points, when a kernel made them just before */
     if (i >= n)
         return;
     Patch<MAXH, true> P;
@@ -1126,14 +1144,18 @@ __global__ void __launch_bounds__(256, 2) lk_points_pair_kernel(const DevPyr *__
 cudaError_t vtg_launch_cells(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, const CellGrid &g, int base_w,
                              int base_h, vtg_lk_out *out, vtg_cell *cells, cudaStream_t s)
 {
-    const dim3 blocks((unsigned)((g.cols + 1) / 2) * (unsigned)((g.rows + 1) / 2)), threads(32 * LK_CTA_CELLS);
+    const bool few = lk_few(g.n);
+    const unsigned rows = few ? LkShape<true>::cell_rows : LkShape<false>::cell_rows;
+    const dim3 blocks((unsigned)((g.cols + 1) / 2) * (((unsigned)g.rows + rows - 1) / rows)), threads(32 * 2 * rows);
     auto launch = [&](auto kernel, int maxh) {
-        return vtg_launch_k(kernel, blocks, threads, lk_t_bytes(maxh, LK_CTA_CELLS), s, true, I, J, top, p, g, base_w, base_h, out,
+        return vtg_launch_k(kernel, blocks, threads, lk_t_bytes(maxh, 2 * (int)rows), s, true, I, J, top, p, g, base_w, base_h, out,
                             cells);
     };
-    return p.H == 21   ? launch(lk_cells_kernel<21, true>, 21)
-           : p.H == 15 ? launch(lk_cells_kernel<15, true>, 15)
-                       : launch(lk_cells_kernel<31, false>, 31);
+    if (p.H == 21)
+        return few ? launch(lk_cells_kernel<21, true, true>, 21) : launch(lk_cells_kernel<21, true, false>, 21);
+    if (p.H == 15)
+        return few ? launch(lk_cells_kernel<15, true, true>, 15) : launch(lk_cells_kernel<15, true, false>, 15);
+    return few ? launch(lk_cells_kernel<31, false, true>, 31) : launch(lk_cells_kernel<31, false, false>, 31);
 }
 
 cudaError_t vtg_launch_points(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, int n, const float *xs,
@@ -1152,12 +1174,15 @@ cudaError_t vtg_launch_points(const DevPyr *I, const DevPyr *J, int top, const L
             lk_points_pair_kernel<16><<<pblocks, 256, lk_t_bytes(16, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
         return cudaGetLastError();
     }
-    const int blocks = (n + 7) / 8;
+    const bool few = lk_few(n);
+    const int per = few ? LkShape<true>::points : LkShape<false>::points;
+    auto launch = [&](auto kernel, int maxh) {
+        return vtg_launch_k(kernel, dim3((n + per - 1) / per), dim3(32 * per), lk_t_bytes(maxh, per), s, true, I, J, top, p, n, xs, ys,
+                            gx, gy, out);
+    };
     if (p.H == 21)
-        lk_points_kernel<21, true><<<blocks, 256, lk_t_bytes(21, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
-    else if (p.H == 15)
-        lk_points_kernel<15, true><<<blocks, 256, lk_t_bytes(15, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
-    else
-        lk_points_kernel<31, false><<<blocks, 256, lk_t_bytes(31, 8), s>>>(I, J, top, p, n, xs, ys, gx, gy, out);
-    return cudaGetLastError();
+        return few ? launch(lk_points_kernel<21, true, true>, 21) : launch(lk_points_kernel<21, true, false>, 21);
+    if (p.H == 15)
+        return few ? launch(lk_points_kernel<15, true, true>, 15) : launch(lk_points_kernel<15, true, false>, 15);
+    return few ? launch(lk_points_kernel<31, false, true>, 31) : launch(lk_points_kernel<31, false, false>, 31);
 }
