@@ -160,10 +160,11 @@ __device__ __forceinline__ f2_t get_t(const Patch<MAXH, TS> &P, int r, int lane)
         return P.t[r];
 }
 
+template <int LANES = 32>
 __device__ __forceinline__ float warp_fold(float v)
 {
 #pragma unroll
-    for (int s = 1; s < 32; s <<= 1)
+    for (int s = 1; s < LANES; s <<= 1)
         v = v + __shfl_xor_sync(VTG_FULL, v, s);
     return v;
 }
@@ -787,6 +788,7 @@ __device__ __forceinline__ void store_out(vtg_lk_out *dst, const vtg_lk_out &o, 
 
 /* Mean |J - I| over one cell of level 0, 8-bit grey (still.c:105-114). The differences are whole Q6 numbers, their sum
  * below 2^24, so the F32 sum is exact and the mean is one rounding, as in the reference. */
+template <int LANES = 32>
 __device__ __forceinline__ float cell_diff(const DevLevel &A, const DevLevel &B, int col, int row, const CellGrid &g,
                                            int lane)
 {
@@ -795,12 +797,12 @@ __device__ __forceinline__ float cell_diff(const DevLevel &A, const DevLevel &B,
     /* a cell's row and column of element k: a shift and a mask for power-of-two widths (the 16 x 8 grid) */
     const bool p2 = (g.cell_w & (g.cell_w - 1)) == 0;
     const int sh = __ffs(g.cell_w) - 1;
-    for (int k = lane; k < g.cell_w * (y1 - y0); k += 32) {
+    for (int k = lane; k < g.cell_w * (y1 - y0); k += LANES) {
         const int kr = p2 ? k >> sh : k / g.cell_w, kc = p2 ? k & (g.cell_w - 1) : k % g.cell_w;
         const int yy = y0 + kr, xx = min(x + kc, A.w - 1);
         s += fabsf(__ldg(B.p + (size_t)yy * B.pitch + xx) - __ldg(A.p + (size_t)yy * A.pitch + xx));
     }
-    s = warp_fold(s);
+    s = warp_fold<LANES>(s);
     return __fdiv_rn(s, (float)((y1 - y0) * g.cell_w)) * LK_Q6_INV;
 }
 
@@ -820,8 +822,7 @@ __device__ __forceinline__ void lk_count(unsigned long long *count, unsigned wor
 template <int MAXH, bool EXACT, bool TS>
 __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int top, const LkPrm &p, const CellGrid &g,
                                         int base_w, int base_h, int i, int lane, vtg_lk_out *__restrict__ out,
-                                        vtg_cell *__restrict__ cells, f2_t *ts, unsigned long long *count = nullptr,
-                                        int *hist = nullptr)
+                                        vtg_cell *__restrict__ cells, f2_t *ts, unsigned long long *count = nullptr)
 {
     const int col = i % g.cols, row = i / g.cols;
     const float mx = (float)(p.W / 2 + 2), my = (float)(p.H / 2 + 2);
@@ -847,8 +848,6 @@ __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int to
             c.sigma = o.status ? 0.0f : sqrtf(o.cov_xx + o.cov_yy);
             c.pad = 0.0f;
             cells[i] = c;
-            if (hist)
-                atomicAdd(hist + vtg_still_bin(diff), 1);
         }
     }
 }
@@ -1059,16 +1058,442 @@ cudaError_t vtg_launch_lk_batch(const LkJob *jobs, const int *item_start, int nj
 /* shared memory of a single-stream CTA: its warps' template intensities (at most 30 KB) */
 static constexpr size_t lk_t_bytes(int maxh, int warps) { return sizeof(f2_t) * (size_t)warps * (size_t)(maxh / 2) * 32; }
 
-/* The still picture's vectors (still.cu): one level, its descriptors by value, and the cells' differences counted. Its 15 x 15
- * patch spills nothing at 128 registers. */
-#define LK_CTA_CELLS LkShape<false>::cells
-__global__ void __launch_bounds__(32 * LK_CTA_CELLS, 16 / LK_CTA_CELLS) lk_still_kernel(DevLevel I, DevLevel J, LkPrm p, CellGrid g,
-                                                                                     vtg_cell *__restrict__ cells, int *hist)
+/* Two points a warp, for a patch of 15 x 15: a half-warp holds the patch's 15 columns and the one left of it, so the same
+ * instructions walk two points, and neither leaves 16 lanes idle as a warp a point does. Lane c of a half is window column c
+ * (lk_build's lanes 0 .. 15); window columns 16 and 17, the patch's right border, have no lane: the window pass reads its right
+ * neighbours from memory instead of the next lane, and the build makes S column 16 beforehand, a row a lane, in shared memory.
+ * Every operation, chain and fold is the one a warp a point runs on those columns (its lanes past 15 add +0), so the bits are
+ * the same.
+ *
+ * The warp stays uniform: a branch is taken when either half wants it. A half that does not want a build or a residual pass
+ * runs it at the level's first allowed pixel and drops it; one that needs no window pass repeats its own last one, which
+ * leaves its sums as they were; a half whose walk has ended keeps its state. */
+#ifdef VTG_CHECKED
+#define DUO_CHECK_WINDOW(L, x0, x1, y0, y1, site, ...)                                                                  \
+    do {                                                                                                               \
+        if (__any_sync(VTG_FULL, !((x0) >= 0 && (y0) >= 0 && (x1) < (L).w && (y1) < (L).h))) {                         \
+            if ((threadIdx.x & 31) == 0) {                                                                             \
+                atomicOr(&g_vtg_check[0], site);                                                                       \
+                atomicAdd(&g_vtg_check[1], 1u);                                                                        \
+            }                                                                                                          \
+            __VA_ARGS__;                                                                                               \
+            return;                                                                                                    \
+        }                                                                                                              \
+    } while (0)
+#else
+#define DUO_CHECK_WINDOW(L, x0, x1, y0, y1, site, ...)                                                                  \
+    do {                                                                                                               \
+    } while (0)
+#endif
+#define DUO_M 15
+#define DUO_HH (DUO_M / 2)
+#define DUO_E (DUO_HH + 2) /* row pairs of S column 16: S rows -1 .. HH and HH - 1 .. 2 HH */
+
+/* warp_fold8 and warp_fold2 within each half */
+template <int N>
+__device__ __forceinline__ void duo_fold8(float (&v)[8])
 {
-    extern __shared__ f2_t s_tc[]; /* the template's T: 4 warps x 7 x 32 pairs */
-    __shared__ DevPyr s_pyr[2];    /* the walk indexes its levels */
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, across = (g.cols + 1) / 2;
-    const int col = 2 * ((int)blockIdx.x % across) + (warp & 1), row = 2 * ((int)blockIdx.x / across) + (warp >> 1);
+    const int lane = threadIdx.x & 31;
+    const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+    float a[4], c[2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float keep = b0 ? v[4 + k] : v[k], send = b0 ? v[k] : v[4 + k];
+        a[k] = keep + __shfl_xor_sync(VTG_FULL, send, 1);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float keep = b1 ? a[2 + k] : a[k], send = b1 ? a[k] : a[2 + k];
+        c[k] = keep + __shfl_xor_sync(VTG_FULL, send, 2);
+    }
+    float t = (b2 ? c[1] : c[0]) + __shfl_xor_sync(VTG_FULL, b2 ? c[0] : c[1], 4);
+    t = t + __shfl_xor_sync(VTG_FULL, t, 8);
+#pragma unroll
+    for (int k = 0; k < N; k++)
+        v[k] = __shfl_sync(VTG_FULL, t, (k >> 2) | (((k >> 1) & 1) << 1) | ((k & 1) << 2), 16);
+}
+
+__device__ __forceinline__ void duo_fold2(float &a, float &b)
+{
+#pragma unroll
+    for (int s = 1; s < 16; s <<= 1) {
+        a = a + __shfl_xor_sync(VTG_FULL, a, s);
+        b = b + __shfl_xor_sync(VTG_FULL, b, s);
+    }
+}
+
+/* hlerp2 with the right neighbours from memory */
+__device__ __forceinline__ f2_t duo_hlerp2(const float *pa, const float *pb, f2_t FX)
+{
+    const f2_t l = f2_pack(__ldg(pa), __ldg(pb)), n = f2_pack(__ldg(pa + 1), __ldg(pb + 1));
+    return f2_fma(f2_sub(n, l), FX, l);
+}
+__device__ __forceinline__ float duo_hlerp(const float *p, float fx)
+{
+    const float l = __ldg(p);
+    return __fmaf_rn(__ldg(p + 1) - l, fx, l);
+}
+
+/* lk_build; e: this half's DUO_E pairs of S column 16 */
+__device__ __forceinline__ void duo_build(const DevLevel &L, int ix, float fx, int iy, float fy, int lane, Patch<DUO_M, true> &P,
+                                          f2_t *e, float &gxx, float &gxy, float &gyy, float &tco, float &cxo, float &cyo)
+{
+    constexpr int HH = DUO_HH;
+    const int c = lane & 15, x0 = ix - DUO_M / 2, y0 = iy - DUO_M / 2;
+    DUO_CHECK_WINDOW(L, x0 - 1, x0 + DUO_M + 1, y0 - 1, y0 + DUO_M + 1, 1u, gxx = gxy = gyy = tco = cxo = cyo = 0.0f);
+    const bool act = c >= 1;
+    const float *col = L.p + (size_t)(y0 - 1) * L.pitch + (x0 - 1);
+    float e15; /* S column 16's last row */
+    {
+        const float *q = col + (size_t)c * L.pitch + 16;
+        const float h0 = duo_hlerp(q, fx), h1 = duo_hlerp(q + L.pitch, fx);
+        const float s = __fmaf_rn(h1 - h0, fy, h0); /* S row c - 1 */
+        float *w = reinterpret_cast<float *>(e);
+        __syncwarp(); /* the last build's reads */
+        if (c <= HH + 1)
+            w[2 * c] = s;
+        if (c >= HH)
+            w[2 * (c - HH) + 1] = s;
+        __syncwarp();
+        const float *z = col + (size_t)(DUO_M + 1) * L.pitch + 16;
+        const float g0 = duo_hlerp(z, fx), g1 = duo_hlerp(z + L.pitch, fx);
+        e15 = __fmaf_rn(g1 - g0, fy, g0);
+    }
+    const f2_t FX = f2_pack(fx, fx), FY = f2_pack(fy, fy), TWO = f2_pack(2.0f, 2.0f);
+    const float *pa = col + c, *pb = pa + (size_t)HH * L.pitch;
+    f2_t prev = duo_hlerp2(pa, pb, FX);
+    f2_t u = 0ull, ul = 0ull, ur = 0ull, m = 0ull, ml = 0ull, mr = 0ull, mdx = 0ull, udx = 0ull;
+    f2_t sxx = 0ull, sxy = 0ull, syy = 0ull, scx = 0ull, scy = 0ull, TC = 0ull, hu2 = 0ull, hm2 = 0ull;
+    float tc = 0.0f;
+#pragma unroll
+    for (int t = 0; t < HH + 2; t++) {
+        pa += L.pitch;
+        pb += L.pitch;
+        const f2_t cur = duo_hlerp2(pa, pb, FX);
+        const f2_t d = f2_fma(f2_sub(cur, prev), FY, prev);
+        prev = cur;
+        float dlo, dhi, elo, ehi;
+        f2_split(d, dlo, dhi);
+        f2_split(e[t], elo, ehi);
+        const f2_t dl = f2_pack(__shfl_up_sync(VTG_FULL, dlo, 1, 16), __shfl_up_sync(VTG_FULL, dhi, 1, 16));
+        const float nlo = __shfl_down_sync(VTG_FULL, dlo, 1, 16), nhi = __shfl_down_sync(VTG_FULL, dhi, 1, 16);
+        const f2_t dr = f2_pack(c == 15 ? elo : nlo, c == 15 ? ehi : nhi);
+        const f2_t ddx = f2_sub(dr, dl);
+        if (t >= 2) {
+            const int k = t - 2; /* rows k and HH + k */
+            const f2_t tx = f2_fma(mdx, TWO, f2_add(udx, ddx));
+            const f2_t ty = f2_sub(f2_fma(d, TWO, f2_add(dl, dr)), hu2);
+            if (k == 0) {
+                float mlo, mhi;
+                f2_split(m, mlo, mhi);
+                tc = __shfl_sync(VTG_FULL, mlo, DUO_M / 2 + 1, 16);
+                TC = f2_pack(tc, tc);
+            }
+            put_t(P, k, lane, m);
+            P.tx[k] = tx;
+            P.ty[k] = ty;
+            sxx = f2_fma(tx, tx, sxx);
+            sxy = f2_fma(tx, ty, sxy);
+            syy = f2_fma(ty, ty, syy);
+            const f2_t tt = f2_sub(m, TC);
+            scx = f2_fma(tt, tx, scx);
+            scy = f2_fma(tt, ty, scy);
+        }
+        hu2 = hm2; hm2 = f2_fma(d, TWO, f2_add(dl, dr));
+        u = m; ul = ml; ur = mr; udx = mdx;
+        m = d; ml = dl; mr = dr; mdx = ddx;
+    }
+    float fv[8] = {f2_sum(sxx), f2_sum(sxy), f2_sum(syy), f2_sum(scx), f2_sum(scy), 0.0f, 0.0f, 0.0f};
+    {
+        const float c1 = duo_hlerp(pb + L.pitch, fx);
+        const float p1 = f2_hi(prev);
+        const float d = __fmaf_rn(c1 - p1, fy, p1);
+        const float dl = __shfl_up_sync(VTG_FULL, d, 1, 16), nr = __shfl_down_sync(VTG_FULL, d, 1, 16);
+        const float dr = c == 15 ? e15 : nr;
+        const float tx = __fmaf_rn(f2_hi(mdx), 2.0f, f2_hi(udx) + (dr - dl));
+        const float ty = __fmaf_rn(d - f2_hi(u), 2.0f, (dl - f2_hi(ul)) + (dr - f2_hi(ur)));
+        const float mt = f2_hi(m);
+        P.tl = mt;
+        P.txl = tx;
+        P.tyl = ty;
+        fv[0] = __fmaf_rn(tx, tx, fv[0]);
+        fv[1] = __fmaf_rn(tx, ty, fv[1]);
+        fv[2] = __fmaf_rn(ty, ty, fv[2]);
+        fv[3] = __fmaf_rn(mt - tc, tx, fv[3]);
+        fv[4] = __fmaf_rn(mt - tc, ty, fv[4]);
+    }
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+        fv[k] = act ? fv[k] : 0.0f;
+    duo_fold8<5>(fv);
+    gxx = fv[0] * (LK_GRAD_SCALE * LK_GRAD_SCALE);
+    gxy = fv[1] * (LK_GRAD_SCALE * LK_GRAD_SCALE);
+    gyy = fv[2] * (LK_GRAD_SCALE * LK_GRAD_SCALE);
+    tco = tc;
+    cxo = fv[3];
+    cyo = fv[4];
+}
+
+/* lk_correlate */
+__device__ __forceinline__ void duo_correlate(const DevLevel &L, int jx, int jy, int lane, const Patch<DUO_M, true> &P, float tc,
+                                              float (&X)[8])
+{
+    constexpr int HH = DUO_HH;
+    const int c = lane & 15, x0 = jx - DUO_M / 2, y0 = jy - DUO_M / 2;
+    DUO_CHECK_WINDOW(L, x0 - 1, x0 + DUO_M, y0, y0 + DUO_M, 2u, for (int k = 0; k < 8; k++) X[k] = 0.0f);
+    const bool act = c >= 1;
+    const float *ra = L.p + (size_t)y0 * L.pitch + (x0 - 1 + c), *rb = ra + (size_t)HH * L.pitch;
+    const f2_t M = f2_pack(-tc, -tc);
+    f2_t pl = f2_add(f2_pack(__ldg(ra), __ldg(rb)), M), pn = f2_add(f2_pack(__ldg(ra + 1), __ldg(rb + 1)), M);
+    f2_t a00 = 0ull, a10 = 0ull, a01 = 0ull, a11 = 0ull, b00 = 0ull, b10 = 0ull, b01 = 0ull, b11 = 0ull;
+#pragma unroll
+    for (int r = 0; r < HH; r++) {
+        ra += L.pitch;
+        rb += L.pitch;
+        const f2_t cl = f2_add(f2_pack(__ldg(ra), __ldg(rb)), M), cn = f2_add(f2_pack(__ldg(ra + 1), __ldg(rb + 1)), M);
+        a00 = f2_fma(pl, P.tx[r], a00);
+        a10 = f2_fma(pn, P.tx[r], a10);
+        a01 = f2_fma(cl, P.tx[r], a01);
+        a11 = f2_fma(cn, P.tx[r], a11);
+        b00 = f2_fma(pl, P.ty[r], b00);
+        b10 = f2_fma(pn, P.ty[r], b10);
+        b01 = f2_fma(cl, P.ty[r], b01);
+        b11 = f2_fma(cn, P.ty[r], b11);
+        pl = cl;
+        pn = cn;
+    }
+    {
+        const float l = __ldg(rb + L.pitch) - tc, n = __ldg(rb + L.pitch + 1) - tc;
+        const float ol = f2_hi(pl), on = f2_hi(pn);
+        X[0] = __fmaf_rn(ol, P.txl, f2_sum(a00));
+        X[1] = __fmaf_rn(on, P.txl, f2_sum(a10));
+        X[2] = __fmaf_rn(l, P.txl, f2_sum(a01));
+        X[3] = __fmaf_rn(n, P.txl, f2_sum(a11));
+        X[4] = __fmaf_rn(ol, P.tyl, f2_sum(b00));
+        X[5] = __fmaf_rn(on, P.tyl, f2_sum(b10));
+        X[6] = __fmaf_rn(l, P.tyl, f2_sum(b01));
+        X[7] = __fmaf_rn(n, P.tyl, f2_sum(b11));
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        X[k] = act ? X[k] : 0.0f;
+    duo_fold8<8>(X);
+}
+
+/* lk_sample's residual sums */
+__device__ __forceinline__ void duo_resid(const DevLevel &L, int jx, float fx, int jy, float fy, int lane,
+                                          const Patch<DUO_M, true> &P, float &b0, float &b1)
+{
+    constexpr int HH = DUO_HH;
+    const int c = lane & 15, x0 = jx - DUO_M / 2, y0 = jy - DUO_M / 2;
+    DUO_CHECK_WINDOW(L, x0 - 1, x0 + DUO_M, y0, y0 + DUO_M, 4u, b0 = b1 = 0.0f);
+    const float q6 = c >= 1 ? LK_Q6_INV : 0.0f;
+    const float *ra = L.p + (size_t)y0 * L.pitch + (x0 - 1 + c), *rb = ra + (size_t)HH * L.pitch;
+    const f2_t FX = f2_pack(fx, fx), FY = f2_pack(fy, fy), Q = f2_pack(q6, q6);
+    f2_t prev = duo_hlerp2(ra, rb, FX);
+    f2_t s0 = 0ull, s1 = 0ull;
+#pragma unroll
+    for (int r = 0; r < HH; r++) {
+        ra += L.pitch;
+        rb += L.pitch;
+        const f2_t cur = duo_hlerp2(ra, rb, FX);
+        const f2_t g = f2_mul(f2_sub(get_t(P, r, lane), f2_fma(f2_sub(cur, prev), FY, prev)), Q);
+        prev = cur;
+        s0 = f2_add(s0, f2_abs(g));
+        s1 = f2_fma(g, g, s1);
+    }
+    float t0 = f2_sum(s0), t1 = f2_sum(s1);
+    const float cur = duo_hlerp(rb + L.pitch, fx);
+    const float pb = f2_hi(prev);
+    const float g = (P.tl - __fmaf_rn(cur - pb, fy, pb)) * q6;
+    b0 = t0 + fabsf(g);
+    b1 = __fmaf_rn(g, g, t1);
+    duo_fold2(b0, b1);
+}
+
+/* lk_track for the two halves' points; live: this half has one to walk */
+__device__ __forceinline__ void duo_track(const DevPyr &I, const DevPyr &J, int top, const LkPrm &p, float x, float y, float gx0,
+                                          float gy0, bool live, int lane, Patch<DUO_M, true> &P, f2_t *e, vtg_lk_out &o)
+{
+    constexpr int mx = DUO_M / 2 + 1, my = mx;
+    const float stop = __int_as_float((127 - top) << 23);
+    float gx = gx0 * stop, gy = gy0 * stop;
+    int status = 0, iters = 0;
+    bool valid0 = false;
+    float eig0 = 0.0f, idet0 = 0.0f, gxx0 = 0.0f, gxy0 = 0.0f, gyy0 = 0.0f;
+    for (int L = top; L >= 0; L--) {
+        const DevLevel IL = I.l[L], JL = J.l[L];
+        const float sl = __int_as_float((127 - L) << 23);
+        const float px = x * sl, py = y * sl;
+        bool on = live && px >= (float)mx && py >= (float)my && px < (float)(IL.w - mx - 1) && py < (float)(IL.h - my - 1);
+        if (L == 0 && !on)
+            status |= VTG_LK_OUT;
+        if (__any_sync(VTG_FULL, on)) {
+            const float fpx = on ? floorf(px) : (float)mx, fpy = on ? floorf(py) : (float)my;
+            const int bx = (int)fpx, by = (int)fpy;
+            const float rx = on ? px - fpx : 0.0f, ry = on ? py - fpy : 0.0f;
+            float gxx, gxy, gyy, tc, cx, cy;
+            duo_build(IL, bx, rx, by, ry, lane, P, e, gxx, gxy, gyy, tc, cx, cy);
+            const float w2 = gxy * gxy;
+            const float e2 = __fmaf_rn(gxy, gxy, -w2);
+            const float det = __fmaf_rn(gxx, gyy, -w2) - e2;
+            const float tr = gxx + gyy, df = gxx - gyy;
+            const float root = sqrtf(__fmaf_rn(df, df, 4.0f * w2));
+            const float lmax = 0.5f * (tr + root);
+            const float eig = lmax > 0.0f ? __fdividef(det, lmax * p.area) : 0.0f;
+            if (L == 0 && on)
+                eig0 = eig;
+            if (on && (eig < p.min_eig || det <= 0.0f)) {
+                if (L == 0)
+                    status |= VTG_LK_LOWEIG;
+                on = false;
+            }
+            const float idet = __frcp_rn(det);
+            if (L == 0 && on) {
+                idet0 = idet;
+                gxx0 = gxx;
+                gxy0 = gxy;
+                gyy0 = gyy;
+                valid0 = true;
+            }
+            const float ia = gyy * idet * LK_Q6_INV * LK_GRAD_SCALE, ib = -gxy * idet * LK_Q6_INV * LK_GRAD_SCALE,
+                        ic = gxx * idet * LK_Q6_INV * LK_GRAD_SCALE;
+            const float lo_x = (float)(mx - bx), lo_y = (float)(my - by);
+            const float hi_x = (float)(JL.w - mx - 1 - bx), hi_y = (float)(JL.h - my - 1 - by);
+            float vx = 0.0f, vy = 0.0f;
+            float X[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            float cfx = __int_as_float(0x7fffffff), cfy = cfx;
+            int jx = mx, jy = my;
+            bool run = on;
+            for (int it = 0; it < p.max_iter && __any_sync(VTG_FULL, run); it++) {
+                const float qx = (rx + gx) + vx, qy = (ry + gy) + vy;
+                float fx = qx - cfx, fy = qy - cfy;
+                const bool cross = run && !(fx >= 0.0f && fy >= 0.0f && fx < 1.0f && fy < 1.0f);
+                if (__any_sync(VTG_FULL, cross)) {
+                    const bool in = qx >= lo_x && qy >= lo_y && qx < hi_x && qy < hi_y;
+                    if (cross && !in) {
+                        if (L == 0) {
+                            status |= VTG_LK_OUT;
+                            valid0 = false;
+                        }
+                        run = false;
+                    }
+                    if (cross && in) {
+                        cfx = floorf(qx);
+                        cfy = floorf(qy);
+                        fx = qx - cfx;
+                        fy = qy - cfy;
+                        jx = bx + (int)cfx;
+                        jy = by + (int)cfy;
+                    }
+                    if (__any_sync(VTG_FULL, cross && in)) {
+                        duo_correlate(JL, jx, jy, lane, P, tc, X);
+                        lk_phase_diffs(X);
+                    }
+                }
+                const float sx = lk_at_phase(X, cx, fx, fy), sy = lk_at_phase(X + 4, cy, fx, fy);
+                const float ex = __fmaf_rn(ia, sx, ib * sy), ey = __fmaf_rn(ib, sx, ic * sy);
+                if (run) {
+                    vx += ex;
+                    vy += ey;
+                    iters++;
+                    run = !(__fmaf_rn(ex, ex, ey * ey) < p.eps2);
+                }
+            }
+            if (on) {
+                gx += vx;
+                gy += vy;
+            }
+        }
+        if (L > 0) {
+            gx *= 2.0f;
+            gy *= 2.0f;
+        }
+    }
+    o.x = x + gx;
+    o.y = y + gy;
+    o.min_eig = eig0;
+    o.iters = (uint16_t)iters;
+    o.residual = 0.0f;
+    o.cov_xx = o.cov_xy = o.cov_yy = 0.0f;
+    const DevLevel J0 = J.l[0];
+    const float fx0 = floorf(x), fy0 = floorf(y);
+    const int bx = (int)fx0, by = (int)fy0;
+    const float qx = (x - fx0) + gx, qy = (y - fy0) + gy;
+    bool good = valid0 && !status;
+    if (good && !(qx >= (float)(mx - bx) && qy >= (float)(my - by) && qx < (float)(J0.w - mx - 1 - bx) &&
+                  qy < (float)(J0.h - my - 1 - by))) {
+        status |= VTG_LK_OUT;
+        good = false;
+    }
+    if (__any_sync(VTG_FULL, good)) {
+        int jx = mx, jy = my;
+        float fx = 0.0f, fy = 0.0f;
+        if (good) {
+            split(bx, qx, jx, fx);
+            split(by, qy, jy, fy);
+        }
+        float sa, ss;
+        duo_resid(J0, jx, fx, jy, fy, lane, P, sa, ss);
+        if (good) {
+            const float r0 = sa / p.area, r1 = ss / p.area;
+            o.residual = r0;
+            if (r0 > p.max_residual)
+                status |= VTG_LK_RESIDUAL;
+            const float s2 = r1 * p.area / (p.area - 2.0f);
+            o.cov_xx = s2 * gyy0 * idet0;
+            o.cov_xy = -s2 * gxy0 * idet0;
+            o.cov_yy = s2 * gxx0 * idet0;
+        }
+    }
+    o.status = (uint16_t)status;
+}
+
+/* lk_point */
+__device__ __forceinline__ void duo_point(const DevPyr &I, const DevPyr &J, int top, const LkPrm &p, float x, float y, float gx,
+                                          float gy, bool live, int lane, Patch<DUO_M, true> &P, f2_t *e, vtg_lk_out &o)
+{
+    const int passes = p.fb_max2 > 0.0f ? 2 : 1;
+    float sx = x, sy = y;
+    for (int pass = 0; pass < passes; pass++) {
+        vtg_lk_out r;
+        duo_track(pass ? J : I, pass ? I : J, top, p, sx, sy, gx, gy, live, lane, P, e, r);
+        if (pass == 0) {
+            o = r;
+            live = live && !o.status;
+            if (!__any_sync(VTG_FULL, live))
+                break;
+            sx = o.x;
+            sy = o.y;
+            gx = x - o.x;
+            gy = y - o.y;
+        } else if (live) {
+            const float ex = r.x - x, ey = r.y - y;
+            if (r.status || !(__fmaf_rn(ex, ex, ey * ey) <= p.fb_max2))
+                o.status |= VTG_LK_FLOWBACK;
+        }
+    }
+}
+
+/* The still picture's vectors (still.cu): one level, its descriptors by value, and the cells' differences counted. A warp takes two
+ * cells of a row, a CTA DUO_ACROSS x DUO_DOWN of these pairs. Bound as the other walks are, by the latency of their chains at 16
+ * warps an SM and the instructions a cell takes; half a warp a cell takes a little over half of them. A 1920 x 1080 frame (this
+ * and the decision), us: one stream 83 with a warp a cell, 62 now; three streams' frames together 66 and 46. Five CTAs an SM (96
+ * registers) 47, pairs one across and four down 47, one across and two down the same as 2 x 2. */
+#define DUO_ACROSS 2
+#define DUO_DOWN 2
+#define DUO_CTAS 4 /* an SM: 128 registers a thread */
+#define DUO_WARPS (DUO_ACROSS * DUO_DOWN)
+__global__ void __launch_bounds__(32 * DUO_WARPS, DUO_CTAS) lk_still_kernel(DevLevel I, DevLevel J, LkPrm p, CellGrid g,
+                                                                         vtg_cell *__restrict__ cells, int *hist)
+{
+    __shared__ f2_t s_t[DUO_WARPS][DUO_HH][32]; /* the templates' T */
+    __shared__ f2_t s_e[DUO_WARPS][2][DUO_E];
+    __shared__ DevPyr s_pyr[2]; /* the walk indexes its levels */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
+    const int across = (g.cols + 2 * DUO_ACROSS - 1) / (2 * DUO_ACROSS);
+    const int col = 2 * (DUO_ACROSS * ((int)blockIdx.x % across) + warp % DUO_ACROSS) + half;
+    const int row = DUO_DOWN * ((int)blockIdx.x / across) + warp / DUO_ACROSS;
     if (threadIdx.x == 0) {
         s_pyr[0].l[0] = I;
         s_pyr[1].l[0] = J;
@@ -1076,19 +1501,40 @@ __global__ void __launch_bounds__(32 * LK_CTA_CELLS, 16 / LK_CTA_CELLS) lk_still
     __syncthreads();
     vtg_grid_launch_dependents();
     vtg_grid_dependency_wait(); /* the mean, when its kernel is the one before on the stream */
-    if (col >= g.cols || row >= g.rows)
+    if (col - half >= g.cols || row >= g.rows)
         return;
-    lk_cell<15, true, true>(s_pyr[0], s_pyr[1], 0, p, g, I.w, I.h, row * g.cols + col, lane, nullptr, cells,
-                            s_tc + (size_t)warp * 7 * 32, nullptr, hist);
+    /* the cell's centre and record: lk_cell's */
+    const bool live = col < g.cols;
+    const float mx = (float)(DUO_M / 2 + 2), my = mx;
+    float x = (float)(col * g.cell_w + g.cell_w / 2), y = (float)(row * g.cell_h + g.cell_h / 2);
+    x = fminf(fmaxf(x, mx), (float)I.w - 1.0f - mx);
+    y = fminf(fmaxf(y, my), (float)I.h - 1.0f - my);
+    Patch<DUO_M, true> P;
+    P.ts = &s_t[warp][0][0];
+    vtg_lk_out o;
+    duo_point(s_pyr[0], s_pyr[1], 0, p, x, y, 0.0f, 0.0f, live, lane, P, s_e[warp][half], o);
+    const float diff = cell_diff<16>(I, J, min(col, g.cols - 1), row, g, lane & 15);
+    if (live && (lane & 15) == 0) {
+        vtg_cell c;
+        c.u = o.x - x;
+        c.v = o.y - y;
+        c.diff = diff;
+        c.state = o.status;
+        c.sigma = o.status ? 0.0f : sqrtf(o.cov_xx + o.cov_yy);
+        c.pad = 0.0f;
+        cells[row * g.cols + col] = c;
+        if (hist)
+            atomicAdd(hist + vtg_still_bin(diff), 1);
+    }
 }
 
 cudaError_t vtg_launch_still_cells(const DevLevel &I, const DevLevel &J, const LkPrm &p, const CellGrid &g, vtg_cell *cells,
                                    int *hist, cudaStream_t s)
 {
-    const unsigned blocks = (unsigned)((g.cols + 1) / 2) * (unsigned)((g.rows + 1) / 2);
-    return p.H == 15 ? vtg_launch_k(lk_still_kernel, dim3(blocks), dim3(32 * LK_CTA_CELLS), lk_t_bytes(15, LK_CTA_CELLS), s, true, I, J,
-                                    p, g, cells, hist)
-                     : cudaErrorInvalidValue;
+    const unsigned blocks = (unsigned)((g.cols + 2 * DUO_ACROSS - 1) / (2 * DUO_ACROSS)) * (unsigned)((g.rows + DUO_DOWN - 1) / DUO_DOWN);
+    return p.H == DUO_M && p.W == DUO_M
+               ? vtg_launch_k(lk_still_kernel, dim3(blocks), dim3(32 * DUO_WARPS), 0, s, true, I, J, p, g, cells, hist)
+               : cudaErrorInvalidValue;
 }
 
 template <int MAXH, bool EXACT, bool FEW>
