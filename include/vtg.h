@@ -96,7 +96,9 @@ int vtg_check_read(uint32_t *out);
 
 /* ---- a tracker: one camera stream's device-resident state (tk_create, src/kern/track.h:22 / track.c:447-572) ---- */
 
-/* Device bytes one tracker of this configuration holds: two pyramid sets, a frame staging buffer, the cell results. */
+/* Device bytes one tracker of this configuration is charged: two pyramid sets, a frame staging buffer, the cell results. In a
+ * context without a budget a frame 256 to 2,080 pixels wide may hold more, as its rows then lie 2,080 floats apart on every
+ * level (vtg_level_device's pitch); such padding is not counted in vtg_ctx_used, and is at most 16 GiB a context. */
 size_t vtg_tracker_bytes(const struct vtg_config *cfg);
 int vtg_tracker_create(vtg_ctx *ctx, const struct vtg_config *cfg, vtg_tracker **out);
 void vtg_tracker_destroy(vtg_tracker *t);

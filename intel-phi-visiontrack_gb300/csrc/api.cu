@@ -34,7 +34,7 @@ void vtg_set_cuda_error(cudaError_t e) { g_last_cuda = (int)e; }
 
 struct vtg_ctx {
     int device;
-    size_t budget, used;
+    size_t budget, used, padding; /* padding: the trackers' rows past their compact layout, not in used */
     std::mutex mu;
     std::vector<vtg_tracker *> trackers;
     std::vector<cudaStream_t> streams; /* of the other objects (search contexts, batches) */
@@ -107,7 +107,7 @@ extern "C" int vtg_ctx_create(int device, size_t hbm_budget, vtg_ctx **out)
         return VTG_ENOMEM;
     c->device = device;
     c->budget = hbm_budget;
-    c->used = 0;
+    c->used = c->padding = 0;
     *out = c;
     return VTG_OK;
 }
@@ -192,14 +192,22 @@ struct Layout {
 
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-static void layout(const vtg_config *c, Layout *L)
+/* Two layouts of a tracker's planes. Compact: each level's rows as far apart as its width asks. Wide: every level of a frame at
+ * most VTG_LK_PITCH pixels wide at that one pitch, which the LK kernels are compiled for (lk.cu: a tenth of their time). Wide
+ * holds more memory (a 1080p tracker of four levels 38.8 MB for 27.0, 640 x 480 15 for 4), so a tracker has it only in a context
+ * without a budget, while the context's padding stays below VTG_PADDING_MAX, and where the device has the room; the budget's
+ * count is the compact size's. Frames under 256 pixels wide, more than eight times their size at that pitch, stay compact. */
+#define VTG_PADDING_MAX ((size_t)16 << 30)
+static bool wide_fits(const vtg_config *c) { return c->width >= 256 && c->width <= VTG_LK_PITCH; }
+
+static void layout(const vtg_config *c, bool wide, Layout *L)
 {
     int w = (int)c->width, h = (int)c->height;
     size_t off = 0;
     for (int i = 0; i < (int)c->levels; i++) {
         L->lw[i] = w;
         L->lh[i] = h;
-        L->lpitch[i] = vtg_pitch(w);
+        L->lpitch[i] = wide ? VTG_LK_PITCH : vtg_pitch(w);
         L->loff[i] = off;
         off += up256((size_t)L->lpitch[i] * (size_t)h * sizeof(float)) / sizeof(float);
         w = (w + 1) / 2;
@@ -232,7 +240,7 @@ extern "C" size_t vtg_tracker_bytes(const vtg_config *cfg)
     if (check_config(cfg) != VTG_OK)
         return 0;
     Layout L;
-    layout(cfg, &L);
+    layout(cfg, false, &L);
     return L.bytes;
 }
 
@@ -263,23 +271,50 @@ extern "C" int vtg_tracker_create(vtg_ctx *ctx, const vtg_config *cfg, vtg_track
     const int chk = check_config(cfg);
     if (chk != VTG_OK)
         return chk;
-    Layout L;
-    layout(cfg, &L);
+    Layout L, wide;
+    layout(cfg, false, &L);
+    layout(cfg, true, &wide);
+    const size_t bytes = L.bytes;
+    size_t padding = wide_fits(cfg) ? wide.bytes - bytes : 0;
     {
         std::lock_guard<std::mutex> g(ctx->mu);
-        if (ctx->budget && ctx->used + L.bytes > ctx->budget)
+        if (ctx->budget && ctx->used + bytes > ctx->budget)
             return VTG_EBUDGET;
-        ctx->used += L.bytes;
+        ctx->used += bytes;
+        if (ctx->budget || ctx->padding + padding > VTG_PADDING_MAX)
+            padding = 0;
+        ctx->padding += padding;
     }
     vtg_tracker *t = new (std::nothrow) vtg_tracker;
     auto undo = [&](int code) {
         std::lock_guard<std::mutex> g(ctx->mu);
-        ctx->used -= L.bytes;
+        ctx->used -= bytes;
+        ctx->padding -= padding;
         delete t;
         return code;
     };
     if (!t)
         return undo(VTG_ENOMEM);
+    if (cudaSetDevice(ctx->device) != cudaSuccess)
+        return undo(VTG_ECUDA);
+    cudaError_t e = cudaSuccess;
+    if (padding) {
+        e = cudaMalloc(&t->mem, wide.bytes);
+        if (e == cudaSuccess) {
+            L = wide;
+        } else { /* the compact layout may still fit */
+            cudaGetLastError();
+            std::lock_guard<std::mutex> g(ctx->mu);
+            ctx->padding -= padding;
+            padding = 0;
+        }
+    }
+    if (!padding)
+        e = cudaMalloc(&t->mem, bytes);
+    if (e != cudaSuccess) {
+        g_last_cuda = (int)e;
+        return undo(VTG_ENOMEM);
+    }
     t->ctx = ctx;
     t->cfg = *cfg;
     t->levels = (int)cfg->levels;
@@ -292,14 +327,8 @@ extern "C" int vtg_tracker_create(vtg_ctx *ctx, const vtg_config *cfg, vtg_track
         t->loff[i] = i < t->levels ? L.loff[i] : 0;
     }
     t->set_floats = L.set_floats;
-    t->bytes = L.bytes;
-    if (cudaSetDevice(ctx->device) != cudaSuccess)
-        return undo(VTG_ECUDA);
-    cudaError_t e = cudaMalloc(&t->mem, L.bytes);
-    if (e != cudaSuccess) {
-        g_last_cuda = (int)e;
-        return undo(VTG_ENOMEM);
-    }
+    t->bytes = bytes;
+    t->padding = padding;
     e = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         cudaFree(t->mem);
@@ -343,6 +372,10 @@ extern "C" int vtg_tracker_create(vtg_ctx *ctx, const vtg_config *cfg, vtg_track
     t->prm.max_residual = cfg->max_residual;
     t->prm.fb_max2 = cfg->fb_max > 0.0f ? cfg->fb_max * cfg->fb_max : 0.0f;
     t->prm.area = (float)(cfg->patch_w * cfg->patch_h);
+    t->prm.pitch = VTG_LK_PITCH;
+    for (int i = 0; i < t->levels; i++)
+        if (t->lpitch[i] != VTG_LK_PITCH)
+            t->prm.pitch = 0;
     {
         std::lock_guard<std::mutex> g(ctx->mu);
         ctx->trackers.push_back(t);
@@ -364,6 +397,7 @@ extern "C" void vtg_tracker_destroy(vtg_tracker *t)
     {
         std::lock_guard<std::mutex> g(ctx->mu);
         ctx->used -= t->bytes;
+        ctx->padding -= t->padding;
         for (size_t i = 0; i < ctx->trackers.size(); i++)
             if (ctx->trackers[i] == t) {
                 ctx->trackers.erase(ctx->trackers.begin() + (long)i);

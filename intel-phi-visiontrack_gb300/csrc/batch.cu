@@ -306,6 +306,9 @@ extern "C" int vtg_batch_prepare(vtg_batch *b, int slot, int n, vtg_tracker *con
     sl.njobs = n;
     sl.max_levels = max_levels;
     sl.prm = trackers[0]->prm;
+    for (int j = 1; j < n; j++) /* one launch for all: the fixed pitch only when every stream has it */
+        if (trackers[j]->prm.pitch != sl.prm.pitch)
+            sl.prm.pitch = 0;
     CU(cudaSetDevice(vtg_ctx_device(b->ctx)));
     CU(cudaMemcpyAsync(sl.d_pyr, pj.data(), sizeof(PyrJob) * (size_t)n, cudaMemcpyHostToDevice, b->stream));
     CU(cudaMemcpyAsync(sl.d_tiles, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice, b->stream));

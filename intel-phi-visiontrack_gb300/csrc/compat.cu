@@ -136,6 +136,7 @@ LkPrm lk_prm(const vtg_ref_lk_cfg *c, float fb_max)
     p.max_residual = c->max_residual;
     p.fb_max2 = fb_max > 0.0f ? fb_max * fb_max : 0.0f;
     p.area = (float)(c->w * c->h);
+    p.pitch = 0;
     return p;
 }
 

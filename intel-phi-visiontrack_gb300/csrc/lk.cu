@@ -132,8 +132,12 @@ __device__ __forceinline__ f2_t f2_abs(f2_t v) { return v & 0x7fffffff7ffffffful
 /* The template of the current level, patch rows paired as (r, HH + r), HH = MAXH / 2, so the sample walks the top and
  * bottom halves of the patch together; an odd MAXH's last row (2 HH) is kept apart. Tx, Ty are the unscaled Sobel sums
  * (the 1/512 is applied to the folded sums, an exact power of two). T is in registers or, with TS, in this warp's
- * rows of shared memory ([HH][32] pairs: a lane reads only what it wrote). */
-template <int MAXH, bool TS>
+ * rows of shared memory ([HH][32] pairs: a lane reads only what it wrote).
+ *
+ * PITCH: the levels' row pitch when it is VTG_LK_PITCH on every level of both pyramids, else 0 (each level's own). With a pitch
+ * known here a pass's rows are immediate offsets of one address, where every row took an addition of 64 bits: a tenth of the
+ * walk's time. Measured: 8 x 1080p cells in one launch 1.7015 -> 1.5416 ms, a 1080p pair 0.234 -> 0.215, the same bits. */
+template <int MAXH, bool TS, int PITCH = 0>
 struct Patch {
     static constexpr int HH = MAXH / 2;
     f2_t tx[HH], ty[HH];
@@ -142,8 +146,8 @@ struct Patch {
     f2_t *ts;
 };
 
-template <int MAXH, bool TS>
-__device__ __forceinline__ void put_t(Patch<MAXH, TS> &P, int r, int lane, f2_t v)
+template <int MAXH, bool TS, int PITCH>
+__device__ __forceinline__ void put_t(Patch<MAXH, TS, PITCH> &P, int r, int lane, f2_t v)
 {
     if constexpr (TS)
         P.ts[r * 32 + lane] = v;
@@ -151,8 +155,8 @@ __device__ __forceinline__ void put_t(Patch<MAXH, TS> &P, int r, int lane, f2_t 
         P.t[r] = v;
 }
 
-template <int MAXH, bool TS>
-__device__ __forceinline__ f2_t get_t(const Patch<MAXH, TS> &P, int r, int lane)
+template <int MAXH, bool TS, int PITCH>
+__device__ __forceinline__ f2_t get_t(const Patch<MAXH, TS, PITCH> &P, int r, int lane)
 {
     if constexpr (TS)
         return P.ts[r * 32 + lane];
@@ -236,13 +240,13 @@ __device__ __forceinline__ f2_t hlerp2(const float *pa, const float *pb, f2_t FX
  * .. 2 HH) run as the two halves of packed pairs, each with its own three-row window, so each pair of rows lands in
  * the patch's pair register directly; an odd height's last row continues the bottom half. Not EXACT: rows from H on
  * read the last image row again and are zero in Tx, Ty. */
-template <int MAXH, bool EXACT, bool TS>
+template <int MAXH, bool EXACT, bool TS, int PITCH>
 __device__ __forceinline__ void lk_build(const DevLevel &L, int ix, float fx, int iy, float fy, int W, int Hr, int lane,
-                                         Patch<MAXH, TS> &P, float &gxx, float &gxy, float &gyy, float &tco,
+                                         Patch<MAXH, TS, PITCH> &P, float &gxx, float &gxy, float &gyy, float &tco,
                                          float &cxo, float &cyo)
 {
     constexpr int HH = MAXH / 2;
-    const int H = EXACT ? MAXH : Hr;
+    const int H = EXACT ? MAXH : Hr, pitch = PITCH ? PITCH : L.pitch;
     const int x0 = ix - W / 2, y0 = iy - H / 2;
     LK_CHECK_WINDOW(L, x0 - 1, x0 + W + 1, y0 - 1, y0 + H + 1, 1u, gxx = gxy = gyy = tco = cxo = cyo = 0.0f);
     /* Lane c samples window column c - 1 (c = 0 .. W + 1; lane W + 2 feeds lane W + 1's right neighbour; the lanes past
@@ -251,7 +255,7 @@ __device__ __forceinline__ void lk_build(const DevLevel &L, int ix, float fx, in
     const bool act = lane >= 1 && lane <= W;
     const float *col = L.p + (x0 - 1 + min(lane, W + 2));
     /* image row y0 + r, r in -1 .. H + 1 (rows past that are read as row H + 1) */
-    auto img = [&](int r) { return col + (size_t)(y0 + (EXACT ? r : min(r, H + 1))) * L.pitch; };
+    auto img = [&](int r) { return col + (size_t)(y0 + (EXACT ? r : min(r, H + 1))) * pitch; };
     const f2_t FX = f2_pack(fx, fx), FY = f2_pack(fy, fy), TWO = f2_pack(2.0f, 2.0f);
     const float *pa = img(-1), *pb = img(HH - 1);
     f2_t prev = hlerp2(pa, pb, FX);
@@ -263,8 +267,8 @@ __device__ __forceinline__ void lk_build(const DevLevel &L, int ix, float fx, in
     for (int t = 0; t < HH + 2; t++) {
         if (EXACT || t < H + 2) {
             if (EXACT) {
-                pa += L.pitch;
-                pb += L.pitch;
+                pa += pitch;
+                pb += pitch;
             } else {
                 pa = img(t);
                 pb = img(HH + t);
@@ -313,7 +317,7 @@ __device__ __forceinline__ void lk_build(const DevLevel &L, int ix, float fx, in
     if constexpr ((MAXH & 1) != 0) {
         /* the last row, 2 HH: one more step of the bottom half (S row 2 HH + 1, image rows H, H + 1) */
         if (EXACT || H == MAXH) {
-            const float c1 = hlerp(EXACT ? pb + L.pitch : img(H + 1), fx);
+            const float c1 = hlerp(EXACT ? pb + pitch : img(H + 1), fx);
             const float p1 = f2_hi(prev);
             const float d = __fmaf_rn(c1 - p1, fy, p1);
             const float dl = __shfl_up_sync(VTG_FULL, d, 1), dr = __shfl_down_sync(VTG_FULL, d, 1);
@@ -371,18 +375,18 @@ __device__ __forceinline__ void lk_build(const DevLevel &L, int ix, float fx, in
  * (X[4..7]); every iteration that stays at the same whole pixel then needs only these eight numbers. Subtracting tc
  * keeps the sums near the patch's contrast, not its brightness, so F32 rounding stays far below 1e-4 px. Rows as in
  * lk_sample: the top and bottom halves of the patch as the two halves of packed pairs. */
-template <int MAXH, bool EXACT, bool TS>
+template <int MAXH, bool EXACT, bool TS, int PITCH>
 __device__ __forceinline__ void lk_correlate(const DevLevel &L, int jx, int jy, int W, int Hr, int lane,
-                                             const Patch<MAXH, TS> &P, float tc, float (&X)[8])
+                                             const Patch<MAXH, TS, PITCH> &P, float tc, float (&X)[8])
 {
     constexpr int HH = MAXH / 2;
-    const int H = EXACT ? MAXH : Hr;
+    const int H = EXACT ? MAXH : Hr, pitch = PITCH ? PITCH : L.pitch;
     const int x0 = jx - W / 2, y0 = jy - H / 2;
     LK_CHECK_WINDOW(L, x0 - 1, x0 + W, y0, y0 + H, 2u, for (int k = 0; k < 8; k++) X[k] = 0.0f);
     const bool act = lane >= 1 && lane <= W;
-    const float *col = L.p + (size_t)y0 * L.pitch + (x0 - 1 + min(lane, W + 1));
+    const float *col = L.p + (size_t)y0 * pitch + (x0 - 1 + min(lane, W + 1));
     const float *ra = col;
-    const float *rb = col + (size_t)(EXACT ? HH : min(HH, H)) * L.pitch;
+    const float *rb = col + (size_t)(EXACT ? HH : min(HH, H)) * pitch;
     const f2_t M = f2_pack(-tc, -tc);
     /* a row pair: l = J' at this lane's column, n = J' at the next column (the next lane's l) */
     auto load = [&](const float *pa, const float *pb, f2_t &l, f2_t &n) {
@@ -397,11 +401,11 @@ __device__ __forceinline__ void lk_correlate(const DevLevel &L, int jx, int jy, 
 #pragma unroll
     for (int r = 0; r < HH; r++) {
         if (EXACT || r < H) {
-            ra += L.pitch;
+            ra += pitch;
             if (EXACT)
-                rb += L.pitch;
+                rb += pitch;
             else
-                rb = col + (size_t)min(HH + 1 + r, H) * L.pitch;
+                rb = col + (size_t)min(HH + 1 + r, H) * pitch;
             f2_t cl, cn;
             load(ra, rb, cl, cn);
             a00 = f2_fma(pl, P.tx[r], a00);
@@ -427,7 +431,7 @@ __device__ __forceinline__ void lk_correlate(const DevLevel &L, int jx, int jy, 
     if constexpr ((MAXH & 1) != 0) {
         if (EXACT || H == MAXH) {
             /* the last row follows the bottom half: its previous row is the pairs' high halves */
-            const float l = __ldg(EXACT ? rb + L.pitch : col + (size_t)H * L.pitch) - tc;
+            const float l = __ldg(EXACT ? rb + pitch : col + (size_t)H * pitch) - tc;
             const float n = __shfl_down_sync(VTG_FULL, l, 1);
             const float ol = f2_hi(pl), on = f2_hi(pn);
             X[0] = __fmaf_rn(ol, P.txl, X[0]);
@@ -467,19 +471,19 @@ __device__ __forceinline__ void lk_phase_diffs(float (&X)[8])
  * The top half's rows (image rows y0 .. y0 + HH) and the bottom half's (y0 + HH .. y0 + 2 HH) run as the two halves
  * of packed pairs, each carrying its own previous row; an odd height's last row follows the bottom half. With a height
  * below MAXH (not EXACT), bottom-half rows past H read row H again and count for nothing (zero Tx, Ty; masked It). */
-template <int MAXH, bool EXACT, bool RESID, bool TS>
+template <int MAXH, bool EXACT, bool RESID, bool TS, int PITCH>
 __device__ __forceinline__ void lk_sample(const DevLevel &L, int jx, float fx, int jy, float fy, int W, int Hr, int lane,
-                                          const Patch<MAXH, TS> &P, float &b0, float &b1)
+                                          const Patch<MAXH, TS, PITCH> &P, float &b0, float &b1)
 {
     constexpr int HH = MAXH / 2;
-    const int H = EXACT ? MAXH : Hr;
+    const int H = EXACT ? MAXH : Hr, pitch = PITCH ? PITCH : L.pitch;
     const int x0 = jx - W / 2, y0 = jy - H / 2;
     LK_CHECK_WINDOW(L, x0 - 1, x0 + W, y0, y0 + H, 4u, b0 = b1 = 0.0f);
     const bool act = lane >= 1 && lane <= W;
     const float q6 = act ? LK_Q6_INV : 0.0f;
-    const float *col = L.p + (size_t)y0 * L.pitch + (x0 - 1 + min(lane, W + 1));
+    const float *col = L.p + (size_t)y0 * pitch + (x0 - 1 + min(lane, W + 1));
     const float *ra = col;
-    const float *rb = col + (size_t)(EXACT ? HH : min(HH, H)) * L.pitch;
+    const float *rb = col + (size_t)(EXACT ? HH : min(HH, H)) * pitch;
     const f2_t FX = f2_pack(fx, fx), FY = f2_pack(fy, fy);
     f2_t prev = hlerp2(ra, rb, FX);
     /* It Tx, It Ty: pairs of even and of odd r in separate chains */
@@ -487,11 +491,11 @@ __device__ __forceinline__ void lk_sample(const DevLevel &L, int jx, float fx, i
 #pragma unroll
     for (int r = 0; r < HH; r++) {
         if (EXACT || r < H) {
-            ra += L.pitch;
+            ra += pitch;
             if (EXACT)
-                rb += L.pitch;
+                rb += pitch;
             else
-                rb = col + (size_t)min(HH + 1 + r, H) * L.pitch;
+                rb = col + (size_t)min(HH + 1 + r, H) * pitch;
             const f2_t cur = hlerp2(ra, rb, FX);
             const f2_t it = f2_sub(get_t(P, r, lane), f2_fma(f2_sub(cur, prev), FY, prev));
             prev = cur;
@@ -515,7 +519,7 @@ __device__ __forceinline__ void lk_sample(const DevLevel &L, int jx, float fx, i
     float t0 = f2_sum(s0), t1 = f2_sum(s1);
     if constexpr ((MAXH & 1) != 0) {
         if (EXACT || H == MAXH) {
-            const float cur = hlerp(EXACT ? rb + L.pitch : col + (size_t)H * L.pitch, fx);
+            const float cur = hlerp(EXACT ? rb + pitch : col + (size_t)H * pitch, fx);
             const float pb = f2_hi(prev);
             const float it = P.tl - __fmaf_rn(cur - pb, fy, pb);
             if (RESID) {
@@ -578,9 +582,9 @@ __device__ __forceinline__ void split(int base, float t, int &i, float &f)
 #define LK_WORK_PASS (1u << 8)
 #define LK_WORK_ITER (1u << 16)
 
-template <int MAXH, bool EXACT, bool TS, int NW = 1>
+template <int MAXH, bool EXACT, bool TS, int NW = 1, int PITCH = 0>
 __device__ __forceinline__ void lk_track(const DevPyr &I, const DevPyr &J, int top, const LkPrm &p, float x, float y,
-                                         float gx0, float gy0, int lane, Patch<MAXH, TS> &P, vtg_lk_out &o,
+                                         float gx0, float gy0, int lane, Patch<MAXH, TS, PITCH> &P, vtg_lk_out &o,
                                          unsigned &work, const LkPair &q = LkPair{nullptr, 0, 0})
 {
     /* NW = 2: the patch's rows split as Ht = ceil(H / 2) on top and the rest below; this warp's Hs rows start `off`
@@ -748,16 +752,16 @@ __device__ __forceinline__ void lk_track(const DevPyr &I, const DevPyr &J, int t
 
 /* lk_track then, when asked and the track is good, the forward-backward check (src/kern/lk_driver.inc:111-121): the
  * found point tracked back from J to I from minus the found flow. One copy of the walk serves both passes. */
-template <int MAXH, bool EXACT, bool TS, int NW = 1>
+template <int MAXH, bool EXACT, bool TS, int NW = 1, int PITCH = 0>
 __device__ __forceinline__ void lk_point(const DevPyr &I, const DevPyr &J, int top, const LkPrm &p, float x, float y,
-                                         float gx, float gy, int lane, Patch<MAXH, TS> &P, vtg_lk_out &o,
+                                         float gx, float gy, int lane, Patch<MAXH, TS, PITCH> &P, vtg_lk_out &o,
                                          unsigned &work, const LkPair &q = LkPair{nullptr, 0, 0})
 {
     const int passes = p.fb_max2 > 0.0f ? 2 : 1;
     float sx = x, sy = y;
     for (int pass = 0; pass < passes; pass++) {
         vtg_lk_out r;
-        lk_track<MAXH, EXACT, TS, NW>(pass ? J : I, pass ? I : J, top, p, sx, sy, gx, gy, lane, P, r, work, q);
+        lk_track<MAXH, EXACT, TS, NW, PITCH>(pass ? J : I, pass ? I : J, top, p, sx, sy, gx, gy, lane, P, r, work, q);
         if (pass == 0) {
             o = r;
             if (o.status)
@@ -819,7 +823,7 @@ __device__ __forceinline__ void lk_count(unsigned long long *count, unsigned wor
     }
 }
 
-template <int MAXH, bool EXACT, bool TS>
+template <int MAXH, bool EXACT, bool TS, int PITCH>
 __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int top, const LkPrm &p, const CellGrid &g,
                                         int base_w, int base_h, int i, int lane, vtg_lk_out *__restrict__ out,
                                         vtg_cell *__restrict__ cells, f2_t *ts, unsigned long long *count = nullptr)
@@ -829,11 +833,11 @@ __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int to
     float x = (float)(col * g.cell_w + g.cell_w / 2), y = (float)(row * g.cell_h + g.cell_h / 2);
     x = fminf(fmaxf(x, mx), (float)base_w - 1.0f - mx);
     y = fminf(fmaxf(y, my), (float)base_h - 1.0f - my);
-    Patch<MAXH, TS> P;
+    Patch<MAXH, TS, PITCH> P;
     P.ts = ts;
     vtg_lk_out o;
     unsigned work = 0;
-    lk_point<MAXH, EXACT, TS>(I, J, top, p, x, y, 0.0f, 0.0f, lane, P, o, work);
+    lk_point<MAXH, EXACT, TS, 1, PITCH>(I, J, top, p, x, y, 0.0f, 0.0f, lane, P, o, work);
     lk_count(count, work, lane);
     if (out)
         store_out(out + i, o, lane);
@@ -870,7 +874,7 @@ static bool lk_few(int n) { return n <= 8 * LK_SMS; }
 /* A warp a cell. Many: 2 x 2 cells a CTA, as neighbours' windows overlap in L1, and a CTA of few warps leaves its place as soon
  * as its few cells are done. A 1080p pair (build and cells, 16,200 cells), by cells a CTA: 8 x 1 0.243 ms, 4 x 2 0.242, 4 x 4
  * 0.249, 4 x 1 0.240, 2 x 2 0.236, 2 x 1 0.240, one 0.242. */
-template <int MAXH, bool EXACT, bool FEW>
+template <int MAXH, bool EXACT, bool FEW, int PITCH>
 __global__ void __launch_bounds__(32 * LkShape<FEW>::cells, LkShape<FEW>::cell_ctas)
     lk_cells_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp, int top, LkPrm p, CellGrid g, int base_w, int base_h,
                     vtg_lk_out *__restrict__ out, vtg_cell *__restrict__ cells)
@@ -882,7 +886,7 @@ __global__ void __launch_bounds__(32 * LkShape<FEW>::cells, LkShape<FEW>::cell_c
     vtg_grid_dependency_wait(); /* the pyramid, when its kernel is the one before on the stream */
     if (col >= g.cols || row >= g.rows)
         return;
-    lk_cell<MAXH, EXACT, true>(*Ip, *Jp, top, p, g, base_w, base_h, row * g.cols + col, lane, out, cells,
+    lk_cell<MAXH, EXACT, true, PITCH>(*Ip, *Jp, top, p, g, base_w, base_h, row * g.cols + col, lane, out, cells,
                                s_tc + (size_t)warp * (MAXH / 2) * 32);
 }
 
@@ -911,7 +915,7 @@ __device__ __forceinline__ int lk_tile_cell(const CellGrid &g, int w)
     return (col < g.cols && row < g.rows) ? row * g.cols + col : -1;
 }
 
-template <int MAXH, bool EXACT, bool PERSISTENT, int WARPS, int MINB, bool TS, bool COUNT = false>
+template <int MAXH, bool EXACT, bool PERSISTENT, int WARPS, int MINB, bool TS, int PITCH, bool COUNT = false>
 __global__ void __launch_bounds__(WARPS * 32, MINB) lk_batch_kernel(const LkJob *__restrict__ jobs,
                                                                     const int *__restrict__ item_start, int njobs,
                                                                     int items, int chunk, LkPrm p,
@@ -967,7 +971,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) lk_batch_kernel(const LkJob 
         for (int c = c0; c < c0 + chunk; c++) {
             const int cell = tiled ? lk_tile_cell(jb.g, c) : (c < jb.g.n ? c : -1);
             if (cell >= 0)
-                lk_cell<MAXH, EXACT, TS>(*jb.I, *jb.J, jb.top, p, jb.g, jb.base_w, jb.base_h, cell, lane, jb.out,
+                lk_cell<MAXH, EXACT, TS, PITCH>(*jb.I, *jb.J, jb.top, p, jb.g, jb.base_w, jb.base_h, cell, lane, jb.out,
                                          jb.cells, ts, COUNT ? count : nullptr);
         }
         if (!PERSISTENT)
@@ -975,7 +979,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) lk_batch_kernel(const LkJob 
     }
 }
 
-template <int MAXH, bool EXACT>
+template <int MAXH, bool EXACT, int PITCH>
 static cudaError_t lk_batch_launch(const LkJob *jobs, const int *item_start, int njobs, int items, const LkPrm &p,
                                    const LkTune &t, int sms, int *counter, cudaStream_t s, bool pdl,
                                    unsigned long long *count)
@@ -983,7 +987,7 @@ static cudaError_t lk_batch_launch(const LkJob *jobs, const int *item_start, int
 #define LKB(P, WARPS, MINB)                                                                                            \
     do {                                                                                                               \
         const int blocks = P ? sms * t.ctas_per_sm : (items + WARPS - 1) / WARPS;                                      \
-        const cudaError_t e = vtg_launch_k(lk_batch_kernel<MAXH, EXACT, P, WARPS, MINB, false>, blocks, WARPS * 32, 0, \
+        const cudaError_t e = vtg_launch_k(lk_batch_kernel<MAXH, EXACT, P, WARPS, MINB, false, PITCH>, blocks, WARPS * 32, 0, \
                                            s, pdl, jobs, item_start, njobs, items, t.chunk, p, counter, count,         \
                                            P ? t.tiled : 0);                                                           \
         if (e != cudaSuccess)                                                                                          \
@@ -994,12 +998,12 @@ static cudaError_t lk_batch_launch(const LkJob *jobs, const int *item_start, int
         /* WARPS x (MAXH / 2) x 32 pairs: at most 60 KB (16 warps, MAXH 31) */                                       \
         const size_t smem = sizeof(f2_t) * WARPS * (MAXH / 2) * 32;                                                  \
         if (smem > 48 * 1024) {                                                                                        \
-            const cudaError_t e = cudaFuncSetAttribute(lk_batch_kernel<MAXH, EXACT, true, WARPS, MINB, true>,          \
+            const cudaError_t e = cudaFuncSetAttribute(lk_batch_kernel<MAXH, EXACT, true, WARPS, MINB, true, PITCH>,          \
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
             if (e != cudaSuccess)                                                                                      \
                 return e;                                                                                              \
         }                                                                                                              \
-        const cudaError_t e2 = vtg_launch_k(lk_batch_kernel<MAXH, EXACT, true, WARPS, MINB, true>,                    \
+        const cudaError_t e2 = vtg_launch_k(lk_batch_kernel<MAXH, EXACT, true, WARPS, MINB, true, PITCH>,                    \
                                             sms * t.ctas_per_sm, WARPS * 32, smem, s, pdl, jobs, item_start, njobs,    \
                                             items, t.chunk, p, counter, count, t.tiled);                               \
         if (e2 != cudaSuccess)                                                                                         \
@@ -1008,7 +1012,7 @@ static cudaError_t lk_batch_launch(const LkJob *jobs, const int *item_start, int
     if (count) {
         /* counting: one shape for every tuning (a cell's work does not depend on it), so that the others carry no counters */
         const size_t smem = sizeof(f2_t) * 16 * (MAXH / 2) * 32;
-        auto kernel = lk_batch_kernel<MAXH, EXACT, true, 16, 1, true, true>;
+        auto kernel = lk_batch_kernel<MAXH, EXACT, true, 16, 1, true, 0, true>;
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         return e != cudaSuccess ? e
                                 : vtg_launch_k(kernel, sms, 16 * 32, smem, s, pdl, jobs, item_start, njobs, items, t.chunk, p,
@@ -1048,11 +1052,13 @@ cudaError_t vtg_launch_lk_batch(const LkJob *jobs, const int *item_start, int nj
 {
     if (njobs < 1 || njobs > LK_BATCH_MAX_JOBS || items <= 0)
         return items <= 0 ? cudaSuccess : cudaErrorInvalidValue;
+    auto launch = [&](auto kernel) { return kernel(jobs, item_start, njobs, items, p, tune, sms, counter, s, pdl, count); };
+    const bool fixed = p.pitch == VTG_LK_PITCH;
     if (p.H == 21)
-        return lk_batch_launch<21, true>(jobs, item_start, njobs, items, p, tune, sms, counter, s, pdl, count);
+        return launch(fixed ? lk_batch_launch<21, true, VTG_LK_PITCH> : lk_batch_launch<21, true, 0>);
     if (p.H == 15)
-        return lk_batch_launch<15, true>(jobs, item_start, njobs, items, p, tune, sms, counter, s, pdl, count);
-    return lk_batch_launch<31, false>(jobs, item_start, njobs, items, p, tune, sms, counter, s, pdl, count);
+        return launch(fixed ? lk_batch_launch<15, true, VTG_LK_PITCH> : lk_batch_launch<15, true, 0>);
+    return launch(lk_batch_launch<31, false, 0>);
 }
 
 /* shared memory of a single-stream CTA: its warps' template intensities (at most 30 KB) */
@@ -1537,7 +1543,7 @@ cudaError_t vtg_launch_still_cells(const DevLevel &I, const DevLevel &J, const L
                : cudaErrorInvalidValue;
 }
 
-template <int MAXH, bool EXACT, bool FEW>
+template <int MAXH, bool EXACT, bool FEW, int PITCH>
 __global__ void __launch_bounds__(32 * LkShape<FEW>::points, LkShape<FEW>::point_ctas)
     lk_points_kernel(const DevPyr *__restrict__ Ip, const DevPyr *__restrict__ Jp, int top, LkPrm p, int n, const float *__restrict__ xs,
                      const float *__restrict__ ys, const float *__restrict__ gxs, const float *__restrict__ gys,
@@ -1548,11 +1554,11 @@ __global__ void __launch_bounds__(32 * LkShape<FEW>::points, LkShape<FEW>::point
     vtg_grid_dependency_wait(); /* the pyramid or the points, when a kernel made them just before */
     if (i >= n)
         return;
-    Patch<MAXH, true> P;
+    Patch<MAXH, true, PITCH> P;
     P.ts = s_tp + (size_t)(threadIdx.x >> 5) * (MAXH / 2) * 32;
     vtg_lk_out o;
     unsigned work = 0;
-    lk_point<MAXH, EXACT, true>(*Ip, *Jp, top, p, xs[i], ys[i], gxs ? gxs[i] : 0.0f, gys ? gys[i] : 0.0f, lane, P, o,
+    lk_point<MAXH, EXACT, true, 1, PITCH>(*Ip, *Jp, top, p, xs[i], ys[i], gxs ? gxs[i] : 0.0f, gys ? gys[i] : 0.0f, lane, P, o,
                                 work);
     store_out(out + i, o, lane);
 }
@@ -1597,11 +1603,15 @@ cudaError_t vtg_launch_cells(const DevPyr *I, const DevPyr *J, int top, const Lk
         return vtg_launch_k(kernel, blocks, threads, lk_t_bytes(maxh, 2 * (int)rows), s, true, I, J, top, p, g, base_w, base_h, out,
                             cells);
     };
+    constexpr int W = VTG_LK_PITCH;
+    const bool fixed = p.pitch == W;
     if (p.H == 21)
-        return few ? launch(lk_cells_kernel<21, true, true>, 21) : launch(lk_cells_kernel<21, true, false>, 21);
+        return few ? launch(fixed ? lk_cells_kernel<21, true, true, W> : lk_cells_kernel<21, true, true, 0>, 21)
+                   : launch(fixed ? lk_cells_kernel<21, true, false, W> : lk_cells_kernel<21, true, false, 0>, 21);
     if (p.H == 15)
-        return few ? launch(lk_cells_kernel<15, true, true>, 15) : launch(lk_cells_kernel<15, true, false>, 15);
-    return few ? launch(lk_cells_kernel<31, false, true>, 31) : launch(lk_cells_kernel<31, false, false>, 31);
+        return few ? launch(fixed ? lk_cells_kernel<15, true, true, W> : lk_cells_kernel<15, true, true, 0>, 15)
+                   : launch(fixed ? lk_cells_kernel<15, true, false, W> : lk_cells_kernel<15, true, false, 0>, 15);
+    return few ? launch(lk_cells_kernel<31, false, true, 0>, 31) : launch(lk_cells_kernel<31, false, false, 0>, 31);
 }
 
 cudaError_t vtg_launch_points(const DevPyr *I, const DevPyr *J, int top, const LkPrm &p, int n, const float *xs,
@@ -1626,9 +1636,13 @@ cudaError_t vtg_launch_points(const DevPyr *I, const DevPyr *J, int top, const L
         return vtg_launch_k(kernel, dim3((n + per - 1) / per), dim3(32 * per), lk_t_bytes(maxh, per), s, true, I, J, top, p, n, xs, ys,
                             gx, gy, out);
     };
+    constexpr int W = VTG_LK_PITCH;
+    const bool fixed = p.pitch == W;
     if (p.H == 21)
-        return few ? launch(lk_points_kernel<21, true, true>, 21) : launch(lk_points_kernel<21, true, false>, 21);
+        return few ? launch(fixed ? lk_points_kernel<21, true, true, W> : lk_points_kernel<21, true, true, 0>, 21)
+                   : launch(fixed ? lk_points_kernel<21, true, false, W> : lk_points_kernel<21, true, false, 0>, 21);
     if (p.H == 15)
-        return few ? launch(lk_points_kernel<15, true, true>, 15) : launch(lk_points_kernel<15, true, false>, 15);
-    return few ? launch(lk_points_kernel<31, false, true>, 31) : launch(lk_points_kernel<31, false, false>, 31);
+        return few ? launch(fixed ? lk_points_kernel<15, true, true, W> : lk_points_kernel<15, true, true, 0>, 15)
+                   : launch(fixed ? lk_points_kernel<15, true, false, W> : lk_points_kernel<15, true, false, 0>, 15);
+    return few ? launch(lk_points_kernel<31, false, true, 0>, 31) : launch(lk_points_kernel<31, false, false, 0>, 31);
 }

@@ -562,6 +562,7 @@ extern "C" int vtg_still_frame(vtg_still *s, const float *cur, int pitch, const 
         p.max_residual = 16.0f;
         p.fb_max2 = 0.25f * 0.25f;
         p.area = 225.0f;
+        p.pitch = 0;
         CellGrid g;
         g.cell_w = 16;
         g.cell_h = 8;

@@ -33,6 +33,7 @@ struct LkPrm {
     float max_residual;
     float fb_max2;  /* fb_max^2; <= 0: no forward-backward check */
     float area;     /* W H */
+    int pitch;      /* VTG_LK_PITCH when every level of the pyramids has that row pitch, else 0 */
 };
 
 /* A cell grid on level 0 of the pyramids handed to the kernel. */
@@ -42,6 +43,9 @@ struct CellGrid {
 };
 
 static inline int vtg_pitch(int w) { return (w + 31) & ~31; }
+/* The row pitch of every level of a tracker up to this many pixels wide, where its context has the room (api.cu): one number the
+ * LK kernels are compiled for. 65 lines of 128 bytes, an odd number, so that a window's rows spread over the caches' sets. */
+#define VTG_LK_PITCH 2080
 
 /* tk_build's optional input steps (VTG_BUILD_CONTRAST / VTG_BUILD_PRE_GAUSS) keep a frame's partial minima and maxima,
  * a ticket and the gain / offset in VTG_MM_WORDS words of device memory. */

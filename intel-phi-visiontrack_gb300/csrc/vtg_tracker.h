@@ -19,7 +19,7 @@ struct vtg_tracker {
     int lw[VTG_MAX_LEVELS], lh[VTG_MAX_LEVELS], lpitch[VTG_MAX_LEVELS];
     size_t loff[VTG_MAX_LEVELS]; /* float offset of each level inside a set */
     size_t set_floats;
-    size_t bytes;
+    size_t bytes, padding; /* charged to the budget; held beside them for the rows' fixed pitch (api.cu) */
     char *mem;            /* the one allocation */
     float *sets[2];       /* pyramid sets */
     uint8_t *staging;     /* frames uploaded from the host: one buffer per set, staging_set bytes apart */
