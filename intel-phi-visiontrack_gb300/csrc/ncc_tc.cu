@@ -15,16 +15,18 @@
  *   search (ncc_prep), shifted so that every tile's row segment starts on a 16-byte boundary.
  *   B_r depends only on r - Y0: the band (Q + T_h - 1 blocks of 8 Q x K_row) is built once per template in the canonical
  *   core-matrix layout.
- * Pipeline: three threads drive it. Six shared-memory stages, each an image-row segment and a band block, arrive by
- * cp.async.bulk on a "full" mbarrier (expected bytes). A producer thread (warp 0) fills a stage again as soon as the
+ * Pipeline: three threads drive it. Six shared-memory stages (five when the CTA makes its factors too), each an image-row segment and a band
+ * block, arrive by cp.async.bulk on a "full" mbarrier (expected bytes). A producer thread (warp 0) fills a stage again as soon as the
  * MMAs of its last use commit to its "empty" mbarrier. Two issuer threads (warps 1 and 2) take alternate stages, each
  * into its own accumulator: issuing a stage's MMAs takes a lone thread longer than the tensor core takes to run them,
  * so one issuer would leave it idle. Every wait is bounded by the global timer; past it the kernel records an error
  * word.
- * Epilogue: four warps cover the accumulator's 128 lanes, one row (8 x-corners by Q y-corners) a thread; at Q = 16
- * eight, two to a lane quarter, each reading half the row's columns. A thread sums the issuers' accumulators for its
+ * Factors: each corner's 1 / sqrt(norm var) from exact integer window sums, by ncc_prep or, where the tensor core is busy for
+ * longer than that takes, by twelve more warps of the map's CTAs while it multiplies (tc_fused).
+ * Epilogue: four warps cover the accumulator's 128 lanes, one row (8 x-corners by Q y-corners) a thread; with more warps
+ * each of a lane quarter's reads its share of the row's columns. A thread sums the issuers' accumulators for its
  * row. Per corner: st = acc - J(x, y) sum t' (the reference's st is relative to the corner's first pixel), times the
- * corner's factor 1 / sqrt(norm var) from ncc_prep (0 for a near-blank window: the exact integer rule), the best
+ * corner's factor (0 for a near-blank window: the exact integer rule), the best
  * per 16 x 16 cell by value then scan order, merged across tiles by a 64-bit atomicMax on (ordered score, inverted scan
  * index). */
 #include <cuda_bf16.h>
@@ -35,7 +37,6 @@
 #define TC_M 128
 #define TC_QMAX 16 /* y-corners of a tile, at most */
 #define TC_XS (8 * TC_M) /* x-corners of a tile */
-#define TC_STAGES 6
 #ifndef TC_ISSUERS
 #define TC_ISSUERS 2 /* MMA-issuing threads, each with its own accumulator, taking every TC_ISSUERS-th stage */
 #endif
@@ -221,41 +222,45 @@ __device__ __forceinline__ void conv_cta(const uint8_t *__restrict__ plane, int 
 
 /* fac[(y - y0) fpitch + (x - x0)] = 1 / sqrt(norm var) from the corner's exact window sums; 0 for a near-blank window
  * (n var <= n norm / 16) or norm <= 0 -- the reference's rule (src/kern/track.c:203-205) on exact integers.
- * The sums come straight from the bytes, a tile of btx x BP_TY corners a CTA (btx = bp_tx(T_w)):
- *   - a thread a column of the tile, down its column: running sums over the template's T_h rows for the tile's BP_TY corner
- *     rows, into shared memory;
- *   - a thread 16 columns of a row: its prefix sums, the row's 16 threads' totals scanned by shuffles;
+ * The sums come straight from the bytes, nx x ny corners (nx + T_w - 1 <= NT, ny <= TY) by NT threads, tid their number: a CTA of
+ * the preparation, or the warps of a map's CTA that do not drive its tensor core (tc_fused).
+ *   - a thread a column, down its column: running sums over the template's T_h rows for the corner rows, into shared memory;
+ *   - a thread NT / 16 columns of a row: its prefix sums, the row's 16 threads' totals scanned by shuffles;
  *   - a corner's window sums are then P(x + T_w) - P(x), four consecutive corners a thread by 16-byte reads.
  * Bytes keep every window sum in 32 bits (sum J^2 <= 255^2 x 128^2 < 2^31). A row's prefix of J^2 may pass 2^32, so
- * the prefixes are unsigned and wrap: their differences are still exact. n var is formed in 64 bits. The kernel is bound by
- * issue and by its loads' latency: 18 us over a 1080p frame at 64 x 64; a shuffle scan of every row by every warp, and a
- * corner a thread, took 13M instructions where this takes 8M, and 23 us. */
-#define BP_TY 16 /* corner rows a CTA: 16 threads each in the scan */
-#define BP_P 260 /* words of a row of prefixes: 0 .. 256, rows 16-byte aligned */
-/* corners a CTA across: the most, a multiple of 32, whose columns (+ T_w - 1) fit the CTA's 256 threads */
-static inline int bp_tx(int tw) { return ((257 - tw) / 32) * 32; }
+ * the prefixes are unsigned and wrap: their differences are still exact. n var is formed in 64 bits. The preparation's CTAs are
+ * bound by issue and by their loads' latency: 16 us over a 1080p frame at 64 x 64; a shuffle scan of every row by every warp,
+ * and a corner a thread, took 13M instructions where this takes 8M, and 23 us. */
+#define BOX_NT 256 /* threads of a preparation's CTA */
+/* corners of such a CTA across: the most, a multiple of 32, whose columns (+ T_w - 1) fit its threads */
+static inline int bp_tx(int tw) { return ((BOX_NT + 1 - tw) / 32) * 32; }
 
+template <int NT>
 struct BoxSmem {
-    __align__(16) unsigned p[2][BP_TY][BP_P]; /* P[r][c]: columns 0 .. c - 1 of row r; of J and of J^2 */
+    __align__(16) unsigned p[2][TC_QMAX][NT + 4]; /* P[r][c]: columns 0 .. c - 1 of row r; of J and of J^2 */
 };
 
-template <bool TOL>
-__device__ void box_cta(const uint8_t *__restrict__ plane, int pitch, const NccPrm &p, int fw, int fpitch, int btx,
-                        float *__restrict__ fac, uint16_t *__restrict__ tol, int bx, int by, BoxSmem &S)
+/* a barrier of the NT threads (the CTA's own is 0) */
+template <int NT>
+__device__ __forceinline__ void box_sync()
 {
-    const int fh = p.y1 - p.y0 + 1;
-    const int tx0 = bx * btx, ty0 = by * BP_TY;
-    const int nx = min(btx, fw - tx0), ny = min(BP_TY, fh - ty0);
-    const int tid = threadIdx.x;
-    const int ncol = nx + p.tw - 1; /* <= 256 */
+    asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+}
+
+template <int NT, int TY, bool TOL>
+__device__ void box_sums(const uint8_t *__restrict__ plane, int pitch, const NccPrm &p, int fpitch, float *__restrict__ fac,
+                                         uint16_t *__restrict__ tol, int tx0, int ty0, int nx, int ny, int tid, BoxSmem<NT> &S)
+{
+    constexpr int SEG = NT / 16;
+    const int ncol = nx + p.tw - 1;
     {
         /* column tid's sums (0 past the tile's columns); every load of the sliding part in flight, before the first window's
          * rows are added */
         const bool in = tid < ncol;
         const uint8_t *col = plane + (size_t)(p.y0 + ty0) * pitch + (p.x0 + tx0 + min(tid, ncol - 1));
-        unsigned leave[BP_TY], enter[BP_TY];
+        unsigned leave[TY], enter[TY];
 #pragma unroll
-        for (int r = 1; r < BP_TY; r++) {
+        for (int r = 1; r < TY; r++) {
             const int k = min(r, ny - 1) - (ny > 1 ? 1 : 0);
             leave[r] = __ldg(col + (size_t)k * pitch);
             enter[r] = __ldg(col + (size_t)(k + p.th) * pitch);
@@ -270,46 +275,48 @@ __device__ void box_cta(const uint8_t *__restrict__ plane, int pitch, const NccP
         S.p[0][0][tid] = in ? sa : 0u;
         S.p[1][0][tid] = in ? sb : 0u;
 #pragma unroll
-        for (int r = 1; r < BP_TY; r++) {
+        for (int r = 1; r < TY; r++) {
             sa += enter[r] - leave[r];
             sb += enter[r] * enter[r] - leave[r] * leave[r];
             S.p[0][r][tid] = in ? sa : 0u;
             S.p[1][r][tid] = in ? sb : 0u;
         }
     }
-    __syncthreads();
-    /* row tid / 16, columns 16 (tid % 16) ..: read, scanned, and (after a barrier) written one place on */
+    box_sync<NT>();
+    /* row tid / 16, columns SEG (tid % 16) ..: read, scanned, and written one place on (a row lies in one half of a warp) */
     const int row = tid >> 4, seg = tid & 15;
+    if (row < TY) {
 #pragma unroll
-    for (int t = 0; t < 2; t++) {
-        unsigned v[16];
+        for (int t = 0; t < 2; t++) {
+            unsigned v[SEG];
+            uint4 *const at = reinterpret_cast<uint4 *>(&S.p[t][row][SEG * seg]);
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-            *reinterpret_cast<uint4 *>(&v[4 * k]) = *reinterpret_cast<const uint4 *>(&S.p[t][row][16 * seg + 4 * k]);
+            for (int k = 0; k < SEG / 4; k++)
+                *reinterpret_cast<uint4 *>(&v[4 * k]) = at[k];
 #pragma unroll
-        for (int k = 1; k < 16; k++)
-            v[k] += v[k - 1];
-        unsigned before = v[15];
+            for (int k = 1; k < SEG; k++)
+                v[k] += v[k - 1];
+            unsigned before = v[SEG - 1];
 #pragma unroll
-        for (int d = 1; d < 16; d <<= 1) {
-            const unsigned u = __shfl_up_sync(VTG_FULL, before, d, 16);
-            before += seg >= d ? u : 0u;
+            for (int d = 1; d < 16; d <<= 1) {
+                const unsigned u = __shfl_up_sync(VTG_FULL, before, d, 16);
+                before += seg >= d ? u : 0u;
+            }
+            before -= v[SEG - 1];
+            __syncwarp();
+            /* P[SEG seg] = before, P[SEG seg + 1 ..] = before + v[0] ..: the SEG places from there on, and NT */
+#pragma unroll
+            for (int k = 0; k < SEG / 4; k++)
+                at[k] = make_uint4(k ? before + v[4 * k - 1] : before, before + v[4 * k], before + v[4 * k + 1], before + v[4 * k + 2]);
+            if (seg == 15)
+                S.p[t][row][NT] = before + v[SEG - 1];
         }
-        before -= v[15];
-        __syncwarp(); /* a row lies in one half of a warp */
-        /* P[16 seg] = before, P[16 seg + 1 ..] = before + v[0] ..: the 16 places from 16 seg on, and 256 */
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            *reinterpret_cast<uint4 *>(&S.p[t][row][16 * seg + 4 * k]) =
-                make_uint4(k ? before + v[4 * k - 1] : before, before + v[4 * k], before + v[4 * k + 1], before + v[4 * k + 2]);
-        if (seg == 15)
-            S.p[t][row][256] = before + v[15];
     }
-    __syncthreads();
+    box_sync<NT>();
     /* four corners a thread of a row (tw is a multiple of 8: both ends 16-byte aligned); fac's rows hold whole tiles, so a
      * group's store stays inside, past the window's last corner too */
     const int groups = (nx + 3) / 4;
-    for (int i = tid; i < ny * groups; i += 256) {
+    for (int i = tid; i < ny * groups; i += NT) {
         const int r = i / groups, x = 4 * (i - r * groups);
         const uint4 l1 = *reinterpret_cast<const uint4 *>(&S.p[0][r][x]), h1 = *reinterpret_cast<const uint4 *>(&S.p[0][r][x + p.tw]);
         const uint4 l2 = *reinterpret_cast<const uint4 *>(&S.p[1][r][x]), h2 = *reinterpret_cast<const uint4 *>(&S.p[1][r][x + p.tw]);
@@ -336,21 +343,24 @@ __device__ void box_cta(const uint8_t *__restrict__ plane, int pitch, const NccP
     }
 }
 
-/* The map's preparation in one launch of 256-thread CTAs: the first nbox sum the windows (the longer work, so they
- * start first), the rest convert the picture, and those also zero the cells' words the map merges into. The two jobs
- * are independent and run side by side. */
-template <int KIND, bool FILTER>
-__global__ void __launch_bounds__(256) ncc_prep(const uint8_t *__restrict__ plane, int pitch, NccPrm p, int fw, int fpitch,
+/* The map's preparation in one launch of 256-thread CTAs: the picture converted, and the cells' words that the map merges into
+ * zeroed. BOX: the first nbox sum the windows (the longer work, so they start first), where the map's CTAs do not. */
+template <int KIND, bool FILTER, bool BOX>
+__global__ void __launch_bounds__(BOX_NT) ncc_prep(const uint8_t *__restrict__ plane, int pitch, NccPrm p, int fw, int fpitch,
                                                 int btx, int bgx, int nbox, float *__restrict__ fac,
                                                 uint16_t *__restrict__ tol, int rows, int cpitch, int cgx, uint16_t *__restrict__ conv, unsigned long long *__restrict__ cellw,
                                                 int cells, unsigned *__restrict__ ncand)
 {
-    __shared__ BoxSmem S;
     vtg_grid_launch_dependents(); /* the map may start its setup as this launch's last CTAs run */
     const int b = (int)blockIdx.x;
-    if (b < nbox) {
-        box_cta<FILTER>(plane, pitch, p, fw, fpitch, btx, fac, tol, b % bgx, b / bgx, S);
-        return;
+    if constexpr (BOX) {
+        __shared__ BoxSmem<BOX_NT> S;
+        if (b < nbox) {
+            const int x = b % bgx * btx, y = b / bgx * TC_QMAX;
+            box_sums<BOX_NT, TC_QMAX, FILTER>(plane, pitch, p, fpitch, fac, tol, x, y, min(btx, fw - x),
+                                              min(TC_QMAX, p.y1 - p.y0 + 1 - y), (int)threadIdx.x, S);
+            return;
+        }
     }
     const int k = b - nbox, g = k * 256 + (int)threadIdx.x;
     if (g < cells)
@@ -449,27 +459,36 @@ __host__ __device__ constexpr uint32_t tc_cols(int q)
 static_assert(8 * TC_QMAX * TC_ISSUERS <= 512, "the accumulators fit the tensor memory");
 static_assert(TC_ISSUERS >= 1 && TC_ISSUERS <= 3, "issuers are warps 1 .. 3 of the CTA's four");
 
+/* A CTA of the map. Four warps cover the accumulator's 128 lanes. Not FUSED: at Q = 16 eight warps, two to a lane quarter, each
+ * reading half the columns. FUSED: sixteen, four to a quarter; while the tensor core multiplies, warps 4 to 15 make the tile's
+ * factors (box_sums), 256 corners a round, with a stage fewer to leave them the shared memory. shares: warps to a quarter;
+ * chunks: 16-column blocks a thread reads. */
+#define TC_BOX_WARP 4
+#define TC_BOX_X 256
+template <int Q, bool FUSED> struct TcShape {
+    static constexpr int threads = FUSED ? 512 : Q == 16 ? 256 : 128;
+    static constexpr int shares = threads / 128;
+    static constexpr int chunks = Q / 2 / shares;
+    static constexpr int stages = FUSED ? 5 : 6;
+    static constexpr int boxes = threads - 32 * TC_BOX_WARP; /* FUSED: the threads that make factors */
+};
+
 struct TcSmem {
     uint32_t a_bytes, b_bytes, stage_bytes, total;
 };
 
-static TcSmem tc_smem(int krow, int q)
+static TcSmem tc_smem(int krow, int q, bool fused)
 {
     TcSmem s;
     s.a_bytes = (uint32_t)(((TC_XS + krow) * 2 + 127) & ~127);
     s.b_bytes = (uint32_t)(8 * q * krow * 2);
     s.stage_bytes = s.a_bytes + s.b_bytes;
-    s.total = TC_STAGES * s.stage_bytes + 256; /* + mbarriers and the tensor-memory address */
+    /* + mbarriers and the tensor-memory address */
+    s.total = (fused ? TcShape<16, true>::stages : TcShape<16, false>::stages) * s.stage_bytes + 256;
+    if (fused)
+        s.total += (uint32_t)sizeof(BoxSmem<TcShape<16, true>::boxes>);
     return s;
 }
-
-/* Threads of a CTA: four warps cover the accumulator's 128 lanes; at Q = 16 eight, two to a lane quarter, each warp
- * of a pair reading half the columns. chunks: 16-column blocks a thread reads. */
-template <int Q> struct TcShape {
-    static constexpr int threads = Q == 16 ? 256 : 128;
-    static constexpr int halves = threads / 128;
-    static constexpr int chunks = Q / 2 / halves;
-};
 
 /* FILTER: the F32 map's first half. Instead of a cell's best, the corners whose score may be it in F32 arithmetic go to
  * cand: a corner's F32 score lies within its tol of its score here (vtg_ncc_filter_bound), so only corners with score + tol
@@ -477,14 +496,17 @@ template <int Q> struct TcShape {
  * = 8, each tile's part is taken by itself, which can only keep more.) On the blurred-noise frames 1.0 to 1.3 corners a cell
  * are left of 256, at 64 x 64 (29 us for this map, where the F32 map took 728). A near-blank window scores exactly 0 either way: the
  * earliest of them goes straight to the cell's word. */
-template <int KIND, int Q, bool FILTER>
-__global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, const uint16_t *__restrict__ band, int krow, int tiles_x,
+template <int KIND, int Q, bool FILTER, bool FUSED>
+__global__ void __launch_bounds__(TcShape<Q, FUSED>::threads, 1) ncc_map_tc(NccPrm p, const uint8_t *__restrict__ plane, int pitch,
+                                                     const uint16_t *__restrict__ band, int krow, int tiles_x,
                                                      uint32_t a_bytes, uint32_t stage_bytes,
                                                      const uint16_t *__restrict__ conv, int cpitch,
-                                                     const float *__restrict__ fac, int fpitch,
+                                                     float *fac, int fpitch,
                                                      unsigned long long *__restrict__ cellw, int *__restrict__ err,
-                                                     const uint16_t *__restrict__ tol, unsigned *__restrict__ cand, unsigned *__restrict__ ncand)
+                                                     uint16_t *tol, unsigned *__restrict__ cand, unsigned *__restrict__ ncand)
 {
+    using Shape = TcShape<Q, FUSED>;
+    constexpr int TC_STAGES = Shape::stages;
     extern __shared__ __align__(1024) uint8_t smem[];
     if (!FILTER)
         vtg_grid_launch_dependents(); /* the top-8 pass may take the SMs this launch leaves free and wait there */
@@ -517,38 +539,57 @@ __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, c
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    const int fh = p.y1 - p.y0 + 1;
+    if constexpr (FUSED) {
+        if (warp >= TC_BOX_WARP) {
+            /* The tile's factors. They need not wait for the preparation: the picture was there before that started (an ordinary
+             * launch), and whatever read the last search's factors was done. */
+            const int nx = min(TC_XS, p.x1 - p.x0 + 1 - tx * TC_XS);
+            BoxSmem<Shape::boxes> &S = *reinterpret_cast<BoxSmem<Shape::boxes> *>(ctl + 256);
+            for (int x = 0; x < nx; x += TC_BOX_X) {
+                if (x)
+                    box_sync<Shape::boxes>(); /* the last round's sums are read */
+                box_sums<Shape::boxes, Q, FILTER>(plane, pitch, p, fpitch, fac, tol, tx * TC_XS + x, ty * Q, min(TC_BOX_X, nx - x),
+                                                  min(Q, fh - ty * Q), tid - 32 * TC_BOX_WARP, S);
+            }
+        }
+    }
     /* Launched as a programmatic dependent of the preparation, the CTA got here (barriers, tensor memory) while that
      * drained; everything below reads what it wrote (the 16-bit rows, the factors, the cells' reset), with ordinary
      * coherent loads: that data was not read-only while this kernel ran. */
     vtg_grid_dependency_wait();
 
-    /* The epilogue's inputs, loaded before the MMAs start: they arrive while those run. Thread
-     * (quad, lane) owns accumulator row m = 32 quad + lane, corners X0 + 8 m + s, and of its y-corners the pair half of
-     * the CTA's reads: 2 chunks each. A y-corner's eight picture values (the converted row holds the bytes exactly) and
-     * eight factors are one 16-byte and two 16-byte loads. */
-    constexpr int CH = TcShape<Q>::chunks;
+    /* The epilogue's inputs: before the MMAs start, so that they arrive while those run, or FUSED after them. Thread
+     * (quad, lane) owns accumulator row m = 32 quad + lane, corners X0 + 8 m + s, and of its y-corners its share's 2 chunks.
+     * A y-corner's eight picture values (the converted row holds the bytes exactly) and eight factors are one 16-byte and two
+     * 16-byte loads. */
+    constexpr int CH = Shape::chunks;
     const int m = (warp & 3) * 32 + lane, c0 = (warp >> 2) * CH;
     const int xr = tx * TC_XS + 8 * m; /* x - x0 of the thread's first corner */
-    const int fh = p.y1 - p.y0 + 1;
     uint4 jr[2 * CH];
     float4 fr[4 * CH];
     uint4 er[FILTER ? 2 * CH : 1];
+    auto inputs = [&]() {
 #pragma unroll
-    for (int i = 0; i < 2 * CH; i++) {
-        const int yr = ty * Q + 2 * c0 + i;
-        if (yr < fh) {
-            jr[i] = __ldca(reinterpret_cast<const uint4 *>(conv + (size_t)(p.y0 + yr) * cpitch + xr));
-            fr[2 * i] = __ldca(reinterpret_cast<const float4 *>(fac + (size_t)yr * fpitch + xr));
-            fr[2 * i + 1] = __ldca(reinterpret_cast<const float4 *>(fac + (size_t)yr * fpitch + xr + 4));
-            if constexpr (FILTER)
-                er[i] = __ldca(reinterpret_cast<const uint4 *>(tol + (size_t)yr * fpitch + xr));
-        } else {
-            if constexpr (FILTER)
-                er[i] = make_uint4(0u, 0u, 0u, 0u);
-            jr[i] = make_uint4(0u, 0u, 0u, 0u);
-            fr[2 * i] = fr[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int i = 0; i < 2 * CH; i++) {
+            const int yr = ty * Q + 2 * c0 + i;
+            if (yr < fh) {
+                const float4 *f = reinterpret_cast<const float4 *>(fac + (size_t)yr * fpitch + xr);
+                jr[i] = __ldca(reinterpret_cast<const uint4 *>(conv + (size_t)(p.y0 + yr) * cpitch + xr));
+                fr[2 * i] = f[0];
+                fr[2 * i + 1] = f[1];
+                if constexpr (FILTER)
+                    er[i] = *reinterpret_cast<const uint4 *>(tol + (size_t)yr * fpitch + xr);
+            } else {
+                if constexpr (FILTER)
+                    er[i] = make_uint4(0u, 0u, 0u, 0u);
+                jr[i] = make_uint4(0u, 0u, 0u, 0u);
+                fr[2 * i] = fr[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
         }
-    }
+    };
+    if constexpr (!FUSED)
+        inputs();
 
     const int fmt = KIND == VTG_NCC_BF16 ? 1 : 0;
     const uint32_t idesc = (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((uint32_t)((8 * Q) >> 3) << 17) |
@@ -621,6 +662,8 @@ __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, c
                     mbar_wait(full0 + 8 * (k % TC_STAGES), (uint32_t)((k / TC_STAGES) & 1));
         }
     } else {
+        if constexpr (FUSED)
+            inputs();
         /* epilogue. The step is a power of two dividing the cell, and X0 - x0 is a multiple of 16, so the corner (x, y)
          * is on the step grid when (8 m + s) and y - y0 are multiples of it. */
         const int sh = __ffs(p.step) - 1;
@@ -700,11 +743,13 @@ __global__ void __launch_bounds__(TcShape<Q>::threads, 1) ncc_map_tc(NccPrm p, c
             });
             lb = fmaxf(lb, __shfl_xor_sync(VTG_FULL, lb, 1));
             zkey = min(zkey, __shfl_xor_sync(VTG_FULL, zkey, 1));
-            if constexpr (TcShape<Q>::halves == 2) { /* the cell's other eight rows: the pair warp's */
-                __shared__ float s_lb[2][128];
+            if constexpr (Shape::shares > 1) { /* the tile's other rows: the other shares' */
+                __shared__ float s_lb[Shape::shares][128];
                 s_lb[warp >> 2][m] = lb;
                 __syncthreads();
-                lb = fmaxf(lb, s_lb[(warp >> 2) ^ 1][m]);
+#pragma unroll
+                for (int k = 0; k < Shape::shares; k++)
+                    lb = fmaxf(lb, s_lb[k][m]);
             }
             if ((m & 1) == 0 && mine && zkey < (1 << 30))
                 atomicMax(cellw + (size_t)crow * p.ccols + ccol, ncc_cell_word(0.0f, zkey));
@@ -801,18 +846,32 @@ bool vtg_ncc_filters(const NccPrm &p, const NccScratch &s)
            (size_t)g.fpitch * g.fh <= s.tol_elems;
 }
 
+/* Whether the map's own CTAs make their tiles' factors, under the MMAs. They do when the tensor core is busy for longer than that
+ * takes (cycles: an MMA of 8 Q columns takes 4 Q; a round of 256 corners measured some 4,000 and 90 a template row, its loads'
+ * latency), or when the preparation would be long by itself: tall templates over most SMs' tiles. Otherwise the preparation,
+ * whose CTAs fill the chip, is the shorter way. Whole searches, us, factors by the preparation / by the map: 96 x 96 over a 1080p
+ * frame 90 / 82, 64 x 64 62.6 / 58.9, 128 x 128 130 / 118, 64 x 64 over 3840 x 2160 153 / 143, over 201 x 201 corners 49.7 /
+ * 47.9; but over 960 x 540 53.5 / 57.7 (30 tiles of four rounds), 32 x 32 over 1080p 52.2 / 53.1, 32 x 21 over 3840 x 2160
+ * 111 / 125. */
+static bool tc_fused(const NccPrm &p, const TcGrid &g)
+{
+    const int rounds = ((g.fw < TC_XS ? g.fw : TC_XS) + TC_BOX_X - 1) / TC_BOX_X;
+    const int mma = (g.q + p.th - 1) * (g.krow / 16) * 4 * g.q, box = rounds * (4000 + 90 * p.th);
+    return mma >= box || (p.th >= 64 && p.tw >= 64 && g.tiles_x * g.tiles_y >= 100);
+}
+
 /* The preparation and the map. The map (and the passes after it) start as programmatic dependents, their launch and
  * setup overlapping the kernel before, except when events around the map time it alone. */
-template <int KIND, bool FILTER>
-static cudaError_t tc_launch(const uint8_t *plane, int pitch, const NccPrm &p, const NccScratch &s, const TcGrid &g,
-                             cudaStream_t st)
+template <int KIND, bool FILTER, bool FUSED>
+static cudaError_t tc_launch_as(const uint8_t *plane, int pitch, const NccPrm &p, const NccScratch &s, const TcGrid &g,
+                                cudaStream_t st)
 {
-    const TcSmem sm = tc_smem(g.krow, g.q);
+    const TcSmem sm = tc_smem(g.krow, g.q, FUSED);
     const int cells = p.ccols * p.crows;
-    const int btx = bp_tx(p.tw), bgx = (g.fw + btx - 1) / btx, nbox = bgx * ((g.fh + BP_TY - 1) / BP_TY);
+    const int btx = bp_tx(p.tw), bgx = (g.fw + btx - 1) / btx, nbox = FUSED ? 0 : bgx * ((g.fh + TC_QMAX - 1) / TC_QMAX);
     const int cgx = (g.cpitch / 8 + 255) / 256, nconv = cgx * g.rows;
-    ncc_prep<KIND, FILTER><<<nbox + nconv, 256, 0, st>>>(plane, pitch, p, g.fw, g.fpitch, btx, bgx, nbox, s.fac, s.tol, g.rows,
-                                                         g.cpitch, cgx, s.conv, s.cellw, cells, s.ncand);
+    ncc_prep<KIND, FILTER, !FUSED><<<nbox + nconv, BOX_NT, 0, st>>>(plane, pitch, p, g.fw, g.fpitch, btx, bgx, nbox, s.fac, s.tol,
+                                                                    g.rows, g.cpitch, cgx, s.conv, s.cellw, cells, s.ncand);
     const bool pdl = !s.map_ev0;
     auto run = [&](auto kernel, int threads) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm.total);
@@ -820,11 +879,20 @@ static cudaError_t tc_launch(const uint8_t *plane, int pitch, const NccPrm &p, c
             e = cudaEventRecord(s.map_ev0, st);
         if (e != cudaSuccess)
             return e;
-        return vtg_launch_k(kernel, dim3(g.tiles_x * g.tiles_y), dim3(threads), sm.total, st, pdl, p,
+        return vtg_launch_k(kernel, dim3(g.tiles_x * g.tiles_y), dim3(threads), sm.total, st, pdl, p, plane, pitch,
                             (const uint16_t *)s.band, g.krow, g.tiles_x, sm.a_bytes, sm.stage_bytes, (const uint16_t *)s.conv,
-                            g.cpitch, (const float *)s.fac, g.fpitch, s.cellw, s.err, (const uint16_t *)s.tol, s.cand, s.ncand);
+                            g.cpitch, s.fac, g.fpitch, s.cellw, s.err, s.tol, s.cand, s.ncand);
     };
-    return g.q == 8 ? run(ncc_map_tc<KIND, 8, FILTER>, TcShape<8>::threads) : run(ncc_map_tc<KIND, 16, FILTER>, TcShape<16>::threads);
+    return g.q == 8 ? run(ncc_map_tc<KIND, 8, FILTER, FUSED>, TcShape<8, FUSED>::threads)
+                    : run(ncc_map_tc<KIND, 16, FILTER, FUSED>, TcShape<16, FUSED>::threads);
+}
+
+template <int KIND, bool FILTER>
+static cudaError_t tc_launch(const uint8_t *plane, int pitch, const NccPrm &p, const NccScratch &s, const TcGrid &g,
+                             cudaStream_t st)
+{
+    return tc_fused(p, g) ? tc_launch_as<KIND, FILTER, true>(plane, pitch, p, s, g, st)
+                          : tc_launch_as<KIND, FILTER, false>(plane, pitch, p, s, g, st);
 }
 
 cudaError_t vtg_launch_ncc_filter(const uint8_t *plane, int pitch, const NccPrm &p, const NccScratch &s, cudaStream_t st)
