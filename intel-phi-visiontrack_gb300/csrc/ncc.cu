@@ -819,7 +819,7 @@ cudaError_t vtg_launch_ncc_top(const NccPrm &p, const NccScratch &s, bool words,
  * 32-bit a thread for byte planes (at most 64 terms of at most 1,020^2 each, for a 128 x 128 template), 64-bit for F32
  * planes and for every sum across threads. The F32 product sum is added in a fixed order (each thread's rows, the
  * warp's butterfly, then warps 0 .. 7), so a corner's score is the same every run. The result is thread 0's. */
-template <typename T>
+template <typename T, int C>
 __device__ float half_score_cta(const T *__restrict__ plane, int pitch, const float *__restrict__ app, const NccPrm &p,
                                 int hx, int hy)
 {
@@ -833,10 +833,10 @@ __device__ float half_score_cta(const T *__restrict__ plane, int pitch, const fl
     const float first = (float)__ldg(plane + (size_t)y * pitch + x);
     float st = 0.0f;
     Q a1 = 0, a2 = 0; /* in quarters */
-    /* A warp's rows four at a time (two past 32 columns), a lane's columns of them (four at most, T_w <= 128) all loaded before
-     * they are summed: one wait for memory for all of them. The order of its sums is still rows, then columns, ascending. */
-    auto rows = [&](auto columns, int i0) {
-        constexpr int C = decltype(columns)::value, R = 4 / C > 2 ? 4 / C : 2;
+    /* A warp's rows four at a time, a lane's C columns of them (4 for T_w to 128, 2 to 64, 1 to 32) all loaded before they are
+     * summed: one wait for memory for all of them. The order of its sums is still rows, then columns, ascending. */
+    constexpr int R = 4;
+    auto rows = [&](int i0) {
         T a[R][C], b[R][C], c[R][C], d[R][C];
         float t[R][C];
 #pragma unroll
@@ -874,15 +874,8 @@ __device__ float half_score_cta(const T *__restrict__ plane, int pitch, const fl
                 st = __fmaf_rn((float)q * 0.25f - first, t[k][u], st);
             }
     };
-    if (p.tw > 64)
-        for (int i = warp; i < p.th; i += 16)
-            rows(std::integral_constant<int, 4>(), i);
-    else if (p.tw > 32)
-        for (int i = warp; i < p.th; i += 16)
-            rows(std::integral_constant<int, 2>(), i);
-    else
-        for (int i = warp; i < p.th; i += 32)
-            rows(std::integral_constant<int, 1>(), i);
+    for (int i = warp; i < p.th; i += 8 * R)
+        rows(i);
     long long q1 = a1, q2 = a2;
 #pragma unroll
     for (int s = 16; s >= 1; s >>= 1) {
@@ -1001,8 +994,11 @@ __device__ void ncc_pick(const NccPrm &p, const int *__restrict__ map_x, const i
  * search_slot compares, and one ring past it, so the parabola's neighbours of any best are already scored. Scores go
  * to hs[candidate][(around + 1 + dy) ring + around + 1 + dx], ring = 2 around + 3. The CTA that arrives last (every
  * CTA counts, those past the candidates too) makes the pick and resets the counter. */
-template <typename T>
-__global__ void __launch_bounds__(NCC_TOP * 32, 4) ncc_half_all(const T *__restrict__ plane, int pitch,
+/* A byte plane's 200 corners are fewer CTAs than two an SM, so past 32 columns a thread may have 128 registers for its loads (C: a
+ * lane's columns). With one kernel of 64 for every width, two rows at a time, a whole 96 x 96 search took 81.4 us; now 75.5. Six
+ * rows in 255 registers: 79.5; at 64 x 64 two, four or eight rows are the same. */
+template <typename T, int C>
+__global__ void __launch_bounds__(NCC_TOP * 32, C > 1 ? 2 : 4) ncc_half_all(const T *__restrict__ plane, int pitch,
                                                              const float *__restrict__ app, NccPrm p,
                                                              const int *__restrict__ map_x, const int *__restrict__ map_y,
                                                              const int *__restrict__ top, const int *__restrict__ ntop,
@@ -1018,7 +1014,7 @@ __global__ void __launch_bounds__(NCC_TOP * 32, 4) ncc_half_all(const T *__restr
     if (c < n) {
         const int cell = __ldca(top + c);
         const int hx = 2 * __ldca(map_x + cell) + (o % ring) - r, hy = 2 * __ldca(map_y + cell) + (o / ring) - r;
-        const float v = half_score_cta(plane, pitch, app, p, hx, hy);
+        const float v = half_score_cta<T, C>(plane, pitch, app, p, hx, hy);
         if (threadIdx.x == 0)
             hs[c * ring * ring + o] = v;
     }
@@ -1137,7 +1133,8 @@ static cudaError_t launch_all(const T *plane, int pitch, const float *app, const
     if (map_kind == VTG_NCC_F32 && (e = vtg_launch_ncc_top(p, s, filtered, st, pdl)) != cudaSuccess)
         return e;
     const int around = p.step > 1 ? 2 * p.step - 1 : 1, ring = 2 * around + 3;
-    return vtg_launch_k(ncc_half_all<T>, dim3(NCC_TOP * ring * ring), dim3(NCC_TOP * 32), 0, st, pdl, plane, pitch, app, p,
+    auto kernel = p.tw > 64 ? ncc_half_all<T, 4> : p.tw > 32 ? ncc_half_all<T, 2> : ncc_half_all<T, 1>;
+    return vtg_launch_k(kernel, dim3(NCC_TOP * ring * ring), dim3(NCC_TOP * 32), 0, st, pdl, plane, pitch, app, p,
                         (const int *)s.map_x, (const int *)s.map_y, (const int *)s.top, (const int *)s.ntop, s.half,
                         s.arrive + 1, out);
 }
