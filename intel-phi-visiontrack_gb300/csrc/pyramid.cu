@@ -461,6 +461,22 @@ __device__ __forceinline__ uint32_t block_minmax(uint32_t mn, uint32_t mx, uint3
     return r;
 }
 
+/* Sixteen bytes at any alignment as four words: from five aligned words, shifted. They read up to three bytes before and after,
+ * so the caller keeps p three bytes clear of its row's ends. */
+__device__ __forceinline__ void load16(const uint8_t *p, uint32_t (&q)[4])
+{
+    const uint32_t *a = reinterpret_cast<const uint32_t *>((uintptr_t)p & ~(uintptr_t)3);
+    const int sh = 8 * (int)((uintptr_t)p & 3);
+    uint32_t w[5];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        w[k] = __ldg(a + k);
+    w[4] = sh ? __ldg(a + 4) : 0u;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        q[k] = __funnelshift_r(w[k], w[k + 1], sh);
+}
+
 /* The frame's byte min and max (x 64 = img_minmax of its Q6 plane): CTA b scans rows b, b + grid, ... four bytes at a
  * time (16 with an aligned frame) and writes its partial to mm[b]; the last CTA to finish (a ticket in
  * mm[VTG_MM_BLOCKS]) combines the partials, writes gain and offset to mm[VTG_MM_BLOCKS + 1 ..] and resets the ticket. */
@@ -481,6 +497,8 @@ __global__ void __launch_bounds__(256) pyr_minmax_kernel(const uint8_t *__restri
                 v[1] = q.y;
                 v[2] = q.z;
                 v[3] = q.w;
+            } else if (x >= 3 && x + 19 <= w) {
+                load16(row + x, v);
             } else {
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
@@ -532,8 +550,11 @@ __global__ void __launch_bounds__(256) pyr_minmax_kernel(const uint8_t *__restri
  * over the block and the halo that level 1 needs (rows Y0 - 14 .. Y0 + 70, columns X0 - 14 .. X0 + 134) by the binomial's two
  * passes, else the staged values are level 0. Past the frame's edge the levels read the clamped index, never the halo's own
  * value there. A value's bit 15 keeps the table's -0, which a level-0 store without GAUSS must (the sums mask it).
- * A 1281 x 719 frame with both steps: 13 us for this launch, where level 0 and each level above took
- * one (27 us). */
+ * The vertical passes run down a column with the last five rows in
+ * registers: a shared load and a tap sum an output, where each output read its five rows. Bound by its phases' issue: two CTAs an
+ * SM. A 1281 x 719 frame with both steps (and the launch for the gain), three streams: 15.4 us as five launches, 9.8 as two, 9.3
+ * with unaligned bytes by shifted words, 8.5 with the running columns. (Started early, under the minimum and maximum's launch, it
+ * fetches its bytes sooner, but a frame alone took 22 us, not 16, at 640 x 480: not done.) */
 #define PI_R 89
 #define PI_C 160
 #define P0_R 85 /* level 0 as level 1 reads it */
@@ -548,41 +569,61 @@ struct InputSmem {
         FusedUpper u;                         /* once they are not needed */
     };
     union {
-        int v0[P0_R][P0_P + 4]; /* GAUSS: vertical sums, columns X0 - 16 .. X0 + 139 */
+        __align__(16) int v0[P0_R][P0_P + 4]; /* GAUSS: vertical sums, columns X0 - 16 .. X0 + 139 */
         int v1[F1_R][P0_P];     /* level 1's vertical sums, columns X0 - 14 .. */
     };
     __align__(16) uint16_t l0[P0_R][P0_P]; /* GAUSS: level 0 (must stay last) */
 };
 
-template <bool GAUSS, bool EDGE>
-__device__ __forceinline__ void input_block(const FusedFrame &f, int X0, int Y0, InputSmem &S)
+#define PI_CHUNKS ((PI_R * (PI_C / 16) + PI_T - 1) / PI_T) /* 16-byte chunks of the staged bytes a thread takes */
+
+template <bool EDGE>
+__device__ __forceinline__ void input_fetch(const FusedFrame &f, int X0, int Y0, uint32_t (&q)[PI_CHUNKS][4])
 {
-    const int tid = threadIdx.x, w = f.w, h = f.h;
+    const int w = f.w, h = f.h;
     const bool vec = (((uintptr_t)f.src | (uintptr_t)f.stride) & 15) == 0;
-    for (int i = tid; i < PI_R * (PI_C / 16); i += PI_T) {
+#pragma unroll
+    for (int j = 0; j < PI_CHUNKS; j++) {
+        const int i = (int)threadIdx.x + j * PI_T;
+        if (i >= PI_R * (PI_C / 16))
+            break;
         const int r = i / (PI_C / 16), k = i - r * (PI_C / 16);
         const int gy = EDGE ? min(max(Y0 - 16 + r, 0), h - 1) : Y0 - 16 + r, gx = X0 - 16 + 16 * k;
         const uint8_t *row = f.src + (size_t)gy * f.stride;
-        uint32_t q[4];
         if (vec && (!EDGE || (gx >= 0 && gx + 16 <= w))) {
             const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + gx));
-            q[0] = v.x;
-            q[1] = v.y;
-            q[2] = v.z;
-            q[3] = v.w;
+            q[j][0] = v.x;
+            q[j][1] = v.y;
+            q[j][2] = v.z;
+            q[j][3] = v.w;
+        } else if (gx >= 3 && gx + 19 <= w) {
+            load16(row + gx, q[j]);
         } else {
 #pragma unroll
             for (int a = 0; a < 4; a++) {
-                q[a] = 0u;
+                q[j][a] = 0u;
 #pragma unroll
                 for (int e = 0; e < 4; e++)
-                    q[a] |= (uint32_t)__ldg(row + (EDGE ? min(max(gx + 4 * a + e, 0), w - 1) : gx + 4 * a + e)) << (8 * e);
+                    q[j][a] |= (uint32_t)__ldg(row + (EDGE ? min(max(gx + 4 * a + e, 0), w - 1) : gx + 4 * a + e)) << (8 * e);
             }
         }
+    }
+}
+
+template <bool GAUSS, bool EDGE>
+__device__ __forceinline__ void input_block(const FusedFrame &f, int X0, int Y0, const uint32_t (&q)[PI_CHUNKS][4], InputSmem &S)
+{
+    const int tid = threadIdx.x, w = f.w, h = f.h;
+#pragma unroll
+    for (int j = 0; j < PI_CHUNKS; j++) {
+        const int i = tid + j * PI_T;
+        if (i >= PI_R * (PI_C / 16))
+            break;
+        const int r = i / (PI_C / 16), k = i - r * (PI_C / 16);
         uint32_t o[8];
 #pragma unroll
         for (int a = 0; a < 8; a++) {
-            const uint32_t two = q[a >> 1] >> (16 * (a & 1));
+            const uint32_t two = q[j][a >> 1] >> (16 * (a & 1));
             o[a] = S.lut[two & 255u] | S.lut[(two >> 8) & 255u] << 16;
         }
         *reinterpret_cast<uint4 *>(&S.n[r][16 * k]) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -595,25 +636,32 @@ __device__ __forceinline__ void input_block(const FusedFrame &f, int X0, int Y0,
                        *reinterpret_cast<const uint32_t *>(&S.n[r + 2][c + 2]) & 0x7fff7fffu;
     };
     if (GAUSS) {
-        for (int i = tid; i < P0_R * (P0_P + 4) / 2; i += PI_T) {
-            const int r = i / ((P0_P + 4) / 2), c = 2 * (i - r * ((P0_P + 4) / 2));
+        /* a thread two columns of a run of rows, the last five rows' values in registers */
+        constexpr int PAIRS = (P0_P + 4) / 2, RUN = (P0_R + PI_T / PAIRS - 1) / (PI_T / PAIRS);
+        const int run = tid / PAIRS, c = 2 * (tid - run * PAIRS), r0 = run * RUN;
+        if (run < PI_T / PAIRS) {
             int a[5], b[5];
 #pragma unroll
-            for (int t = 0; t < 5; t++) {
-                const uint32_t q = *reinterpret_cast<const uint32_t *>(&S.n[r + t][c]);
-                a[t] = (int)(q & 0x7fffu);
-                b[t] = (int)((q >> 16) & 0x7fffu);
+            for (int k = -4; k < RUN; k++) {
+                if (r0 + k >= P0_R)
+                    break;
+                const uint32_t q = *reinterpret_cast<const uint32_t *>(&S.n[r0 + k + 4][c]);
+                a[(k + 5) % 5] = (int)(q & 0x7fffu);
+                b[(k + 5) % 5] = (int)((q >> 16) & 0x7fffu);
+                if (k >= 0) /* rows r .. r + 4 sit from (k + 1) % 5 on */
+                    *reinterpret_cast<int2 *>(&S.v0[r0 + k][c]) =
+                        make_int2(tap5(a[(k + 1) % 5], a[(k + 2) % 5], a[(k + 3) % 5], a[(k + 4) % 5], a[k % 5]),
+                                  tap5(b[(k + 1) % 5], b[(k + 2) % 5], b[(k + 3) % 5], b[(k + 4) % 5], b[k % 5]));
             }
-            *reinterpret_cast<int2 *>(&S.v0[r][c]) = make_int2(tap5(a[0], a[1], a[2], a[3], a[4]), tap5(b[0], b[1], b[2], b[3], b[4]));
         }
         __syncthreads();
         /* level 0's column c (frame column X0 - 14 + c) centres on vertical sum c + 2 */
-        for (int i = tid; i < P0_R * P0_P / 2; i += PI_T) {
-            const int r = i / (P0_P / 2), c = 2 * (i - r * (P0_P / 2));
-            const int2 q0 = *reinterpret_cast<const int2 *>(&S.v0[r][c]), q1 = *reinterpret_cast<const int2 *>(&S.v0[r][c + 2]),
-                       q2 = *reinterpret_cast<const int2 *>(&S.v0[r][c + 4]);
-            const int o0 = (tap5(q0.x, q0.y, q1.x, q1.y, q2.x) + 128) >> 8, o1 = (tap5(q0.y, q1.x, q1.y, q2.x, q2.y) + 128) >> 8;
-            *reinterpret_cast<uint32_t *>(&S.l0[r][c]) = (uint32_t)o0 | (uint32_t)o1 << 16;
+        for (int i = tid; i < P0_R * P0_P / 4; i += PI_T) {
+            const int r = i / (P0_P / 4), c = 4 * (i - r * (P0_P / 4));
+            const int4 u = *reinterpret_cast<const int4 *>(&S.v0[r][c]), v = *reinterpret_cast<const int4 *>(&S.v0[r][c + 4]);
+            const int o0 = (tap5(u.x, u.y, u.z, u.w, v.x) + 128) >> 8, o1 = (tap5(u.y, u.z, u.w, v.x, v.y) + 128) >> 8,
+                      o2 = (tap5(u.z, u.w, v.x, v.y, v.z) + 128) >> 8, o3 = (tap5(u.w, v.x, v.y, v.z, v.w) + 128) >> 8;
+            *reinterpret_cast<uint2 *>(&S.l0[r][c]) = make_uint2((uint32_t)o0 | (uint32_t)o1 << 16, (uint32_t)o2 | (uint32_t)o3 << 16);
         }
         __syncthreads();
     }
@@ -636,7 +684,32 @@ __device__ __forceinline__ void input_block(const FusedFrame &f, int X0, int Y0,
         return;
     /* level 1: its local origin is X0 / 2 - 6, Y0 / 2 - 6, level 0's X0 - 14, Y0 - 14 */
     /* (v1 takes v0's place: nothing of v0 is read after the barrier above) */
-    for (int i = tid; i < F1_R * (P0_P / 2); i += PI_T) {
+    if constexpr (!EDGE) { /* runs of rows again: two new ones an output */
+        constexpr int PAIRS = P0_P / 2, RUN = (F1_R + PI_T / PAIRS - 1) / (PI_T / PAIRS);
+        const int run = tid / PAIRS, c = 2 * (tid - run * PAIRS), y0 = run * RUN;
+        if (run < PI_T / PAIRS) {
+            int a[5], b[5];
+            auto take = [&](int slot, int r) {
+                const uint32_t q = l0_pair(r, c);
+                a[slot] = (int)(q & 0xffffu);
+                b[slot] = (int)(q >> 16);
+            };
+#pragma unroll
+            for (int t = 0; t < 3; t++)
+                take(t, 2 * y0 + t);
+#pragma unroll
+            for (int k = 0; k < RUN; k++) {
+                if (y0 + k >= F1_R)
+                    break;
+                take((2 * k + 3) % 5, 2 * (y0 + k) + 3);
+                take((2 * k + 4) % 5, 2 * (y0 + k) + 4);
+                *reinterpret_cast<int2 *>(&S.v1[y0 + k][c]) =
+                    make_int2(tap5(a[2 * k % 5], a[(2 * k + 1) % 5], a[(2 * k + 2) % 5], a[(2 * k + 3) % 5], a[(2 * k + 4) % 5]),
+                              tap5(b[2 * k % 5], b[(2 * k + 1) % 5], b[(2 * k + 2) % 5], b[(2 * k + 3) % 5], b[(2 * k + 4) % 5]));
+            }
+        }
+    }
+    for (int i = tid; EDGE && i < F1_R * (P0_P / 2); i += PI_T) {
         const int y = i / (P0_P / 2), c = 2 * (i - y * (P0_P / 2));
         int a[5], b[5];
 #pragma unroll
@@ -668,8 +741,15 @@ __global__ void __launch_bounds__(PI_T) pyr_input_kernel(FusedFrame f, bool cont
 {
     extern __shared__ __align__(16) unsigned char s_input[];
     InputSmem &S = *reinterpret_cast<InputSmem *>(s_input);
-    const int tid = threadIdx.x;
-    vtg_grid_dependency_wait(); /* the gain and offset, when launched as the minimum and maximum's dependent */
+    const int tid = threadIdx.x, X0 = blockIdx.x * FP_X, Y0 = blockIdx.y * FP_Y;
+    const bool inside = X0 >= 16 && X0 + 144 <= f.w && Y0 >= 16 && Y0 + 73 <= f.h;
+    /* the bytes, which were there before the minimum and maximum's launch (an ordinary one) */
+    uint32_t q[PI_CHUNKS][4];
+    if (inside)
+        input_fetch<false>(f, X0, Y0, q);
+    else
+        input_fetch<true>(f, X0, Y0, q);
+    vtg_grid_dependency_wait(); /* the gain and offset, when launched as that launch's dependent */
     if (tid < 256) {
         float v = (float)(64 * tid);
         if (contrast) {
@@ -685,11 +765,10 @@ __global__ void __launch_bounds__(PI_T) pyr_input_kernel(FusedFrame f, bool cont
         S.lut[tid] = (uint32_t)fabsf(v) | (__float_as_uint(v) >> 31 << 15);
     }
     __syncthreads();
-    const int X0 = blockIdx.x * FP_X, Y0 = blockIdx.y * FP_Y;
-    if (X0 >= 16 && X0 + 144 <= f.w && Y0 >= 16 && Y0 + 73 <= f.h)
-        input_block<GAUSS, false>(f, X0, Y0, S);
+    if (inside)
+        input_block<GAUSS, false>(f, X0, Y0, q, S);
     else
-        input_block<GAUSS, true>(f, X0, Y0, S);
+        input_block<GAUSS, true>(f, X0, Y0, q, S);
 }
 
 static FusedFrame fused_frame(const uint8_t *frame, int stride, int w, int h, float *const *levels, const int *pitches, int nlevels)
