@@ -1,4 +1,4 @@
-"""The input steps' byte loads at every alignment of the frame's first byte and of its rows (sixteen bytes from shifted words, whole
+"""The builds' byte loads, plain and under the input steps, at every alignment of the frame's first byte and of its rows (sixteen bytes from shifted words, whole
 vectors or single bytes), with guard bytes around the frame that a wrong one would take for its minimum or maximum. Bit for bit
 against the oracle."""
 import numpy as np
@@ -10,7 +10,7 @@ import vtg_synth as S
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("opts", [1, 2, 3])
+@pytest.mark.parametrize("opts", [0, 1, 2, 3])
 @pytest.mark.parametrize("w,h,start,pad", [(275, 130, 1, 0), (275, 130, 2, 2), (275, 130, 3, 13), (272, 130, 16, 0), (272, 130, 4, 4),
                                            (290, 90, 7, 1), (51, 70, 5, 0), (35, 33, 1, 2), (34, 33, 0, 0)])
 def test_any_alignment(vtg_lib, ctx, w, h, start, pad, opts):
