@@ -713,7 +713,8 @@ __global__ void __launch_bounds__(32 * NCR_WARPS) ncc_rescore(const uint8_t *__r
         if (on && !odd) {
             const float v = ncc_score(acc + acc1, (long long)s1, (long long)s2, p) + 0.0f;
             const int key = ((b % NCC_CELL) >> sh) * per + ((a % NCC_CELL) >> sh);
-            atomicMax(cellw + (size_t)(b / NCC_CELL) * p.ccols + a / NCC_CELL, ncc_cell_word(v, key));
+            if (v > -2.0f) /* a cell with nothing above -2 keeps that and its origin, as ncc_map_f32q's does */
+                atomicMax(cellw + (size_t)(b / NCC_CELL) * p.ccols + a / NCC_CELL, ncc_cell_word(v, key));
         }
     }
 }
