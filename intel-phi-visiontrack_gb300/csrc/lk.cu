@@ -790,24 +790,35 @@ __device__ __forceinline__ void store_out(vtg_lk_out *dst, const vtg_lk_out &o, 
         reinterpret_cast<uint32_t *>(dst)[lane] = w;
 }
 
-/* Mean |J - I| over one cell of level 0, 8-bit grey (still.c:105-114). The differences are whole Q6 numbers, their sum
- * below 2^24, so the F32 sum is exact and the mean is one rounding, as in the reference. */
+/* Mean |J - I| over one cell of level 0, 8-bit grey (still.c:105-114). Between frames the differences are whole Q6 numbers, their
+ * sum below 2^24, so the F32 sum is exact and the mean is one rounding, as in the reference. A still picture's mean is not
+ * whole, so there the order of the additions shows: element k in partial sum k % 32, the partial sums by warp_fold's butterfly.
+ * Sixteen lanes keep two of a warp's partial sums each, and add in the same order. */
 template <int LANES = 32>
 __device__ __forceinline__ float cell_diff(const DevLevel &A, const DevLevel &B, int col, int row, const CellGrid &g,
                                            int lane)
 {
-    const int x = col * g.cell_w, y0 = row * g.cell_h, y1 = min(y0 + g.cell_h, A.h);
-    float s = 0.0f;
+    constexpr int PARTS = 32 / LANES;
+    const int x = col * g.cell_w, y0 = row * g.cell_h, y1 = min(y0 + g.cell_h, A.h), n = g.cell_w * (y1 - y0);
+    float s[PARTS] = {};
     /* a cell's row and column of element k: a shift and a mask for power-of-two widths (the 16 x 8 grid) */
     const bool p2 = (g.cell_w & (g.cell_w - 1)) == 0;
     const int sh = __ffs(g.cell_w) - 1;
-    for (int k = lane; k < g.cell_w * (y1 - y0); k += LANES) {
-        const int kr = p2 ? k >> sh : k / g.cell_w, kc = p2 ? k & (g.cell_w - 1) : k % g.cell_w;
-        const int yy = y0 + kr, xx = min(x + kc, A.w - 1);
-        s += fabsf(__ldg(B.p + (size_t)yy * B.pitch + xx) - __ldg(A.p + (size_t)yy * A.pitch + xx));
-    }
-    s = warp_fold<LANES>(s);
-    return __fdiv_rn(s, (float)((y1 - y0) * g.cell_w)) * LK_Q6_INV;
+    for (int k0 = lane; k0 < n; k0 += 32)
+#pragma unroll
+        for (int u = 0; u < PARTS; u++) {
+            const int k = k0 + u * LANES;
+            if (u && k >= n)
+                break;
+            const int kr = p2 ? k >> sh : k / g.cell_w, kc = p2 ? k & (g.cell_w - 1) : k % g.cell_w;
+            const int yy = y0 + kr, xx = min(x + kc, A.w - 1);
+            s[u] += fabsf(__ldg(B.p + (size_t)yy * B.pitch + xx) - __ldg(A.p + (size_t)yy * A.pitch + xx));
+        }
+    float sum = warp_fold<LANES>(s[0]);
+#pragma unroll
+    for (int u = 1; u < PARTS; u++)
+        sum += warp_fold<LANES>(s[u]);
+    return __fdiv_rn(sum, (float)n) * LK_Q6_INV;
 }
 
 /* One cell of a grid: its centre (cw c + cw / 2, ch r + ch / 2), clamped to where the patch fits (still.c:127-130),
