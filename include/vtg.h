@@ -93,6 +93,9 @@ int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms);
  * pass, 4 sample pass), out[1] = how many times; then clears it. Returns 1 in the checked build, 0 (out zeroed) in the
  * production build, which has no checks. */
 int vtg_check_read(uint32_t *out);
+/* The checked build's injected failure: while on, every tensor-core search map ends as one whose bounded wait gave up. Returns 1
+ * in the checked build, 0 (nothing done) in the production build. */
+int vtg_check_give_up(int on);
 
 /* ---- a tracker: one camera stream's device-resident state (tk_create, src/kern/track.h:22 / track.c:447-572) ---- */
 
@@ -248,7 +251,8 @@ enum { VTG_NCC_F32 = 0, VTG_NCC_BF16 = 1, VTG_NCC_FP16 = 2 };
 /* What a search found: struct found (src/kern/track.c:1608-1612) plus take_back's parabola offsets
  * (track.c:1741-1742). hx, hy: the template's corner in half pixels of the plane; ncc: its score; second: the best
  * score clear of it by half a template (-2 if none); ox, oy: sub-half-pixel offsets in [-0.5, 0.5]; ntop: candidates
- * looked at; cells: cells of the map. */
+ * looked at; cells: cells of the map. ntop -1 (and both scores -2): a bounded wait in the search's map gave up, so its result is
+ * not whole. */
 struct vtg_found {
     int hx, hy;
     float ncc, second, ox, oy;
@@ -270,7 +274,8 @@ int vtg_search_template(vtg_search *s, const float *app, int tw, int th, float n
 /* search_slot (src/kern/track.c:1661-1726) over corners [x0, x1] x [y0, y1] of a plane (w x h, rows `pitch` elements
  * apart, device memory, type VTG_PLANE_*), at `step`; the window is clamped to where the template fits as the
  * reference clamps it. `precision` VTG_NCC_*. *found (and, if not NULL, the per-cell map of `cells` entries) in host
- * or device memory as `where` says. */
+ * or device memory as `where` says. VTG_ETIMEOUT (host results) or ntop -1 (host and device results): this search's map gave up;
+ * the next search is not affected. */
 int vtg_search_run(vtg_search *s, const void *plane, int w, int h, int pitch, int plane_type, int x0, int x1, int y0,
                    int y1, int step, int precision, struct vtg_found *found, float *map_v, int *map_x, int *map_y,
                    int where, void *stream);

@@ -19,10 +19,7 @@ struct vtg_search {
     NccScratch sc;
     uint16_t *band[2]; /* BF16 and FP16 bands */
     vtg_found *found;  /* device result slot (vtg_search_profile) */
-    struct Host {
-        vtg_found found;
-        int err; /* the tensor-core map's status word */
-    } *host, *host_dev; /* pinned host memory that the kernels write: a host caller's result needs no copy */
+    vtg_found *host, *host_dev; /* pinned host memory that the kernels write: a host caller's result needs no copy */
     int *xy;           /* corners for vtg_correlate from the host */
     float *vals;
     int tw, th;
@@ -150,7 +147,6 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
         delete s;
         return VTG_ECUDA;
     }
-    s->host->err = 0;
     s->app = (float *)(s->mem + L.app);
     s->stats = (NccBandStats *)(s->mem + L.sum);
     s->sc.S1 = (long long *)(s->mem + L.S1);
@@ -161,7 +157,6 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
     s->sc.map_y = (int *)(s->mem + L.map_y);
     s->sc.top = (int *)(s->mem + L.top);
     s->sc.ntop = (int *)(s->mem + L.ntop);
-    s->sc.err = &s->host_dev->err;
     s->sc.half = (float *)(s->mem + L.half);
     s->band[0] = (uint16_t *)(s->mem + L.band0);
     s->band[1] = (uint16_t *)(s->mem + L.band1);
@@ -179,6 +174,7 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
     s->sc.tol = (uint16_t *)s->sc.S2;
     s->sc.tol_elems = 4 * (size_t)L.tp * (max_h + 1);
     s->sc.ncand = s->sc.arrive + 2;
+    s->sc.err = (int *)(s->sc.arrive + 3);
     s->sc.map_ev0 = s->sc.map_ev1 = nullptr;
     s->found = (vtg_found *)(s->mem + L.found);
     s->xy = nullptr;
@@ -276,7 +272,7 @@ extern "C" int vtg_search_run(vtg_search *s, const void *plane, int w, int h, in
     if (chk != VTG_OK)
         return chk;
     const cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
-    vtg_found *dst = where == VTG_DEVICE ? found : &s->host_dev->found;
+    vtg_found *dst = where == VTG_DEVICE ? found : s->host_dev;
     if (empty) {
         vtg_found f = {0, 0, -2.0f, -2.0f, 0.0f, 0.0f, 0, 0};
         if (where == VTG_HOST)
@@ -298,11 +294,9 @@ extern "C" int vtg_search_run(vtg_search *s, const void *plane, int w, int h, in
         CU(cudaMemcpyAsync(map_y, sc.map_y, cells * sizeof(int), k, st));
     if (where == VTG_HOST) {
         CU(cudaStreamSynchronize(st));
-        *found = s->host->found;
-        if (s->host->err) {
-            s->host->err = 0;
+        *found = *s->host;
+        if (found->ntop < 0)
             return VTG_ETIMEOUT;
-        }
     }
     return VTG_OK;
 }

@@ -918,14 +918,20 @@ __device__ __forceinline__ float parabola(float l, float c, float r)
 /* The best of each candidate's window (row-major first maximum, as search_slot's strict > over hy then hx: the
  * smallest index among equal scores), one warp a candidate; then, on one thread, the best over candidates in rank
  * order, the second peak half a template away, and the parabola through the four neighbours of the best (take_back's
- * peak_offset), all from hs (read through L2: other CTAs wrote it). Run by a CTA of NCC_TOP warps. */
+ * peak_offset), all from hs (read through L2: other CTAs wrote it). Run by a CTA of NCC_TOP warps. gave_up: the map is not
+ * whole (a bounded wait in it ended), so there is no best: ntop -1 says so. */
 __device__ void ncc_pick(const NccPrm &p, const int *__restrict__ map_x, const int *__restrict__ map_y,
-                         const int *__restrict__ top, int n, const float *__restrict__ hs, vtg_found *__restrict__ out)
+                         const int *__restrict__ top, int n, const float *__restrict__ hs, bool gave_up, vtg_found *__restrict__ out)
 {
     __shared__ float s_score[NCC_TOP];
     __shared__ int s_hx[NCC_TOP], s_hy[NCC_TOP], s_at[NCC_TOP];
     const int around = p.step > 1 ? 2 * p.step - 1 : 1, side = 2 * around + 1, ring = side + 2;
     const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (gave_up) {
+        if (threadIdx.x == 0)
+            *out = vtg_found{0, 0, -2.0f, -2.0f, 0.0f, 0.0f, -1, p.ccols * p.crows};
+        return;
+    }
     if (c < n) {
         const float *h = hs + (size_t)c * ring * ring;
         float best = -2.0f;
@@ -994,8 +1000,9 @@ __device__ void ncc_pick(const NccPrm &p, const int *__restrict__ map_x, const i
 /* The half-pixel corners around every candidate, one CTA each: the window of +-around half pixels that
  * search_slot compares, and one ring past it, so the parabola's neighbours of any best are already scored. Scores go
  * to hs[candidate][(around + 1 + dy) ring + around + 1 + dx], ring = 2 around + 3. The CTA that arrives last (every
- * CTA counts, those past the candidates too) makes the pick and resets the counter. */
-/* A byte plane's 200 corners are fewer CTAs than two an SM, so past 32 columns a thread may have 128 registers for its loads (C: a
+ * CTA counts, those past the candidates too) makes the pick and resets the counter. err: the tensor-core map's status word
+ * (NULL after the maps that have none).
+ * A byte plane's 200 corners are fewer CTAs than two an SM, so past 32 columns a thread may have 128 registers for its loads (C: a
  * lane's columns). With one kernel of 64 for every width, two rows at a time, a whole 96 x 96 search took 81.4 us; now 75.5. Six
  * rows in 255 registers: 79.5; at 64 x 64 two, four or eight rows are the same. */
 template <typename T, int C>
@@ -1004,7 +1011,7 @@ __global__ void __launch_bounds__(NCC_TOP * 32, C > 1 ? 2 : 4) ncc_half_all(cons
                                                              const int *__restrict__ map_x, const int *__restrict__ map_y,
                                                              const int *__restrict__ top, const int *__restrict__ ntop,
                                                              float *__restrict__ hs, unsigned *__restrict__ arrive,
-                                                             vtg_found *__restrict__ out)
+                                                             const int *err, vtg_found *__restrict__ out)
 {
     __shared__ bool s_last;
     vtg_grid_dependency_wait(); /* the candidates, when launched as the top-8 pass's programmatic dependent */
@@ -1028,7 +1035,7 @@ __global__ void __launch_bounds__(NCC_TOP * 32, C > 1 ? 2 : 4) ncc_half_all(cons
     if (!s_last)
         return;
     __threadfence();
-    ncc_pick(p, map_x, map_y, top, n, hs, out);
+    ncc_pick(p, map_x, map_y, top, n, hs, err && __ldcg(err) != 0, out);
     if (threadIdx.x == 0)
         *arrive = 0u;
 }
@@ -1137,7 +1144,7 @@ static cudaError_t launch_all(const T *plane, int pitch, const float *app, const
     auto kernel = p.tw > 64 ? ncc_half_all<T, 4> : p.tw > 32 ? ncc_half_all<T, 2> : ncc_half_all<T, 1>;
     return vtg_launch_k(kernel, dim3(NCC_TOP * ring * ring), dim3(NCC_TOP * 32), 0, st, pdl, plane, pitch, app, p,
                         (const int *)s.map_x, (const int *)s.map_y, (const int *)s.top, (const int *)s.ntop, s.half,
-                        s.arrive + 1, out);
+                        s.arrive + 1, map_kind != VTG_NCC_F32 || filtered ? (const int *)s.err : (const int *)nullptr, out);
 }
 
 cudaError_t vtg_launch_ncc(const void *plane, int pitch, int plane_type, const float *app, const NccPrm &p,

@@ -344,12 +344,13 @@ __device__ void box_sums(const uint8_t *__restrict__ plane, int pitch, const Ncc
 }
 
 /* The map's preparation in one launch of 256-thread CTAs: the picture converted, and the cells' words that the map merges into
- * zeroed. BOX: the first nbox sum the windows (the longer work, so they start first), where the map's CTAs do not. */
+ * and the status word zeroed. BOX: the first nbox sum the windows (the longer work, so they start first), where the map's CTAs do not. */
 template <int KIND, bool FILTER, bool BOX>
 __global__ void __launch_bounds__(BOX_NT) ncc_prep(const uint8_t *__restrict__ plane, int pitch, NccPrm p, int fw, int fpitch,
                                                 int btx, int bgx, int nbox, float *__restrict__ fac,
-                                                uint16_t *__restrict__ tol, int rows, int cpitch, int cgx, uint16_t *__restrict__ conv, unsigned long long *__restrict__ cellw,
-                                                int cells, unsigned *__restrict__ ncand)
+                                                uint16_t *__restrict__ tol, int rows, int cpitch, int cgx, uint16_t *__restrict__ conv,
+                                                unsigned long long *__restrict__ cellw, int cells, unsigned *__restrict__ ncand,
+                                                int *__restrict__ err)
 {
     vtg_grid_launch_dependents(); /* the map may start its setup as this launch's last CTAs run */
     const int b = (int)blockIdx.x;
@@ -365,6 +366,8 @@ __global__ void __launch_bounds__(BOX_NT) ncc_prep(const uint8_t *__restrict__ p
     const int k = b - nbox, g = k * 256 + (int)threadIdx.x;
     if (g < cells)
         cellw[g] = 0ull;
+    if (g == 0)
+        *err = 0; /* the map's, for this search */
     if (FILTER && g == 0)
         *ncand = 0u;
     conv_cta<KIND>(plane, pitch, p.w, p.h, p.x0, rows, cpitch, FILTER ? 128.0f : 0.0f, conv, k % cgx, k / cgx);
@@ -488,6 +491,21 @@ static TcSmem tc_smem(int krow, int q, bool fused)
     if (fused)
         s.total += (uint32_t)sizeof(BoxSmem<TcShape<16, true>::boxes>);
     return s;
+}
+
+/* The checked build's failure: while on, the map's first CTA ends as if one of its waits had given up (all have ended by then).
+ * Returns 1 there, 0 in the production build, which has no such word. */
+#ifdef VTG_CHECKED
+__device__ int g_vtg_give_up;
+#endif
+extern "C" int vtg_check_give_up(int on)
+{
+#ifdef VTG_CHECKED
+    return cudaMemcpyToSymbol(g_vtg_give_up, &on, sizeof on) == cudaSuccess ? 1 : VTG_ECUDA;
+#else
+    (void)on;
+    return 0;
+#endif
 }
 
 /* FILTER: the F32 map's first half. Instead of a cell's best, the corners whose score may be it in F32 arithmetic go to
@@ -640,6 +658,10 @@ __global__ void __launch_bounds__(TcShape<Q, FUSED>::threads, 1) ncc_map_tc(NccP
         if (good && last >= 0)
             good = mbar_wait(empty0 + 8 * (last % TC_STAGES), (uint32_t)((last / TC_STAGES) & 1)) ? 1 : 0;
     }
+#ifdef VTG_CHECKED
+    if (g_vtg_give_up && blockIdx.x == 0)
+        good = 0;
+#endif
     const int ok_all = __syncthreads_and(good);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!ok_all) {
@@ -871,7 +893,7 @@ static cudaError_t tc_launch_as(const uint8_t *plane, int pitch, const NccPrm &p
     const int btx = bp_tx(p.tw), bgx = (g.fw + btx - 1) / btx, nbox = FUSED ? 0 : bgx * ((g.fh + TC_QMAX - 1) / TC_QMAX);
     const int cgx = (g.cpitch / 8 + 255) / 256, nconv = cgx * g.rows;
     ncc_prep<KIND, FILTER, !FUSED><<<nbox + nconv, BOX_NT, 0, st>>>(plane, pitch, p, g.fw, g.fpitch, btx, bgx, nbox, s.fac, s.tol,
-                                                                    g.rows, g.cpitch, cgx, s.conv, s.cellw, cells, s.ncand);
+                                                                    g.rows, g.cpitch, cgx, s.conv, s.cellw, cells, s.ncand, s.err);
     const bool pdl = !s.map_ev0;
     auto run = [&](auto kernel, int threads) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm.total);
