@@ -86,6 +86,8 @@ int vtg_ctx_create(int device, size_t hbm_budget, vtg_ctx **out);
 void vtg_ctx_destroy(vtg_ctx *ctx);
 /* Bytes of the budget in use. */
 size_t vtg_ctx_used(const vtg_ctx *ctx);
+/* Device bytes the context's objects hold: vtg_ctx_used, and the trackers' padding (below). */
+size_t vtg_ctx_held(const vtg_ctx *ctx);
 /* Waits for all of the context's work, at most timeout_ms (VTG_ETIMEOUT after that). */
 int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms);
 /* The bounds record of the checked build (libvtg_checked.so, built with VTG_CHECKED): after the device is idle,
@@ -101,7 +103,8 @@ int vtg_check_give_up(int on);
 
 /* Device bytes one tracker of this configuration is charged: two pyramid sets, a frame staging buffer, the cell results. In a
  * context without a budget a frame 256 to 2,080 pixels wide may hold more, as its rows then lie 2,080 floats apart on every
- * level (vtg_level_device's pitch); such padding is not counted in vtg_ctx_used, and is at most 16 GiB a context. */
+ * level (vtg_level_device's pitch); such padding is not counted in vtg_ctx_used but in vtg_ctx_held, and is at
+ * most 16 GiB a context. */
 size_t vtg_tracker_bytes(const struct vtg_config *cfg);
 int vtg_tracker_create(vtg_ctx *ctx, const struct vtg_config *cfg, vtg_tracker **out);
 void vtg_tracker_destroy(vtg_tracker *t);

@@ -113,7 +113,7 @@ struct vtg_serve_cfg {
     double duration_s;     /* the arrival window; the loop gives up 10 s after it */
     int max_batch;         /* streams in one batch at most */
     int inflight;          /* batches on the GPU at once, 1 or 2 */
-    size_t hbm_budget;     /* device bytes for the streams' trackers; 0: no limit */
+    size_t hbm_budget;     /* device bytes that the streams' trackers hold at most; 0: no limit */
     float ncc_share;       /* share of frame pairs followed by an appearance search on their level 1 */
     int plain;             /* 1: the plain form, one frame pair at a time in arrival order, no batching */
     uint64_t seed;

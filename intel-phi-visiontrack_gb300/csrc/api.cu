@@ -16,6 +16,7 @@
 #include "vtg_internal.cuh"
 #include "vtg_tracker.h"
 #include "x87.cuh"
+#include "../host/vtg_host.h"
 
 static thread_local int g_last_cuda = 0;
 
@@ -128,6 +129,8 @@ extern "C" void vtg_ctx_destroy(vtg_ctx *ctx)
 
 extern "C" size_t vtg_ctx_used(const vtg_ctx *ctx) { return ctx ? ctx->used : 0; }
 
+extern "C" size_t vtg_ctx_held(const vtg_ctx *ctx) { return ctx ? ctx->used + ctx->padding : 0; }
+
 extern "C" int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms)
 {
     if (!ctx)
@@ -195,8 +198,8 @@ static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 /* Two layouts of a tracker's planes. Compact: each level's rows as far apart as its width asks. Wide: every level of a frame at
  * most VTG_LK_PITCH pixels wide at that one pitch, which the LK kernels are compiled for (lk.cu: a tenth of their time). Wide
  * holds more memory (a 1080p tracker of four levels 38.8 MB for 27.0, 640 x 480 15 for 4), so a tracker has it only in a context
- * without a budget, while the context's padding stays below VTG_PADDING_MAX, and where the device has the room; the budget's
- * count is the compact size's. Frames under 256 pixels wide, more than eight times their size at that pitch, stay compact. */
+ * without a budget, while the context's padding stays below VTG_PADDING_MAX, where the device has the room, and not in a served
+ * loop whose own limit the wide trackers would pass (serve.c); the budget's count is the compact size's. Frames under 256 pixels wide, more than eight times their size at that pitch, stay compact. */
 #define VTG_PADDING_MAX ((size_t)16 << 30)
 static bool wide_fits(const vtg_config *c) { return c->width >= 256 && c->width <= VTG_LK_PITCH; }
 
@@ -263,7 +266,21 @@ static DevPyr pyr_from(const vtg_tracker *t, int set, int from)
     return p;
 }
 
+extern "C" size_t vtg_tracker_held(const vtg_config *cfg)
+{
+    if (check_config(cfg) != VTG_OK)
+        return 0;
+    Layout L;
+    layout(cfg, wide_fits(cfg), &L);
+    return L.bytes;
+}
+
 extern "C" int vtg_tracker_create(vtg_ctx *ctx, const vtg_config *cfg, vtg_tracker **out)
+{
+    return vtg_tracker_create_as(ctx, cfg, 0, out);
+}
+
+extern "C" int vtg_tracker_create_as(vtg_ctx *ctx, const vtg_config *cfg, int compact, vtg_tracker **out)
 {
     if (!ctx || !out)
         return VTG_EINVAL;
@@ -275,7 +292,7 @@ extern "C" int vtg_tracker_create(vtg_ctx *ctx, const vtg_config *cfg, vtg_track
     layout(cfg, false, &L);
     layout(cfg, true, &wide);
     const size_t bytes = L.bytes;
-    size_t padding = wide_fits(cfg) ? wide.bytes - bytes : 0;
+    size_t padding = wide_fits(cfg) && !compact ? wide.bytes - bytes : 0;
     {
         std::lock_guard<std::mutex> g(ctx->mu);
         if (ctx->budget && ctx->used + bytes > ctx->budget)

@@ -4,8 +4,8 @@
  * The reference's card session takes frames from a DMA ring as the host publishes them, skips frames under LIVE
  * priority and backs off when device memory is full (src/card/session_track.c:1-10, 37-53, 187-225). This drives the
  * request API the same way, on the host, in C:
- *   - streams start over time; each is admitted when its tracker's device memory fits the budget (vtg_tracker_bytes),
- *     else it waits for a stream that finishes to free memory; a stream whose description is malformed is refused and
+ *   - streams start over time; each is admitted when its tracker's device memory fits the budget (vtg_tracker_bytes; with a
+ *     limit the trackers hold no more than that, unless all of them fit it with their padding too), else it waits for a stream that finishes to free memory; a stream whose description is malformed is refused and
  *     the run goes on;
  *   - each stream's frame pairs arrive on a seeded Poisson schedule at its rate and are submitted when they arrive
  *     (a frame that meets a full queue is dropped); with `live`, a stream's newer frame goes ahead of its queued older
@@ -22,7 +22,7 @@
 #include <string.h>
 #include <time.h>
 
-#include "vtg_serve.h"
+#include "vtg_host.h"
 
 #define SERVE_DRAIN_S 10.0
 #define SERVE_POLL 256
@@ -186,6 +186,17 @@ int vtg_serve_run(vtg_ctx *ctx, const struct vtg_serve_cfg *c, struct vtg_serve_
         for (int i = 0; i < 32 * 21; i++)
             app[i] = (float)((int)(urand(&seed) * 255.0) - 127) * 64.0f;
         rc = vtg_server_template(srv, app, 32, 21, 1.0e9f);
+    }
+    if (rc == VTG_OK && c->hbm_budget) {
+        /* the limit is on what the trackers hold: the wide layout, which holds more than is counted, only where every stream's
+         * together stays within it */
+        size_t held = 0;
+        for (int s = 0; s < ns; s++) {
+            struct vtg_config g = stream_cfg(c, s);
+            held += st[s].valid ? vtg_tracker_held(&g) : 0;
+        }
+        if (held > c->hbm_budget)
+            vtg_server_compact(srv);
     }
     const size_t used0 = vtg_ctx_used(ctx);
     const double stall_to = c->stall_timeout_s > 0.0 ? c->stall_timeout_s : 2.0;

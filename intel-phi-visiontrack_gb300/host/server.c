@@ -28,7 +28,7 @@
 
 #include <cuda_runtime.h>
 
-#include "vtg_serve.h"
+#include "vtg_host.h"
 
 #define SRV_SLOTS 2
 #define SRV_QMAX 64
@@ -88,6 +88,7 @@ struct srv_slot {
 struct vtg_server {
     vtg_ctx *ctx;
     struct vtg_server_cfg cfg;
+    int compact; /* streams opened from now on: vtg_server_compact */
     struct srv_stream *st;
     int nst, cap;
     struct srv_slot sl[SRV_SLOTS];
@@ -194,6 +195,8 @@ int vtg_server_create(vtg_ctx *ctx, const struct vtg_server_cfg *cfg, vtg_server
     return VTG_OK;
 }
 
+void vtg_server_compact(vtg_server *s) { s->compact = 1; }
+
 void vtg_server_destroy(vtg_server *s)
 {
     if (!s)
@@ -292,7 +295,7 @@ int vtg_server_open(vtg_server *s, uint32_t width, uint32_t height, uint32_t flo
     }
     struct srv_stream *ss = &s->st[id];
     memset(ss, 0, sizeof *ss);
-    int rc = vtg_tracker_create(s->ctx, &g, &ss->t); /* VTG_EINVAL (malformed) or VTG_EBUDGET (no room now) */
+    int rc = vtg_tracker_create_as(s->ctx, &g, s->compact, &ss->t); /* VTG_EINVAL (malformed) or VTG_EBUDGET (no room now) */
     if (rc != VTG_OK) {
         ss->t = NULL;
         return rc;

@@ -129,6 +129,12 @@ class Context:
     def used(self) -> int:
         return lib().vtg_ctx_used(self.h)
 
+    def held(self) -> int:
+        L = lib()
+        L.vtg_ctx_held.argtypes = [C.c_void_p]
+        L.vtg_ctx_held.restype = C.c_size_t
+        return L.vtg_ctx_held(self.h)
+
     def sync(self, timeout_ms: int = 10000):
         check(lib().vtg_ctx_sync(self.h, timeout_ms), "vtg_ctx_sync")
 
