@@ -31,7 +31,7 @@ void vtg_set_cuda_error(cudaError_t e) { g_last_cuda = (int)e; }
         }                                                                                                              \
     } while (0)
 
-#define POINTS_KEPT 16384 /* points of a list whose scratch a tracker keeps: 1.5 MB at most */
+#define POINTS_KEPT 16384 /* points of a list whose scratch a tracker keeps: 1.5 MB, and the outgrown ones, 3 MB at most */
 
 struct vtg_ctx {
     int device;
@@ -363,6 +363,7 @@ extern "C" int vtg_tracker_create_as(vtg_ctx *ctx, const vtg_config *cfg, int co
     t->d_app = (float *)(t->mem + L.app_off);
     t->points = nullptr;
     t->points_bytes = 0;
+    t->outgrown_n = 0;
     t->build_opts = 0;
     t->point_warps = 0;
     DevPyr d[4] = {pyr_from(t, 0, 0), pyr_from(t, 0, (int)cfg->flow_level), pyr_from(t, 1, 0),
@@ -411,6 +412,8 @@ extern "C" void vtg_tracker_destroy(vtg_tracker *t)
     cudaStreamDestroy(t->stream);
     cudaFree(t->mem);
     cudaFree(t->points);
+    for (int k = 0; k < t->outgrown_n; k++)
+        cudaFree(t->outgrown[k]);
     {
         std::lock_guard<std::mutex> g(ctx->mu);
         ctx->used -= t->bytes;
@@ -538,7 +541,9 @@ extern "C" int vtg_points(vtg_tracker *t, int prev, int cur, int top, int n, con
     /* Host arrays go through device scratch: on the tracker's own stream, which orders the calls, its own (kept, grown to the
      * longest list up to POINTS_KEPT); on another stream, for longer lists and in a capture, where nothing may be allocated
      * otherwise, a stream-ordered allocation of the call's. The pool gives its memory back at every device-wide wait, so an
-     * allocation a call can take longer than the call's work (200 us of 270 for 512 points). */
+     * allocation a call can take longer than the call's work (200 us of 270 for 512 points). A buffer that a longer list has
+     * outgrown stays until the tracker goes, as to free it now would wait for every stream of the device; each holds more
+     * than twice the one before, so together they hold less than the newest. */
     const size_t fbytes = (size_t)n * sizeof(float), need = 4 * fbytes + (size_t)n * sizeof(vtg_lk_out);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(s, &cap));
@@ -550,8 +555,9 @@ extern "C" int vtg_points(vtg_tracker *t, int prev, int cur, int top, int n, con
         if (t->points_bytes < need) {
             CU(cudaSetDevice(t->ctx->device));
             char *more = nullptr;
-            if (cudaMalloc(&more, 2 * need) == cudaSuccess) {
-                cudaFree(t->points); /* waits for the work that reads it */
+            if (t->outgrown_n < VTG_POINTS_OUTGROWN && cudaMalloc(&more, 2 * need) == cudaSuccess) {
+                if (t->points)
+                    t->outgrown[t->outgrown_n++] = t->points;
                 t->points = more;
                 t->points_bytes = 2 * need;
             } else {

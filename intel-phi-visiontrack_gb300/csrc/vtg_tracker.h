@@ -11,6 +11,8 @@
 
 #include "vtg_internal.cuh"
 
+#define VTG_POINTS_OUTGROWN 16 /* 96 bytes, doubled as often, are past the longest list's 1.5 MB */
+
 struct vtg_tracker {
     vtg_ctx *ctx;
     vtg_config cfg;
@@ -32,6 +34,8 @@ struct vtg_tracker {
     float *d_app;         /* an appearance template and its norm (VTG_APP_W x VTG_APP_H + 1 floats), for host reads */
     char *points; /* the host point lists' scratch, allocated at the first one, and the calls that use it in turn */
     size_t points_bytes;
+    char *outgrown[VTG_POINTS_OUTGROWN]; /* the buffers before it, each less than half the next */
+    int outgrown_n;
     std::mutex points_mu;
     LkPrm prm;
     int point_warps; /* warps a point of the point list: 0 by the list's length, 1 or 2 */
