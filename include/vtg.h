@@ -86,7 +86,8 @@ int vtg_ctx_create(int device, size_t hbm_budget, vtg_ctx **out);
 void vtg_ctx_destroy(vtg_ctx *ctx);
 /* Bytes of the budget in use. */
 size_t vtg_ctx_used(const vtg_ctx *ctx);
-/* Device bytes the context's objects hold: vtg_ctx_used, and the trackers' padding (below). */
+/* Device bytes the context's objects hold: vtg_ctx_used, and, in a context without a budget, the trackers' padding (below) and the
+ * scratch they keep for host point lists (at most 3 MB a tracker). */
 size_t vtg_ctx_held(const vtg_ctx *ctx);
 /* Waits for all of the context's work, at most timeout_ms (VTG_ETIMEOUT after that). */
 int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms);

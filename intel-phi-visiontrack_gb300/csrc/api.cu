@@ -35,7 +35,8 @@ void vtg_set_cuda_error(cudaError_t e) { g_last_cuda = (int)e; }
 
 struct vtg_ctx {
     int device;
-    size_t budget, used, padding; /* padding: the trackers' rows past their compact layout, not in used */
+    size_t budget, used;
+    size_t padding, kept; /* not in used: the trackers' rows past their compact layout; their kept scratch of point lists */
     std::mutex mu;
     std::vector<vtg_tracker *> trackers;
     std::vector<cudaStream_t> streams; /* of the other objects (search contexts, batches) */
@@ -108,7 +109,7 @@ extern "C" int vtg_ctx_create(int device, size_t hbm_budget, vtg_ctx **out)
         return VTG_ENOMEM;
     c->device = device;
     c->budget = hbm_budget;
-    c->used = c->padding = 0;
+    c->used = c->padding = c->kept = 0;
     *out = c;
     return VTG_OK;
 }
@@ -129,7 +130,7 @@ extern "C" void vtg_ctx_destroy(vtg_ctx *ctx)
 
 extern "C" size_t vtg_ctx_used(const vtg_ctx *ctx) { return ctx ? ctx->used : 0; }
 
-extern "C" size_t vtg_ctx_held(const vtg_ctx *ctx) { return ctx ? ctx->used + ctx->padding : 0; }
+extern "C" size_t vtg_ctx_held(const vtg_ctx *ctx) { return ctx ? ctx->used + ctx->padding + ctx->kept : 0; }
 
 extern "C" int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms)
 {
@@ -362,7 +363,7 @@ extern "C" int vtg_tracker_create_as(vtg_ctx *ctx, const vtg_config *cfg, int co
     t->d_mm = (uint32_t *)(t->mem + L.mm_off);
     t->d_app = (float *)(t->mem + L.app_off);
     t->points = nullptr;
-    t->points_bytes = 0;
+    t->points_bytes = t->points_held = 0;
     t->outgrown_n = 0;
     t->build_opts = 0;
     t->point_warps = 0;
@@ -418,6 +419,7 @@ extern "C" void vtg_tracker_destroy(vtg_tracker *t)
         std::lock_guard<std::mutex> g(ctx->mu);
         ctx->used -= t->bytes;
         ctx->padding -= t->padding;
+        ctx->kept -= t->points_held;
         for (size_t i = 0; i < ctx->trackers.size(); i++)
             if (ctx->trackers[i] == t) {
                 ctx->trackers.erase(ctx->trackers.begin() + (long)i);
@@ -543,13 +545,14 @@ extern "C" int vtg_points(vtg_tracker *t, int prev, int cur, int top, int n, con
      * otherwise, a stream-ordered allocation of the call's. The pool gives its memory back at every device-wide wait, so an
      * allocation a call can take longer than the call's work (200 us of 270 for 512 points). A buffer that a longer list has
      * outgrown stays until the tracker goes, as to free it now would wait for every stream of the device; each holds more
-     * than twice the one before, so together they hold less than the newest. */
+     * than twice the one before, so together they hold less than the newest. A context with a budget holds nothing past it, so
+     * there every list has an allocation of its call's. */
     const size_t fbytes = (size_t)n * sizeof(float), need = 4 * fbytes + (size_t)n * sizeof(vtg_lk_out);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(s, &cap));
     std::unique_lock<std::mutex> own(t->points_mu, std::defer_lock);
     char *d = nullptr;
-    bool kept = s == t->stream && n <= POINTS_KEPT && cap == cudaStreamCaptureStatusNone;
+    bool kept = s == t->stream && n <= POINTS_KEPT && cap == cudaStreamCaptureStatusNone && !t->ctx->budget;
     if (kept) {
         own.lock(); /* to the end of the call: its copies and kernel follow each other on the stream */
         if (t->points_bytes < need) {
@@ -560,6 +563,9 @@ extern "C" int vtg_points(vtg_tracker *t, int prev, int cur, int top, int n, con
                     t->outgrown[t->outgrown_n++] = t->points;
                 t->points = more;
                 t->points_bytes = 2 * need;
+                t->points_held += 2 * need;
+                std::lock_guard<std::mutex> g(t->ctx->mu);
+                t->ctx->kept += 2 * need;
             } else {
                 cudaGetLastError();
                 kept = false;

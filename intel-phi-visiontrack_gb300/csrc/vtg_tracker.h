@@ -33,7 +33,7 @@ struct vtg_tracker {
     int build_opts;       /* VTG_BUILD_CONTRAST | VTG_BUILD_PRE_GAUSS */
     float *d_app;         /* an appearance template and its norm (VTG_APP_W x VTG_APP_H + 1 floats), for host reads */
     char *points; /* the host point lists' scratch, allocated at the first one, and the calls that use it in turn */
-    size_t points_bytes;
+    size_t points_bytes, points_held; /* its size, and with the outgrown ones' */
     char *outgrown[VTG_POINTS_OUTGROWN]; /* the buffers before it, each less than half the next */
     int outgrown_n;
     std::mutex points_mu;
