@@ -314,33 +314,35 @@ __device__ __forceinline__ void nmq_col_slide(const float *s_img, int ip, int th
     r2 += vn * vn - vo * vo;
 }
 
-/* With SUMS, six CTAs an SM: the sums' phase would otherwise take the registers to 48 and small templates to five CTAs
- * an SM. Without it no bound: the integral images' variant runs large templates, which shared memory already holds to
- * one or two CTAs an SM, and the bound slowed it (96 x 96 by 4 %). */
-template <typename T, int ST, bool SUMS, int CY>
-__global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q(const T *__restrict__ plane, int pitch, const float *__restrict__ app,
-                                                    NccPrm p, const long long *__restrict__ S1,
-                                                    const long long *__restrict__ S2, int tp, int bcols,
-                                                    float *__restrict__ map_v, int *__restrict__ map_x,
-                                                    int *__restrict__ map_y)
+/* A CTA's barrier. */
+struct NmqCta {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+    __device__ __forceinline__ bool all(bool v) const { return __syncthreads_and(v ? 1 : 0) != 0; }
+};
+/* The corners of block `block` of the map, bcols to a row, by 8 CY threads, t their number: a CTA's, or a part of one with shared
+ * memory of its own (sm, s_best: a word a cell of the block) and its barrier (sync, sync.all). Each cell's best goes to out(cell, its origin, its
+ * word as ncc_cell_word makes it, 0 where no corner was scored). */
+template <typename T, int ST, bool SUMS, int CY, typename Sync, typename Out>
+__device__ __forceinline__ void nmq_block(const T *__restrict__ plane, int pitch, const float *__restrict__ app, const NccPrm &p,
+                                          const long long *__restrict__ S1, const long long *__restrict__ S2, int tp, int bcols,
+                                          int block, int t, float *sm, unsigned long long *s_best, Sync sync, Out out)
 {
     constexpr int BC = NMQ_CORNERS * ST / NCC_CELL, BR = CY * ST / NCC_CELL; /* cells a CTA's sides */
     constexpr int PER = NCC_CELL / ST;             /* corners a cell's side */
     constexpr int M = (NMQ_K - 1) * ST + 2;        /* the sliding window */
-    extern __shared__ __align__(16) float sm[];
-    __shared__ unsigned long long s_best[BC * BR];
-    const int bx = blockIdx.x % bcols, by = blockIdx.x / bcols;
+    constexpr int NT = 8 * CY;
+    const int bx = block % bcols, by = block / bcols;
     const int ccx0 = BC * bx, ccy0 = BR * by; /* the CTA's first cell column and row */
     const int X0 = p.x0 + ccx0 * NCC_CELL, Y0 = p.y0 + ccy0 * NCC_CELL;
     const int iw = nmq_cols(ST, p.tw), ip = nmq_pitch(ST, p.tw), ih = nmq_rows(ST, p.th, CY);
     /* a multiple of 8 floats either way: s_img stays 16-byte aligned. Without SUMS nothing takes the template's place, and
      * the launch sizes the head by the template alone (shorter than the column sums for a wide, low template). */
     float *s_app = sm, *s_img = sm + (SUMS ? nmq_head(ST, p.tw, p.th) : p.tw * p.th);
-    for (int i = threadIdx.x; i < p.tw * p.th; i += blockDim.x)
+    for (int i = t; i < p.tw * p.th; i += NT)
         s_app[i] = app[i];
     bool small = true; /* every value this thread staged converts to the same integer in 32 bits */
     if constexpr (CY == 32) {
-        for (int i = threadIdx.x; i < iw * ih; i += blockDim.x) {
+        for (int i = t; i < iw * ih; i += NT) {
             const int r = i / iw, c = i - r * iw;
             const int yy = min(Y0 + r, p.h - 1), xx = min(X0 + c, p.w - 1);
             const float v = (float)__ldg(plane + (size_t)yy * pitch + xx);
@@ -350,8 +352,8 @@ __global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q
     } else {
         /* few CTAs, whose wait for the picture nothing hides: a warp two rows at a time, both rows' loads in flight */
         constexpr int CH = 4; /* 32-column chunks: nmq_narrow's windows have at most 130 columns */
-        const int lane = threadIdx.x & 31;
-        for (int r = threadIdx.x >> 5; r < ih; r += 2 * (8 * CY / 32)) {
+        const int lane = t & 31;
+        for (int r = t >> 5; r < ih; r += 2 * (8 * CY / 32)) {
             T v[2][CH + 1];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
@@ -372,11 +374,10 @@ __global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q
                     }
         }
     }
-    if (threadIdx.x < BC * BR)
-        s_best[threadIdx.x] = 0ull;
-    const bool w32 = __syncthreads_and(small ? 1 : 0) != 0 || sizeof(T) == 1;
+    if (t < BC * BR)
+        s_best[t] = 0ull;
+    const bool w32 = sync.all(small) || sizeof(T) == 1;
     constexpr int GROUPS = NMQ_CORNERS / NMQ_K;
-    const int t = threadIdx.x;
     const int b = t / GROUPS, a0 = (t - b * GROUPS) * NMQ_K; /* corner row, first corner column in the CTA */
     const float *rowb = s_img + (b * ST) * ip + a0 * ST;
     float first[NMQ_K], s0[NMQ_K], s1[NMQ_K];
@@ -421,7 +422,7 @@ __global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q
         }
     } else {
         /* the window sums, eight corner rows at a time, in the template's place */
-        __syncthreads();
+        sync();
         const int ncols = nmq_sum_cols(ST, p.tw);
         long long *cs1 = reinterpret_cast<long long *>(sm), *cs2 = cs1 + 8 * ncols;
         long long r1 = 0, r2 = 0; /* thread t < ncols: column t's sums over the current corner row's window rows */
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q
                         column(k);
                 }
             }
-            __syncthreads();
+            sync();
             if (b / 8 == q) {
                 const long long *c1 = cs1 + (b % 8) * ncols + a0 * ST, *c2 = cs2 + (b % 8) * ncols + a0 * ST;
                 long long x1 = 0, x2 = 0, y1 = 0, y2 = 0; /* two chains; tw is even */
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q
                     sc[c] = ncc_score(sc[c], x1, x2, p) + 0.0f;
                 }
             }
-            __syncthreads();
+            sync();
         }
     }
 #pragma unroll
@@ -494,30 +495,43 @@ __global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q
         u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
         atomicMax(&s_best[(b / PER) * BC + a / PER], ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)key));
     }
-    __syncthreads();
+    sync();
     if (t < BC * BR) {
         const int ccx = ccx0 + t % BC, ccy = ccy0 + t / BC;
-        if (ccx < p.ccols && ccy < p.crows) {
-            const int cell = ccy * p.ccols + ccx;
-            const int cx0 = p.x0 + ccx * NCC_CELL, cy0 = p.y0 + ccy * NCC_CELL;
-            const unsigned long long wd = s_best[t];
-            if (wd == 0ull) { /* no corner: the reference leaves top at -2 and the cell origin */
-                map_v[cell] = -2.0f;
-                map_x[cell] = cx0;
-                map_y[cell] = cy0;
-            } else {
-                unsigned u = (unsigned)(wd >> 32);
-                u = (u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u;
-                const float bv = __uint_as_float(u);
-                const int bk = (int)(0xFFFFFFFFu - (unsigned)(wd & 0xFFFFFFFFull));
-                /* a cell whose every corner reads -1 (out of bounds) keeps -2 and its origin, as `v > top` never fires */
-                const bool fired = bv > -2.0f;
-                map_v[cell] = fired ? bv : -2.0f;
-                map_x[cell] = fired ? cx0 + (bk % PER) * ST : cx0;
-                map_y[cell] = fired ? cy0 + (bk / PER) * ST : cy0;
-            }
-        }
+        if (ccx < p.ccols && ccy < p.crows)
+            out(ccy * p.ccols + ccx, p.x0 + ccx * NCC_CELL, p.y0 + ccy * NCC_CELL, s_best[t]);
     }
+}
+
+/* With SUMS, six CTAs an SM: the sums' phase would otherwise take the registers to 48 and small templates to five CTAs
+ * an SM. Without it no bound: the integral images' variant runs large templates, which shared memory already holds to
+ * one or two CTAs an SM, and the bound slowed it (96 x 96 by 4 %). */
+template <typename T, int ST, bool SUMS, int CY>
+__global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q(const T *__restrict__ plane, int pitch, const float *__restrict__ app,
+                                                    NccPrm p, const long long *__restrict__ S1,
+                                                    const long long *__restrict__ S2, int tp, int bcols,
+                                                    float *__restrict__ map_v, int *__restrict__ map_x,
+                                                    int *__restrict__ map_y)
+{
+    constexpr int PER = NCC_CELL / ST;
+    extern __shared__ __align__(16) float sm[];
+    __shared__ unsigned long long s_best[NMQ_CORNERS * CY / (PER * PER)];
+    nmq_block<T, ST, SUMS, CY>(plane, pitch, app, p, S1, S2, tp, bcols, blockIdx.x, threadIdx.x, sm, s_best, NmqCta{},
+                               [&](int cell, int cx0, int cy0, unsigned long long wd) {
+        if (wd == 0ull) { /* no corner: the reference leaves top at -2 and the cell origin */
+            map_v[cell] = -2.0f;
+            map_x[cell] = cx0;
+            map_y[cell] = cy0;
+        } else {
+            const float bv = ncc_word_score(wd);
+            const int bk = (int)(0xFFFFFFFFu - (unsigned)(wd & 0xFFFFFFFFull));
+            /* a cell whose every corner reads -1 (out of bounds) keeps -2 and its origin, as `v > top` never fires */
+            const bool fired = bv > -2.0f;
+            map_v[cell] = fired ? bv : -2.0f;
+            map_x[cell] = fired ? cx0 + (bk % PER) * ST : cx0;
+            map_y[cell] = fired ? cy0 + (bk / PER) * ST : cy0;
+        }
+    });
 }
 
 /* Whether a search's F32 map at steps 1 and 2 takes CTAs of 16 corner rows: up to four CTAs of 32 rows an SM, whose barriers and
@@ -587,35 +601,102 @@ static size_t ncr_smem(const NccPrm &p)
     return sizeof(float) * 32 * (size_t)steps * p.th + (size_t)NCR_WARPS * NCR_DEPTH * NCR_RUN * ncr_stride(steps);
 }
 
+/* The longest list that is scored corner by corner. A longer one (a ramp, where every window is its neighbours' plus a constant and
+ * the filter rules nothing out) has every corner scored by ncc_map_f32q's blocks, whose words replace the cells': a corner of the
+ * list costs some three of theirs at step 1, two at step 2, where a block stages more picture a corner. Measured, the share of the
+ * corners at which both take the same: step 1, 16 x 16 .27, 32 x 32 .34, 48 x 48 .27, 64 x 64 .34, 96 x 96 .32, 128 x 128 .36, 32 x
+ * 128 .26, 128 x 32 .38; step 2, 32 x 32 .46, 64 x 64 .48, 96 x 96 .60, 128 x 128 .36. Whole searches of a 1080p ramp, us, by the
+ * list / by the blocks: 16 x 16 503 / 198, 32 x 32 726 / 358, 64 x 64 1,404 / 954, 96 x 96 4,450 / 1,700, 128 x 128 7,533 / 3,210,
+ * at step 2 2,082 / 993; by ncc_map_f32q alone 121, 252, 774, 1,535, 2,954 and 873. The blocks are made in the rescoring's own
+ * launch, by two parts of a CTA: a launch of their own behind it, four CTAs an SM, took 814 at 64 x 64 and 1,590 at 96 x 96, but
+ * 1.1 us of every search that the filter does decide, and two CTAs of the rescoring's an SM took 10 us of those, as the first half of
+ * its CTAs then shared SMs. */
+static unsigned ncr_crowd(const NccPrm &p)
+{
+    const unsigned nx = (unsigned)((p.x1 - p.x0) / p.step + 1), ny = (unsigned)((p.y1 - p.y0) / p.step + 1);
+    return p.step == 1 ? nx * ny / 10 * 3 : nx * ny / 20 * 9;
+}
+
+/* a block's shared memory, in 16-byte steps (its head is a multiple of 8 floats) */
+static size_t ncr_all_smem(const NccPrm &p)
+{
+    return sizeof(float) * ((size_t)nmq_head(p.step, p.tw, p.th) +
+                            (((size_t)nmq_pitch(p.step, p.tw) * nmq_rows(p.step, p.th, NMQ_CORNERS) + 3) & ~(size_t)3));
+}
+
+/* Parts of a CTA, a block each; only as many of them work (`parts`) as the shared memory holds blocks. */
+#define NCR_PARTS 2
+#define NCR_THREADS (8 * NMQ_CORNERS * NCR_PARTS)
+struct NcrPart { /* a part's barrier; its staged values are bytes, which all fit 32 bits */
+    int bar;
+    __device__ __forceinline__ void operator()() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NCR_THREADS / NCR_PARTS) : "memory"); }
+    __device__ __forceinline__ bool all(bool) const
+    {
+        (*this)();
+        return true;
+    }
+};
+template <int ST>
+__device__ __noinline__ void ncr_all(const uint8_t *plane, int pitch, const float *app, const NccPrm &p, int parts,
+                                     unsigned long long *cellw)
+{
+    constexpr int B = NMQ_CORNERS * ST / NCC_CELL, NT = NCR_THREADS / NCR_PARTS;
+    extern __shared__ __align__(16) float sm[];
+    __shared__ unsigned long long s_best[NCR_PARTS][B * B];
+    const int part = threadIdx.x / NT;
+    if (part >= parts)
+        return;
+    float *const mine = sm + part * (nmq_head(ST, p.tw, p.th) + ((nmq_pitch(ST, p.tw) * nmq_rows(ST, p.th, NMQ_CORNERS) + 3) & ~3));
+    const int bcols = (p.ccols + B - 1) / B, blocks = bcols * ((p.crows + B - 1) / B);
+    const NcrPart sync{1 + part};
+    for (int block = (int)blockIdx.x * parts + part; block < blocks; block += (int)gridDim.x * parts) {
+        nmq_block<uint8_t, ST, true, NMQ_CORNERS>(plane, pitch, app, p, nullptr, nullptr, 0, bcols, block, threadIdx.x % NT, mine,
+                                                  s_best[part], sync, [&](int cell, int, int, unsigned long long wd) {
+                                                      cellw[cell] = wd != 0ull && ncc_word_score(wd) > -2.0f ? wd : 0ull;
+                                                  });
+        sync(); /* the shared memory is the next block's */
+    }
+}
+
 struct NcrStep {
     unsigned w[9]; /* the words from the corner's first one of these 32 columns */
     float4 t[4];   /* the template at the lane's columns */
 };
 
 template <int STEPS, bool FULL>
-__global__ void __launch_bounds__(32 * NCR_WARPS) ncc_rescore(const uint8_t *__restrict__ plane, int pitch,
-                                                              const float *__restrict__ app, NccPrm p,
+__global__ void __launch_bounds__(NCR_THREADS, 1) ncc_rescore(const uint8_t *__restrict__ plane, int pitch,
+                                                              const float *__restrict__ app, const __grid_constant__ NccPrm p,
                                                               const unsigned *__restrict__ cand,
-                                                              const unsigned *__restrict__ ncand,
+                                                              const unsigned *__restrict__ ncand, unsigned crowd, int parts,
                                                               unsigned long long *__restrict__ cellw)
 {
     extern __shared__ __align__(16) float sm[]; /* the template, 32 columns at a time: 16 even ones, then 16 odd ones */
     constexpr int COLS = 32 * STEPS, STRIDE = ncr_stride(STEPS), SLOT = NCR_RUN * STRIDE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, odd = lane & 1;
-    for (int i = threadIdx.x; i < COLS * p.th; i += 32 * NCR_WARPS) {
+    const unsigned listed = __ldcg(ncand);
+    if (listed > crowd) {
+        if (p.step == 1)
+            ncr_all<1>(plane, pitch, app, p, parts, cellw);
+        else
+            ncr_all<2>(plane, pitch, app, p, parts, cellw);
+        return;
+    }
+    for (int i = threadIdx.x; i < COLS * p.th; i += NCR_THREADS) {
         const int r = i / COLS, c = i % COLS;
         sm[r * COLS + (c & ~31) + 16 * (c & 1) + ((c & 31) >> 1)] = c < p.tw ? __ldg(app + r * p.tw + c) : 0.0f;
     }
     __syncthreads();
+    if (warp >= NCR_WARPS)
+        return;
     /* the pair's rows in the warp's ring */
     const uint8_t *const ring = reinterpret_cast<const uint8_t *>(sm + COLS * p.th) + warp * NCR_DEPTH * SLOT + (lane >> 1) * STRIDE;
     const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring) + 16u * odd;
-    const int count = (int)__ldcg(ncand);
+    const int count = (int)listed;
     const int sh = __ffs(p.step) - 1, per = NCC_CELL >> sh;
     const unsigned lo = 0x7440u + odd, hi = 0x7442u + odd; /* the lane's two bytes of a word */
     const int groups = (p.tw - 32 * (STEPS - 1)) / 8;      /* of the last step; the others have 4 */
     /* runs of 16 corners, one a CTA before any CTA takes a second */
-    for (int base = (warp * gridDim.x + blockIdx.x) * NCR_RUN; base < count; base += NCR_WARPS * gridDim.x * NCR_RUN) {
+    for (int base = (warp * NCR_CTAS + (int)blockIdx.x) * NCR_RUN; base < count; base += NCR_WARPS * NCR_CTAS * NCR_RUN) {
         const int mine = base + (lane >> 1);
         const bool on = mine < count;
         const unsigned xy = __ldcg(cand + (on ? mine : base));
@@ -724,12 +805,14 @@ static cudaError_t launch_rescore(const uint8_t *plane, int pitch, const float *
                                   cudaStream_t st)
 {
     auto kernel = p.tw % 32 ? ncc_rescore<STEPS, false> : ncc_rescore<STEPS, true>;
-    const size_t smem = ncr_smem(p);
+    const size_t one = ncr_all_smem(p), room = (227u << 10) - 1024;
+    const int parts = NCR_PARTS * one <= room ? NCR_PARTS : 1;
+    const size_t list = ncr_smem(p), smem = list > parts * one ? list : parts * one;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
     /* an ordinary launch: as the map's programmatic dependent its CTAs would all start on the SMs that the map leaves free */
-    kernel<<<NCR_CTAS, 32 * NCR_WARPS, smem, st>>>(plane, pitch, app, p, s.cand, s.ncand, s.cellw);
+    kernel<<<NCR_CTAS, NCR_THREADS, smem, st>>>(plane, pitch, app, p, s.cand, s.ncand, ncr_crowd(p), parts, s.cellw);
     return cudaGetLastError();
 }
 

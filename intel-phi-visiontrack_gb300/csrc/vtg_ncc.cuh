@@ -87,6 +87,12 @@ __device__ __forceinline__ unsigned long long ncc_cell_word(float v, int key)
     return ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)key);
 }
 
+__device__ __forceinline__ float ncc_word_score(unsigned long long w)
+{
+    const unsigned u = (unsigned)(w >> 32);
+    return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
+}
+
 /* A cell of the tensor-core map from its 64-bit word (ordered score, inverted scan index): value and corner, or -2 and
  * the cell's origin where no corner was scored (the F32 map's convention). */
 __device__ __forceinline__ void ncc_cell_decode(const NccPrm &p, int cell, unsigned long long w, float &v, int &x, int &y)
@@ -99,10 +105,8 @@ __device__ __forceinline__ void ncc_cell_decode(const NccPrm &p, int cell, unsig
         y = cy0;
         return;
     }
-    unsigned u = (unsigned)(w >> 32);
-    u = (u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u;
     const int key = (int)(0xFFFFFFFFu - (unsigned)(w & 0xFFFFFFFFull));
-    v = __uint_as_float(u);
+    v = ncc_word_score(w);
     x = cx0 + (key % per) * p.step;
     y = cy0 + (key / per) * p.step;
 }
