@@ -867,7 +867,10 @@ __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int to
     }
 }
 
-/* How a single stream's cells and a point list launch. Many: 128 registers a thread, 16 warps an SM. Few: as many points as
+/* How a single stream's cells and a point list launch. The walk reads the planes by the read-only path (coherent loads take 2.6 %
+ * more). The cells may still be a programmatic dependent: they read only a tracker's planes, which this library's builds write, and
+ * those let a dependent start only as their last CTAs end, so nothing writes a plane while a cell's CTA runs. A point list is an
+ * ordinary launch, as a caller's kernel may have made it just before. Many: 128 registers a thread, 16 warps an SM. Few: as many points as
  * the chip has places for two-warp CTAs at eight warps an SM; then nothing but a point's own latency counts, and with 256
  * registers a thread it spills nothing and keeps more loads in flight. Measured, us, few against many: 512 points at 1920 x
  * 1080 28 / 33, 128 at 640 x 480 22 / 24, 1,024 at 1080p 34 / 38; past one wave, 2,048 at 1080p, 55 / 46. A whole 640 x 480 pair
@@ -1493,7 +1496,9 @@ __device__ __forceinline__ void duo_point(const DevPyr &I, const DevPyr &J, int 
 }
 
 /* The still picture's vectors (still.cu): one level, its descriptors by value, and the cells' differences counted. A warp takes two
- * cells of a row, a CTA DUO_ACROSS x DUO_DOWN of these pairs. Bound as the other walks are, by the latency of their chains at 16
+ * cells of a row, a CTA DUO_ACROSS x DUO_DOWN of these pairs. An ordinary launch: the frame is the caller's, whose kernel may have
+ * let its dependents start before it wrote it, and the walk reads by the read-only path; as a dependent the frames of three
+ * streams together took 46.4 us, so 43.9. Bound as the other walks are, by the latency of their chains at 16
  * warps an SM and the instructions a cell takes; half a warp a cell takes a little over half of them. A 1920 x 1080 frame (this
  * and the decision), us: one stream 83 with a warp a cell, 62 now; three streams' frames together 66 and 46. Five CTAs an SM (96
  * registers) 47, pairs one across and four down 47, one across and two down the same as 2 x 2. */
@@ -1517,7 +1522,6 @@ __global__ void __launch_bounds__(32 * DUO_WARPS, DUO_CTAS) lk_still_kernel(DevL
     }
     __syncthreads();
     vtg_grid_launch_dependents();
-    vtg_grid_dependency_wait(); /* the mean, when its kernel is the one before on the stream */
     if (col - half >= g.cols || row >= g.rows)
         return;
     /* the cell's centre and record: lk_cell's */
@@ -1550,7 +1554,7 @@ cudaError_t vtg_launch_still_cells(const DevLevel &I, const DevLevel &J, const L
 {
     const unsigned blocks = (unsigned)((g.cols + 2 * DUO_ACROSS - 1) / (2 * DUO_ACROSS)) * (unsigned)((g.rows + DUO_DOWN - 1) / DUO_DOWN);
     return p.H == DUO_M && p.W == DUO_M
-               ? vtg_launch_k(lk_still_kernel, dim3(blocks), dim3(32 * DUO_WARPS), 0, s, true, I, J, p, g, cells, hist)
+               ? vtg_launch_k(lk_still_kernel, dim3(blocks), dim3(32 * DUO_WARPS), 0, s, false, I, J, p, g, cells, hist)
                : cudaErrorInvalidValue;
 }
 
@@ -1562,7 +1566,6 @@ __global__ void __launch_bounds__(32 * LkShape<FEW>::points, LkShape<FEW>::point
 {
     extern __shared__ f2_t s_tp[]; /* the template's T: a warp (MAXH / 2) x 32 pairs */
     const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    vtg_grid_dependency_wait(); /* the pyramid or the points, when a kernel made them just before */
     if (i >= n)
         return;
     Patch<MAXH, true, PITCH> P;
@@ -1644,7 +1647,7 @@ cudaError_t vtg_launch_points(const DevPyr *I, const DevPyr *J, int top, const L
     const bool few = lk_few(n);
     const int per = few ? LkShape<true>::points : LkShape<false>::points;
     auto launch = [&](auto kernel, int maxh) {
-        return vtg_launch_k(kernel, dim3((n + per - 1) / per), dim3(32 * per), lk_t_bytes(maxh, per), s, true, I, J, top, p, n, xs, ys,
+        return vtg_launch_k(kernel, dim3((n + per - 1) / per), dim3(32 * per), lk_t_bytes(maxh, per), s, false, I, J, top, p, n, xs, ys,
                             gx, gy, out);
     };
     constexpr int W = VTG_LK_PITCH;

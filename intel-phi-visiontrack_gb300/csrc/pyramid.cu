@@ -45,35 +45,35 @@ __device__ __forceinline__ void reduce_tile(const float *src, int sw, int sh, in
                                             int dpitch, int ox, int oy, float (*s_f)[SF_P], float (*s_v)[SF_P])
 {
     const int tid = threadIdx.x;
-    const int sy0 = 2 * oy - 2;
-                    const int gx0 = 2 * ox - 4;
-            for (int i = tid; i < RS_Y * (SF_X / 4); i += blockDim.x) {
-                const int r = i / (SF_X / 4), k = i - r * (SF_X / 4);
-                const int gy = min(max(sy0 + r, 0), sh - 1), gx = gx0 + 4 * k;
-                const float *row = src + (size_t)gy * spitch;
-                float4 v;
-                if (gx >= 0 && gx + 4 <= sw)
-                    v = __ldg(reinterpret_cast<const float4 *>(row + gx));
-                else
-                    v = make_float4(__ldg(row + min(max(gx, 0), sw - 1)), __ldg(row + min(max(gx + 1, 0), sw - 1)),
-                                    __ldg(row + min(max(gx + 2, 0), sw - 1)), __ldg(row + min(max(gx + 3, 0), sw - 1)));
-                *reinterpret_cast<float4 *>(&s_f[r][4 * k]) = v;
-            }
-            __syncthreads();
-            for (int i = tid; i < RT_Y * (SF_X / 4); i += blockDim.x) {
-                const int r = i / (SF_X / 4), g = i - r * (SF_X / 4);
-                /* F32 as the reference sums: whole numbers below 2^24, so every sum is exact */
-                float4 t[5];
-    #pragma unroll
-                for (int q = 0; q < 5; q++)
-                    t[q] = *reinterpret_cast<const float4 *>(&s_f[2 * r + q][4 * g]);
-                float4 o;
-                o.x = t[0].x + t[4].x + 4.0f * (t[1].x + t[3].x) + 6.0f * t[2].x;
-                o.y = t[0].y + t[4].y + 4.0f * (t[1].y + t[3].y) + 6.0f * t[2].y;
-                o.z = t[0].z + t[4].z + 4.0f * (t[1].z + t[3].z) + 6.0f * t[2].z;
-                o.w = t[0].w + t[4].w + 4.0f * (t[1].w + t[3].w) + 6.0f * t[2].w;
-                *reinterpret_cast<float4 *>(&s_v[r][4 * g]) = o;
-            }
+    const int sy0 = 2 * oy - 2, gx0 = 2 * ox - 4;
+    /* coherent loads: the level below may have been written while this launch, its dependent, had begun */
+    for (int i = tid; i < RS_Y * (SF_X / 4); i += blockDim.x) {
+        const int r = i / (SF_X / 4), k = i - r * (SF_X / 4);
+        const int gy = min(max(sy0 + r, 0), sh - 1), gx = gx0 + 4 * k;
+        const float *row = src + (size_t)gy * spitch;
+        float4 v;
+        if (gx >= 0 && gx + 4 <= sw)
+            v = __ldca(reinterpret_cast<const float4 *>(row + gx));
+        else
+            v = make_float4(__ldca(row + min(max(gx, 0), sw - 1)), __ldca(row + min(max(gx + 1, 0), sw - 1)),
+                            __ldca(row + min(max(gx + 2, 0), sw - 1)), __ldca(row + min(max(gx + 3, 0), sw - 1)));
+        *reinterpret_cast<float4 *>(&s_f[r][4 * k]) = v;
+    }
+    __syncthreads();
+    for (int i = tid; i < RT_Y * (SF_X / 4); i += blockDim.x) {
+        const int r = i / (SF_X / 4), g = i - r * (SF_X / 4);
+        /* F32 as the reference sums: whole numbers below 2^24, so every sum is exact */
+        float4 t[5];
+#pragma unroll
+        for (int q = 0; q < 5; q++)
+            t[q] = *reinterpret_cast<const float4 *>(&s_f[2 * r + q][4 * g]);
+        float4 o;
+        o.x = t[0].x + t[4].x + 4.0f * (t[1].x + t[3].x) + 6.0f * t[2].x;
+        o.y = t[0].y + t[4].y + 4.0f * (t[1].y + t[3].y) + 6.0f * t[2].y;
+        o.z = t[0].z + t[4].z + 4.0f * (t[1].z + t[3].z) + 6.0f * t[2].z;
+        o.w = t[0].w + t[4].w + 4.0f * (t[1].w + t[3].w) + 6.0f * t[2].w;
+        *reinterpret_cast<float4 *>(&s_v[r][4 * g]) = o;
+    }
     __syncthreads();
     /* horizontal: output x takes vertical sums 2 x + 2 .. 2 x + 6; four outputs a thread (sums 8 g .. 8 g + 15) */
     for (int i = tid; i < RT_Y * (RT_X / 4); i += blockDim.x) {
