@@ -120,6 +120,8 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
     s->max_th = max_th;
     s->bytes = L.bytes;
     s->has_template = false;
+    s->stream = nullptr;
+    s->host = nullptr;
     cudaError_t e = cudaSetDevice(vtg_ctx_device(ctx));
     if (e == cudaSuccess)
         e = cudaMalloc(&s->mem, L.bytes);
@@ -134,13 +136,14 @@ extern "C" int vtg_search_create(vtg_ctx *ctx, int max_w, int max_h, int max_tw,
         e = cudaMemsetAsync(s->mem, 0, L.bytes, s->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s->stream);
-    s->host = nullptr;
     if (e == cudaSuccess)
         e = cudaHostAlloc(&s->host, sizeof *s->host, cudaHostAllocMapped);
     if (e == cudaSuccess)
         e = cudaHostGetDevicePointer(&s->host_dev, s->host, 0);
     if (e != cudaSuccess) {
         vtg_set_cuda_error(e);
+        if (s->stream)
+            cudaStreamDestroy(s->stream);
         cudaFreeHost(s->host);
         cudaFree(s->mem);
         vtg_ctx_release(ctx, L.bytes);
