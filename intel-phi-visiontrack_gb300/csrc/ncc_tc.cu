@@ -161,7 +161,7 @@ void vtg_ncc_filter_bound(NccPrm &p, const NccBandStats &b)
     const double spread = (double)b.sum_dd * 1.001 - sd * sd * 0.999 / n;
     const double t = sqrt((double)b.sum_tt / norm); /* 1 for a caller's true norm */
     const double core = t * steps * 0x1p-21, chain = t * (n * 0.5 + 16.0) * 0x1p-24;
-    const double a = sqrt((spread > 0.0 ? spread : 0.0) / norm) + core + chain + 4e-6;
+    const double a = sqrt((spread <= 0.0 ? 0.0 : spread) / norm) + core + chain + 4e-6; /* NaN stays: a value past FP16's */
     const bool good = norm > 0.0 && a <= 0.01; /* false for NaN */
     p.flt_a = good ? (float)(a * 1.02) : -1.0f;
     p.flt_m = good ? (float)(core * 1.02) : 0.0f;
