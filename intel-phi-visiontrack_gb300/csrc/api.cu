@@ -200,7 +200,8 @@ static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
  * most VTG_LK_PITCH pixels wide at that one pitch, which the LK kernels are compiled for (lk.cu: a tenth of their time). Wide
  * holds more memory (a 1080p tracker of four levels 38.8 MB for 27.0, 640 x 480 15 for 4), so a tracker has it only in a context
  * without a budget, while the context's padding stays below VTG_PADDING_MAX, where the device has the room, and not in a served
- * loop whose own limit the wide trackers would pass (serve.c); the budget's count is the compact size's. Frames under 256 pixels wide, more than eight times their size at that pitch, stay compact. */
+ * loop whose own limit the wide trackers would pass (serve.c); the budget's count is the compact size's. Frames under 256 pixels
+ * wide, more than eight times their size at that pitch, stay compact. */
 #define VTG_PADDING_MAX ((size_t)16 << 30)
 static bool wide_fits(const vtg_config *c) { return c->width >= 256 && c->width <= VTG_LK_PITCH; }
 

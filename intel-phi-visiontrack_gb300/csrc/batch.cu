@@ -267,14 +267,14 @@ extern "C" int vtg_batch_prepare(vtg_batch *b, int slot, int n, vtg_tracker *con
         if (it != b->tuned.end())
             b->tune = it->second;
     }
-    /* tile offsets per level launch (level L of the launch makes level L, L = 1 also level 0) */
-    for (int L = 1; L < VTG_MAX_LEVELS; L++) {
+    /* tile offsets per level launch: level L's in row L - 1 (levels 0 to 3 are the fused launch's, below) */
+    for (int L = 4; L < VTG_MAX_LEVELS; L++) {
         int acc = 0;
         int *row = tiles.data() + (size_t)(L - 1) * (n + 1);
         for (int j = 0; j < n; j++) {
             row[j] = acc;
             const PyrJob &p = pj[(size_t)j];
-            if (L == 1 || L < p.levels)
+            if (L < p.levels)
                 acc += vtg_pyr_tiles(p.w, p.h, L);
         }
         row[n] = acc;

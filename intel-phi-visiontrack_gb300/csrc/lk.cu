@@ -1544,8 +1544,7 @@ __global__ void __launch_bounds__(32 * DUO_WARPS, DUO_CTAS) lk_still_kernel(DevL
         c.sigma = o.status ? 0.0f : sqrtf(o.cov_xx + o.cov_yy);
         c.pad = 0.0f;
         cells[row * g.cols + col] = c;
-        if (hist)
-            atomicAdd(hist + vtg_still_bin(diff), 1);
+        atomicAdd(hist + vtg_still_bin(diff), 1);
     }
 }
 

@@ -320,8 +320,8 @@ struct NmqCta {
     __device__ __forceinline__ bool all(bool v) const { return __syncthreads_and(v ? 1 : 0) != 0; }
 };
 /* The corners of block `block` of the map, bcols to a row, by 8 CY threads, t their number: a CTA's, or a part of one with shared
- * memory of its own (sm, s_best: a word a cell of the block) and its barrier (sync, sync.all). Each cell's best goes to out(cell, its origin, its
- * word as ncc_cell_word makes it, 0 where no corner was scored). */
+ * memory of its own (sm; s_best: a word a cell of the block) and its barrier (sync, sync.all). Each cell's best goes to
+ * out(cell, its origin, its word as ncc_cell_word makes it, 0 where no corner was scored). */
 template <typename T, int ST, bool SUMS, int CY, typename Sync, typename Out>
 __device__ __forceinline__ void nmq_block(const T *__restrict__ plane, int pitch, const float *__restrict__ app, const NccPrm &p,
                                           const long long *__restrict__ S1, const long long *__restrict__ S2, int tp, int bcols,
@@ -507,11 +507,10 @@ __device__ __forceinline__ void nmq_block(const T *__restrict__ plane, int pitch
  * an SM. Without it no bound: the integral images' variant runs large templates, which shared memory already holds to
  * one or two CTAs an SM, and the bound slowed it (96 x 96 by 4 %). */
 template <typename T, int ST, bool SUMS, int CY>
-__global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1) ncc_map_f32q(const T *__restrict__ plane, int pitch, const float *__restrict__ app,
-                                                    NccPrm p, const long long *__restrict__ S1,
-                                                    const long long *__restrict__ S2, int tp, int bcols,
-                                                    float *__restrict__ map_v, int *__restrict__ map_x,
-                                                    int *__restrict__ map_y)
+__global__ void __launch_bounds__(8 * CY, SUMS && CY == 32 ? 6 : 1)
+    ncc_map_f32q(const T *__restrict__ plane, int pitch, const float *__restrict__ app, NccPrm p, const long long *__restrict__ S1,
+                 const long long *__restrict__ S2, int tp, int bcols, float *__restrict__ map_v, int *__restrict__ map_x,
+                 int *__restrict__ map_y)
 {
     constexpr int PER = NCC_CELL / ST;
     extern __shared__ __align__(16) float sm[];
@@ -629,7 +628,10 @@ static size_t ncr_all_smem(const NccPrm &p)
 #define NCR_THREADS (8 * NMQ_CORNERS * NCR_PARTS)
 struct NcrPart { /* a part's barrier; its staged values are bytes, which all fit 32 bits */
     int bar;
-    __device__ __forceinline__ void operator()() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NCR_THREADS / NCR_PARTS) : "memory"); }
+    __device__ __forceinline__ void operator()() const
+    {
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NCR_THREADS / NCR_PARTS) : "memory");
+    }
     __device__ __forceinline__ bool all(bool) const
     {
         (*this)();

@@ -874,7 +874,7 @@ cudaError_t vtg_launch_pyramid_opts(const uint8_t *frame, int stride, int w, int
 
 int vtg_pyr_tiles(int w, int h, int level)
 {
-    /* tiles of the launch that makes `level` (1: levels 0 and 1) from a w x h frame */
+    /* tiles of the launch that makes `level` (4 and up) of a w x h frame */
     int sw = w, sh = h;
     for (int L = 1; L < level; L++) {
         sw = (sw + 1) / 2;

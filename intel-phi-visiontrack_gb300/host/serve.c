@@ -5,8 +5,8 @@
  * priority and backs off when device memory is full (src/card/session_track.c:1-10, 37-53, 187-225). This drives the
  * request API the same way, on the host, in C:
  *   - streams start over time; each is admitted when its tracker's device memory fits the budget (vtg_tracker_bytes; with a
- *     limit the trackers hold no more than that, unless all of them fit it with their padding too), else it waits for a stream that finishes to free memory; a stream whose description is malformed is refused and
- *     the run goes on;
+ *     limit the trackers hold no more than that, unless all of them fit it with their padding too), else it waits for a
+ *     stream that finishes to free memory; a stream whose description is malformed is refused and the run goes on;
  *   - each stream's frame pairs arrive on a seeded Poisson schedule at its rate and are submitted when they arrive
  *     (a frame that meets a full queue is dropped); with `live`, a stream's newer frame goes ahead of its queued older
  *     ones, which are skipped;
