@@ -807,12 +807,11 @@ __device__ __forceinline__ float cell_diff(const DevLevel &A, const DevLevel &B,
     for (int k0 = lane; k0 < n; k0 += 32)
 #pragma unroll
         for (int u = 0; u < PARTS; u++) {
-            const int k = k0 + u * LANES;
-            if (u && k >= n)
-                break;
+            const int k = min(k0 + u * LANES, n - 1);
             const int kr = p2 ? k >> sh : k / g.cell_w, kc = p2 ? k & (g.cell_w - 1) : k % g.cell_w;
             const int yy = y0 + kr, xx = min(x + kc, A.w - 1);
-            s[u] += fabsf(__ldg(B.p + (size_t)yy * B.pitch + xx) - __ldg(A.p + (size_t)yy * A.pitch + xx));
+            const float d = fabsf(__ldg(B.p + (size_t)yy * B.pitch + xx) - __ldg(A.p + (size_t)yy * A.pitch + xx));
+            s[u] += k0 + u * LANES < n ? d : 0.0f;
         }
     float sum = warp_fold<LANES>(s[0]);
 #pragma unroll
@@ -867,15 +866,16 @@ __device__ __forceinline__ void lk_cell(const DevPyr &I, const DevPyr &J, int to
     }
 }
 
-/* How a single stream's cells and a point list launch. The walk reads the planes by the read-only path (coherent loads take 2.6 %
- * more). The cells may still be a programmatic dependent: they read only a tracker's planes, which this library's builds write, and
- * those let a dependent start only as their last CTAs end, so nothing writes a plane while a cell's CTA runs. A point list is an
- * ordinary launch, as a caller's kernel may have made it just before. Many: 128 registers a thread, 16 warps an SM. Few: as many points as
+/* How a single stream's cells and a point list launch. Many: 128 registers a thread, 16 warps an SM. Few: as many points as
  * the chip has places for two-warp CTAs at eight warps an SM; then nothing but a point's own latency counts, and with 256
  * registers a thread it spills nothing and keeps more loads in flight. Measured, us, few against many: 512 points at 1920 x
  * 1080 28 / 33, 128 at 640 x 480 22 / 24, 1,024 at 1080p 34 / 38; past one wave, 2,048 at 1080p, 55 / 46. A whole 640 x 480 pair
  * from host memory (1,200 cells) 64.4 / 66.7. The shape before both, for point lists of any length, was 8 warps a CTA of 128
- * registers and no launch ahead of the kernel before: 28, 37 and 39 for the three lists above. */
+ * registers: 28, 37 and 39 for the three lists above.
+ * The walk reads the planes by the read-only path (coherent loads take 2.6 % more of 8 x 1080p cells). The cells may still be a
+ * programmatic dependent (1.6 us of a whole 640 x 480 pair): they read only a tracker's planes, which this library's builds write,
+ * and those let a dependent start only as their last CTAs end, so nothing writes a plane while a cell's CTA runs. A point list is
+ * an ordinary launch, as a caller's kernel may have made it just before. */
 #define LK_SMS 152
 template <bool FEW>
 struct LkShape {
@@ -1496,12 +1496,12 @@ __device__ __forceinline__ void duo_point(const DevPyr &I, const DevPyr &J, int 
 }
 
 /* The still picture's vectors (still.cu): one level, its descriptors by value, and the cells' differences counted. A warp takes two
- * cells of a row, a CTA DUO_ACROSS x DUO_DOWN of these pairs. An ordinary launch: the frame is the caller's, whose kernel may have
- * let its dependents start before it wrote it, and the walk reads by the read-only path; as a dependent the frames of three
- * streams together took 46.4 us, so 43.9. Bound as the other walks are, by the latency of their chains at 16
+ * cells of a row, a CTA DUO_ACROSS x DUO_DOWN of these pairs. Bound as the other walks are, by the latency of their chains at 16
  * warps an SM and the instructions a cell takes; half a warp a cell takes a little over half of them. A 1920 x 1080 frame (this
  * and the decision), us: one stream 83 with a warp a cell, 62 now; three streams' frames together 66 and 46. Five CTAs an SM (96
- * registers) 47, pairs one across and four down 47, one across and two down the same as 2 x 2. */
+ * registers) 47, pairs one across and four down 47, one across and two down the same as 2 x 2. An ordinary launch: the frame is
+ * the caller's, whose kernel may have let its dependents start before it wrote it, and the walk reads by the read-only path; as a
+ * dependent three streams' frames took those 46, so 44 to 45. */
 #define DUO_ACROSS 2
 #define DUO_DOWN 2
 #define DUO_CTAS 4 /* an SM: 128 registers a thread */
