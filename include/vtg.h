@@ -89,7 +89,8 @@ size_t vtg_ctx_used(const vtg_ctx *ctx);
 /* Device bytes the context's objects hold: vtg_ctx_used, and, in a context without a budget, the trackers' padding (below) and the
  * scratch they keep for host point lists (at most 3 MB a tracker). */
 size_t vtg_ctx_held(const vtg_ctx *ctx);
-/* Waits for all of the context's work, at most timeout_ms (VTG_ETIMEOUT after that). */
+/* Waits for all of the context's work, at most timeout_ms (VTG_ETIMEOUT after that). The calling thread asks without pause for the
+ * first 300 us, then every 50. */
 int vtg_ctx_sync(vtg_ctx *ctx, int timeout_ms);
 /* The bounds record of the checked build (libvtg_checked.so, built with VTG_CHECKED): after the device is idle,
  * out[0] = the LK patch operations whose pixel rectangle would have left its level (bit 1 template build, 2 window

@@ -405,7 +405,8 @@ struct DetSelectSmem {
  * into, which ends as keys differ), so nothing is ordered that the walk never reaches; the histogram's prefix sums also place
  * the members, a bin's few among themselves by counting. Whatever of it is too close to a corner
  * taken before it is out at once, a thread a member; up to 256 may be left (a block with more is tried again with fewer
- * members; the share left sets the next block's size). Those are settled by conflict masks, 32 candidates at a time by one warp: a candidate is taken once no earlier one in conflict with it is taken or open, out once
+ * members; the share left sets the next block's size). Those are settled by conflict masks, 32 candidates at a time by one warp:
+ * a candidate is taken once no earlier one in conflict with it is taken or open, out once
  * one is taken. 128 corners of a 384 x 307 box (2,673 candidates): 13 us, where four radix passes over the candidates and
  * blocks settled in passes took 32. Latency of one SM's barriers and shared memory bounds it. */
 __global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, const int *ncand, const float *best, const unsigned *keys,

@@ -578,7 +578,7 @@ static bool ncc_sums_in_map(const NccPrm &p)
  * step's latency. The picture comes in by 16-byte asynchronous copies, NCR_DEPTH rows ahead, the pair's lanes taking a corner
  * row's chunks in turn; a step is 32 columns, its words and template values read from shared memory while the step before
  * runs. Byte b becomes the float 2^23 + b by one byte permute, then less 2^23 + first: b - first, exact. The window's sums
- * are byte dot products, each lane of a pair on half the words. Measured at 1080p: 11 us at 32 x 32, 21 at 64 x 64, 53 at
+ * are byte dot products, each lane of a pair on half the words. Measured at 1080p: 11 us at 32 x 32, 19 at 64 x 64, 51 at
  * 96 x 96, three times less than a lane a corner reading the picture itself; the wait between a step's dependent
  * instructions bounds it (an instruction every three cycles of a scheduler). Columns past the template's in a last step (not FULL) hold
  * zeros in the staged template and are masked from the sums: they add exact zeros.
