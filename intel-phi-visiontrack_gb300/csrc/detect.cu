@@ -364,25 +364,33 @@ __global__ void __launch_bounds__(32 * DET_SEGS) det_collect(DetPrm q, const flo
 }
 
 /* Whether the corner at (x, y) keeps the spacing from every corner in the grid: the 3 x 3 grid cells around its own
- * (a cell's side is at least the spacing, so no corner farther out can be too close). */
+ * (a cell's side is at least the spacing, so no corner farther out can be too close). The whole warp asks together, a lane
+ * without a corner with far = false, and steps through the lists by votes, so that no lane can leave a list on its own. With
+ * nested loops left by a return, compiled into det_select, a lane was measured to come back after the warp's next ballots and
+ * barriers: det_select then counted a block twice and wrote past its arrays. */
 __device__ __forceinline__ bool det_far(const DetPrm &q, const int *s_head, const int *s_next, const int *s_tx,
-                                        const int *s_ty, int x, int y)
+                                        const int *s_ty, int x, int y, bool far)
 {
     const int gx = (x - q.g.ax) / q.gs, gy = (y - q.g.y0) / q.gs;
     int h[9];
 #pragma unroll
     for (int j = 0; j < 9; j++) {
         const int a = gx + j % 3 - 1, b = gy + j / 3 - 1;
-        h[j] = a >= 0 && a < q.gw && b >= 0 && b < q.gh ? s_head[b * q.gw + a] : -1;
+        h[j] = far && a >= 0 && a < q.gw && b >= 0 && b < q.gh ? s_head[b * q.gw + a] : -1;
     }
 #pragma unroll
-    for (int j = 0; j < 9; j++)
-        for (int t = h[j]; t >= 0; t = s_next[t]) {
-            const int dx = s_tx[t] - x, dy = s_ty[t] - y;
-            if (dx * dx + dy * dy < q.need)
-                return false;
+    for (int j = 0; j < 9; j++) {
+        int t = far ? h[j] : -1;
+        while (__any_sync(VTG_FULL, t >= 0)) {
+            if (t >= 0) {
+                const int dx = s_tx[t] - x, dy = s_ty[t] - y;
+                far = dx * dx + dy * dy >= q.need;
+                t = far ? s_next[t] : -1;
+            }
+            __syncwarp();
         }
-    return true;
+    }
+    return far;
 }
 
 struct DetSelectSmem {
@@ -407,7 +415,7 @@ struct DetSelectSmem {
  * taken before it is out at once, a thread a member; up to 256 may be left (a block with more is tried again with fewer
  * members; the share left sets the next block's size). Those are settled by conflict masks, 32 candidates at a time by one warp:
  * a candidate is taken once no earlier one in conflict with it is taken or open, out once
- * one is taken. 128 corners of a 384 x 307 box (2,673 candidates): 13 us, where four radix passes over the candidates and
+ * one is taken. 128 corners of a 384 x 307 box (2,673 candidates): 16 us, where four radix passes over the candidates and
  * blocks settled in passes took 32. Latency of one SM's barriers and shared memory bounds it. */
 __global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, const int *ncand, const float *best, const unsigned *keys,
                                                                  const int2 *cxy, float *__restrict__ xs,
@@ -520,11 +528,9 @@ __global__ void __launch_bounds__(DET_SELECT_THREADS, 1) det_select(DetPrm q, co
         __syncthreads();
         /* of them, those clear of every corner taken */
         int2 me = make_int2(0, 0);
-        bool clear = false;
-        if (tid < members) {
+        if (tid < members)
             me = __ldca(cxy + (int)(S.order[tid] & 8191ull));
-            clear = det_far(q, S.head, S.next, S.tx, S.ty, me.x, me.y);
-        }
+        const bool clear = det_far(q, S.head, S.next, S.tx, S.ty, me.x, me.y, tid < members);
         const unsigned bal = __ballot_sync(VTG_FULL, clear);
         if (lane == 0)
             S.wsum[warp] = __popc(bal);
